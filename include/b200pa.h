@@ -191,6 +191,23 @@ int b200pa_paged_attention_v2(const b200pa_attn_args* args, void* stream);
 int b200pa_paged_attention_v2_noalloc(const b200pa_attn_args* args, void* stream);
 
 /*
+ * Attention of an engine step: request r brings the query rows
+ * [query_start_loc[r], query_start_loc[r+1]) of `query` and `out`, the last positions of its
+ * sequence, and each of them attends to the cached positions up to its own (causal).  The step's
+ * own K and V have to be in the cache.  (What the reference's paged-attention backends compute for
+ * chunked prefill, vllm/v1/attention/backends/rocm_attn.py:275-362.)
+ *   args: as for v1, with one entry of seq_lens / block_tables per REQUEST (num_seqs requests);
+ *     out_lse and block-sparse arguments are not supported.
+ *   query_start_loc: device, int32 [num_seqs + 1]
+ *   num_tokens: query rows of the step
+ *   num_decodes: the first `num_decodes` requests bring exactly one row each (decode kernel)
+ * Returns B200PA_EUNSUPPORTED, with nothing launched, for shapes that it has no kernel for (fp32
+ * queries, block size 8, unaligned tensors, more than 2048 requests with several rows).
+ */
+int b200pa_paged_attention_varlen(const b200pa_attn_args* args, const int32_t* query_start_loc,
+                                  int32_t num_tokens, int32_t num_decodes, void* stream);
+
+/*
  * Arguments of reshape_and_cache / reshape_and_cache_flash.
  * Replaces: csrc/cache.h:21-32, launchers csrc/cache_kernels.cu:656-683 and :700-738.
  *

@@ -1,0 +1,124 @@
+"""Attention of steps whose requests bring several query tokens (paged_attention_varlen), against
+fp32 dense causal attention over the same cache contents."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _gather(key_cache, value_cache, table, n, kv, scale):
+    """K and V [n, Hkv, D] of one request's first n positions, as fp32."""
+    def plain(t):
+        if kv == "auto":
+            return t.float()
+        return t.view(torch.float8_e5m2 if kv == "fp8_e5m2" else torch.float8_e4m3fn).float() * scale
+    nb, hk, dx, B, x = key_cache.shape
+    blocks = table[: (n + B - 1) // B].long()
+    k = plain(key_cache[blocks]).permute(0, 3, 1, 2, 4).reshape(-1, hk, dx * x)[:n]
+    v = plain(value_cache[blocks]).permute(0, 3, 1, 2).reshape(-1, hk, dx * x)[:n]
+    return k, v
+
+
+def _case(q_lens, ctx, H, HK, D, B, dtype, kv, alibi=False, seed=0, poison=True):
+    from vllm_b200 import _custom_ops as ops
+    gen = torch.Generator(device=DEV).manual_seed(seed)
+    rng = np.random.default_rng(seed)
+    q_lens, ctx = np.asarray(q_lens), np.asarray(ctx)
+    lens = q_lens + ctx
+    need = np.maximum(1, -(-lens // B))
+    nb = int(need.sum()) + 3
+    perm = rng.permutation(nb).astype(np.int32)
+    table = np.zeros((len(lens), int(need.max())), np.int32)
+    off = 0
+    for r, k in enumerate(need):
+        table[r, :k] = perm[off:off + k]
+        off += k
+    table = torch.from_numpy(table).to(DEV)
+    fp8 = kv != "auto"
+    x = 16 if fp8 else 16 // torch.empty((), dtype=dtype).element_size()
+    scale = 0.02 if fp8 else 1.0
+    kf = torch.randn((nb, HK, D // x, B, x), generator=gen, device=DEV)
+    vf = torch.randn((nb, HK, D, B), generator=gen, device=DEV)
+    if fp8:
+        t = torch.float8_e5m2 if kv == "fp8_e5m2" else torch.float8_e4m3fn
+        kc, vc = ((f / scale).clamp(-448, 448).to(t).view(torch.uint8) for f in (kf, vf))
+    else:
+        kc, vc = kf.to(dtype), vf.to(dtype)
+    n = int(q_lens.sum())
+    q = (2 * torch.randn((n, H, D), generator=gen, device=DEV)).to(dtype)
+    out = torch.full((n, H, D), float("nan"), dtype=dtype, device=DEV)
+    slopes = torch.tensor([2.0 ** (-(i + 1) / 2) for i in range(H)], device=DEV) if alibi else None
+    if poison:  # stale bytes behind the end of a sequence must not reach the result
+        bad = 0x7F if fp8 else float("nan")
+        for r, k in enumerate(lens):
+            if k % B:
+                blk = table[r, k // B].long()
+                kc[blk, :, :, k % B:] = bad
+                vc[blk, :, :, k % B:] = bad
+    qsl = torch.from_numpy(np.concatenate([[0], np.cumsum(q_lens)]).astype(np.int32)).to(DEV)
+    lens_t = torch.from_numpy(lens.astype(np.int32)).to(DEV)
+    nd = int(np.argmax(q_lens != 1)) if (q_lens != 1).any() else len(q_lens)
+    ks = torch.tensor(scale, device=DEV)
+    took = ops.paged_attention_varlen(out, q, kc, vc, HK, D ** -0.5, table, lens_t, qsl, nd, B,
+                                      int(lens.max()), slopes, kv, ks, ks)
+    assert took
+    torch.cuda.synchronize()
+    off = 0
+    for r, (t, c) in enumerate(zip(q_lens, ctx)):
+        if t == 0:
+            continue
+        k, v = _gather(kc, vc, table[r], int(t + c), kv, scale)
+        g = H // HK
+        qq = q[off:off + t].float().view(t, HK, g, D)
+        s = torch.einsum("tkgd,lkd->kgtl", qq, k) * D ** -0.5
+        pos = torch.arange(c, c + t, device=DEV)
+        key = torch.arange(c + t, device=DEV)
+        if alibi:
+            s = s + slopes.view(HK, g, 1, 1) * (key.view(1, -1) - pos.view(-1, 1)).float()
+        s = s.masked_fill(key.view(1, -1) > pos.view(-1, 1), float("-inf"))
+        want = torch.einsum("kgtl,lkd->tkgd", torch.softmax(s, -1), v).reshape(t, H, D)
+        got = out[off:off + t].float()
+        err = (got - want).norm() / want.norm()
+        assert err < 6e-3, (r, t, c, float(err))
+        torch.testing.assert_close(got, want, atol=2e-2, rtol=2e-2)
+        off += t
+    from vllm_b200 import capi
+    assert capi.device_status() == 0
+
+
+@pytest.mark.parametrize("D", [32, 64, 80, 96, 112, 120, 128, 192, 256])
+@pytest.mark.parametrize("kv,dtype", [("auto", torch.bfloat16), ("auto", torch.float16),
+                                      ("fp8", torch.bfloat16), ("fp8_e5m2", torch.float16)])
+@pytest.mark.parametrize("B", [16, 32])
+def test_head_sizes_types_and_blocks(D, kv, dtype, B):
+    if D == 120 and kv != "auto":
+        pytest.skip("an fp8 cache keeps 16 head dimensions together")
+    _case([1, 1, 70, 3, 200], [5, 300, 0, 129, 61], 8, 2, D, B, dtype, kv, alibi=D == 96, seed=D)
+
+
+# row tiles hold 128 // (H // HK) tokens, two to an item; key tiles 128 (64 above head size 128)
+@pytest.mark.parametrize("H,HK", [(4, 4), (12, 4), (28, 4), (32, 2), (33, 1)])
+@pytest.mark.parametrize("q,ctx", [(2, 0), (15, 1), (16, 112), (17, 112), (31, 97), (127, 1), (128, 0),
+                                   (129, 127), (255, 2), (256, 128), (257, 511)])
+def test_tile_edges(H, HK, q, ctx):
+    _case([q, 0, q], [ctx, 7, 0], H, HK, 128, 16, torch.bfloat16, "auto", seed=q)
+
+
+@pytest.mark.parametrize("kv", ["auto", "fp8"])
+def test_few_rows_behind_long_contexts_are_split(kv):
+    _case([5, 2, 40], [9000, 3000, 20000], 8, 2, 128, 16, torch.bfloat16, kv)
+
+
+def test_many_requests_and_single_rows_among_them():
+    rng = np.random.default_rng(3)
+    q = rng.integers(1, 40, size=300)
+    q[:20] = 1
+    q[100] = 1
+    _case(q, rng.integers(0, 400, size=300), 8, 2, 64, 16, torch.bfloat16, "auto")
+
+
+@pytest.mark.parametrize("kv", ["auto", "fp8"])
+def test_a_long_prompt(kv):
+    _case([1500, 900], [700, 0], 8, 2, 128, 16, torch.bfloat16, kv)

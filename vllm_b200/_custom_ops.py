@@ -175,6 +175,34 @@ def paged_attention_with_lse(
         block_size, max_seq_len, alibi_slopes, kv_cache_dtype, k_scale, v_scale)
 
 
+def paged_attention_varlen(
+    out: torch.Tensor,
+    query: torch.Tensor,
+    key_cache: torch.Tensor,
+    value_cache: torch.Tensor,
+    num_kv_heads: int,
+    scale: float,
+    block_tables: torch.Tensor,
+    seq_lens: torch.Tensor,
+    query_start_loc: torch.Tensor,
+    num_decodes: int,
+    block_size: int,
+    max_seq_len: int,
+    alibi_slopes: torch.Tensor | None,
+    kv_cache_dtype: str,
+    k_scale: torch.Tensor,
+    v_scale: torch.Tensor,
+) -> bool:
+    """Causal attention of an engine step: request r brings the rows
+    ``query_start_loc[r]:query_start_loc[r + 1]`` of `query`, the last positions of its sequence;
+    the first `num_decodes` requests bring one each.  False when there is no kernel for the shape
+    (nothing was launched then)."""
+    return _ops.paged_attention_varlen(
+        out, query, key_cache, value_cache, num_kv_heads, scale, block_tables, seq_lens,
+        query_start_loc, num_decodes, block_size, max_seq_len, alibi_slopes, kv_cache_dtype, k_scale,
+        v_scale)
+
+
 def merge_attn_states(
     output: torch.Tensor,
     prefix_output: torch.Tensor,

@@ -14,18 +14,21 @@ module also works stand-alone; inside vLLM it is registered with::
 
 Decode steps (one query token per sequence) go straight to
 ``PagedAttention.forward_decode``.  Steps that contain prefill or chunked-prefill
-tokens are served by the same decode kernels: after the KV write every query
-token is presented as its own single-token "sequence" that shares its request's
-block-table row and sees the cache up to its own position (causal).  That reads
-the cache once per query token - fine for short prompts and for correctness; a
-dedicated prefill kernel is outside this path.
+tokens go to ``paged_attention_varlen``: the leading single-token requests to the
+decode kernel, the others to the prefill kernel.  Shapes that the prefill kernel
+is not built for (fp32, block size 8, unaligned tensors) are served by the decode
+kernels alone: every query token is presented as its own single-token "sequence"
+that shares its request's block-table row and sees the cache up to its own
+position (causal), which reads the cache once per query token.
 """
 from __future__ import annotations
 
 import dataclasses
 
+import numpy as np
 import torch
 
+from vllm_b200 import _custom_ops as ops
 from vllm_b200.paged_attn import PagedAttention
 
 
@@ -42,6 +45,16 @@ class B200PagedAttentionMetadata:
     block_table: torch.Tensor       # [num_reqs, max_blocks] int32
     slot_mapping: torch.Tensor      # [num_tokens] int64, cache slot of every new token
     use_cascade: bool = False
+    num_decodes: int = 0            # requests in front of the batch that bring exactly one token
+
+
+def leading_decodes(query_start_loc_cpu: torch.Tensor | None) -> int:
+    """How many requests in front of the batch bring exactly one query token (0 when the host does
+    not know the offsets)."""
+    if query_start_loc_cpu is None:
+        return 0
+    more = np.flatnonzero(np.diff(query_start_loc_cpu.numpy()) != 1)
+    return int(more[0]) if more.size else len(query_start_loc_cpu) - 1
 
 
 def expand_to_token_sequences(query_start_loc: torch.Tensor, seq_lens: torch.Tensor,
@@ -99,7 +112,9 @@ class B200PagedAttentionMetadataBuilder:
         return B200PagedAttentionMetadata(
             num_actual_tokens=m.num_actual_tokens, max_query_len=m.max_query_len,
             query_start_loc=m.query_start_loc, max_seq_len=m.max_seq_len, seq_lens=m.seq_lens,
-            block_table=m.block_table_tensor, slot_mapping=m.slot_mapping)
+            block_table=m.block_table_tensor, slot_mapping=m.slot_mapping,
+            num_decodes=(m.num_reqs if m.max_query_len == 1
+                         else leading_decodes(getattr(m, "query_start_loc_cpu", None))))
 
     def build_for_cudagraph_capture(self, common_attn_metadata) -> B200PagedAttentionMetadata:
         """Metadata for a capture run: real shapes, every sequence one token long so that the
@@ -160,6 +175,12 @@ class B200PagedAttentionImpl:
         q = query[:n].view(n, self.num_heads, self.head_size)
         if attn_metadata.max_query_len == 1:
             seq_lens, block_table = attn_metadata.seq_lens, attn_metadata.block_table
+        elif ops.paged_attention_varlen(
+                output[:n].view(n, self.num_heads, self.head_size), q, key_cache, value_cache,
+                self.num_kv_heads, self.scale, attn_metadata.block_table, attn_metadata.seq_lens,
+                attn_metadata.query_start_loc, attn_metadata.num_decodes, value_cache.shape[3],
+                attn_metadata.max_seq_len, alibi, self.kv_cache_dtype, layer._k_scale, layer._v_scale):
+            return output
         else:
             seq_lens, block_table = expand_to_token_sequences(
                 attn_metadata.query_start_loc, attn_metadata.seq_lens, attn_metadata.block_table, n)

@@ -1,0 +1,25 @@
+// Device-side state that the launchers of the attention kernels share: the split-KV workspace and
+// arrival counters of a stream, the self-resetting scheduler words, the SM count.  Defined in
+// paged_attention.cu.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstddef>
+
+namespace b200pa {
+
+constexpr int kArrivePerRegion = 32768;
+
+struct StreamRegion {
+  unsigned char* ws;   // split-KV workspace of this stream
+  size_t ws_bytes;
+  unsigned* arrive;    // arrival counters of this stream (kArrivePerRegion, zero between launches)
+  unsigned* arrive2;   // ... of its merge groups
+};
+
+bool stream_region(cudaStream_t stream, StreamRegion* out);
+unsigned* sched_words();
+int sm_count();
+
+}  // namespace b200pa

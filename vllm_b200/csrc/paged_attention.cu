@@ -13,6 +13,7 @@
 #include <mutex>
 
 #include "decode_inst.cuh"
+#include "launch_state.cuh"
 
 namespace b200pa {
 
@@ -212,7 +213,6 @@ __device__ unsigned g_sched_words[256][2];  // zero-initialised; self-resetting 
 // Arrival counters of the fused split-KV merge: one per (sequence, kv head, head
 // group); zero-initialised and re-armed by the warp that performs the merge.
 constexpr int kStreamSlots = 8;
-constexpr int kArrivePerRegion = 32768;
 __device__ unsigned g_arrive[kStreamSlots][kArrivePerRegion];
 // ... and one per group of pieces of a sequence that is merged in two levels
 constexpr int kArrive2PerRegion = 65536;
@@ -232,13 +232,6 @@ constexpr size_t kBigRegionBytes = size_t(32) << 20;
 constexpr size_t kSmallRegionBytes = size_t(4) << 20;
 constexpr size_t kWorkspaceBytes = kBigRegionBytes + (kStreamSlots - 1) * kSmallRegionBytes;
 static __device__ __align__(256) unsigned char g_workspace[kWorkspaceBytes];
-
-struct StreamRegion {
-  unsigned char* ws;   // split-KV workspace of this stream
-  size_t ws_bytes;
-  unsigned* arrive;    // arrival counters of this stream
-  unsigned* arrive2;   // ... of its merge groups
-};
 
 // Developer knobs, read from the environment once per process (B200PA_TUNE_RELOAD=1 at
 // that first read makes every call read them again, for parameter sweeps in one process).
@@ -279,7 +272,7 @@ static Tuning tuning() {
 // scratch and counters).  A slot whose stream has not been used for the longest time is
 // handed to a new stream, so streams that have been destroyed do not use the slots up;
 // more than eight streams calling concurrently are not kept apart.
-static bool stream_region(cudaStream_t stream, StreamRegion* out) {
+bool stream_region(cudaStream_t stream, StreamRegion* out) {
   constexpr int kMaxDev = 64;
   struct DevState {
     unsigned char* ws = nullptr;
@@ -335,7 +328,7 @@ static bool stream_region(cudaStream_t stream, StreamRegion* out) {
 
 // Scheduler words of one launch (256 rotating slots; only unsplit launches with more than
 // three items per warp use them).
-static unsigned* sched_words() {
+unsigned* sched_words() {
   constexpr int kMaxDev = 64;
   static unsigned* sbase[kMaxDev] = {};
   static std::atomic<unsigned> rr{0};
@@ -352,7 +345,7 @@ static unsigned* sched_words() {
   return sb + 2 * (rr.fetch_add(1, std::memory_order_relaxed) & 255u);
 }
 
-static int sm_count() {
+int sm_count() {
   static int cache[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;

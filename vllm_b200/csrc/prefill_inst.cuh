@@ -1,0 +1,60 @@
+// Explicit-instantiation helper of the prefill kernel: each prefill_*.cu file builds it for some
+// head sizes so that the files compile in parallel.
+#pragma once
+
+#include "prefill_kernel.cuh"
+
+namespace b200pa {
+
+using PrefillLaunchFn = cudaError_t (*)(const PrefillParams&, int grid, cudaStream_t stream);
+
+struct PrefillKernelInfo {
+  PrefillLaunchFn fn;
+  int piece_bytes;  // workspace of one piece of an item
+};
+
+template <typename QT, int KV, int D>
+cudaError_t prefill_launch(const PrefillParams& p, int grid, cudaStream_t stream) {
+  auto kern = pa_prefill_kernel<QT, KV, D>;
+  constexpr int smem = PrefillShape<D>::kSmem;
+  // opt in to large dynamic shared memory once per device
+  static bool done[64] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64 || !done[dev]) {
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) {
+      (void)cudaGetLastError();  // do not leave the error for the next caller
+      return e;
+    }
+    if (dev >= 0 && dev < 64) done[dev] = true;
+  }
+  kern<<<grid, kPrefillThreads, smem, stream>>>(p);
+  return cudaGetLastError();
+}
+
+template <typename QT, int D>
+PrefillKernelInfo find_prefill_kv(int kv_dtype) {
+  constexpr int piece = PrefillShape<D>::NQ * 128 * (D * 2 + 8);
+  if (kv_dtype == B200PA_KV_AUTO) return {prefill_launch<QT, kCache16, D>, piece};
+  if constexpr (D % 16 == 0) {
+    if (kv_dtype == B200PA_KV_FP8_E4M3) return {prefill_launch<QT, kCacheE4M3, D>, piece};
+    if (kv_dtype == B200PA_KV_FP8_E5M2) return {prefill_launch<QT, kCacheE5M2, D>, piece};
+  }
+  return {nullptr, 0};
+}
+
+template <int D>
+PrefillKernelInfo find_prefill_for(int q_dtype, int kv_dtype) {
+  if (q_dtype == B200PA_BF16) return find_prefill_kv<__nv_bfloat16, D>(kv_dtype);
+  if (q_dtype == B200PA_F16) return find_prefill_kv<__half, D>(kv_dtype);
+  return {nullptr, 0};
+}
+
+// Defined in prefill_small.cu (32 .. 96), prefill_mid.cu (112 .. 128), prefill_large.cu (192, 256).
+PrefillKernelInfo find_prefill_small(int d, int q_dtype, int kv_dtype);
+PrefillKernelInfo find_prefill_mid(int d, int q_dtype, int kv_dtype);
+PrefillKernelInfo find_prefill_large(int d, int q_dtype, int kv_dtype);
+
+}  // namespace b200pa

@@ -1,0 +1,823 @@
+// Attention of query chunks (prefill, chunked prefill) over the paged cache, on the fifth-generation
+// tensor cores.  Every request r of a step brings q_len tokens, the last q_len positions of its
+// sequence; token i attends to the cached positions up to its own (causal).  The new tokens' K and V
+// are in the cache already.
+//
+// What bounds it: the two contractions are 4 * D flops per (query head, query, key), so with a few
+// hundred query rows per K/V tile the tensor cores and the exponentials are the limit, not HBM.
+// The decode kernel reads the whole context once per query TOKEN; here a K/V tile is read once per
+// 256 query rows.
+//
+//   * One persistent CTA per SM, 13 warps: two softmax warpgroups (one thread per query row), one
+//     producer warpgroup, one warp that issues the MMAs.
+//   * A work item is (request, 2 x 128 query rows, kv head).  A row is one (token, query head of the
+//     group): the heads that share a kv head are packed into the rows of a tile, so K/V are fetched
+//     once for all of them, and the causal edge of a tile is only 128 / group tokens wide.
+//   * S = Q.K^T and O += P.V are tcgen05.mma (M = 128, fp32 accumulators in TMEM).  Q, K and V sit in
+//     shared memory as [16-byte granule along K][row][16 bytes]: the no-swizzle K-major operand
+//     layout, which is what the x-layout of the K cache and 8-token pieces of V rows give without any
+//     transposition.  P goes back to TMEM as the A operand of the second product, over S.
+//   * The two row tiles take turns: while the softmax of one runs, the tensor cores work for the
+//     other.
+//   * The running maximum is only raised (and O rescaled in TMEM) when a row's maximum grew by more
+//     than 2^8: until then P is merely larger than 1, which fp32 sums and 16-bit P hold as exactly.
+//   * fp8 caches are widened to f16 (exact) by the producers on their way to shared memory.
+//   * Few items (short chunks behind long contexts): the keys of an item are cut into pieces, every
+//     piece leaves a normalised partial, and the warp that delivers the last piece of its rows merges
+//     them.  Nobody waits for another CTA.
+//   * Every mbarrier wait is bounded; on expiry a status code is recorded and all roles leave.
+//
+// Measured on B200, a step of 4 chunks (8192 tokens, contexts up to 4096, 32 / 8 heads of 128, bf16;
+// KV write included): 8990 us with one decode work item per token, 686 us here (586 TFLOP/s).
+#pragma once
+
+#include <type_traits>
+
+#include "decode_kernel.cuh"
+#include "tcgen05.cuh"
+
+namespace b200pa {
+
+struct PrefillParams {
+  void* out;                  // [num_tokens, num_heads, D]
+  const void* q;              // [num_tokens, num_heads, D], token stride q_stride
+  const void* kc;
+  const void* vc;
+  const int* block_tables;
+  const int* seq_lens;        // per request, this step's tokens included
+  const int* q_start;         // [num_reqs + 1]
+  const float* alibi;
+  const float* k_scale;
+  const float* v_scale;
+  unsigned* sched;            // [0] ticket, [1] CTAs done (self-resetting)
+  unsigned* arrive;           // arrival counters of split row tiles
+  unsigned char* ws;          // partials of split row tiles
+  int* status;
+  int64_t q_stride;
+  int64_t kv_block_stride;    // elements
+  int64_t kv_head_stride;
+  int num_reqs;
+  int num_heads;
+  int num_kv_heads;
+  int group;
+  int block_size;
+  int max_blocks_per_seq;
+  int ws_slots;               // pieces that the workspace has room for
+  float scale;
+};
+
+constexpr int kPrefillThreads = 13 * 32;
+constexpr int kPrefillMaxReqs = 2048;   // prefix table in shared memory
+
+template <int D>
+struct PrefillShape {
+  static constexpr int DP = (D + 15) / 16 * 16;     // operand width (head size 120 is padded)
+  static constexpr int NQ = D > 192 ? 1 : 2;        // row tiles per item: TMEM holds NQ * (KT + DP) columns
+  static constexpr int KT = D > 128 ? 64 : 128;     // keys per tile
+  static constexpr int kQBytes = 128 * DP * 2;
+  static constexpr int kTileBytes = KT * DP * 2;
+  static constexpr int kStages = 2;
+  static constexpr int kSmem = NQ * kQBytes + 2 * kStages * kTileBytes;
+  static_assert(NQ * (KT + DP) <= 512, "TMEM columns");
+};
+
+struct PrefillItem {
+  int req, kvh, piece, npieces;
+  int tok0;        // first query token of the item inside its request
+  int q_len, ctx;  // ctx: cached positions in front of the chunk (seq_len - q_len)
+  int seq_len, q0; // q0: row of the request's first token
+  int first;       // number of the item's piece 0
+  int b, e0, e1;   // key tiles [b, e0) of row tile 0, [b, e1) of row tile 1
+};
+
+template <typename QT, int KV, int D>
+__global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const PrefillParams p) {
+  using SH = PrefillShape<D>;
+  constexpr bool kFp8 = KV != kCache16;
+  constexpr bool kE5 = KV == kCacheE5M2;
+  constexpr bool kBf = !kFp8 && std::is_same_v<QT, __nv_bfloat16>;  // operand type: bf16, else f16
+  constexpr bool kOutBf = std::is_same_v<QT, __nv_bfloat16>;
+  constexpr int DP = SH::DP, NQ = SH::NQ, KT = SH::KT, NST = SH::kStages;
+  constexpr int kWs = 128 * (D * 2 + 8);  // workspace of one row tile's partial: O, then (m, l)
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ int cum[kPrefillMaxReqs + 1];  // items before request r
+  __shared__ uint64_t s_bar[4 * NST + 3 * 2 + 2 + 4];
+  __shared__ int s_item[2];
+  __shared__ uint32_t s_tmem;
+  __shared__ int s_red[3][13];
+
+  const int tid = threadIdx.x, lane = tid & 31;
+  // (through a shuffle, so that the compiler knows it is uniform in the warp)
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const uint32_t bar0 = smem_u32(s_bar);
+  auto k_full = [&](int s) { return bar0 + 8u * s; };
+  auto k_empty = [&](int s) { return bar0 + 8u * (NST + s); };
+  auto v_full = [&](int s) { return bar0 + 8u * (2 * NST + s); };
+  auto v_empty = [&](int s) { return bar0 + 8u * (3 * NST + s); };
+  auto s_full = [&](int i) { return bar0 + 8u * (4 * NST + i); };
+  auto p_full = [&](int i) { return bar0 + 8u * (4 * NST + 2 + i); };
+  auto pv_done = [&](int i) { return bar0 + 8u * (4 * NST + 4 + i); };
+  auto q_full = [&](int i) { return bar0 + 8u * (4 * NST + 6 + i); };
+  auto item_full = [&](int i) { return bar0 + 8u * (4 * NST + 8 + i); };
+  auto item_empty = [&](int i) { return bar0 + 8u * (4 * NST + 10 + i); };
+
+  const uint32_t sq = smem_u32(smem_raw);
+  const uint32_t sk = sq + NQ * SH::kQBytes;
+  const uint32_t sv = sk + NST * SH::kTileBytes;
+
+  if (warp == 12) {
+    if (lane == 0) {
+      for (int s = 0; s < NST; ++s) {
+        mbar_init(k_full(s), 128);
+        mbar_init(k_empty(s), 1);
+        mbar_init(v_full(s), 128);
+        mbar_init(v_empty(s), 1);
+      }
+      for (int i = 0; i < 2; ++i) {
+        mbar_init(s_full(i), 1);
+        mbar_init(p_full(i), 128);
+        mbar_init(pv_done(i), 1);
+        mbar_init(q_full(i), 128);
+        mbar_init(item_full(i), 1);
+        mbar_init(item_empty(i), 384);
+      }
+      fence_barrier_init();
+    }
+    __syncwarp();
+    tmem_alloc(smem_u32(&s_tmem), 512);
+  }
+  if constexpr (DP != D) {
+    // the padding granules of Q and K take part in the product: zero, once (nobody writes them)
+    for (int i = tid; i < NQ * 128 + NST * KT; i += kPrefillThreads) {
+      unsigned char* at = i < NQ * 128
+          ? smem_raw + (i / 128) * SH::kQBytes + (D / 8) * 128 * 16 + (i % 128) * 16
+          : smem_raw + NQ * SH::kQBytes + ((i - NQ * 128) / KT) * SH::kTileBytes + (D / 8) * KT * 16 +
+                ((i - NQ * 128) % KT) * 16;
+      *reinterpret_cast<uint4*>(at) = make_uint4(0, 0, 0, 0);
+    }
+    // ... and V's padding columns (their results are dropped, but the operand has to be defined)
+    for (int i = tid; i < NST * (KT / 8) * (DP - D); i += kPrefillThreads) {
+      const int st = i / ((KT / 8) * (DP - D)), r = i % ((KT / 8) * (DP - D));
+      *reinterpret_cast<uint4*>(smem_raw + NQ * SH::kQBytes + (NST + st) * SH::kTileBytes +
+                                ((r / (DP - D)) * DP + D + r % (DP - D)) * 16) = make_uint4(0, 0, 0, 0);
+    }
+    fence_proxy_async();
+  }
+
+  // ---- plan.  T tokens fill a row tile; a request has ceil(q_len / (NQ T)) row-tile groups per kv
+  // head, and each of them npieces pieces.
+  const int G = p.group, HK = p.num_kv_heads, S = p.num_reqs, B = p.block_size;
+  const int b_shift = 31 - __clz(B);  // 16 or 32 tokens per block
+  const int T = 128 / G, TT = NQ * T;
+  int split_tiles;  // key tiles per piece (INT_MAX: one piece per group)
+  auto q_len_of = [&](int r) { return p.q_start[r + 1] - p.q_start[r]; };
+  auto tiles_of = [&](int len) { return (max(len, 0) + KT - 1) / KT; };
+  {
+    // groups and key tiles of all requests: with fewer than four groups per SM the groups are cut
+    // into pieces of about half an SM's share of the key tiles (at least four tiles: a piece costs
+    // a Q load, a pipeline fill and a partial)
+    int groups = 0, work = 0, most = 0;
+    for (int r = tid; r < S; r += kPrefillThreads) {
+      const int ql = q_len_of(r);
+      const int n = (ql + TT - 1) / TT;
+      const int len = p.seq_lens[r];
+      groups += n;
+      work += n * ((tiles_of(len) + tiles_of(len - ql + min(ql, TT)) + 1) / 2);
+      most += n * tiles_of(len);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      groups += __shfl_xor_sync(0xffffffffu, groups, o);
+      work += __shfl_xor_sync(0xffffffffu, work, o);
+      most += __shfl_xor_sync(0xffffffffu, most, o);
+    }
+    if (lane == 0) {
+      s_red[0][warp] = groups;
+      s_red[1][warp] = work;
+      s_red[2][warp] = most;
+    }
+    __syncthreads();
+    groups = work = most = 0;
+    for (int w = 0; w < 13; ++w) {
+      groups += s_red[0][w];
+      work += s_red[1][w];
+      most += s_red[2][w];
+    }
+    __syncthreads();  // (s_red is written again below)
+    const int64_t all_work = int64_t(work) * HK, all_groups = int64_t(groups) * HK;
+    split_tiles = INT32_MAX;
+    if (all_groups < 4 * int64_t(gridDim.x)) {
+      int64_t c = max(int64_t(4), (all_work + 2 * int64_t(gridDim.x) - 1) / (2 * int64_t(gridDim.x)));
+      // every piece needs a slot of the workspace: a group of n tiles has at most n / c + 1 pieces
+      const int64_t room = p.ws_slots - all_groups;
+      if (room > 0) split_tiles = int(min(max(c, int64_t(most) * HK / room + 1), int64_t(INT32_MAX)));
+    }
+  }
+  auto pieces_of = [&](int len) { return split_tiles == INT32_MAX ? 1 : max(1, (tiles_of(len) + split_tiles - 1) / split_tiles); };
+  {
+    const int per = (S + kPrefillThreads - 1) / kPrefillThreads;
+    const int r0 = min(S, tid * per), r1 = min(S, r0 + per);
+    auto items_of = [&](int r) { return ((q_len_of(r) + TT - 1) / TT) * pieces_of(p.seq_lens[r]) * HK; };
+    int mine = 0;
+    for (int r = r0; r < r1; ++r) mine += items_of(r);
+    int incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (lane == 31) s_red[2][warp] = incl;
+    __syncthreads();
+    int run = incl - mine;
+    for (int w = 0; w < warp; ++w) run += s_red[2][w];
+    for (int r = r0; r < r1; ++r) {
+      cum[r] = run;
+      run += items_of(r);
+    }
+    if (tid == kPrefillThreads - 1) cum[S] = run;
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = s_tmem;
+  const int total = cum[S];
+
+  // item number -> what it covers.  Inside a request the row tiles run from the last to the first
+  // (longest first), then the pieces, then the kv heads.
+  auto decode = [&](int item) {
+    PrefillItem it;
+    int lo = 0, hi = S;
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (cum[mid] <= item) lo = mid; else hi = mid;
+    }
+    it.req = lo;
+    it.q0 = p.q_start[lo];
+    it.q_len = p.q_start[lo + 1] - it.q0;
+    it.seq_len = p.seq_lens[lo];
+    it.ctx = it.seq_len - it.q_len;
+    const int rel = item - cum[lo];
+    it.kvh = rel % HK;
+    const int gp = rel / HK;
+    it.npieces = pieces_of(it.seq_len);
+    it.piece = gp % it.npieces;
+    const int ngroups = (it.q_len + TT - 1) / TT;
+    const int grp = ngroups - 1 - gp / it.npieces;
+    it.first = item - it.piece * HK;
+    it.tok0 = grp * TT;
+    const int n = tiles_of(it.ctx + min(it.q_len, it.tok0 + TT));
+    it.b = int(int64_t(n) * it.piece / it.npieces);
+    const int e = int(int64_t(n) * (it.piece + 1) / it.npieces);
+    auto end_of = [&](int i) {
+      const int t0 = it.tok0 + i * T;
+      return i < NQ && t0 < it.q_len ? max(it.b, min(e, tiles_of(it.ctx + min(it.q_len, t0 + T)))) : it.b;
+    };
+    it.e0 = end_of(0);
+    it.e1 = end_of(1);
+    return it;
+  };
+  bool ok = true;
+  auto wait = [&](uint32_t bar, uint32_t parity) {
+    if (ok && !mbar_wait(bar, parity)) {
+      ok = false;
+      atomicExch(p.status, kStatusMbarTimeout);
+    }
+    return ok;
+  };
+  // the same for a whole warp: TMEM accesses are warp-collective, so its threads leave together
+  auto wait_warp = [&](uint32_t bar, uint32_t parity) { return ok = __all_sync(0xffffffffu, wait(bar, parity)); };
+  // next item of this CTA, for the roles that do not draw it themselves
+  int n_item = 0;  // items received so far
+  auto next_item = [&]() -> int {
+    const int slot = n_item & 1;
+    if (!wait(item_full(slot), (n_item >> 1) & 1)) return INT32_MAX;
+    const int v = *reinterpret_cast<volatile int*>(&s_item[slot]);
+    mbar_arrive(item_empty(slot));
+    ++n_item;
+    return v;
+  };
+
+  if (warp < 8) {
+    // ================================================= softmax: one thread per row of tile wg
+    const int wg = warp >> 2;
+    const int row = tid & 127;
+    const uint32_t lane_off = uint32_t((warp & 3) * 32) << 16;
+    const uint32_t t_s = tmem + lane_off + uint32_t(wg * KT);
+    const uint32_t t_o = tmem + lane_off + uint32_t(NQ * KT + wg * DP);
+    const float c = p.scale * kLog2e * (kFp8 ? *p.k_scale : 1.f);
+    const float v_scale = kFp8 ? *p.v_scale : 1.f;
+    const bool row_used = wg < NQ && row < T * G;
+    const int row_tok = row / G, row_head = row % G;
+    uint32_t n_s = 0, n_pv = 0;  // S tiles received, PV products issued for this row tile
+
+    auto load_q = [&](const PrefillItem& it) {
+      if (wg < NQ) {
+        const int tok = it.tok0 + wg * T + row_tok;
+        if (row_used && tok < it.q_len) {
+          const QT* src = static_cast<const QT*>(p.q) + int64_t(it.q0 + tok) * p.q_stride +
+                          int64_t(it.kvh * G + row_head) * D;
+          const uint32_t dst = sq + wg * SH::kQBytes + row * 16;
+#pragma unroll
+          for (int g = 0; g < D / 8; ++g) {
+            if constexpr (kFp8 && kOutBf) {  // the operands of an fp8 cache are f16
+              const uint4 v = __ldg(reinterpret_cast<const uint4*>(src) + g);
+              const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+              uint32_t o[4];
+#pragma unroll
+              for (int k = 0; k < 4; ++k)
+                o[k] = pack2<false>(__uint_as_float(w[k] << 16), __uint_as_float(w[k] & 0xffff0000u));
+              st_shared16(dst + g * 128 * 16, make_uint4(o[0], o[1], o[2], o[3]));
+            } else {
+              cp_async16(dst + g * 128 * 16, reinterpret_cast<const uint4*>(src) + g, 16);
+            }
+          }
+          if constexpr (!(kFp8 && kOutBf)) cp_async_wait_all();
+        }
+      }
+      fence_proxy_async();
+      mbar_arrive(q_full(wg));
+    };
+
+    int item = blockIdx.x < unsigned(total) ? int(blockIdx.x) : INT32_MAX;
+    PrefillItem it{};
+    if (item < total) {
+      it = decode(item);
+      load_q(it);
+    }
+    while (item < total && ok) {
+      const int b = it.b, e = wg == 0 ? it.e0 : it.e1;
+      const int tok = it.tok0 + wg * T + row_tok;
+      const bool valid = row_used && tok < it.q_len;
+      const int pos = valid ? it.ctx + tok : -1;                     // last key of this row
+      const int pos_first = it.ctx + it.tok0 + wg * T;               // ... of the tile's first row
+      const int head = it.kvh * G + row_head;
+      const float slope = (p.alibi != nullptr && valid) ? p.alibi[head] * kLog2e : 0.f;
+      float m = -INFINITY, l = 0.f;
+      for (int j = b; j < e; ++j) {
+        if (!wait_warp(s_full(wg), n_s & 1)) break;
+        ++n_s;
+        tc_fence_after();
+        const int key0 = j * KT;
+        // full tiles without a bias need no per-element work besides the scale
+        const bool plain = key0 + KT - 1 <= pos_first && p.alibi == nullptr && c > 0.f;
+        float mx = -INFINITY;
+        float v[32];
+        if (plain) {
+#pragma unroll
+          for (int ch = 0; ch < KT / 32; ++ch) {
+            tmem_ld32(t_s + ch * 32, v);
+            tmem_landed(v);
+            float m4[4] = {v[0], v[1], v[2], v[3]};
+#pragma unroll
+            for (int k = 4; k < 32; ++k) m4[k & 3] = fmaxf(m4[k & 3], v[k]);
+            mx = fmaxf(mx, fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])));
+          }
+          mx *= c;
+        } else {
+#pragma unroll 1
+          for (int ch = 0; ch < KT / 32; ++ch) {
+            tmem_ld32(t_s + ch * 32, v);
+            tmem_landed(v);
+            const int k0 = key0 + ch * 32;
+#pragma unroll
+            for (int k = 0; k < 32; ++k)
+              if (k0 + k <= pos) mx = fmaxf(mx, v[k] * c + slope * float(k0 + k - pos));
+          }
+        }
+        // raise the maximum (and rescale what has been summed) only when it grew by more than 8
+        const bool grow = mx > m + 8.f || (m == -INFINITY && mx > m);
+        if (__any_sync(0xffffffffu, grow)) {
+          const float m_new = fmaxf(m, mx);
+          const float alpha = m_new == -INFINITY ? 1.f : fast_exp2(m - m_new);
+          m = m_new;
+          l *= alpha;
+          if (j > b) {
+            if (!wait_warp(pv_done(wg), (n_pv - 1) & 1)) break;
+            tc_fence_after();
+#pragma unroll 1
+            for (int ch = 0; ch < DP / 16; ++ch) {
+              float o[16];
+              tmem_ld16(t_o + ch * 16, o);
+#pragma unroll
+              for (int k = 0; k < 16; ++k) o[k] *= alpha;
+              tmem_st16(t_o + ch * 16, o);
+            }
+            tmem_wait_st();
+          }
+        }
+        const float mm = m == -INFINITY ? 0.f : m;
+        float sum = 0.f;
+        if (plain) {
+#pragma unroll
+          for (int ch = 0; ch < KT / 32; ++ch) {
+            tmem_ld32(t_s + ch * 32, v);
+            tmem_landed(v);
+            float s4[4] = {0.f, 0.f, 0.f, 0.f};
+            uint32_t w[16];
+#pragma unroll
+            for (int k = 0; k < 32; k += 2) {
+              const float p0 = fast_exp2(fmaf(v[k], c, -mm)), p1 = fast_exp2(fmaf(v[k + 1], c, -mm));
+              s4[k & 2] += p0;
+              s4[(k & 2) + 1] += p1;
+              w[k / 2] = pack2<kBf>(p0, p1);
+            }
+            sum += (s4[0] + s4[1]) + (s4[2] + s4[3]);
+            tmem_st16(t_s + ch * 16, w);
+          }
+        } else {
+#pragma unroll 1
+          for (int ch = 0; ch < KT / 32; ++ch) {
+            tmem_ld32(t_s + ch * 32, v);
+            tmem_landed(v);
+            const int k0 = key0 + ch * 32;
+            uint32_t w[16];
+#pragma unroll
+            for (int k = 0; k < 32; k += 2) {
+              const float p0 = k0 + k <= pos ? fast_exp2(v[k] * c + slope * float(k0 + k - pos) - mm) : 0.f;
+              const float p1 = k0 + k + 1 <= pos ? fast_exp2(v[k + 1] * c + slope * float(k0 + k + 1 - pos) - mm) : 0.f;
+              sum += p0 + p1;
+              w[k / 2] = pack2<kBf>(p0, p1);
+            }
+            tmem_st16(t_s + ch * 16, w);
+          }
+        }
+        l += sum;
+        tmem_wait_st();
+        tc_fence_before();
+        mbar_arrive(p_full(wg));
+        ++n_pv;
+      }
+      if (!ok) break;
+      // ---- the next item's Q goes in while this one's last product runs (S of the last tile has
+      // been received, so nothing reads this tile's Q any more)
+      const PrefillItem cur = it;
+      item = next_item();
+      ok = __all_sync(0xffffffffu, ok);
+      if (item < total) {
+        it = decode(item);
+        load_q(it);
+      }
+      if (!ok) break;
+      if (wg >= NQ) continue;
+      // ---- results
+      const bool any = e > b;
+      if (any) {
+        if (!wait_warp(pv_done(wg), (n_pv - 1) & 1)) break;
+        tc_fence_after();
+      }
+      const bool whole = cur.npieces == 1;
+      const float inv = v_scale * __fdividef(1.f, l + 1e-6f);
+      const int64_t out_row = (int64_t(cur.q0 + tok) * p.num_heads + head) * D;
+      unsigned char* part = p.ws + (size_t(cur.first + cur.piece * HK) * NQ + wg) * kWs;
+      QT* dst = whole ? static_cast<QT*>(p.out) + out_row
+                      : reinterpret_cast<QT*>(part) + row * D;
+      if (any || whole) {
+#pragma unroll 1
+        for (int ch = 0; ch < DP / 16; ++ch) {
+          float o[16];
+          if (any) {
+            tmem_ld16(t_o + ch * 16, o);
+          } else {
+#pragma unroll
+            for (int k = 0; k < 16; ++k) o[k] = 0.f;
+          }
+          if (valid) {
+            uint32_t w[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) w[k] = pack2<kOutBf>(o[2 * k] * inv, o[2 * k + 1] * inv);
+            uint4* d4 = reinterpret_cast<uint4*>(dst + ch * 16);
+            d4[0] = make_uint4(w[0], w[1], w[2], w[3]);
+            if (ch * 16 + 8 < D) d4[1] = make_uint4(w[4], w[5], w[6], w[7]);
+          }
+        }
+        tc_fence_before();  // (ordered before the next item's p_full, which frees O)
+      }
+      if (!whole) {
+        float* stats = reinterpret_cast<float*>(part + 128 * D * 2);
+        if (valid) reinterpret_cast<float2*>(stats)[row] = make_float2(m, any ? l : 0.f);
+        // the rows of a warp are merged by the warp that delivers their last piece
+        __threadfence();
+        __syncwarp();
+        unsigned old = 0;
+        unsigned* cnt = p.arrive + (size_t(cur.first) * NQ + wg) * 4 + (warp & 3);
+        if (lane == 0) {
+          old = atomicAdd(cnt, 1u);
+          if (old == unsigned(cur.npieces - 1)) *cnt = 0;  // re-arm for the next launch
+        }
+        old = __shfl_sync(0xffffffffu, old, 0);
+        if (old == unsigned(cur.npieces - 1) && valid) {
+          __threadfence();
+          const unsigned char* base = p.ws + (size_t(cur.first) * NQ + wg) * kWs;
+          const size_t step = size_t(HK) * NQ * kWs;
+          float mx = -INFINITY;
+          for (int k = 0; k < cur.npieces; ++k) {
+            const float2 ml = __ldcg(reinterpret_cast<const float2*>(base + k * step + 128 * D * 2) + row);
+            if (ml.y > 0.f) mx = fmaxf(mx, ml.x);
+          }
+          float total_l = 0.f;
+          for (int k = 0; k < cur.npieces; ++k) {
+            const float2 ml = __ldcg(reinterpret_cast<const float2*>(base + k * step + 128 * D * 2) + row);
+            if (ml.y > 0.f) total_l += ml.y * fast_exp2(ml.x - mx);
+          }
+          const float winv = __fdividef(1.f, total_l + 1e-6f);
+          QT* od = static_cast<QT*>(p.out) + out_row;
+#pragma unroll 1
+          for (int d0 = 0; d0 < D; d0 += 8 * 4) {
+            float acc[4][8];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+              for (int k = 0; k < 8; ++k) acc[u][k] = 0.f;
+            for (int k = 0; k < cur.npieces; ++k) {
+              const float2 ml = __ldcg(reinterpret_cast<const float2*>(base + k * step + 128 * D * 2) + row);
+              if (!(ml.y > 0.f)) continue;
+              const float w = ml.y * fast_exp2(ml.x - mx) * winv;
+              const QT* src = reinterpret_cast<const QT*>(base + k * step) + row * D + d0;
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                if (d0 + u * 8 < D) {
+                  const uint4 x = __ldcg(reinterpret_cast<const uint4*>(src) + u);
+                  const QT* xe = reinterpret_cast<const QT*>(&x);
+#pragma unroll
+                  for (int z = 0; z < 8; ++z) acc[u][z] += w * to_f32(xe[z]);
+                }
+              }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              if (d0 + u * 8 < D)
+                reinterpret_cast<uint4*>(od + d0)[u] =
+                    make_uint4(pack2<kOutBf>(acc[u][0], acc[u][1]), pack2<kOutBf>(acc[u][2], acc[u][3]),
+                               pack2<kOutBf>(acc[u][4], acc[u][5]), pack2<kOutBf>(acc[u][6], acc[u][7]));
+          }
+        }
+        __syncwarp();
+      }
+    }
+  } else if (warp < 12) {
+    // ================================================= producers: K and V tiles into shared memory
+    const int pt = tid - 256;  // 0 .. 127
+    uint32_t n_half = 0;       // halves (K or V tiles) put on their way
+    uint32_t n_done = 0;       // ... and announced
+    const char* kb = static_cast<const char*>(p.kc);
+    const char* vb = static_cast<const char*>(p.vc);
+    constexpr int ES = kFp8 ? 1 : 2;
+    auto full_of = [&](uint32_t h) { return (h & 1) ? v_full((h >> 1) % NST) : k_full((h >> 1) % NST); };
+    auto empty_of = [&](uint32_t h) { return (h & 1) ? v_empty((h >> 1) % NST) : k_empty((h >> 1) % NST); };
+    auto wait_slot = [&](uint32_t h) {
+      const uint32_t use = (h >> 1) / NST;  // times the slot has been filled before
+      return use == 0 || wait(empty_of(h), (use - 1) & 1);
+    };
+    auto announce = [&]() {
+      fence_proxy_async();
+      mbar_arrive(full_of(n_done));
+      ++n_done;
+    };
+    int item = blockIdx.x < unsigned(total) ? int(blockIdx.x) : INT32_MAX;
+    while (item < total && ok) {
+      const PrefillItem it = decode(item);
+      const int* bt = p.block_tables + int64_t(it.req) * p.max_blocks_per_seq;
+      const int64_t head_off = int64_t(it.kvh) * p.kv_head_stride * ES;
+      const int e = max(it.e0, it.e1);
+      // the page byte address of key `key` (its block's start), or of block 0 past the end
+      auto page = [&](const char* base, int key) -> const char* {
+        const int blk = key < it.seq_len ? __ldg(bt + (key >> b_shift)) : 0;
+        return base + int64_t(blk) * p.kv_block_stride * ES + head_off;
+      };
+      if constexpr (!kFp8) {
+        // K: a thread owns one key and walks along its 16-byte granules; V: a thread owns 8 keys
+        // and every 8th head dimension (128 bytes of shared memory per 8 threads in both cases)
+        const int kt = pt % KT, kg = pt / KT;
+        constexpr int VJ = KT / 8;              // 8-key groups per tile
+        const int vj = pt / 8 % VJ, vd = pt % 8 + 8 * (pt / 8 / VJ);
+        for (int j = it.b; j < e && ok; ++j) {
+          {
+            const int key = j * KT + kt;
+            const char* src = page(kb, key) + (key & (B - 1)) * 16;
+            const int bytes = key < it.seq_len ? 16 : 0;
+            if (!wait_slot(n_half)) break;
+            const uint32_t dst = sk + ((n_half >> 1) % NST) * SH::kTileBytes + kt * 16;
+#pragma unroll
+            for (int g = kg; g < D / 8; g += 128 / KT)
+              cp_async16(dst + g * KT * 16, src + int64_t(g) * B * 16, bytes);
+            cp_async_commit();
+            ++n_half;
+            if (n_half - n_done > 2) {
+              cp_async_wait<2>();
+              announce();
+            }
+          }
+          {
+            const int key = j * KT + vj * 8;
+            const char* src = page(vb, key) + (key & (B - 1)) * 2;
+            const int bytes = max(0, min(16, (it.seq_len - key) * 2));  // keys past the end: zeros
+            if (!wait_slot(n_half)) break;
+            const uint32_t dst = sv + ((n_half >> 1) % NST) * SH::kTileBytes + vj * DP * 16;
+#pragma unroll
+            for (int d = 0; d < D; d += 8 * (16 / VJ))
+              if (D % (8 * (16 / VJ)) == 0 || d + vd < D)
+                cp_async16(dst + (d + vd) * 16, src + int64_t(d + vd) * B * 2, bytes);
+            cp_async_commit();
+            ++n_half;
+            if (n_half - n_done > 2) {
+              cp_async_wait<2>();
+              announce();
+            }
+          }
+        }
+      } else {
+        // fp8: 16-byte loads into registers (the next half is always in flight), widened to two
+        // 16-byte granules of f16.  K: a thread owns one key; V: 16 keys and every 16th dimension.
+        const int kt = pt % KT, kg = pt / KT;
+        constexpr int KN = (D / 16 + 128 / KT - 1) / (128 / KT);
+        constexpr int VJ = KT / 16;
+        constexpr int VDS = 128 / VJ;           // threads that share a 16-key group
+        const int vj = pt / VDS, vd = pt % VDS;
+        constexpr int VN = (D + VDS - 1) / VDS;
+        uint4 kr[KN], vr[VN];
+        auto get_k = [&](int j) {
+          const int key = j * KT + kt;
+          const char* src = page(kb, key) + (key & (B - 1)) * 16;
+#pragma unroll
+          for (int i = 0; i < KN; ++i) {
+            const int g = kg + i * (128 / KT);
+            if (key < it.seq_len && g < D / 16) kr[i] = __ldg(reinterpret_cast<const uint4*>(src + int64_t(g) * B * 16));
+            else kr[i] = make_uint4(0, 0, 0, 0);
+          }
+        };
+        auto get_v = [&](int j) {
+          const int key = j * KT + vj * 16;
+          const char* src = page(vb, key) + (key & (B - 1));
+#pragma unroll
+          for (int i = 0; i < VN; ++i) {
+            const int d = vd + i * VDS;
+            if (key < it.seq_len && d < D) vr[i] = __ldg(reinterpret_cast<const uint4*>(src + int64_t(d) * B));
+            else vr[i] = make_uint4(0, 0, 0, 0);
+          }
+        };
+        auto widen = [&](const uint4& x, uint4& lo, uint4& hi) {
+          fp8x4_to_f16<kE5>(x.x, lo.x, lo.y);
+          fp8x4_to_f16<kE5>(x.y, lo.z, lo.w);
+          fp8x4_to_f16<kE5>(x.z, hi.x, hi.y);
+          fp8x4_to_f16<kE5>(x.w, hi.z, hi.w);
+        };
+        if (it.b < e) {
+          get_k(it.b);
+          get_v(it.b);
+        }
+        for (int j = it.b; j < e && ok; ++j) {
+          if (!wait_slot(n_half)) break;
+          {
+            const uint32_t dst = sk + ((n_half >> 1) % NST) * SH::kTileBytes + kt * 16;
+#pragma unroll
+            for (int i = 0; i < KN; ++i) {
+              const int g = kg + i * (128 / KT);
+              if (D / 16 % (128 / KT) == 0 || g < D / 16) {
+                uint4 lo, hi;
+                widen(kr[i], lo, hi);
+                st_shared16(dst + (2 * g) * KT * 16, lo);
+                st_shared16(dst + (2 * g + 1) * KT * 16, hi);
+              }
+            }
+            ++n_half;
+            announce();
+            if (j + 1 < e) get_k(j + 1);
+          }
+          if (!wait_slot(n_half)) break;
+          {
+            const uint32_t dst = sv + ((n_half >> 1) % NST) * SH::kTileBytes + 2 * vj * DP * 16;
+            const int left = it.seq_len - (j * KT + vj * 16);  // keys of the group that exist
+#pragma unroll
+            for (int i = 0; i < VN; ++i) {
+              const int d = vd + i * VDS;
+              if (D % VDS == 0 || d < D) {
+                uint4 x = vr[i];
+                if (left < 16) {  // keys past the end: zeros
+                  auto keep = [&](uint32_t w, int at) {
+                    const int n = left - at;
+                    return n >= 4 ? w : (n <= 0 ? 0u : w & (0xffffffffu >> (32 - 8 * n)));
+                  };
+                  x = make_uint4(keep(x.x, 0), keep(x.y, 4), keep(x.z, 8), keep(x.w, 12));
+                }
+                uint4 lo, hi;
+                widen(x, lo, hi);
+                st_shared16(dst + d * 16, lo);
+                st_shared16(dst + (DP + d) * 16, hi);
+              }
+            }
+            ++n_half;
+            announce();
+            if (j + 1 < e) get_v(j + 1);
+          }
+        }
+      }
+      if (!ok) break;
+      if constexpr (!kFp8) {
+        // (an item without key tiles announces nothing, and the item after it is only drawn when
+        // the MMAs have come here: what is on its way has to be announced first)
+        if (it.b >= e) {
+          cp_async_wait<0>();
+          while (n_done < n_half) announce();
+        }
+      }
+      item = next_item();
+    }
+    if constexpr (!kFp8) {
+      cp_async_wait<0>();
+      while (ok && n_done < n_half) announce();
+    }
+  } else if (lane == 0) {
+    // ================================================= the MMA thread
+    const uint32_t idesc_s = mma_idesc(kBf, 128, KT);
+    const uint32_t idesc_o = mma_idesc(kBf, 128, DP);
+    uint32_t n_k = 0, n_v = 0, n_it = 0, n_p[2] = {0, 0};
+    auto qk = [&](int i, uint32_t st) {
+#pragma unroll
+      for (int ks = 0; ks < DP / 16; ++ks)
+        mma_ss(tmem + i * KT, smem_desc(sq + i * SH::kQBytes + ks * 2 * 128 * 16, 128 * 16, 128),
+               smem_desc(sk + st * SH::kTileBytes + ks * 2 * KT * 16, KT * 16, 128), idesc_s, ks > 0);
+      mma_commit(s_full(i));
+    };
+    auto pv = [&](int i, uint32_t st, bool more) {
+#pragma unroll
+      for (int ks = 0; ks < KT / 16; ++ks)
+        mma_ts(tmem + NQ * KT + i * DP, tmem + i * KT + ks * 8,
+               smem_desc(sv + st * SH::kTileBytes + ks * 2 * DP * 16, DP * 16, 128), idesc_o, more || ks > 0);
+      mma_commit(pv_done(i));
+    };
+    int item = blockIdx.x < unsigned(total) ? int(blockIdx.x) : INT32_MAX;
+    while (item < total && ok) {
+      // draw the next item now; the other roles pick it up when they are through with this one
+      const unsigned ticket = atomicAdd(p.sched, 1u);
+      const PrefillItem it = decode(item);
+      const int nxt = int(min(ticket + gridDim.x, unsigned(INT32_MAX)));
+      {
+        const int slot = n_it & 1;
+        if (n_it >= 2 && !wait(item_empty(slot), ((n_it >> 1) - 1) & 1)) break;
+        *reinterpret_cast<volatile int*>(&s_item[slot]) = nxt;
+        mbar_arrive(item_full(slot));
+      }
+      const int e = max(it.e0, it.e1);
+      if (!wait(q_full(0), n_it & 1) || !wait(q_full(1), n_it & 1)) break;
+      ++n_it;
+      tc_fence_after();
+      if (it.b < e) {
+        if (!wait(k_full(n_k % NST), (n_k / NST) & 1)) break;
+        tc_fence_after();
+#pragma unroll
+        for (int i = 0; i < NQ; ++i)
+          if (it.b < (i == 0 ? it.e0 : it.e1)) qk(i, n_k % NST);
+        mma_commit(k_empty(n_k % NST));
+        ++n_k;
+      }
+      for (int j = it.b; j < e && ok; ++j) {
+        if (!wait(v_full(n_v % NST), (n_v / NST) & 1)) break;
+        bool have_k = false;
+#pragma unroll
+        for (int i = 0; i < NQ; ++i) {
+          const int ei = i == 0 ? it.e0 : it.e1;
+          if (!ok || j >= ei) continue;
+          if (!wait(p_full(i), n_p[i] & 1)) continue;
+          ++n_p[i];
+          tc_fence_after();
+          pv(i, n_v % NST, j > it.b);
+          if (j + 1 < ei) {
+            if (!have_k) {
+              if (!wait(k_full(n_k % NST), (n_k / NST) & 1)) continue;
+              tc_fence_after();
+              have_k = true;
+            }
+            qk(i, n_k % NST);
+          }
+        }
+        if (!ok) break;
+        mma_commit(v_empty(n_v % NST));
+        ++n_v;
+        if (have_k) {
+          mma_commit(k_empty(n_k % NST));
+          ++n_k;
+        }
+      }
+      item = nxt;
+    }
+  }
+
+  // ---- everything issued has been waited for by the softmax warpgroups (or a wait ran out)
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 12) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 512);
+  }
+  if (tid == 0) {
+    __threadfence();
+    const unsigned prev = atomicAdd(p.sched + 1, 1u);
+    if (prev == gridDim.x - 1) {
+      p.sched[0] = 0;
+      p.sched[1] = 0;
+      __threadfence();
+    }
+  }
+}
+
+}  // namespace b200pa

@@ -194,6 +194,32 @@ void paged_attention_v2(torch::Tensor& out, torch::Tensor& exp_sums, torch::Tens
   check_rc(b200pa_paged_attention_v2(&a, at::cuda::getCurrentCUDAStream().stream()));
 }
 
+// Attention of a step whose requests bring several query rows (not an op of the reference).
+// False: no kernel for this shape, nothing was launched.
+bool paged_attention_varlen(torch::Tensor& out, torch::Tensor& query, torch::Tensor& key_cache,
+                            torch::Tensor& value_cache, int64_t num_kv_heads, double scale,
+                            torch::Tensor& block_tables, torch::Tensor& seq_lens,
+                            torch::Tensor& query_start_loc, int64_t num_decodes, int64_t block_size,
+                            int64_t max_seq_len, const std::optional<torch::Tensor>& alibi_slopes,
+                            const std::string& kv_cache_dtype, torch::Tensor& k_scale,
+                            torch::Tensor& v_scale) {
+  b200pa_attn_args a;
+  fill_attn(a, out, query, key_cache, value_cache, num_kv_heads, scale, block_tables, seq_lens,
+            block_size, max_seq_len, alibi_slopes, kv_cache_dtype, k_scale, v_scale, 0, 0, 0, 64, 0);
+  TORCH_CHECK(query_start_loc.is_cuda() && query_start_loc.scalar_type() == at::ScalarType::Int &&
+                  query_start_loc.is_contiguous() && query_start_loc.numel() == seq_lens.numel() + 1,
+              "query_start_loc must be a contiguous int32 CUDA tensor [num_requests + 1]");
+  a.num_seqs = static_cast<int32_t>(seq_lens.size(0));
+  const at::cuda::OptionalCUDAGuard device_guard(device_of(query));
+  const int rc = b200pa_paged_attention_varlen(&a, query_start_loc.data_ptr<int>(),
+                                               static_cast<int32_t>(query.size(0)),
+                                               static_cast<int32_t>(num_decodes),
+                                               at::cuda::getCurrentCUDAStream().stream());
+  if (rc == B200PA_EUNSUPPORTED) return false;
+  check_rc(rc);
+  return true;
+}
+
 void fill_cache(b200pa_cache_args& a, torch::Tensor& key, torch::Tensor& value,
                 torch::Tensor& key_cache, torch::Tensor& value_cache, torch::Tensor& slot_mapping,
                 const std::string& kv_cache_dtype, torch::Tensor& k_scale, torch::Tensor& v_scale) {
@@ -457,6 +483,16 @@ TORCH_LIBRARY(_C_b200, ops) {
       " int block_size, int max_seq_len, Tensor? alibi_slopes, str kv_cache_dtype,"
       " Tensor k_scale, Tensor v_scale) -> ()");
   ops.impl("paged_attention_with_lse", torch::kCUDA, &paged_attention_with_lse);
+}
+
+// (see b200pa_paged_attention_varlen)
+TORCH_LIBRARY_FRAGMENT(_C_b200, ops) {
+  ops.def(
+      "paged_attention_varlen(Tensor! out, Tensor query, Tensor key_cache, Tensor value_cache,"
+      " int num_kv_heads, float scale, Tensor block_tables, Tensor seq_lens, Tensor query_start_loc,"
+      " int num_decodes, int block_size, int max_seq_len, Tensor? alibi_slopes, str kv_cache_dtype,"
+      " Tensor k_scale, Tensor v_scale) -> bool");
+  ops.impl("paged_attention_varlen", torch::kCUDA, &paged_attention_varlen);
 }
 
 TORCH_LIBRARY(_C_b200_cache_ops, cache_ops) {

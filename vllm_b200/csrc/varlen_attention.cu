@@ -1,0 +1,97 @@
+// Host entry of attention over a step whose requests bring several query tokens each: the requests
+// in front that bring one go to the decode kernel, the others to the prefill kernel.
+#include <algorithm>
+#include <cstdint>
+
+#include "launch_state.cuh"
+#include "prefill_inst.cuh"
+
+extern "C" int b200pa_paged_attention_varlen(const b200pa_attn_args* a, const int32_t* query_start_loc,
+                                             int32_t num_tokens, int32_t num_decodes, void* stream) {
+  using namespace b200pa;
+  B200PA_CHECK_ARG(a != nullptr, "args is NULL");
+  B200PA_CHECK_ARG(a->num_seqs >= 0 && a->num_heads > 0 && a->num_kv_heads > 0 && a->head_size > 0 &&
+                       a->num_heads % a->num_kv_heads == 0,
+                   "bad sizes: num_seqs=%d num_heads=%d num_kv_heads=%d head_size=%d", a->num_seqs,
+                   a->num_heads, a->num_kv_heads, a->head_size);
+  B200PA_CHECK_ARG(num_decodes >= 0 && num_decodes <= a->num_seqs && num_tokens >= num_decodes,
+                   "bad counts: %d requests, %d decodes, %d tokens", a->num_seqs, num_decodes, num_tokens);
+  const int reqs = a->num_seqs - num_decodes;
+  PrefillKernelInfo ki{nullptr, 0};
+  if (reqs > 0) {
+    B200PA_CHECK_ARG(a->out && a->query && a->key_cache && a->value_cache && a->block_tables &&
+                         a->seq_lens && query_start_loc,
+                     "null tensor pointer");
+    B200PA_CHECK_ARG(a->kv_dtype == B200PA_KV_AUTO || (a->k_scale && a->v_scale),
+                     "fp8 kv cache needs k_scale and v_scale");
+    B200PA_CHECK_ARG(a->max_num_blocks_per_seq > 0, "max_num_blocks_per_seq must be positive");
+    // 16-byte accesses: pages, rows of Q and of the output; cache offsets inside a block are shifts
+    const int es = a->kv_dtype == B200PA_KV_AUTO ? 2 : 1;
+    auto al = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr) % 16 == 0; };
+    const bool fits = (a->block_size == 16 || a->block_size == 32) && a->num_heads / a->num_kv_heads <= 128 &&
+                      reqs <= kPrefillMaxReqs && al(a->key_cache) && al(a->value_cache) && al(a->query) &&
+                      al(a->out) && (a->kv_block_stride * es) % 16 == 0 && (a->kv_head_stride * es) % 16 == 0 &&
+                      a->q_stride % 8 == 0 && a->blocksparse_vert_stride <= 1 && a->out_lse == nullptr;
+    if (fits) {
+      ki = a->head_size <= 96 ? find_prefill_small(a->head_size, a->q_dtype, a->kv_dtype)
+           : a->head_size <= 128 ? find_prefill_mid(a->head_size, a->q_dtype, a->kv_dtype)
+                                 : find_prefill_large(a->head_size, a->q_dtype, a->kv_dtype);
+    }
+    if (ki.fn == nullptr) {
+      set_error("paged_attention_varlen: no kernel for head_size=%d block_size=%d q_dtype=%d kv_dtype=%d, "
+                "%d requests, or unaligned tensors",
+                a->head_size, a->block_size, a->q_dtype, a->kv_dtype, reqs);
+      return B200PA_EUNSUPPORTED;
+    }
+  }
+  if (num_decodes > 0) {
+    // the decode rows are the first rows of query and out: an ordinary decode batch
+    b200pa_attn_args d = *a;
+    d.num_seqs = num_decodes;
+    const int rc = b200pa_paged_attention_v1(&d, stream);
+    if (rc != B200PA_OK) return rc;
+  }
+  if (reqs == 0) return B200PA_OK;
+
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  PrefillParams p{};
+  p.out = a->out;
+  p.q = a->query;
+  p.kc = a->key_cache;
+  p.vc = a->value_cache;
+  p.block_tables = a->block_tables + int64_t(num_decodes) * a->max_num_blocks_per_seq;
+  p.seq_lens = a->seq_lens + num_decodes;
+  p.q_start = query_start_loc + num_decodes;
+  p.alibi = a->alibi_slopes;
+  p.k_scale = a->k_scale;
+  p.v_scale = a->v_scale;
+  p.q_stride = a->q_stride;
+  p.kv_block_stride = a->kv_block_stride;
+  p.kv_head_stride = a->kv_head_stride;
+  p.num_reqs = reqs;
+  p.num_heads = a->num_heads;
+  p.num_kv_heads = a->num_kv_heads;
+  p.group = a->num_heads / a->num_kv_heads;
+  p.block_size = a->block_size;
+  p.max_blocks_per_seq = a->max_num_blocks_per_seq;
+  p.scale = a->scale;
+  StreamRegion region{};
+  if (stream_region(s, &region)) {  // (without one the keys of an item are not split)
+    p.ws = region.ws;
+    p.arrive = region.arrive;
+    p.ws_slots = int(std::min<int64_t>(int64_t(region.ws_bytes) / ki.piece_bytes, kArrivePerRegion / 8));
+  }
+  p.sched = sched_words();
+  p.status = device_status_ptr();
+  if (p.sched == nullptr || p.status == nullptr) {
+    set_error("could not resolve device-side scheduler/status words");
+    return B200PA_ECUDA;
+  }
+  const cudaError_t e = ki.fn(p, sm_count(), s);
+  count_launch();
+  if (e != cudaSuccess) {
+    set_error("prefill kernel launch failed: %s", cudaGetErrorString(e));
+    return B200PA_ECUDA;
+  }
+  return B200PA_OK;
+}
