@@ -25,6 +25,12 @@ def _load() -> None:
 
 
 _load()
+from vllm_b200 import _C_b200 as _direct  # noqa: E402  (the same library, loaded above)
+
+# The direct bindings below save the host time of a call through the dispatcher.  They return
+# False, with nothing done, for whatever is not a plain eager call on CUDA tensors; under tracing
+# the operators themselves have to be seen.
+_compiling = torch.compiler.is_compiling
 
 # Always-present private namespaces.
 _ops = torch.ops._C_b200
@@ -77,6 +83,12 @@ def paged_attention_v1(
     blocksparse_block_size: int = 64,
     blocksparse_head_sliding_step: int = 0,
 ) -> None:
+    if not _compiling() and _direct.paged_attention_v1(
+            out, query, key_cache, value_cache, num_kv_heads, scale, block_tables, seq_lens,
+            block_size, max_seq_len, alibi_slopes, kv_cache_dtype, k_scale, v_scale, tp_rank,
+            blocksparse_local_blocks, blocksparse_vert_stride, blocksparse_block_size,
+            blocksparse_head_sliding_step):
+        return
     _ops.paged_attention_v1(
         out, query, key_cache, value_cache, num_kv_heads, scale, block_tables, seq_lens,
         block_size, max_seq_len, alibi_slopes, kv_cache_dtype, k_scale, v_scale, tp_rank,
@@ -108,6 +120,12 @@ def paged_attention_v2(
     blocksparse_block_size: int = 64,
     blocksparse_head_sliding_step: int = 0,
 ) -> None:
+    if not _compiling() and _direct.paged_attention_v2(
+            out, exp_sum, max_logits, tmp_out, query, key_cache, value_cache, num_kv_heads, scale,
+            block_tables, seq_lens, block_size, max_seq_len, alibi_slopes, kv_cache_dtype, k_scale,
+            v_scale, tp_rank, blocksparse_local_blocks, blocksparse_vert_stride,
+            blocksparse_block_size, blocksparse_head_sliding_step):
+        return
     _ops.paged_attention_v2(
         out, exp_sum, max_logits, tmp_out, query, key_cache, value_cache, num_kv_heads, scale,
         block_tables, seq_lens, block_size, max_seq_len, alibi_slopes, kv_cache_dtype, k_scale,
@@ -125,6 +143,9 @@ def reshape_and_cache(
     k_scale: torch.Tensor,
     v_scale: torch.Tensor,
 ) -> None:
+    if not _compiling() and _direct.reshape_and_cache(
+            key, value, key_cache, value_cache, slot_mapping, kv_cache_dtype, k_scale, v_scale):
+        return
     _cache_ops.reshape_and_cache(
         key, value, key_cache, value_cache, slot_mapping, kv_cache_dtype, k_scale, v_scale)
 
@@ -139,6 +160,9 @@ def reshape_and_cache_flash(
     k_scale: torch.Tensor,
     v_scale: torch.Tensor,
 ) -> None:
+    if not _compiling() and _direct.reshape_and_cache_flash(
+            key, value, key_cache, value_cache, slot_mapping, kv_cache_dtype, k_scale, v_scale):
+        return
     _cache_ops.reshape_and_cache_flash(
         key, value, key_cache, value_cache, slot_mapping, kv_cache_dtype, k_scale, v_scale)
 
@@ -201,6 +225,13 @@ def paged_attention_varlen(
         out, query, key_cache, value_cache, num_kv_heads, scale, block_tables, seq_lens,
         query_start_loc, num_decodes, block_size, max_seq_len, alibi_slopes, kv_cache_dtype, k_scale,
         v_scale)
+
+
+def attention_step(*args) -> bool:
+    """KV write and attention of one layer of an engine step in one native call; the arguments are
+    those of ``B200PagedAttentionImpl.forward`` (the only caller), in its order.  False when the
+    call is not a plain one: the caller then goes through the operators one by one."""
+    return not _compiling() and _direct.attention_step(*args)
 
 
 def merge_attn_states(

@@ -161,17 +161,25 @@ class B200PagedAttentionImpl:
             raise NotImplementedError("fused output quantisation is not supported")
         if attn_metadata is None:  # profiling run
             return output.fill_(0)
-        assert attn_metadata.use_cascade is False
-        n = attn_metadata.num_actual_tokens
+        md = attn_metadata
+        assert md.use_cascade is False
+        n = md.num_actual_tokens
+        alibi = self.alibi_slopes
+        if alibi is not None and alibi.device != query.device:
+            alibi = self.alibi_slopes = alibi.to(query.device)
+        if ops.attention_step(
+                output, query, key, value, kv_cache, md.block_table, md.seq_lens, md.slot_mapping,
+                md.query_start_loc, layer._k_scale, layer._v_scale, alibi, n, md.num_decodes,
+                md.max_query_len, md.max_seq_len, self.num_heads, self.num_kv_heads, self.head_size,
+                self.scale, self.kv_cache_dtype, self.kv_sharing_target_layer_name is None):
+            return output
+        # not a plain call (fp32, odd strides, tracing, ...): operator by operator
         key_cache, value_cache = PagedAttention.split_kv_cache(kv_cache, self.num_kv_heads,
                                                                self.head_size)
         if self.kv_sharing_target_layer_name is None:
             PagedAttention.write_to_paged_cache(key[:n], value[:n], key_cache, value_cache,
                                                 attn_metadata.slot_mapping[:n], self.kv_cache_dtype,
                                                 layer._k_scale, layer._v_scale)
-        alibi = self.alibi_slopes
-        if alibi is not None and alibi.device != query.device:
-            alibi = self.alibi_slopes = alibi.to(query.device)
         q = query[:n].view(n, self.num_heads, self.head_size)
         if attn_metadata.max_query_len == 1:
             seq_lens, block_table = attn_metadata.seq_lens, attn_metadata.block_table

@@ -83,7 +83,7 @@ def build_shim(force: bool = False, verbose: bool = False) -> Path:
                                                    "-I/usr/local/cuda/include"]
     cmd = ["g++", "-shared", "-fPIC", "-O2", "-std=c++17", "-D_GLIBCXX_USE_CXX11_ABI=1",
            str(src), "-o", str(SHIM)] + inc + [
-        f"-L{PKG}", "-lb200pa", f"-L{tlib}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10",
+        f"-L{PKG}", "-lb200pa", f"-L{tlib}", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10",
         "-lc10_cuda", "-L/usr/local/cuda/lib64", "-lcudart",
         "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{tlib}"]
     _run(cmd, verbose)

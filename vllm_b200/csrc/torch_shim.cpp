@@ -9,7 +9,12 @@
 // registered as torch.ops._C_b200.* / torch.ops._C_b200_cache_ops.*; on request
 // (b200_claim_reference_names) also under the reference's own names
 // (_C / _C_cache_ops), so code written against vllm._custom_ops runs unchanged.
+#include <torch/csrc/autograd/python_variable.h>  // (Python.h comes first)
+
+#include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/core/dispatch/Dispatcher.h>
+#include <ATen/record_function.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/all.h>
@@ -570,3 +575,274 @@ extern "C" int b200_claim_reference_names(char* err, int err_len) {
     return -1;
   }
 }
+
+// ------------------------------------------------------------------ direct Python bindings
+// A call through torch.ops costs 4-8 us of host time with arguments as many as these (boxing, schema
+// matching, dispatch), more than the small launches take on the GPU.  The module below binds the
+// same functions directly.  Every function returns True when it has done the work, and False when
+// the call is not the plain case - tensor subclasses, tracing or dispatch modes, profiling, autograd,
+// anything that a check objects to: the wrapper then goes through torch.ops, which handles it or
+// raises.
+namespace {
+
+// The calling thread's state allows a call that the dispatcher does not see.
+bool plain_state() {
+  return !c10::impl::TorchDispatchModeTLS::any_modes_set() && !at::impl::torch_function_mode_enabled() &&
+         !at::hasCallbacks();
+}
+
+bool plain_tensor(PyObject* o) {
+  if (!THPVariable_CheckExact(o)) return false;
+  const at::Tensor& t = THPVariable_Unpack(o);
+  return t.defined() && t.is_cuda() && !t.key_set().has(c10::DispatchKey::Python) &&
+         !(t.requires_grad() && c10::GradMode::is_enabled());
+}
+
+// Reads positional arguments in order; `ok` turns false at the first one that is not plain.
+struct Args {
+  PyObject* const* a;
+  Py_ssize_t n, i = 0;
+  bool ok = true;
+  PyObject* next() {
+    if (i >= n) ok = false;
+    return ok ? a[i++] : nullptr;
+  }
+  at::Tensor tensor() {
+    PyObject* o = next();
+    if (o == nullptr || !plain_tensor(o)) return ok = false, at::Tensor();
+    return THPVariable_Unpack(o);
+  }
+  std::optional<at::Tensor> optional_tensor() {
+    PyObject* o = next();
+    if (o == nullptr || o == Py_None) return std::nullopt;
+    if (!plain_tensor(o)) return ok = false, std::nullopt;
+    return THPVariable_Unpack(o);
+  }
+  int64_t integer() {
+    PyObject* o = next();
+    if (o == nullptr || !PyLong_Check(o)) return ok = false, 0;
+    const long long v = PyLong_AsLongLong(o);
+    if (v == -1 && PyErr_Occurred()) PyErr_Clear(), ok = false;
+    return v;
+  }
+  double real() {
+    PyObject* o = next();
+    if (o == nullptr || !PyFloat_Check(o)) return ok = false, 0.0;
+    return PyFloat_AS_DOUBLE(o);
+  }
+  std::string text() {
+    PyObject* o = next();
+    if (o == nullptr || !PyUnicode_Check(o)) return ok = false, std::string();
+    Py_ssize_t len = 0;
+    const char* s = PyUnicode_AsUTF8AndSize(o, &len);
+    if (s == nullptr) return PyErr_Clear(), ok = false, std::string();
+    return std::string(s, size_t(len));
+  }
+};
+
+template <typename F>
+PyObject* direct(Args& in, F&& call) {
+  bool done = false;
+  if (in.ok && in.i == in.n) {
+    PyThreadState* ts = PyEval_SaveThread();
+    try {
+      done = call();
+    } catch (...) {
+      // the wrapper's call through torch.ops raises it again, with everything a caller expects
+      (void)cudaGetLastError();
+    }
+    PyEval_RestoreThread(ts);
+  }
+  return PyBool_FromLong(done);
+}
+
+PyObject* py_paged_attention(PyObject* const* a, Py_ssize_t n, bool v2) {
+  if (!plain_state()) Py_RETURN_FALSE;
+  Args in{a, n};
+  at::Tensor out = in.tensor(), es, ml, tmp;
+  if (v2) {
+    es = in.tensor();
+    ml = in.tensor();
+    tmp = in.tensor();
+  }
+  at::Tensor q = in.tensor(), kc = in.tensor(), vc = in.tensor();
+  const int64_t hk = in.integer();
+  const double scale = in.real();
+  at::Tensor bt = in.tensor(), sl = in.tensor();
+  const int64_t bs = in.integer(), max_len = in.integer();
+  const auto alibi = in.optional_tensor();
+  const std::string kv = in.text();
+  at::Tensor ks = in.tensor(), vs = in.tensor();
+  const int64_t tp = in.integer(), b0 = in.integer(), b1 = in.integer(), b2 = in.integer(), b3 = in.integer();
+  return direct(in, [&] {
+    if (v2)
+      paged_attention_v2(out, es, ml, tmp, q, kc, vc, hk, scale, bt, sl, bs, max_len, alibi, kv, ks, vs, tp, b0,
+                         b1, b2, b3);
+    else
+      paged_attention_v1(out, q, kc, vc, hk, scale, bt, sl, bs, max_len, alibi, kv, ks, vs, tp, b0, b1, b2, b3);
+    return true;
+  });
+}
+PyObject* py_v1(PyObject*, PyObject* const* a, Py_ssize_t n) { return py_paged_attention(a, n, false); }
+PyObject* py_v2(PyObject*, PyObject* const* a, Py_ssize_t n) { return py_paged_attention(a, n, true); }
+
+PyObject* py_write(PyObject* const* a, Py_ssize_t n, bool flash) {
+  if (!plain_state()) Py_RETURN_FALSE;
+  Args in{a, n};
+  at::Tensor k = in.tensor(), v = in.tensor(), kc = in.tensor(), vc = in.tensor(), slots = in.tensor();
+  const std::string kv = in.text();
+  at::Tensor ks = in.tensor(), vs = in.tensor();
+  return direct(in, [&] {
+    if (flash) reshape_and_cache_flash(k, v, kc, vc, slots, kv, ks, vs);
+    else reshape_and_cache(k, v, kc, vc, slots, kv, ks, vs);
+    return true;
+  });
+}
+PyObject* py_write_x(PyObject*, PyObject* const* a, Py_ssize_t n) { return py_write(a, n, false); }
+PyObject* py_write_flash(PyObject*, PyObject* const* a, Py_ssize_t n) { return py_write(a, n, true); }
+
+// One attention layer of an engine step: KV write, then attention, straight from the tensors that
+// the engine hands over (no views, no copies, no scratch tensors where the library's workspace does).
+PyObject* py_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (!plain_state()) Py_RETURN_FALSE;
+  Args in{a, n};
+  at::Tensor out = in.tensor(), q = in.tensor(), k = in.tensor(), v = in.tensor(), cache = in.tensor();
+  at::Tensor bt = in.tensor(), sl = in.tensor(), slots = in.tensor(), qsl = in.tensor();
+  at::Tensor ks = in.tensor(), vs = in.tensor();
+  const auto alibi = in.optional_tensor();
+  const int64_t tokens = in.integer(), decodes = in.integer(), max_q = in.integer(), max_len = in.integer();
+  const int64_t H = in.integer(), HK = in.integer(), D = in.integer();
+  const double scale = in.real();
+  const std::string kv = in.text();
+  const int64_t write = in.integer();
+  return direct(in, [&]() -> bool {
+    using at::ScalarType;
+    const auto type = q.scalar_type();
+    const bool fp8 = kv != "auto";
+    // rows of q, k, v: heads and head dimensions contiguous
+    auto rows = [&](const at::Tensor& t, int64_t heads) {
+      return t.dim() == 3 && t.size(0) >= tokens && t.size(1) == heads && t.size(2) == D && t.stride(2) == 1 &&
+             t.stride(1) == D && t.scalar_type() == type;
+    };
+    if (type != ScalarType::BFloat16 && type != ScalarType::Half) return false;
+    if (tokens <= 0 || H <= 0 || HK <= 0 || D <= 0 || H % HK != 0) return false;
+    if (!rows(q, H) || !rows(k, HK) || !rows(v, HK)) return false;
+    if (!out.is_contiguous() || out.numel() < tokens * H * D || out.scalar_type() != type) return false;
+    if (cache.dim() != 3 || cache.size(0) != 2 || !cache.is_contiguous() || cache.size(2) % (HK * D) != 0)
+      return false;
+    if (fp8 ? cache.element_size() != 1 : cache.scalar_type() != type) return false;
+    const int64_t B = cache.size(2) / (HK * D), x = 16 / cache.element_size();
+    if (B <= 0 || D % x != 0) return false;
+    const int64_t reqs = sl.numel();
+    if (bt.dim() != 2 || bt.size(0) < reqs || !bt.is_contiguous() || bt.scalar_type() != ScalarType::Int ||
+        !sl.is_contiguous() || sl.scalar_type() != ScalarType::Int || slots.dim() != 1 ||
+        !slots.is_contiguous() || slots.numel() < tokens || slots.scalar_type() != ScalarType::Long ||
+        ks.scalar_type() != ScalarType::Float || vs.scalar_type() != ScalarType::Float)
+      return false;
+    if (alibi.has_value() && (alibi->scalar_type() != ScalarType::Float || alibi->numel() != H)) return false;
+    if (max_q == 1) {
+      if (reqs < tokens) return false;
+    } else if (decodes < 0 || decodes > reqs || !qsl.is_contiguous() || qsl.scalar_type() != ScalarType::Int ||
+               qsl.numel() != reqs + 1) {
+      return false;
+    }
+    const auto dev = q.device();
+    for (const at::Tensor* t : {&out, &k, &v, &cache, &bt, &sl, &slots, &qsl, &ks, &vs})
+      if (t->device() != dev) return false;
+
+    char* base = static_cast<char*>(cache.data_ptr());
+    char* vbase = base + cache.stride(0) * cache.element_size();
+    const int in_type = type == ScalarType::BFloat16 ? B200PA_BF16 : B200PA_F16;
+    const int kv_type = kv_code(kv);
+    const at::cuda::OptionalCUDAGuard device_guard(dev);
+    void* stream = at::cuda::getCurrentCUDAStream().stream();
+    if (write) {
+      b200pa_cache_args c;
+      std::memset(&c, 0, sizeof(c));
+      c.in_dtype = in_type;
+      c.kv_dtype = kv_type;
+      c.key = k.data_ptr();
+      c.value = v.data_ptr();
+      c.key_cache = base;
+      c.value_cache = vbase;
+      c.slot_mapping = slots.data_ptr<int64_t>();
+      c.k_scale = ks.data_ptr<float>();
+      c.v_scale = vs.data_ptr<float>();
+      c.key_stride = k.stride(0);
+      c.value_stride = v.stride(0);
+      c.num_tokens = static_cast<int32_t>(tokens);
+      c.num_heads = static_cast<int32_t>(HK);
+      c.head_size = static_cast<int32_t>(D);
+      c.block_size = static_cast<int32_t>(B);
+      c.x = static_cast<int32_t>(x);
+      check_rc(b200pa_reshape_and_cache(&c, stream));
+    }
+    b200pa_attn_args p;
+    std::memset(&p, 0, sizeof(p));
+    p.q_dtype = in_type;
+    p.kv_dtype = kv_type;
+    p.out = out.data_ptr();
+    p.query = q.data_ptr();
+    p.key_cache = base;
+    p.value_cache = vbase;
+    p.block_tables = bt.data_ptr<int>();
+    p.seq_lens = sl.data_ptr<int>();
+    p.alibi_slopes = alibi.has_value() ? alibi->data_ptr<float>() : nullptr;
+    p.k_scale = ks.data_ptr<float>();
+    p.v_scale = vs.data_ptr<float>();
+    p.q_stride = q.stride(0);
+    p.kv_block_stride = HK * D * B;
+    p.kv_head_stride = D * B;
+    p.num_seqs = static_cast<int32_t>(max_q == 1 ? tokens : reqs);
+    p.num_heads = static_cast<int32_t>(H);
+    p.num_kv_heads = static_cast<int32_t>(HK);
+    p.head_size = static_cast<int32_t>(D);
+    p.block_size = static_cast<int32_t>(B);
+    p.max_seq_len = static_cast<int32_t>(max_len);
+    p.max_num_blocks_per_seq = static_cast<int32_t>(bt.size(1));
+    p.scale = static_cast<float>(scale);
+    p.blocksparse_block_size = 64;
+    if (max_q > 1) {
+      const int rc = b200pa_paged_attention_varlen(&p, qsl.data_ptr<int>(), static_cast<int32_t>(tokens),
+                                                   static_cast<int32_t>(decodes), stream);
+      if (rc == B200PA_EUNSUPPORTED) return false;
+      check_rc(rc);
+      return true;
+    }
+    // PagedAttention.forward_decode's rule for v1 / v2; and v1 whenever the partials of v2 fit the
+    // library's own workspace (4 MiB for any stream), which saves the scratch allocations
+    const int64_t parts = (max_len + 511) / 512, rows_n = tokens * H;
+    const bool use_v1 = (max_len <= 8192 && (parts == 1 || rows_n > 512)) ||
+                        rows_n * parts * (8 + 2 * D) <= (int64_t(4) << 20) - 1024;
+    if (use_v1) {
+      check_rc(b200pa_paged_attention_v1(&p, stream));
+      return true;
+    }
+    const int64_t stat = (rows_n * parts * 4 + 255) & ~int64_t(255);
+    const at::Tensor scratch =
+        at::empty({2 * stat + rows_n * parts * D * 2}, q.options().dtype(ScalarType::Byte));
+    char* sp = static_cast<char*>(scratch.data_ptr());
+    p.exp_sums = reinterpret_cast<float*>(sp);
+    p.max_logits = reinterpret_cast<float*>(sp + stat);
+    p.tmp_out = sp + 2 * stat;
+    p.max_num_partitions = static_cast<int32_t>(parts);
+    check_rc(b200pa_paged_attention_v2(&p, stream));
+    return true;
+  });
+}
+
+PyMethodDef kMethods[] = {
+    {"paged_attention_v1", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_v1)), METH_FASTCALL, nullptr},
+    {"paged_attention_v2", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_v2)), METH_FASTCALL, nullptr},
+    {"reshape_and_cache", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_write_x)), METH_FASTCALL,
+     nullptr},
+    {"reshape_and_cache_flash", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_write_flash)),
+     METH_FASTCALL, nullptr},
+    {"attention_step", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_step)), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_C_b200", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+extern "C" __attribute__((visibility("default"))) PyObject* PyInit__C_b200() { return PyModule_Create(&kModule); }
