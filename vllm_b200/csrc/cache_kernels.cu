@@ -383,6 +383,7 @@ reshape_and_cache_kernel(const in_t* __restrict__ key, const in_t* __restrict__ 
                          int block_size, int x, const float* __restrict__ k_scale_ptr,
                          const float* __restrict__ v_scale_ptr) {
   __shared__ TileSlots ts;
+  grid_dependency();
   const int tok0 = blockIdx.x * kTokTile;
   const int ntok = min(kTokTile, num_tokens - tok0);
   load_tile_slots(ts, slot_mapping, tok0, ntok, block_size, int(sizeof(cache_t)));
@@ -541,6 +542,7 @@ reshape_and_cache_flash_kernel(const in_t* __restrict__ key, const in_t* __restr
                                int block_size, int vec_ok, const float* __restrict__ k_scale_ptr,
                                const float* __restrict__ v_scale_ptr) {
   __shared__ TileSlots ts;
+  grid_dependency();
   const int tok0 = blockIdx.x * kTokTile;
   const int ntok = min(kTokTile, num_tokens - tok0);
   load_tile_slots(ts, slot_mapping, tok0, ntok, block_size, int(sizeof(cache_t)));
@@ -726,9 +728,8 @@ static bool launch_staged_as(const b200pa_cache_args& a, cudaStream_t stream, in
       (void)cudaGetLastError();
       return false;
     }
-    kern<<<grid, per_cta * 32, smem, stream>>>(p);
+    e = launch_dependent(kern, dim3(grid), dim3(per_cta * 32), smem, stream, p);
     count_launch();
-    e = cudaGetLastError();
     if (e != cudaSuccess) {
       set_error("KV write kernel launch failed: %s", cudaGetErrorString(e));
       *rc = B200PA_ECUDA;
@@ -780,14 +781,15 @@ static int launch_reshape(const b200pa_cache_args& a, cudaStream_t stream, bool 
                             : launch_staged<in_t, cache_t, KV, false>(a, stream, &rc);
     if (took) return rc;
   }
+  cudaError_t e;
   if (!flash) {
     // small writes (decode steps): split the heads over grid.y so that the write still spreads
     // over the GPU (about two CTAs per SM)
     const int tiles = (a.num_tokens + kTokTile - 1) / kTokTile;
     const int parts = std::max(1, std::min(a.num_heads, (2 * 148 + tiles - 1) / tiles));
     dim3 grid(tiles, parts);
-    reshape_and_cache_kernel<in_t, cache_t, KV><<<grid, 256, 0, stream>>>(
-        static_cast<const in_t*>(a.key), static_cast<const in_t*>(a.value),
+    e = launch_dependent(
+        reshape_and_cache_kernel<in_t, cache_t, KV>, grid, dim3(256), 0, stream, static_cast<const in_t*>(a.key), static_cast<const in_t*>(a.value),
         static_cast<cache_t*>(a.key_cache), static_cast<cache_t*>(a.value_cache), a.slot_mapping,
         a.key_stride, a.value_stride, a.num_tokens, a.num_heads, a.head_size, a.block_size, a.x,
         a.k_scale, a.v_scale);
@@ -801,14 +803,14 @@ static int launch_reshape(const b200pa_cache_args& a, cudaStream_t stream, bool 
         a.block_stride % VEC == 0 && a.page_stride % VEC == 0 && a.head_stride % VEC == 0;
     const int threads = 256;
     dim3 grid((a.num_tokens + kTokTile - 1) / kTokTile);
-    reshape_and_cache_flash_kernel<in_t, cache_t, KV><<<grid, threads, 0, stream>>>(
-        static_cast<const in_t*>(a.key), static_cast<const in_t*>(a.value),
+    e = launch_dependent(
+        reshape_and_cache_flash_kernel<in_t, cache_t, KV>, grid, dim3(threads), 0, stream, static_cast<const in_t*>(a.key), static_cast<const in_t*>(a.value),
         static_cast<cache_t*>(a.key_cache), static_cast<cache_t*>(a.value_cache), a.slot_mapping,
         a.block_stride, a.page_stride, a.head_stride, a.key_stride, a.value_stride, a.num_tokens,
         a.num_heads, a.head_size, a.block_size, vec_ok ? 1 : 0, a.k_scale, a.v_scale);
   }
   count_launch();
-  B200PA_CHECK_CUDA(cudaGetLastError());
+  B200PA_CHECK_CUDA(e);
   return B200PA_OK;
 }
 

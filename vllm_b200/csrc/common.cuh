@@ -43,7 +43,35 @@ inline int dtype_size(int dt) { return dt == B200PA_F32 ? 4 : 2; }
 // text) if the address cannot be resolved.  Defined in capi.cu.
 int* device_status_ptr();
 
+// Launches a kernel that may start while the kernel in front of it in the stream is still running
+// (programmatic dependent launch).  Such a kernel calls grid_dependency() before its first access to
+// global memory: up to there only its own set-up overlaps.  What it saves is the launch latency
+// between two kernels of a stream, which small launches are mostly made of.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                    cudaStream_t stream, Args... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+
 // ---------------------------------------------------------------- device side
+// Waits until everything in front of this grid in the stream is complete and visible, then lets
+// the next grid be launched.  Every thread of every block calls it, before any global access, so
+// that a finished grid implies that all before it have finished.
+__device__ __forceinline__ void grid_dependency() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __device__ __forceinline__ float to_f32(float v) { return v; }
 __device__ __forceinline__ float to_f32(__half v) { return __half2float(v); }
 __device__ __forceinline__ float to_f32(__nv_bfloat16 v) { return __bfloat162float(v); }

@@ -45,8 +45,7 @@ cudaError_t decode_launch(const DecodeParams& p, int grid, int threads, size_t s
     }
     if (dev >= 0 && dev < 64) done[dev] = true;
   }
-  kern<<<grid, threads, smem, stream>>>(p);
-  return cudaGetLastError();
+  return launch_dependent(kern, dim3(grid), dim3(threads), smem, stream, p);
 }
 
 template <typename QT, int KV, int D, int GP>

@@ -568,6 +568,7 @@ __global__ void __launch_bounds__(MAXW * 32, 1) pa_decode_kernel(const DecodePar
   __shared__ int4 s_iter[MAXW];  // per warp: units left, block offset, sequence, head
   __shared__ int4 s_todo[MAXW][2];  // per warp: merges owed (sequence, head item, pieces, piece | level)
   __shared__ int s_ntodo[MAXW];
+  grid_dependency();
   const bool flat = p.use_table != 0;
   const int hsubs = p.num_kv_heads * p.head_groups;
   if (flat) {

@@ -122,6 +122,7 @@ __global__ void __launch_bounds__(kStagedMaxWarps * 32, 1) kv_write_staged_kerne
     fence_barrier_init();
   }
   __syncwarp();
+  grid_dependency();
 
   const char* key_b = static_cast<const char*>(p.key);
   const char* val_b = static_cast<const char*>(p.value);

@@ -30,8 +30,7 @@ cudaError_t prefill_launch(const PrefillParams& p, int grid, cudaStream_t stream
     }
     if (dev >= 0 && dev < 64) done[dev] = true;
   }
-  kern<<<grid, kPrefillThreads, smem, stream>>>(p);
-  return cudaGetLastError();
+  return launch_dependent(kern, dim3(grid), dim3(kPrefillThreads), smem, stream, p);
 }
 
 template <typename QT, int D>

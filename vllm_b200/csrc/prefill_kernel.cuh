@@ -164,6 +164,8 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
     fence_proxy_async();
   }
 
+  grid_dependency();
+
   // ---- plan.  T tokens fill a row tile; a request has ceil(q_len / (NQ T)) row-tile groups per kv
   // head, and each of them npieces pieces.
   const int G = p.group, HK = p.num_kv_heads, S = p.num_reqs, B = p.block_size;
