@@ -13,6 +13,7 @@
 #include <mutex>
 
 #include "decode_inst.cuh"
+#include "direct_inst.cuh"
 #include "launch_state.cuh"
 
 namespace b200pa {
@@ -241,6 +242,8 @@ struct Tuning {
   int min_tokens = 0;    // B200PA_TUNE_MIN_TOKENS: smallest range, in tokens (multiple of 32)
   int warps = 0;         // B200PA_TUNE_WARPS: warps per CTA
   int stages = 0;        // B200PA_TUNE_STAGES: ring slots per warp
+  int direct = 0;        // B200PA_TUNE_DIRECT: 1 always the direct kernel where it is built, 2 never
+  int cluster = 0;       // B200PA_TUNE_CLUSTER: its CTAs per cluster
   int reload = 0;
 };
 
@@ -258,6 +261,8 @@ static Tuning read_tuning() {
   t.min_tokens = env_int("B200PA_TUNE_MIN_TOKENS", 32, 1 << 20) & ~31;
   t.warps = env_int("B200PA_TUNE_WARPS", 1, 16);
   t.stages = env_int("B200PA_TUNE_STAGES", 1, 8);
+  t.direct = env_int("B200PA_TUNE_DIRECT", 0, 2);
+  t.cluster = env_int("B200PA_TUNE_CLUSTER", 1, 16);
   t.reload = env_int("B200PA_TUNE_RELOAD", 0, 1);
   return t;
 }
@@ -370,6 +375,35 @@ static DecodeKernelInfo find_decode(int d, int qdt, int kv, int gp, int nt) {
     case 256: return find_decode_d256(qdt, kv, gp, nt);
   }
   return {nullptr, 0, 1};
+}
+
+static DirectKernelInfo find_direct(int d, int qdt, int kv, int gp) {
+  return d <= 96 ? find_direct_small(d, qdt, kv, gp)
+                 : d <= 128 ? find_direct_mid(d, qdt, kv, gp) : find_direct_large(d, qdt, kv, gp);
+}
+
+// CTAs per cluster for the direct kernel, or 0 when the persistent kernel is the better one.  Only
+// the bound on the lengths is known here.  Measured on B200, persistent / direct, us: 1 sequence of
+// 1500 (32 / 8 heads of 128, bf16) 21.2 / 7.4, of 8000 23.8 / 15.4, of 32000 37.8 / 44.8; 8 sequences
+// up to 1024 (32 heads) 22.7 / 20.5; 16 up to 4096 37.2 / 34.0; 16 up to 2000 with 16 heads on one kv
+// head 41.7 / 9.8; 256 up to 800 76.9 / 73.3; 600 up to 80 (40 heads) 117.7 / 206.
+static int direct_plan(const DirectKernelInfo& ki, int64_t items, int max_seq_len, const Tuning& tune) {
+  const int64_t slots = int64_t(sm_count()) * ki.ctas_per_sm;
+  const int64_t tiles = (int64_t(std::max(max_seq_len, 1)) + 15) / 16;
+  // as many CTAs as the GPU takes at once (a fifth more: short sequences make room early), but no
+  // more warps than the longest sequence can have tiles.  Clusters of 16 are placed one to a GPC:
+  // worth it for eight items at most, when it takes tiles off the warps.
+  int cluster = 1;
+  while (cluster < 8 && items * cluster * 10 <= slots * 6 && cluster * kDirectWarps < tiles) cluster *= 2;
+  if (cluster == 8 && items <= 8 && tiles >= 128) cluster = 16;
+  if (tune.cluster) cluster = tune.cluster;
+  if (tune.direct == 1) return cluster;
+  // A tile costs a warp about 1 us whatever else runs, a CTA 4 us besides; the persistent kernel
+  // pays about 15 us once.
+  const int64_t per_warp = (tiles + cluster * kDirectWarps - 1) / (cluster * kDirectWarps);
+  const int64_t ctas = items * cluster;
+  if (ctas * 10 <= slots * 12) return per_warp <= 20 ? cluster : 0;
+  return ctas <= 5 * slots && per_warp >= 3 && per_warp <= 16 ? cluster : 0;
 }
 
 template <typename QT>
@@ -541,7 +575,7 @@ static int attention_entry(const b200pa_attn_args* a, void* stream, Scratch mode
   // block-sparse attention (unused by any in-tree caller of the reference) runs on the
   // generic kernel only
   bool fast = !force_generic() && !sparse && a->q_dtype != B200PA_F32 &&
-              (a->block_size == 16 || a->block_size == 32) && a->head_size % 16 == 0 &&
+              (a->block_size == 16 || a->block_size == 32) &&
               aligned(a->key_cache, 16) && aligned(a->value_cache, 16) && aligned(a->query, 16) &&
               aligned(a->out, 16) && (!split || aligned(a->tmp_out, 16)) &&
               (a->kv_block_stride * es) % 16 == 0 && (a->kv_head_stride * es) % 16 == 0 &&
@@ -550,6 +584,27 @@ static int attention_entry(const b200pa_attn_args* a, void* stream, Scratch mode
   DecodeLaunchFn fn = ki.fn;
   int rc;
   bool fused = false;
+  if (fast && tune.direct != 2) {
+    // small batches: the latency-bound form (and head size 120, which only it is built for)
+    const DirectKernelInfo di = find_direct(a->head_size, a->q_dtype, a->kv_dtype, gp);
+    const int head_groups = (p.group + 8 * gp - 1) / (8 * gp);
+    const int64_t items = int64_t(p.num_seqs) * p.num_kv_heads * head_groups;
+    int cluster = di.fn == nullptr ? 0 : direct_plan(di, items, a->max_seq_len, tune);
+    if (di.fn != nullptr && fn == nullptr) cluster = std::max(cluster, 1);
+    if (cluster > 0 && items * cluster < INT32_MAX) {
+      p.head_groups = head_groups;
+      // (lengths beyond what the caller's scratch was sized for are ignored, see below)
+      if (split && mode == Scratch::kCaller)
+        p.len_cap = int(std::min<int64_t>(int64_t(a->max_num_partitions) * kPartitionTokens, INT32_MAX));
+      const cudaError_t e = di.fn(p, int(items), cluster, s);
+      count_launch();
+      if (e != cudaSuccess) {
+        set_error("direct decode kernel launch failed: %s", cudaGetErrorString(e));
+        return B200PA_ECUDA;
+      }
+      return B200PA_OK;
+    }
+  }
   if (fn != nullptr) {
     p.head_groups = (p.group + 8 * gp - 1) / (8 * gp);
     const size_t page_bytes = size_t(a->head_size) * a->block_size * es;
