@@ -202,7 +202,7 @@ int b200pa_paged_attention_v2_noalloc(const b200pa_attn_args* args, void* stream
  *   num_tokens: query rows of the step
  *   num_decodes: the first `num_decodes` requests bring exactly one row each (decode kernel)
  * Returns B200PA_EUNSUPPORTED, with nothing launched, for shapes that it has no kernel for (fp32
- * queries, block size 8, unaligned tensors, more than 2048 requests with several rows).
+ * queries, block size 8, unaligned tensors).
  */
 int b200pa_paged_attention_varlen(const b200pa_attn_args* args, const int32_t* query_start_loc,
                                   int32_t num_tokens, int32_t num_decodes, void* stream);

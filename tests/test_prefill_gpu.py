@@ -113,10 +113,10 @@ def test_few_rows_behind_long_contexts_are_split(kv):
 
 def test_many_requests_and_single_rows_among_them():
     rng = np.random.default_rng(3)
-    q = rng.integers(1, 40, size=300)
+    q = rng.integers(1, 40, size=600)  # (512 requests to a launch)
     q[:20] = 1
     q[100] = 1
-    _case(q, rng.integers(0, 400, size=300), 8, 2, 64, 16, torch.bfloat16, "auto")
+    _case(q, rng.integers(0, 400, size=600), 8, 2, 64, 16, torch.bfloat16, "auto")
 
 
 @pytest.mark.parametrize("kv", ["auto", "fp8"])

@@ -8,7 +8,7 @@
 // The decode kernel reads the whole context once per query TOKEN; here a K/V tile is read once per
 // 256 query rows.
 //
-//   * One persistent CTA per SM, 13 warps: two softmax warpgroups (one thread per query row), one
+//   * One persistent CTA per SM: two softmax warpgroups (one thread per query row), one
 //     producer warpgroup, one warp that issues the MMAs.
 //   * A work item is (request, 2 x 128 query rows, kv head).  A row is one (token, query head of the
 //     group): the heads that share a kv head are packed into the rows of a tile, so K/V are fetched
@@ -66,8 +66,15 @@ struct PrefillParams {
   float scale;
 };
 
-constexpr int kPrefillThreads = 13 * 32;
-constexpr int kPrefillMaxReqs = 2048;   // prefix table in shared memory
+constexpr int kPrefillThreads = 16 * 32;  // (three warps beside the MMA warp only complete its warpgroup)
+// Registers per thread: 512 threads start with 128 each; the softmax warpgroups take over what the
+// others give back.  (The producers of an fp8 cache hold a K and a V tile in registers.)
+template <bool kFp8>
+struct PrefillRegs {
+  static constexpr int kSoftmax = kFp8 ? 168 : 184, kProducer = kFp8 ? 120 : 88, kMma = 56;
+  static_assert(2 * kSoftmax + kProducer + kMma == 4 * 128, "register split");
+};
+constexpr int kPrefillMaxReqs = 512;    // requests per launch: prefix table in shared memory
 
 template <int D>
 struct PrefillShape {
@@ -76,8 +83,12 @@ struct PrefillShape {
   static constexpr int KT = D > 128 ? 64 : 128;     // keys per tile
   static constexpr int kQBytes = 128 * DP * 2;
   static constexpr int kTileBytes = KT * DP * 2;
-  static constexpr int kStages = 2;
-  static constexpr int kSmem = NQ * kQBytes + 2 * kStages * kTileBytes;
+  // ring of K and V tiles in turns (K0, V0, K1, V1, ...): what shared memory holds besides Q.  Five
+  // instead of four at head size 128: ~10 % (the loads of a tile take about as long as its products)
+  static constexpr int kRoom = 223 * 1024 - NQ * kQBytes;
+  static constexpr int kSlots = kRoom / kTileBytes < 8 ? kRoom / kTileBytes : 8;
+  static constexpr int kSmem = NQ * kQBytes + kSlots * kTileBytes;
+  static_assert(kSlots >= 4, "a K and a V tile in use, another of each on its way");
   static_assert(NQ * (KT + DP) <= 512, "TMEM columns");
 };
 
@@ -97,49 +108,45 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
   constexpr bool kE5 = KV == kCacheE5M2;
   constexpr bool kBf = !kFp8 && std::is_same_v<QT, __nv_bfloat16>;  // operand type: bf16, else f16
   constexpr bool kOutBf = std::is_same_v<QT, __nv_bfloat16>;
-  constexpr int DP = SH::DP, NQ = SH::NQ, KT = SH::KT, NST = SH::kStages;
+  constexpr int DP = SH::DP, NQ = SH::NQ, KT = SH::KT, NS = SH::kSlots;
   constexpr int kWs = 128 * (D * 2 + 8);  // workspace of one row tile's partial: O, then (m, l)
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ int cum[kPrefillMaxReqs + 1];  // items before request r
-  __shared__ uint64_t s_bar[4 * NST + 3 * 2 + 2 + 4];
+  __shared__ uint64_t s_bar[2 * NS + 12];
   __shared__ int s_item[2];
   __shared__ uint32_t s_tmem;
-  __shared__ int s_red[3][13];
+  __shared__ int s_red[3][16];
 
   const int tid = threadIdx.x, lane = tid & 31;
   // (through a shuffle, so that the compiler knows it is uniform in the warp)
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const uint32_t bar0 = smem_u32(s_bar);
-  auto k_full = [&](int s) { return bar0 + 8u * s; };
-  auto k_empty = [&](int s) { return bar0 + 8u * (NST + s); };
-  auto v_full = [&](int s) { return bar0 + 8u * (2 * NST + s); };
-  auto v_empty = [&](int s) { return bar0 + 8u * (3 * NST + s); };
-  auto s_full = [&](int i) { return bar0 + 8u * (4 * NST + i); };
-  auto p_full = [&](int i) { return bar0 + 8u * (4 * NST + 2 + i); };
-  auto pv_done = [&](int i) { return bar0 + 8u * (4 * NST + 4 + i); };
-  auto q_full = [&](int i) { return bar0 + 8u * (4 * NST + 6 + i); };
-  auto item_full = [&](int i) { return bar0 + 8u * (4 * NST + 8 + i); };
-  auto item_empty = [&](int i) { return bar0 + 8u * (4 * NST + 10 + i); };
+  auto kv_full = [&](uint32_t s) { return bar0 + 8u * s; };
+  auto kv_empty = [&](uint32_t s) { return bar0 + 8u * (NS + s); };
+  auto s_full = [&](int i) { return bar0 + 8u * (2 * NS + i); };
+  auto p_full = [&](int i) { return bar0 + 8u * (2 * NS + 2 + i); };
+  auto pv_done = [&](int i) { return bar0 + 8u * (2 * NS + 4 + i); };
+  auto q_full = [&](int i) { return bar0 + 8u * (2 * NS + 6 + i); };
+  auto item_full = [&](int i) { return bar0 + 8u * (2 * NS + 8 + i); };
+  auto item_empty = [&](int i) { return bar0 + 8u * (2 * NS + 10 + i); };
 
   const uint32_t sq = smem_u32(smem_raw);
-  const uint32_t sk = sq + NQ * SH::kQBytes;
-  const uint32_t sv = sk + NST * SH::kTileBytes;
+  const uint32_t skv = sq + NQ * SH::kQBytes;
 
   if (warp == 12) {
     if (lane == 0) {
-      for (int s = 0; s < NST; ++s) {
-        mbar_init(k_full(s), 128);
-        mbar_init(k_empty(s), 1);
-        mbar_init(v_full(s), 128);
-        mbar_init(v_empty(s), 1);
+      // (a warp arrives once, by its first lane: 128 arrivals on one barrier take a while)
+      for (int s = 0; s < NS; ++s) {
+        mbar_init(kv_full(s), 4);
+        mbar_init(kv_empty(s), 1);
       }
       for (int i = 0; i < 2; ++i) {
         mbar_init(s_full(i), 1);
-        mbar_init(p_full(i), 128);
+        mbar_init(p_full(i), 4);
         mbar_init(pv_done(i), 1);
-        mbar_init(q_full(i), 128);
+        mbar_init(q_full(i), 4);
         mbar_init(item_full(i), 1);
-        mbar_init(item_empty(i), 384);
+        mbar_init(item_empty(i), 12);
       }
       fence_barrier_init();
     }
@@ -147,23 +154,13 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
     tmem_alloc(smem_u32(&s_tmem), 512);
   }
   if constexpr (DP != D) {
-    // the padding granules of Q and K take part in the product: zero, once (nobody writes them)
-    for (int i = tid; i < NQ * 128 + NST * KT; i += kPrefillThreads) {
-      unsigned char* at = i < NQ * 128
-          ? smem_raw + (i / 128) * SH::kQBytes + (D / 8) * 128 * 16 + (i % 128) * 16
-          : smem_raw + NQ * SH::kQBytes + ((i - NQ * 128) / KT) * SH::kTileBytes + (D / 8) * KT * 16 +
-                ((i - NQ * 128) % KT) * 16;
-      *reinterpret_cast<uint4*>(at) = make_uint4(0, 0, 0, 0);
-    }
-    // ... and V's padding columns (their results are dropped, but the operand has to be defined)
-    for (int i = tid; i < NST * (KT / 8) * (DP - D); i += kPrefillThreads) {
-      const int st = i / ((KT / 8) * (DP - D)), r = i % ((KT / 8) * (DP - D));
-      *reinterpret_cast<uint4*>(smem_raw + NQ * SH::kQBytes + (NST + st) * SH::kTileBytes +
-                                ((r / (DP - D)) * DP + D + r % (DP - D)) * 16) = make_uint4(0, 0, 0, 0);
-    }
+    // Q's padding granules take part in the product: zero, once (nobody writes them; K's are zeroed
+    // with every tile, V's padding only gives columns that are dropped)
+    for (int i = tid; i < NQ * 128; i += kPrefillThreads)
+      *reinterpret_cast<uint4*>(smem_raw + (i / 128) * SH::kQBytes + (D / 8) * 128 * 16 + (i % 128) * 16) =
+          make_uint4(0, 0, 0, 0);
     fence_proxy_async();
   }
-
   grid_dependency();
 
   // ---- plan.  T tokens fill a row tile; a request has ceil(q_len / (NQ T)) row-tile groups per kv
@@ -200,7 +197,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
     }
     __syncthreads();
     groups = work = most = 0;
-    for (int w = 0; w < 13; ++w) {
+    for (int w = 0; w < 16; ++w) {
       groups += s_red[0][w];
       work += s_red[1][w];
       most += s_red[2][w];
@@ -279,28 +276,33 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
     return it;
   };
   bool ok = true;
-  auto wait = [&](uint32_t bar, uint32_t parity) {
-    if (ok && !mbar_wait(bar, parity)) {
+  // All roles wait as whole warps and leave as whole warps (TMEM accesses are warp-collective).
+  auto wait = [&](uint32_t bar, uint32_t parity) -> bool {
+    const bool got = __all_sync(0xffffffffu, mbar_spin(bar, parity));
+    if (!got) {
       ok = false;
-      atomicExch(p.status, kStatusMbarTimeout);
+      if (lane == 0) atomicExch(p.status, kStatusMbarTimeout);
     }
-    return ok;
+    return got;
   };
-  // the same for a whole warp: TMEM accesses are warp-collective, so its threads leave together
-  auto wait_warp = [&](uint32_t bar, uint32_t parity) { return ok = __all_sync(0xffffffffu, wait(bar, parity)); };
+  auto arrive = [&](uint32_t bar) {  // once per warp, for everything its lanes have done
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
+  };
   // next item of this CTA, for the roles that do not draw it themselves
   int n_item = 0;  // items received so far
   auto next_item = [&]() -> int {
     const int slot = n_item & 1;
     if (!wait(item_full(slot), (n_item >> 1) & 1)) return INT32_MAX;
     const int v = *reinterpret_cast<volatile int*>(&s_item[slot]);
-    mbar_arrive(item_empty(slot));
+    arrive(item_empty(slot));
     ++n_item;
     return v;
   };
 
   if (warp < 8) {
     // ================================================= softmax: one thread per row of tile wg
+    reg_inc<PrefillRegs<kFp8>::kSoftmax>();
     const int wg = warp >> 2;
     const int row = tid & 127;
     const uint32_t lane_off = uint32_t((warp & 3) * 32) << 16;
@@ -337,7 +339,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
         }
       }
       fence_proxy_async();
-      mbar_arrive(q_full(wg));
+      arrive(q_full(wg));
     };
 
     int item = blockIdx.x < unsigned(total) ? int(blockIdx.x) : INT32_MAX;
@@ -356,34 +358,52 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
       const float slope = (p.alibi != nullptr && valid) ? p.alibi[head] * kLog2e : 0.f;
       float m = -INFINITY, l = 0.f;
       for (int j = b; j < e; ++j) {
-        if (!wait_warp(s_full(wg), n_s & 1)) break;
+        if (!wait(s_full(wg), n_s & 1)) break;
         ++n_s;
         tc_fence_after();
         const int key0 = j * KT;
-        // full tiles without a bias need no per-element work besides the scale
-        const bool plain = key0 + KT - 1 <= pos_first && p.alibi == nullptr && c > 0.f;
+        // No bias: only the tiles at the causal edge of a row tile need a mask.
+        const bool plain = p.alibi == nullptr && c > 0.f;
+        const bool edge = key0 + KT - 1 > pos_first;
+        auto mask = [&](float (&x)[32], int ch) {
+          if (edge) {
+            const int last = pos - key0 - ch * 32;  // last column of the chunk that counts
+#pragma unroll
+            for (int k = 0; k < 32; ++k) x[k] = k <= last ? x[k] : -INFINITY;
+          }
+        };
+        // with a bias: t = x c + slope (key - pos), and the mask
+        auto biased = [&](float x, int ch, int k) {
+          const int first = key0 + ch * 32 - pos;  // (of this row: key - pos of column 0)
+          return first + k <= 0 ? fmaf(slope, float(k), fmaf(x, c, slope * float(first))) : -INFINITY;
+        };
         float mx = -INFINITY;
-        float v[32];
+        // 32-column chunks: one is on its way while another is worked on.  (Registers that a load is
+        // on its way to are not to be moved: the loads span straight-line code only.)
+        constexpr int NC = KT / 32;
+        float v[2][32];
+        tmem_ld32(t_s, v[0]);
         if (plain) {
 #pragma unroll
-          for (int ch = 0; ch < KT / 32; ++ch) {
-            tmem_ld32(t_s + ch * 32, v);
-            tmem_landed(v);
-            float m4[4] = {v[0], v[1], v[2], v[3]};
+          for (int ch = 0; ch < NC; ++ch) {
+            float (&x)[32] = v[ch & 1];
+            tmem_landed(x);
+            if (ch + 1 < NC) tmem_ld32(t_s + (ch + 1) * 32, v[(ch + 1) & 1]);
+            mask(x, ch);
+            float m4[4] = {x[0], x[1], x[2], x[3]};
 #pragma unroll
-            for (int k = 4; k < 32; ++k) m4[k & 3] = fmaxf(m4[k & 3], v[k]);
+            for (int k = 4; k < 32; ++k) m4[k & 3] = fmaxf(m4[k & 3], x[k]);
             mx = fmaxf(mx, fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])));
           }
           mx *= c;
         } else {
 #pragma unroll 1
-          for (int ch = 0; ch < KT / 32; ++ch) {
-            tmem_ld32(t_s + ch * 32, v);
-            tmem_landed(v);
-            const int k0 = key0 + ch * 32;
+          for (int ch = 0; ch < NC; ++ch) {
+            float (&x)[32] = v[0];
+            tmem_landed(x);
 #pragma unroll
-            for (int k = 0; k < 32; ++k)
-              if (k0 + k <= pos) mx = fmaxf(mx, v[k] * c + slope * float(k0 + k - pos));
+            for (int k = 0; k < 32; ++k) mx = fmaxf(mx, biased(x[k], ch, k));
+            if (ch + 1 < NC) tmem_ld32(t_s + (ch + 1) * 32, x);
           }
         }
         // raise the maximum (and rescale what has been summed) only when it grew by more than 8
@@ -394,7 +414,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
           m = m_new;
           l *= alpha;
           if (j > b) {
-            if (!wait_warp(pv_done(wg), (n_pv - 1) & 1)) break;
+            if (!wait(pv_done(wg), (n_pv - 1) & 1)) break;
             tc_fence_after();
 #pragma unroll 1
             for (int ch = 0; ch < DP / 16; ++ch) {
@@ -409,16 +429,19 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
         }
         const float mm = m == -INFINITY ? 0.f : m;
         float sum = 0.f;
+        tmem_ld32(t_s, v[0]);
         if (plain) {
 #pragma unroll
-          for (int ch = 0; ch < KT / 32; ++ch) {
-            tmem_ld32(t_s + ch * 32, v);
-            tmem_landed(v);
+          for (int ch = 0; ch < NC; ++ch) {
+            float (&x)[32] = v[ch & 1];
+            tmem_landed(x);
+            if (ch + 1 < NC) tmem_ld32(t_s + (ch + 1) * 32, v[(ch + 1) & 1]);
+            mask(x, ch);
             float s4[4] = {0.f, 0.f, 0.f, 0.f};
             uint32_t w[16];
 #pragma unroll
             for (int k = 0; k < 32; k += 2) {
-              const float p0 = fast_exp2(fmaf(v[k], c, -mm)), p1 = fast_exp2(fmaf(v[k + 1], c, -mm));
+              const float p0 = fast_exp2(fmaf(x[k], c, -mm)), p1 = fast_exp2(fmaf(x[k + 1], c, -mm));
               s4[k & 2] += p0;
               s4[(k & 2) + 1] += p1;
               w[k / 2] = pack2<kBf>(p0, p1);
@@ -428,25 +451,26 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
           }
         } else {
 #pragma unroll 1
-          for (int ch = 0; ch < KT / 32; ++ch) {
-            tmem_ld32(t_s + ch * 32, v);
-            tmem_landed(v);
-            const int k0 = key0 + ch * 32;
+          for (int ch = 0; ch < NC; ++ch) {
+            float (&x)[32] = v[0];
+            tmem_landed(x);
             uint32_t w[16];
 #pragma unroll
             for (int k = 0; k < 32; k += 2) {
-              const float p0 = k0 + k <= pos ? fast_exp2(v[k] * c + slope * float(k0 + k - pos) - mm) : 0.f;
-              const float p1 = k0 + k + 1 <= pos ? fast_exp2(v[k + 1] * c + slope * float(k0 + k + 1 - pos) - mm) : 0.f;
+              const float p0 = fast_exp2(biased(x[k], ch, k) - mm);
+              const float p1 = fast_exp2(biased(x[k + 1], ch, k + 1) - mm);
               sum += p0 + p1;
               w[k / 2] = pack2<kBf>(p0, p1);
             }
+            // (P's columns lie over S columns that have been read: 16 a chunk over 32)
+            if (ch + 1 < NC) tmem_ld32(t_s + (ch + 1) * 32, x);
             tmem_st16(t_s + ch * 16, w);
           }
         }
         l += sum;
         tmem_wait_st();
         tc_fence_before();
-        mbar_arrive(p_full(wg));
+        arrive(p_full(wg));
         ++n_pv;
       }
       if (!ok) break;
@@ -454,7 +478,6 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
       // been received, so nothing reads this tile's Q any more)
       const PrefillItem cur = it;
       item = next_item();
-      ok = __all_sync(0xffffffffu, ok);
       if (item < total) {
         it = decode(item);
         load_q(it);
@@ -464,7 +487,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
       // ---- results
       const bool any = e > b;
       if (any) {
-        if (!wait_warp(pv_done(wg), (n_pv - 1) & 1)) break;
+        if (!wait(pv_done(wg), (n_pv - 1) & 1)) break;
         tc_fence_after();
       }
       const bool whole = cur.npieces == 1;
@@ -558,50 +581,71 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
     }
   } else if (warp < 12) {
     // ================================================= producers: K and V tiles into shared memory
+    reg_dec<PrefillRegs<kFp8>::kProducer>();
     const int pt = tid - 256;  // 0 .. 127
     uint32_t n_half = 0;       // halves (K or V tiles) put on their way
-    uint32_t n_done = 0;       // ... and announced
+    uint32_t n_done = 0;       // ... and announced (16-bit caches)
     const char* kb = static_cast<const char*>(p.kc);
     const char* vb = static_cast<const char*>(p.vc);
     constexpr int ES = kFp8 ? 1 : 2;
-    auto full_of = [&](uint32_t h) { return (h & 1) ? v_full((h >> 1) % NST) : k_full((h >> 1) % NST); };
-    auto empty_of = [&](uint32_t h) { return (h & 1) ? v_empty((h >> 1) % NST) : k_empty((h >> 1) % NST); };
-    auto wait_slot = [&](uint32_t h) {
-      const uint32_t use = (h >> 1) / NST;  // times the slot has been filled before
-      return use == 0 || wait(empty_of(h), (use - 1) & 1);
-    };
+    // 16-bit caches: halves are announced in order, when their copies have landed.  Up to two stay on
+    // their way while there is something else to issue; before the warp waits for anything, all of
+    // them are announced (the MMAs may be waiting for just those).
     auto announce = [&]() {
       fence_proxy_async();
-      mbar_arrive(full_of(n_done));
+      arrive(kv_full(n_done % NS));
       ++n_done;
     };
+    auto announce_all = [&]() {
+      if (n_half - n_done >= 2) {
+        cp_async_wait<1>();
+        while (n_half - n_done > 1) announce();
+      }
+      if (n_half != n_done) {
+        cp_async_wait<0>();
+        announce();
+      }
+    };
+    auto wait_slot = [&](uint32_t h) -> bool {
+      const uint32_t use = h / NS;  // times the slot has been filled before
+      if (use == 0) return true;
+      if constexpr (!kFp8) {
+        if (!__all_sync(0xffffffffu, mbar_test(kv_empty(h % NS), (use - 1) & 1))) announce_all();
+      }
+      return wait(kv_empty(h % NS), (use - 1) & 1);
+    };
+    auto slot_of = [&](uint32_t h) { return skv + (h % NS) * SH::kTileBytes; };
     int item = blockIdx.x < unsigned(total) ? int(blockIdx.x) : INT32_MAX;
     while (item < total && ok) {
       const PrefillItem it = decode(item);
       const int* bt = p.block_tables + int64_t(it.req) * p.max_blocks_per_seq;
       const int64_t head_off = int64_t(it.kvh) * p.kv_head_stride * ES;
       const int e = max(it.e0, it.e1);
-      // the page byte address of key `key` (its block's start), or of block 0 past the end
-      auto page = [&](const char* base, int key) -> const char* {
-        const int blk = key < it.seq_len ? __ldg(bt + (key >> b_shift)) : 0;
+      auto block_of = [&](int key) { return key < it.seq_len ? __ldg(bt + (key >> b_shift)) : 0; };
+      auto page = [&](const char* base, int blk) {
         return base + int64_t(blk) * p.kv_block_stride * ES + head_off;
       };
       if constexpr (!kFp8) {
         // K: a thread owns one key and walks along its 16-byte granules; V: a thread owns 8 keys
-        // and every 8th head dimension (128 bytes of shared memory per 8 threads in both cases)
+        // and every 8th head dimension (128 bytes of shared memory per 8 threads in both cases).
         const int kt = pt % KT, kg = pt / KT;
         constexpr int VJ = KT / 8;              // 8-key groups per tile
         const int vj = pt / 8 % VJ, vd = pt % 8 + 8 * (pt / 8 / VJ);
-        for (int j = it.b; j < e && ok; ++j) {
+        int k_blk = block_of(it.b * KT + kt), v_blk = block_of(it.b * KT + vj * 8);
+        for (int j = it.b; j < e; ++j) {
           {
             const int key = j * KT + kt;
-            const char* src = page(kb, key) + (key & (B - 1)) * 16;
+            const char* src = page(kb, k_blk) + (kg * B + (key & (B - 1))) * 16;
             const int bytes = key < it.seq_len ? 16 : 0;
+            if (j + 1 < e) k_blk = block_of(key + KT);
             if (!wait_slot(n_half)) break;
-            const uint32_t dst = sk + ((n_half >> 1) % NST) * SH::kTileBytes + kt * 16;
-#pragma unroll
-            for (int g = kg; g < D / 8; g += 128 / KT)
-              cp_async16(dst + g * KT * 16, src + int64_t(g) * B * 16, bytes);
+            uint32_t dst = slot_of(n_half) + (kg * KT + kt) * 16;
+#pragma unroll 4
+            for (int g = kg; g < DP / 8; g += 128 / KT) {
+              cp_async16(dst, src, DP == D || g < D / 8 ? bytes : 0);
+              dst += 128 * 16;
+              src += (128 / KT) * B * 16;
+            }
             cp_async_commit();
             ++n_half;
             if (n_half - n_done > 2) {
@@ -611,14 +655,18 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
           }
           {
             const int key = j * KT + vj * 8;
-            const char* src = page(vb, key) + (key & (B - 1)) * 2;
+            const char* src = page(vb, v_blk) + (vd * B + (key & (B - 1))) * 2;
             const int bytes = max(0, min(16, (it.seq_len - key) * 2));  // keys past the end: zeros
+            if (j + 1 < e) v_blk = block_of(key + KT);
             if (!wait_slot(n_half)) break;
-            const uint32_t dst = sv + ((n_half >> 1) % NST) * SH::kTileBytes + vj * DP * 16;
-#pragma unroll
-            for (int d = 0; d < D; d += 8 * (16 / VJ))
-              if (D % (8 * (16 / VJ)) == 0 || d + vd < D)
-                cp_async16(dst + (d + vd) * 16, src + int64_t(d + vd) * B * 2, bytes);
+            uint32_t dst = slot_of(n_half) + (vj * DP + vd) * 16;
+            constexpr int VS = 8 * (16 / VJ);
+#pragma unroll 4
+            for (int d = 0; d < D; d += VS) {
+              if (D % VS == 0 || d + vd < D) cp_async16(dst, src, bytes);
+              dst += VS * 16;
+              src += VS * B * 2;
+            }
             cp_async_commit();
             ++n_half;
             if (n_half - n_done > 2) {
@@ -639,7 +687,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
         uint4 kr[KN], vr[VN];
         auto get_k = [&](int j) {
           const int key = j * KT + kt;
-          const char* src = page(kb, key) + (key & (B - 1)) * 16;
+          const char* src = page(kb, block_of(key)) + (key & (B - 1)) * 16;
 #pragma unroll
           for (int i = 0; i < KN; ++i) {
             const int g = kg + i * (128 / KT);
@@ -649,7 +697,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
         };
         auto get_v = [&](int j) {
           const int key = j * KT + vj * 16;
-          const char* src = page(vb, key) + (key & (B - 1));
+          const char* src = page(vb, block_of(key)) + (key & (B - 1));
 #pragma unroll
           for (int i = 0; i < VN; ++i) {
             const int d = vd + i * VDS;
@@ -670,7 +718,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
         for (int j = it.b; j < e && ok; ++j) {
           if (!wait_slot(n_half)) break;
           {
-            const uint32_t dst = sk + ((n_half >> 1) % NST) * SH::kTileBytes + kt * 16;
+            const uint32_t dst = slot_of(n_half) + kt * 16;
 #pragma unroll
             for (int i = 0; i < KN; ++i) {
               const int g = kg + i * (128 / KT);
@@ -681,13 +729,14 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
                 st_shared16(dst + (2 * g + 1) * KT * 16, hi);
               }
             }
+            fence_proxy_async();
+            arrive(kv_full(n_half % NS));
             ++n_half;
-            announce();
             if (j + 1 < e) get_k(j + 1);
           }
           if (!wait_slot(n_half)) break;
           {
-            const uint32_t dst = sv + ((n_half >> 1) % NST) * SH::kTileBytes + 2 * vj * DP * 16;
+            const uint32_t dst = slot_of(n_half) + 2 * vj * DP * 16;
             const int left = it.seq_len - (j * KT + vj * 16);  // keys of the group that exist
 #pragma unroll
             for (int i = 0; i < VN; ++i) {
@@ -707,100 +756,113 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
                 st_shared16(dst + (DP + d) * 16, hi);
               }
             }
+            fence_proxy_async();
+            arrive(kv_full(n_half % NS));
             ++n_half;
-            announce();
             if (j + 1 < e) get_v(j + 1);
           }
         }
       }
       if (!ok) break;
-      if constexpr (!kFp8) {
-        // (an item without key tiles announces nothing, and the item after it is only drawn when
-        // the MMAs have come here: what is on its way has to be announced first)
-        if (it.b >= e) {
-          cp_async_wait<0>();
-          while (n_done < n_half) announce();
-        }
-      }
+      if constexpr (!kFp8) announce_all();  // (the next item may be drawn only when they have arrived)
       item = next_item();
     }
-    if constexpr (!kFp8) {
-      cp_async_wait<0>();
-      while (ok && n_done < n_half) announce();
-    }
-  } else if (lane == 0) {
-    // ================================================= the MMA thread
+    if constexpr (!kFp8) cp_async_wait_all();
+  } else {
+    reg_dec<PrefillRegs<kFp8>::kMma>();
+    if (warp == 12) {
+    // ================================================= the MMA warp.  All lanes run along, so that
+    // operand descriptors stay in uniform registers, and one elected lane issues: with a single
+    // lane running, moving them there cost 95 cycles an MMA of 64.
+    const bool leader = elect_one();
     const uint32_t idesc_s = mma_idesc(kBf, 128, KT);
     const uint32_t idesc_o = mma_idesc(kBf, 128, DP);
-    uint32_t n_k = 0, n_v = 0, n_it = 0, n_p[2] = {0, 0};
-    auto qk = [&](int i, uint32_t st) {
-#pragma unroll
-      for (int ks = 0; ks < DP / 16; ++ks)
-        mma_ss(tmem + i * KT, smem_desc(sq + i * SH::kQBytes + ks * 2 * 128 * 16, 128 * 16, 128),
-               smem_desc(sk + st * SH::kTileBytes + ks * 2 * KT * 16, KT * 16, 128), idesc_s, ks > 0);
-      mma_commit(s_full(i));
+    uint32_t n_h = 0, n_it = 0, n_p0 = 0, n_p1 = 0;  // halves consumed, items, P tiles received
+    auto uniform = [](uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); };
+    auto commit = [&](uint32_t bar) {
+      if (leader) mma_commit(bar);
     };
-    auto pv = [&](int i, uint32_t st, bool more) {
+    const uint64_t q_desc = smem_desc(sq, 128 * 16, 128);
+    const uint64_t k_desc = smem_desc(skv, KT * 16, 128);
+    const uint64_t v_desc = smem_desc(skv, DP * 16, 128);
+    auto wait_half = [&](uint32_t h) { return wait(kv_full(h % NS), (h / NS) & 1); };
+    auto qk = [&](int i, uint32_t h) {
+      const uint64_t kd = k_desc + uniform((h % NS) * (SH::kTileBytes >> 4));
+      const uint64_t qd = q_desc + i * (SH::kQBytes >> 4);
+      if (leader) {
 #pragma unroll
-      for (int ks = 0; ks < KT / 16; ++ks)
-        mma_ts(tmem + NQ * KT + i * DP, tmem + i * KT + ks * 8,
-               smem_desc(sv + st * SH::kTileBytes + ks * 2 * DP * 16, DP * 16, 128), idesc_o, more || ks > 0);
-      mma_commit(pv_done(i));
+        for (int ks = 0; ks < DP / 16; ++ks)
+          mma_ss(tmem + i * KT, qd + ks * 2 * 128, kd + ks * 2 * KT, idesc_s, ks > 0);
+        mma_commit(s_full(i));
+      }
+    };
+    auto pv = [&](int i, uint32_t h, bool more) {
+      const uint64_t vd = v_desc + uniform((h % NS) * (SH::kTileBytes >> 4));
+      if (leader) {
+#pragma unroll
+        for (int ks = 0; ks < KT / 16; ++ks)
+          mma_ts(tmem + NQ * KT + i * DP, tmem + i * KT + ks * 8, vd + ks * 2 * DP, idesc_o, more || ks > 0);
+        mma_commit(pv_done(i));
+      }
     };
     int item = blockIdx.x < unsigned(total) ? int(blockIdx.x) : INT32_MAX;
     while (item < total && ok) {
       // draw the next item now; the other roles pick it up when they are through with this one
-      const unsigned ticket = atomicAdd(p.sched, 1u);
+      unsigned ticket = 0;
+      if (leader) ticket = atomicAdd(p.sched, 1u);
       const PrefillItem it = decode(item);
+      ticket = __reduce_max_sync(0xffffffffu, ticket);
       const int nxt = int(min(ticket + gridDim.x, unsigned(INT32_MAX)));
       {
         const int slot = n_it & 1;
         if (n_it >= 2 && !wait(item_empty(slot), ((n_it >> 1) - 1) & 1)) break;
-        *reinterpret_cast<volatile int*>(&s_item[slot]) = nxt;
-        mbar_arrive(item_full(slot));
+        if (leader) {
+          *reinterpret_cast<volatile int*>(&s_item[slot]) = nxt;
+          mbar_arrive(item_full(slot));
+        }
       }
       const int e = max(it.e0, it.e1);
       if (!wait(q_full(0), n_it & 1) || !wait(q_full(1), n_it & 1)) break;
       ++n_it;
       tc_fence_after();
       if (it.b < e) {
-        if (!wait(k_full(n_k % NST), (n_k / NST) & 1)) break;
+        if (!wait_half(n_h)) break;
         tc_fence_after();
 #pragma unroll
         for (int i = 0; i < NQ; ++i)
-          if (it.b < (i == 0 ? it.e0 : it.e1)) qk(i, n_k % NST);
-        mma_commit(k_empty(n_k % NST));
-        ++n_k;
+          if (it.b < (i == 0 ? it.e0 : it.e1)) qk(i, n_h);
+        commit(kv_empty(n_h % NS));
+        ++n_h;
       }
-      for (int j = it.b; j < e && ok; ++j) {
-        if (!wait(v_full(n_v % NST), (n_v / NST) & 1)) break;
+      for (int j = it.b; j < e; ++j) {
+        // V tile j is half n_h, K tile j + 1 half n_h + 1
+        if (!wait_half(n_h)) break;
         bool have_k = false;
 #pragma unroll
         for (int i = 0; i < NQ; ++i) {
           const int ei = i == 0 ? it.e0 : it.e1;
+          uint32_t& n_p = i == 0 ? n_p0 : n_p1;
           if (!ok || j >= ei) continue;
-          if (!wait(p_full(i), n_p[i] & 1)) continue;
-          ++n_p[i];
+          if (!wait(p_full(i), n_p & 1)) continue;
+          ++n_p;
           tc_fence_after();
-          pv(i, n_v % NST, j > it.b);
+          pv(i, n_h, j > it.b);
           if (j + 1 < ei) {
-            if (!have_k) {
-              if (!wait(k_full(n_k % NST), (n_k / NST) & 1)) continue;
-              tc_fence_after();
-              have_k = true;
-            }
-            qk(i, n_k % NST);
+            if (!have_k && !wait_half(n_h + 1)) continue;
+            have_k = true;
+            qk(i, n_h + 1);
           }
         }
         if (!ok) break;
-        mma_commit(v_empty(n_v % NST));
-        ++n_v;
+        commit(kv_empty(n_h % NS));
+        ++n_h;
         if (have_k) {
-          mma_commit(k_empty(n_k % NST));
-          ++n_k;
+          commit(kv_empty(n_h % NS));
+          ++n_h;
         }
       }
       item = nxt;
+    }
     }
   }
 

@@ -29,7 +29,7 @@ extern "C" int b200pa_paged_attention_varlen(const b200pa_attn_args* a, const in
     const int es = a->kv_dtype == B200PA_KV_AUTO ? 2 : 1;
     auto al = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr) % 16 == 0; };
     const bool fits = (a->block_size == 16 || a->block_size == 32) && a->num_heads / a->num_kv_heads <= 128 &&
-                      reqs <= kPrefillMaxReqs && al(a->key_cache) && al(a->value_cache) && al(a->query) &&
+                      al(a->key_cache) && al(a->value_cache) && al(a->query) &&
                       al(a->out) && (a->kv_block_stride * es) % 16 == 0 && (a->kv_head_stride * es) % 16 == 0 &&
                       a->q_stride % 8 == 0 && a->blocksparse_vert_stride <= 1 && a->out_lse == nullptr;
     if (fits) {
@@ -39,8 +39,8 @@ extern "C" int b200pa_paged_attention_varlen(const b200pa_attn_args* a, const in
     }
     if (ki.fn == nullptr) {
       set_error("paged_attention_varlen: no kernel for head_size=%d block_size=%d q_dtype=%d kv_dtype=%d, "
-                "%d requests, or unaligned tensors",
-                a->head_size, a->block_size, a->q_dtype, a->kv_dtype, reqs);
+                "or unaligned tensors",
+                a->head_size, a->block_size, a->q_dtype, a->kv_dtype);
       return B200PA_EUNSUPPORTED;
     }
   }
@@ -59,16 +59,12 @@ extern "C" int b200pa_paged_attention_varlen(const b200pa_attn_args* a, const in
   p.q = a->query;
   p.kc = a->key_cache;
   p.vc = a->value_cache;
-  p.block_tables = a->block_tables + int64_t(num_decodes) * a->max_num_blocks_per_seq;
-  p.seq_lens = a->seq_lens + num_decodes;
-  p.q_start = query_start_loc + num_decodes;
   p.alibi = a->alibi_slopes;
   p.k_scale = a->k_scale;
   p.v_scale = a->v_scale;
   p.q_stride = a->q_stride;
   p.kv_block_stride = a->kv_block_stride;
   p.kv_head_stride = a->kv_head_stride;
-  p.num_reqs = reqs;
   p.num_heads = a->num_heads;
   p.num_kv_heads = a->num_kv_heads;
   p.group = a->num_heads / a->num_kv_heads;
@@ -81,17 +77,23 @@ extern "C" int b200pa_paged_attention_varlen(const b200pa_attn_args* a, const in
     p.arrive = region.arrive;
     p.ws_slots = int(std::min<int64_t>(int64_t(region.ws_bytes) / ki.piece_bytes, kArrivePerRegion / 8));
   }
-  p.sched = sched_words();
   p.status = device_status_ptr();
-  if (p.sched == nullptr || p.status == nullptr) {
-    set_error("could not resolve device-side scheduler/status words");
-    return B200PA_ECUDA;
-  }
-  const cudaError_t e = ki.fn(p, sm_count(), s);
-  count_launch();
-  if (e != cudaSuccess) {
-    set_error("prefill kernel launch failed: %s", cudaGetErrorString(e));
-    return B200PA_ECUDA;
+  for (int r = num_decodes; r < a->num_seqs; r += kPrefillMaxReqs) {
+    p.num_reqs = std::min(kPrefillMaxReqs, a->num_seqs - r);
+    p.block_tables = a->block_tables + int64_t(r) * a->max_num_blocks_per_seq;
+    p.seq_lens = a->seq_lens + r;
+    p.q_start = query_start_loc + r;
+    p.sched = sched_words();
+    if (p.sched == nullptr || p.status == nullptr) {
+      set_error("could not resolve device-side scheduler/status words");
+      return B200PA_ECUDA;
+    }
+    const cudaError_t e = ki.fn(p, sm_count(), s);
+    count_launch();
+    if (e != cudaSuccess) {
+      set_error("prefill kernel launch failed: %s", cudaGetErrorString(e));
+      return B200PA_ECUDA;
+    }
   }
   return B200PA_OK;
 }
