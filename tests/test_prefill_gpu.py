@@ -119,6 +119,14 @@ def test_many_requests_and_single_rows_among_them():
     _case(q, rng.integers(0, 400, size=600), 8, 2, 64, 16, torch.bfloat16, "auto")
 
 
+@pytest.mark.parametrize("kv,dtype", [("auto", torch.bfloat16), ("fp8_e5m2", torch.bfloat16), ("fp8", torch.float16)])
+@pytest.mark.parametrize("alibi", [False, True])
+@pytest.mark.parametrize("HK", [2, 8])
+def test_short_chunks_with_and_without_bias(kv, dtype, alibi, HK):
+    _case([37, 120, 203, 25, 108, 191, 96, 179, 300], [16, 17, 18, 13, 14, 15, 11, 12, 400], 32, HK, 128, 16,
+          dtype, kv, alibi=alibi)
+
+
 @pytest.mark.parametrize("kv", ["auto", "fp8"])
 def test_a_long_prompt(kv):
     _case([1500, 900], [700, 0], 8, 2, 128, 16, torch.bfloat16, kv)

@@ -71,7 +71,7 @@ constexpr int kPrefillThreads = 16 * 32;  // (three warps beside the MMA warp on
 // others give back.  (The producers of an fp8 cache hold a K and a V tile in registers.)
 template <bool kFp8>
 struct PrefillRegs {
-  static constexpr int kSoftmax = kFp8 ? 168 : 184, kProducer = kFp8 ? 120 : 88, kMma = 56;
+  static constexpr int kSoftmax = kFp8 ? 176 : 184, kProducer = kFp8 ? 104 : 88, kMma = 56;
   static_assert(2 * kSoftmax + kProducer + kMma == 4 * 128, "register split");
 };
 constexpr int kPrefillMaxReqs = 512;    // requests per launch: prefix table in shared memory
@@ -314,15 +314,23 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
     const int row_tok = row / G, row_head = row % G;
     uint32_t n_s = 0, n_pv = 0;  // S tiles received, PV products issued for this row tile
 
+    // Each warp brings its own 32 rows: eight rows and four 16-byte granules at a time, 64-byte pieces
+    // of global memory into 128-byte runs of the operand layout.  (One row per thread: 8000 cycles
+    // an item instead of ~2000.)
     auto load_q = [&](const PrefillItem& it) {
       if (wg < NQ) {
-        const int tok = it.tok0 + wg * T + row_tok;
-        if (row_used && tok < it.q_len) {
-          const QT* src = static_cast<const QT*>(p.q) + int64_t(it.q0 + tok) * p.q_stride +
-                          int64_t(it.kvh * G + row_head) * D;
-          const uint32_t dst = sq + wg * SH::kQBytes + row * 16;
 #pragma unroll
-          for (int g = 0; g < D / 8; ++g) {
+        for (int rb = 0; rb < 4; ++rb) {
+          const int from = rb * 8 + (lane & 7);  // the row: this lane's copy of its token and head
+          const int tok = it.tok0 + wg * T + __shfl_sync(0xffffffffu, row_tok, from);
+          const int head = it.kvh * G + __shfl_sync(0xffffffffu, row_head, from);
+          const bool used = __shfl_sync(0xffffffffu, int(row_used), from) != 0 && tok < it.q_len;
+          const QT* src = static_cast<const QT*>(p.q) + int64_t(it.q0 + tok) * p.q_stride + int64_t(head) * D;
+          const uint32_t dst = sq + wg * SH::kQBytes + ((row & ~31) + from) * 16;
+#pragma unroll
+          for (int g0 = 0; g0 < D / 8; g0 += 4) {
+            const int g = g0 + (lane >> 3);
+            if (!used || (D / 8 % 4 != 0 && g >= D / 8)) continue;
             if constexpr (kFp8 && kOutBf) {  // the operands of an fp8 cache are f16
               const uint4 v = __ldg(reinterpret_cast<const uint4*>(src) + g);
               const uint32_t w[4] = {v.x, v.y, v.z, v.w};
@@ -335,8 +343,8 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
               cp_async16(dst + g * 128 * 16, reinterpret_cast<const uint4*>(src) + g, 16);
             }
           }
-          if constexpr (!(kFp8 && kOutBf)) cp_async_wait_all();
         }
+        if constexpr (!(kFp8 && kOutBf)) cp_async_wait_all();
       }
       fence_proxy_async();
       arrive(q_full(wg));
@@ -365,46 +373,81 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
         // No bias: only the tiles at the causal edge of a row tile need a mask.
         const bool plain = p.alibi == nullptr && c > 0.f;
         const bool edge = key0 + KT - 1 > pos_first;
+        int last = pos - key0;  // last column of this row that counts
+        float cc = c;           // (goes through the waits for TMEM loads, see tmem_landed)
         auto mask = [&](float (&x)[32], int ch) {
           if (edge) {
-            const int last = pos - key0 - ch * 32;  // last column of the chunk that counts
 #pragma unroll
-            for (int k = 0; k < 32; ++k) x[k] = k <= last ? x[k] : -INFINITY;
+            for (int k = 0; k < 32; ++k) x[k] = k <= last - ch * 32 ? x[k] : -INFINITY;
           }
         };
         // with a bias: t = x c + slope (key - pos), and the mask
         auto biased = [&](float x, int ch, int k) {
-          const int first = key0 + ch * 32 - pos;  // (of this row: key - pos of column 0)
-          return first + k <= 0 ? fmaf(slope, float(k), fmaf(x, c, slope * float(first))) : -INFINITY;
+          const int first = ch * 32 - last;  // (of this row: key - pos of column 0)
+          return first + k <= 0 ? fmaf(slope, float(k), fmaf(x, cc, slope * float(first))) : -INFINITY;
         };
         float mx = -INFINITY;
-        // 32-column chunks: one is on its way while another is worked on.  (Registers that a load is
-        // on its way to are not to be moved: the loads span straight-line code only.)
-        constexpr int NC = KT / 32;
+        constexpr int NC = KT / 32;  // 32-column chunks: one is on its way while another is worked on
+        float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        float s4[4] = {0.f, 0.f, 0.f, 0.f};
         float v[2][32];
-        tmem_ld32(t_s, v[0]);
-        if (plain) {
+        if (!kFp8 && plain && j > b) {
+          // After the first tile the running maximum mostly stands: take it as it is, and look at this
+          // tile's maximum while the exponentials run.  P waits in registers, S stays intact; a
+          // maximum that grew sends the tile through the two passes below.  (3 % at head size 128; not
+          // for fp8 caches, whose producers need the registers.)
+          const float mm = m == -INFINITY ? 0.f : m;
+          uint32_t w[NC][16];
+          tmem_ld32(t_s, v[0]);
 #pragma unroll
           for (int ch = 0; ch < NC; ++ch) {
             float (&x)[32] = v[ch & 1];
-            tmem_landed(x);
+            tmem_landed(m4, cc, last);
             if (ch + 1 < NC) tmem_ld32(t_s + (ch + 1) * 32, v[(ch + 1) & 1]);
             mask(x, ch);
-            float m4[4] = {x[0], x[1], x[2], x[3]};
 #pragma unroll
-            for (int k = 4; k < 32; ++k) m4[k & 3] = fmaxf(m4[k & 3], x[k]);
-            mx = fmaxf(mx, fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])));
+            for (int k = 0; k < 32; k += 2) {
+              m4[k & 2] = fmaxf(m4[k & 2], x[k]);
+              m4[(k & 2) + 1] = fmaxf(m4[(k & 2) + 1], x[k + 1]);
+              const float p0 = fast_exp2(fmaf(x[k], cc, -mm)), p1 = fast_exp2(fmaf(x[k + 1], cc, -mm));
+              s4[k & 2] += p0;
+              s4[(k & 2) + 1] += p1;
+              w[ch][k / 2] = pack2<kBf>(p0, p1);
+            }
           }
-          mx *= c;
+          mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * c;
+          if (!__any_sync(0xffffffffu, mx > m + 8.f || (m == -INFINITY && mx > m))) {
+#pragma unroll
+            for (int ch = 0; ch < NC; ++ch) tmem_st16(t_s + ch * 16, w[ch]);
+            l += (s4[0] + s4[1]) + (s4[2] + s4[3]);
+            tmem_wait_st();
+            tc_fence_before();
+            arrive(p_full(wg));
+            ++n_pv;
+            continue;
+          }
+          s4[0] = s4[1] = s4[2] = s4[3] = 0.f;
+        } else if (plain) {
+          tmem_ld32(t_s, v[0]);
+#pragma unroll
+          for (int ch = 0; ch < NC; ++ch) {
+            float (&x)[32] = v[ch & 1];
+            tmem_landed(m4, cc, last);
+            if (ch + 1 < NC) tmem_ld32(t_s + (ch + 1) * 32, v[(ch + 1) & 1]);
+            mask(x, ch);
+#pragma unroll
+            for (int k = 0; k < 32; ++k) m4[k & 3] = fmaxf(m4[k & 3], x[k]);
+          }
+          mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * c;
         } else {
 #pragma unroll 1
           for (int ch = 0; ch < NC; ++ch) {
-            float (&x)[32] = v[0];
-            tmem_landed(x);
+            tmem_ld32(t_s + ch * 32, v[0]);
+            tmem_landed(m4, cc, last);
 #pragma unroll
-            for (int k = 0; k < 32; ++k) mx = fmaxf(mx, biased(x[k], ch, k));
-            if (ch + 1 < NC) tmem_ld32(t_s + (ch + 1) * 32, x);
+            for (int k = 0; k < 32; ++k) m4[k & 3] = fmaxf(m4[k & 3], biased(v[0][k], ch, k));
           }
+          mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
         }
         // raise the maximum (and rescale what has been summed) only when it grew by more than 8
         const bool grow = mx > m + 8.f || (m == -INFINITY && mx > m);
@@ -428,45 +471,43 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
           }
         }
         const float mm = m == -INFINITY ? 0.f : m;
-        float sum = 0.f;
-        tmem_ld32(t_s, v[0]);
+        // (P's columns lie over S columns that have been read: 16 a chunk over 32)
         if (plain) {
+          tmem_ld32(t_s, v[0]);
 #pragma unroll
           for (int ch = 0; ch < NC; ++ch) {
             float (&x)[32] = v[ch & 1];
-            tmem_landed(x);
+            tmem_landed(s4, cc, last);
             if (ch + 1 < NC) tmem_ld32(t_s + (ch + 1) * 32, v[(ch + 1) & 1]);
             mask(x, ch);
-            float s4[4] = {0.f, 0.f, 0.f, 0.f};
             uint32_t w[16];
 #pragma unroll
             for (int k = 0; k < 32; k += 2) {
-              const float p0 = fast_exp2(fmaf(x[k], c, -mm)), p1 = fast_exp2(fmaf(x[k + 1], c, -mm));
+              const float p0 = fast_exp2(fmaf(x[k], cc, -mm)), p1 = fast_exp2(fmaf(x[k + 1], cc, -mm));
               s4[k & 2] += p0;
               s4[(k & 2) + 1] += p1;
               w[k / 2] = pack2<kBf>(p0, p1);
             }
-            sum += (s4[0] + s4[1]) + (s4[2] + s4[3]);
             tmem_st16(t_s + ch * 16, w);
           }
         } else {
 #pragma unroll 1
           for (int ch = 0; ch < NC; ++ch) {
-            float (&x)[32] = v[0];
-            tmem_landed(x);
+            tmem_ld32(t_s + ch * 32, v[0]);
+            tmem_landed(s4, cc, last);
             uint32_t w[16];
 #pragma unroll
             for (int k = 0; k < 32; k += 2) {
-              const float p0 = fast_exp2(biased(x[k], ch, k) - mm);
-              const float p1 = fast_exp2(biased(x[k + 1], ch, k + 1) - mm);
-              sum += p0 + p1;
+              const float p0 = fast_exp2(biased(v[0][k], ch, k) - mm);
+              const float p1 = fast_exp2(biased(v[0][k + 1], ch, k + 1) - mm);
+              s4[k & 2] += p0;
+              s4[(k & 2) + 1] += p1;
               w[k / 2] = pack2<kBf>(p0, p1);
             }
-            // (P's columns lie over S columns that have been read: 16 a chunk over 32)
-            if (ch + 1 < NC) tmem_ld32(t_s + (ch + 1) * 32, x);
             tmem_st16(t_s + ch * 16, w);
           }
         }
+        const float sum = (s4[0] + s4[1]) + (s4[2] + s4[3]);
         l += sum;
         tmem_wait_st();
         tc_fence_before();
@@ -773,14 +814,15 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
     if (warp == 12) {
     // ================================================= the MMA warp.  All lanes run along, so that
     // operand descriptors stay in uniform registers, and one elected lane issues: with a single
-    // lane running, moving them there cost 95 cycles an MMA of 64.
-    const bool leader = elect_one();
+    // lane running, moving them there cost 95 cycles an MMA of 64.  Uniform registers belong to the
+    // warp: after every block of the elected lane the warp converges before anything else runs.
     const uint32_t idesc_s = mma_idesc(kBf, 128, KT);
     const uint32_t idesc_o = mma_idesc(kBf, 128, DP);
     uint32_t n_h = 0, n_it = 0, n_p0 = 0, n_p1 = 0;  // halves consumed, items, P tiles received
     auto uniform = [](uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); };
     auto commit = [&](uint32_t bar) {
-      if (leader) mma_commit(bar);
+      if (elect_one()) mma_commit(bar);
+      __syncwarp();
     };
     const uint64_t q_desc = smem_desc(sq, 128 * 16, 128);
     const uint64_t k_desc = smem_desc(skv, KT * 16, 128);
@@ -789,37 +831,40 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
     auto qk = [&](int i, uint32_t h) {
       const uint64_t kd = k_desc + uniform((h % NS) * (SH::kTileBytes >> 4));
       const uint64_t qd = q_desc + i * (SH::kQBytes >> 4);
-      if (leader) {
+      if (elect_one()) {
 #pragma unroll
         for (int ks = 0; ks < DP / 16; ++ks)
           mma_ss(tmem + i * KT, qd + ks * 2 * 128, kd + ks * 2 * KT, idesc_s, ks > 0);
         mma_commit(s_full(i));
       }
+      __syncwarp();
     };
     auto pv = [&](int i, uint32_t h, bool more) {
       const uint64_t vd = v_desc + uniform((h % NS) * (SH::kTileBytes >> 4));
-      if (leader) {
+      if (elect_one()) {
 #pragma unroll
         for (int ks = 0; ks < KT / 16; ++ks)
           mma_ts(tmem + NQ * KT + i * DP, tmem + i * KT + ks * 8, vd + ks * 2 * DP, idesc_o, more || ks > 0);
         mma_commit(pv_done(i));
       }
+      __syncwarp();
     };
     int item = blockIdx.x < unsigned(total) ? int(blockIdx.x) : INT32_MAX;
     while (item < total && ok) {
       // draw the next item now; the other roles pick it up when they are through with this one
       unsigned ticket = 0;
-      if (leader) ticket = atomicAdd(p.sched, 1u);
+      if (lane == 0) ticket = atomicAdd(p.sched, 1u);
       const PrefillItem it = decode(item);
-      ticket = __reduce_max_sync(0xffffffffu, ticket);
+      ticket = __shfl_sync(0xffffffffu, ticket, 0);
       const int nxt = int(min(ticket + gridDim.x, unsigned(INT32_MAX)));
       {
         const int slot = n_it & 1;
         if (n_it >= 2 && !wait(item_empty(slot), ((n_it >> 1) - 1) & 1)) break;
-        if (leader) {
+        if (lane == 0) {
           *reinterpret_cast<volatile int*>(&s_item[slot]) = nxt;
           mbar_arrive(item_full(slot));
         }
+        __syncwarp();
       }
       const int e = max(it.e0, it.e1);
       if (!wait(q_full(0), n_it & 1) || !wait(q_full(1), n_it & 1)) break;

@@ -66,9 +66,9 @@ __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
-// 32 consecutive columns of this thread's TMEM lane.  The load only starts here: the values may
-// be used after tmem_landed() on the same array (which ties them to the wait, so that no use
-// can be scheduled in front of it).
+// 32 consecutive columns of this thread's TMEM lane.  The load only starts here: until tmem_landed()
+// the destination registers belong to the load, and nothing - no copy, no loop-carried move - may
+// touch them.
 __device__ __forceinline__ void tmem_ld32(uint32_t addr, float (&v)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -81,17 +81,12 @@ __device__ __forceinline__ void tmem_ld32(uint32_t addr, float (&v)[32]) {
       : "r"(addr)
       : "memory");
 }
-__device__ __forceinline__ void tmem_landed(float (&v)[32]) {
+// Waits for this thread's TMEM loads.  The arguments are what the loaded values will be combined
+// with: passing them through the wait keeps every use behind it, without an operand that names (and
+// might copy) the registers of a load still on its way.
+__device__ __forceinline__ void tmem_landed(float (&with)[4], float& c, int& last) {
   asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]),
-                 "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]),
-                 "+f"(v[15])
-               :
-               : "memory");
-  asm volatile(""
-               : "+f"(v[16]), "+f"(v[17]), "+f"(v[18]), "+f"(v[19]), "+f"(v[20]), "+f"(v[21]), "+f"(v[22]),
-                 "+f"(v[23]), "+f"(v[24]), "+f"(v[25]), "+f"(v[26]), "+f"(v[27]), "+f"(v[28]), "+f"(v[29]),
-                 "+f"(v[30]), "+f"(v[31])
+               : "+f"(with[0]), "+f"(with[1]), "+f"(with[2]), "+f"(with[3]), "+f"(c), "+r"(last)
                :
                : "memory");
 }
