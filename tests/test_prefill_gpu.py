@@ -128,5 +128,13 @@ def test_short_chunks_with_and_without_bias(kv, dtype, alibi, HK):
 
 
 @pytest.mark.parametrize("kv", ["auto", "fp8"])
+@pytest.mark.parametrize("alibi", [False, True])
+def test_items_whose_second_row_tile_is_empty(kv, alibi):
+    # (the warpgroup of the second row tile runs items ahead of everybody else)
+    _case([20 + i % 12 + 64 * (i % 3) for i in range(60)], [i % 19 for i in range(60)], 32, 8, 128, 16,
+          torch.bfloat16, kv, alibi=alibi)
+
+
+@pytest.mark.parametrize("kv", ["auto", "fp8"])
 def test_a_long_prompt(kv):
     _case([1500, 900], [700, 0], 8, 2, 128, 16, torch.bfloat16, kv)

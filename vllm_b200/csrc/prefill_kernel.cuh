@@ -317,8 +317,10 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
     // Each warp brings its own 32 rows: eight rows and four 16-byte granules at a time, 64-byte pieces
     // of global memory into 128-byte runs of the operand layout.  (One row per thread: 8000 cycles
     // an item instead of ~2000.)
+    // Only for a row tile that has key tiles in this item: a warpgroup without work may be items ahead
+    // of the MMAs, and must not complete a phase of q_full that they have not waited for.
     auto load_q = [&](const PrefillItem& it) {
-      if (wg < NQ) {
+      if ((wg == 0 ? it.e0 : it.e1) > it.b) {
 #pragma unroll
         for (int rb = 0; rb < 4; ++rb) {
           const int from = rb * 8 + (lane & 7);  // the row: this lane's copy of its token and head
@@ -345,9 +347,9 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
           }
         }
         if constexpr (!(kFp8 && kOutBf)) cp_async_wait_all();
+        fence_proxy_async();
+        arrive(q_full(wg));
       }
-      fence_proxy_async();
-      arrive(q_full(wg));
     };
 
     int item = blockIdx.x < unsigned(total) ? int(blockIdx.x) : INT32_MAX;
@@ -732,7 +734,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
 #pragma unroll
           for (int i = 0; i < KN; ++i) {
             const int g = kg + i * (128 / KT);
-            if (key < it.seq_len && g < D / 16) kr[i] = __ldg(reinterpret_cast<const uint4*>(src + int64_t(g) * B * 16));
+            if (key < it.seq_len && g < D / 16) kr[i] = __ldcg(reinterpret_cast<const uint4*>(src + int64_t(g) * B * 16));
             else kr[i] = make_uint4(0, 0, 0, 0);
           }
         };
@@ -742,7 +744,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
 #pragma unroll
           for (int i = 0; i < VN; ++i) {
             const int d = vd + i * VDS;
-            if (key < it.seq_len && d < D) vr[i] = __ldg(reinterpret_cast<const uint4*>(src + int64_t(d) * B));
+            if (key < it.seq_len && d < D) vr[i] = __ldcg(reinterpret_cast<const uint4*>(src + int64_t(d) * B));
             else vr[i] = make_uint4(0, 0, 0, 0);
           }
         };
@@ -818,7 +820,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
     // warp: after every block of the elected lane the warp converges before anything else runs.
     const uint32_t idesc_s = mma_idesc(kBf, 128, KT);
     const uint32_t idesc_o = mma_idesc(kBf, 128, DP);
-    uint32_t n_h = 0, n_it = 0, n_p0 = 0, n_p1 = 0;  // halves consumed, items, P tiles received
+    uint32_t n_h = 0, n_it = 0, n_q0 = 0, n_q1 = 0, n_p0 = 0, n_p1 = 0;  // halves, items, Q tiles, P tiles
     auto uniform = [](uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); };
     auto commit = [&](uint32_t bar) {
       if (elect_one()) mma_commit(bar);
@@ -867,7 +869,8 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
         __syncwarp();
       }
       const int e = max(it.e0, it.e1);
-      if (!wait(q_full(0), n_it & 1) || !wait(q_full(1), n_it & 1)) break;
+      if (it.b < it.e0 && !wait(q_full(0), n_q0++ & 1)) break;
+      if (it.b < it.e1 && !wait(q_full(1), n_q1++ & 1)) break;
       ++n_it;
       tc_fence_after();
       if (it.b < e) {
