@@ -329,20 +329,31 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
           const bool used = __shfl_sync(0xffffffffu, int(row_used), from) != 0 && tok < it.q_len;
           const QT* src = static_cast<const QT*>(p.q) + int64_t(it.q0 + tok) * p.q_stride + int64_t(head) * D;
           const uint32_t dst = sq + wg * SH::kQBytes + ((row & ~31) + from) * 16;
+          constexpr int NG = (D / 8 + 3) / 4;
+          if constexpr (kFp8 && kOutBf) {  // the operands of an fp8 cache are f16
+            uint4 v[NG];
 #pragma unroll
-          for (int g0 = 0; g0 < D / 8; g0 += 4) {
-            const int g = g0 + (lane >> 3);
-            if (!used || (D / 8 % 4 != 0 && g >= D / 8)) continue;
-            if constexpr (kFp8 && kOutBf) {  // the operands of an fp8 cache are f16
-              const uint4 v = __ldg(reinterpret_cast<const uint4*>(src) + g);
-              const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+            for (int i = 0; i < NG; ++i) {
+              const int g = 4 * i + (lane >> 3);
+              v[i] = used && (D / 8 % 4 == 0 || g < D / 8) ? __ldg(reinterpret_cast<const uint4*>(src) + g)
+                                                            : make_uint4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (int i = 0; i < NG; ++i) {
+              const int g = 4 * i + (lane >> 3);
+              const uint32_t w[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
               uint32_t o[4];
 #pragma unroll
               for (int k = 0; k < 4; ++k)
                 o[k] = pack2<false>(__uint_as_float(w[k] << 16), __uint_as_float(w[k] & 0xffff0000u));
-              st_shared16(dst + g * 128 * 16, make_uint4(o[0], o[1], o[2], o[3]));
-            } else {
-              cp_async16(dst + g * 128 * 16, reinterpret_cast<const uint4*>(src) + g, 16);
+              if (D / 8 % 4 == 0 || g < D / 8) st_shared16(dst + g * 128 * 16, make_uint4(o[0], o[1], o[2], o[3]));
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < NG; ++i) {
+              const int g = 4 * i + (lane >> 3);
+              if (used && (D / 8 % 4 == 0 || g < D / 8))
+                cp_async16(dst + g * 128 * 16, reinterpret_cast<const uint4*>(src) + g, 16);
             }
           }
         }
@@ -577,46 +588,61 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
           __threadfence();
           const unsigned char* base = p.ws + (size_t(cur.first) * NQ + wg) * kWs;
           const size_t step = size_t(HK) * NQ * kWs;
-          float mx = -INFINITY;
-          for (int k = 0; k < cur.npieces; ++k) {
-            const float2 ml = __ldcg(reinterpret_cast<const float2*>(base + k * step + 128 * D * 2) + row);
-            if (ml.y > 0.f) mx = fmaxf(mx, ml.x);
-          }
-          float total_l = 0.f;
-          for (int k = 0; k < cur.npieces; ++k) {
-            const float2 ml = __ldcg(reinterpret_cast<const float2*>(base + k * step + 128 * D * 2) + row);
-            if (ml.y > 0.f) total_l += ml.y * fast_exp2(ml.x - mx);
+          // statistics of eight pieces at a time (independent loads), online
+          float mx = -INFINITY, total_l = 0.f;
+#pragma unroll 1
+          for (int k0 = 0; k0 < cur.npieces; k0 += 8) {
+            float2 ml[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+              ml[k] = __ldcg(reinterpret_cast<const float2*>(base + min(k0 + k, cur.npieces - 1) * step + 128 * D * 2) + row);
+            float m_new = mx;
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+              if (k0 + k < cur.npieces && ml[k].y > 0.f) m_new = fmaxf(m_new, ml[k].x);
+            if (m_new == -INFINITY) continue;
+            total_l *= fast_exp2(mx - m_new);
+            mx = m_new;
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+              if (k0 + k < cur.npieces && ml[k].y > 0.f) total_l += ml[k].y * fast_exp2(ml[k].x - mx);
           }
           const float winv = __fdividef(1.f, total_l + 1e-6f);
           QT* od = static_cast<QT*>(p.out) + out_row;
 #pragma unroll 1
-          for (int d0 = 0; d0 < D; d0 += 8 * 4) {
-            float acc[4][8];
+          for (int d0 = 0; d0 < D; d0 += 16) {
+            float acc[16];
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
+            for (int z = 0; z < 16; ++z) acc[z] = 0.f;
+            // four pieces at a time: eight independent loads on their way
+#pragma unroll 1
+            for (int k0 = 0; k0 < cur.npieces; k0 += 4) {
+              uint4 x[4][2];
+              float w[4];
 #pragma unroll
-              for (int k = 0; k < 8; ++k) acc[u][k] = 0.f;
-            for (int k = 0; k < cur.npieces; ++k) {
-              const float2 ml = __ldcg(reinterpret_cast<const float2*>(base + k * step + 128 * D * 2) + row);
-              if (!(ml.y > 0.f)) continue;
-              const float w = ml.y * fast_exp2(ml.x - mx) * winv;
-              const QT* src = reinterpret_cast<const QT*>(base + k * step) + row * D + d0;
+              for (int k = 0; k < 4; ++k) {
+                const unsigned char* pk = base + min(k0 + k, cur.npieces - 1) * step;
+                const float2 ml = __ldcg(reinterpret_cast<const float2*>(pk + 128 * D * 2) + row);
+                const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const QT*>(pk) + row * D + d0);
+                x[k][0] = __ldcg(src);
+                x[k][1] = D % 16 == 0 || d0 + 8 < D ? __ldcg(src + 1) : make_uint4(0, 0, 0, 0);
+                // (a piece in which this row has no key has written no output)
+                w[k] = k0 + k < cur.npieces && ml.y > 0.f ? ml.y * fast_exp2(ml.x - mx) * winv : 0.f;
+              }
 #pragma unroll
-              for (int u = 0; u < 4; ++u) {
-                if (d0 + u * 8 < D) {
-                  const uint4 x = __ldcg(reinterpret_cast<const uint4*>(src) + u);
-                  const QT* xe = reinterpret_cast<const QT*>(&x);
+              for (int k = 0; k < 4; ++k) {
+                if (w[k] == 0.f) continue;
+                const QT* xe = reinterpret_cast<const QT*>(x[k]);
 #pragma unroll
-                  for (int z = 0; z < 8; ++z) acc[u][z] += w * to_f32(xe[z]);
-                }
+                for (int z = 0; z < 16; ++z) acc[z] += w[k] * to_f32(xe[z]);
               }
             }
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-              if (d0 + u * 8 < D)
-                reinterpret_cast<uint4*>(od + d0)[u] =
-                    make_uint4(pack2<kOutBf>(acc[u][0], acc[u][1]), pack2<kOutBf>(acc[u][2], acc[u][3]),
-                               pack2<kOutBf>(acc[u][4], acc[u][5]), pack2<kOutBf>(acc[u][6], acc[u][7]));
+            uint4* o4 = reinterpret_cast<uint4*>(od + d0);
+            o4[0] = make_uint4(pack2<kOutBf>(acc[0], acc[1]), pack2<kOutBf>(acc[2], acc[3]),
+                               pack2<kOutBf>(acc[4], acc[5]), pack2<kOutBf>(acc[6], acc[7]));
+            if (D % 16 == 0 || d0 + 8 < D)
+              o4[1] = make_uint4(pack2<kOutBf>(acc[8], acc[9]), pack2<kOutBf>(acc[10], acc[11]),
+                                 pack2<kOutBf>(acc[12], acc[13]), pack2<kOutBf>(acc[14], acc[15]));
           }
         }
         __syncwarp();
