@@ -383,7 +383,7 @@ reshape_and_cache_kernel(const in_t* __restrict__ key, const in_t* __restrict__ 
                          int block_size, int x, const float* __restrict__ k_scale_ptr,
                          const float* __restrict__ v_scale_ptr) {
   __shared__ TileSlots ts;
-  grid_dependency();
+  grid_dependency_wait();
   const int tok0 = blockIdx.x * kTokTile;
   const int ntok = min(kTokTile, num_tokens - tok0);
   load_tile_slots(ts, slot_mapping, tok0, ntok, block_size, int(sizeof(cache_t)));
@@ -542,7 +542,7 @@ reshape_and_cache_flash_kernel(const in_t* __restrict__ key, const in_t* __restr
                                int block_size, int vec_ok, const float* __restrict__ k_scale_ptr,
                                const float* __restrict__ v_scale_ptr) {
   __shared__ TileSlots ts;
-  grid_dependency();
+  grid_dependency_wait();
   const int tok0 = blockIdx.x * kTokTile;
   const int ntok = min(kTokTile, num_tokens - tok0);
   load_tile_slots(ts, slot_mapping, tok0, ntok, block_size, int(sizeof(cache_t)));
@@ -750,7 +750,10 @@ static bool launch_staged(const b200pa_cache_args& a, cudaStream_t stream, int* 
   // tokens 14.0 -> 11.2 us); large ones pay for the doubled per-item bookkeeping (27 -> 35 us).
   const int64_t items1 = int64_t((a.num_tokens + kStagedTile - 1) / kStagedTile) * a.num_heads * 2;
   const bool small = 2 * items1 <= int64_t(cache_sm_count()) * kStagedMaxWarps;
-  const int hsplit = (a.head_size % 128 == 0 && (kn_hsplit == 2 || (kn_hsplit == 0 && small))) ? 2 : 1;
+  // Heads wider than 128 are always cut: a whole row of them takes so much shared memory that only 12
+  // to 16 warps fit (head size 256, fp8, 27 500 tokens of one head: 27.9 -> 19.8 us).
+  const bool cut = a.head_size > 128 ? a.head_size % 32 == 0 : a.head_size == 128 && small;
+  const int hsplit = kn_hsplit == 0 ? (cut ? 2 : 1) : (kn_hsplit == 2 && a.head_size % 32 == 0 ? 2 : 1);
   // Large x-layout writes use the variant that moves tiles onto 16-slot boundaries of the cache
   // (prefill chunks that start inside a block: 16 384 tokens x 8 heads, fp8 51 -> 38 us, 16-bit
   // cache 67 -> 36 us; chunks that start on a boundary are not affected).  Its extra code costs
