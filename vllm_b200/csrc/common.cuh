@@ -71,8 +71,11 @@ __device__ __forceinline__ void grid_dependency() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
-// The same without the second half: for grids of many small blocks, where the next grid's blocks
+// Its halves.  The wait alone: for grids of many small blocks, where the next grid's blocks
 // would take the places of this one's.
+__device__ __forceinline__ void grid_launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ float to_f32(float v) { return v; }

@@ -7,6 +7,8 @@
 
 #include <cstddef>
 
+#include "../../include/b200pa.h"
+
 namespace b200pa {
 
 constexpr int kArrivePerRegion = 32768;
@@ -21,5 +23,8 @@ struct StreamRegion {
 bool stream_region(cudaStream_t stream, StreamRegion* out);
 unsigned* sched_words();
 int sm_count();
+
+// paged_attention_v1 on the first half of the stream's workspace and arrival counters.
+int attention_half_region(const b200pa_attn_args* a, void* stream);
 
 }  // namespace b200pa

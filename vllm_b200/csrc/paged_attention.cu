@@ -466,7 +466,9 @@ enum class Scratch {
               // slots per (sequence, head), not tied to 512 tokens; nothing else is used
 };
 
-static int attention_entry(const b200pa_attn_args* a, void* stream, Scratch mode) {
+// `share`: the call may use one `share`-th of the stream's workspace and arrival counters (another
+// launch that may run at the same time has the rest).
+static int attention_entry(const b200pa_attn_args* a, void* stream, Scratch mode, int share = 1) {
   const bool v2 = mode != Scratch::kNone;
   B200PA_CHECK_ARG(a != nullptr, "args is NULL");
   B200PA_CHECK_ARG(a->num_seqs >= 0 && a->num_heads > 0 && a->num_kv_heads > 0 && a->head_size > 0,
@@ -643,7 +645,7 @@ static int attention_entry(const b200pa_attn_args* a, void* stream, Scratch mode
     // the unit table lives in shared memory (4 bytes per sequence) and the merge needs one
     // arrival counter per (sequence, head); batches beyond either have more than enough
     // sequences to fill the GPU unsplit
-    const bool can_split = table_full <= 48 * 1024 && units_hs <= kArrivePerRegion &&
+    const bool can_split = table_full <= 48 * 1024 && units_hs <= kArrivePerRegion / share &&
                            pages_max > min_chunk && stream_region(s, &region);
     bool own_ws = false;
     if (!can_split) {
@@ -657,7 +659,7 @@ static int attention_entry(const b200pa_attn_args* a, void* stream, Scratch mode
       const int p_cap = tune.max_parts ? tune.max_parts : 128;
       // what the stream's region of the library workspace can hold
       const int64_t per_slot = int64_t(p.num_seqs) * p.num_heads * (8 + int64_t(a->head_size) * 2);
-      int64_t p_ws = (int64_t(region.ws_bytes) - 3 * 256) / std::max<int64_t>(per_slot, 1);
+      int64_t p_ws = (int64_t(region.ws_bytes / share) - 3 * 256) / std::max<int64_t>(per_slot, 1);
       p_ws = std::min<int64_t>({p_ws, int64_t(p_cap), pages_max / min_chunk + 2});
       if (tune.no_split || mode == Scratch::kOwnArray) p_ws = 0;
       const int64_t p_caller = split ? std::min<int64_t>(a->max_num_partitions, p_cap) : 0;
@@ -762,6 +764,10 @@ static int attention_entry(const b200pa_attn_args* a, void* stream, Scratch mode
     }
   }
   return B200PA_OK;
+}
+
+int attention_half_region(const b200pa_attn_args* a, void* stream) {
+  return attention_entry(a, stream, Scratch::kNone, 2);
 }
 
 }  // namespace b200pa

@@ -63,6 +63,8 @@ struct PrefillParams {
   int block_size;
   int max_blocks_per_seq;
   int ws_slots;               // pieces that the workspace has room for
+  int late_wait;              // 1: independent of the launch in front, waits for it at the end only (the launch in
+                              // front has itself waited for all before it)
   float scale;
 };
 
@@ -161,7 +163,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
           make_uint4(0, 0, 0, 0);
     fence_proxy_async();
   }
-  grid_dependency();
+  if (p.late_wait) grid_launch_dependents(); else grid_dependency();
 
   // ---- plan.  T tokens fill a row tile; a request has ceil(q_len / (NQ T)) row-tile groups per kv
   // head, and each of them npieces pieces.
@@ -940,6 +942,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
     }
   }
 
+  if (p.late_wait) grid_dependency_wait();
   // ---- everything issued has been waited for by the softmax warpgroups (or a wait ran out)
   tc_fence_before();
   __syncthreads();

@@ -48,7 +48,7 @@ extern "C" int b200pa_paged_attention_varlen(const b200pa_attn_args* a, const in
     // the decode rows are the first rows of query and out: an ordinary decode batch
     b200pa_attn_args d = *a;
     d.num_seqs = num_decodes;
-    const int rc = b200pa_paged_attention_v1(&d, stream);
+    const int rc = reqs > 0 ? attention_half_region(&d, stream) : b200pa_paged_attention_v1(&d, stream);
     if (rc != B200PA_OK) return rc;
   }
   if (reqs == 0) return B200PA_OK;
@@ -73,13 +73,20 @@ extern "C" int b200pa_paged_attention_varlen(const b200pa_attn_args* a, const in
   p.scale = a->scale;
   StreamRegion region{};
   if (stream_region(s, &region)) {  // (without one the keys of an item are not split)
-    p.ws = region.ws;
-    p.arrive = region.arrive;
-    p.ws_slots = int(std::min<int64_t>(int64_t(region.ws_bytes) / ki.piece_bytes, kArrivePerRegion / 8));
+    // (the second half: the first belongs to the decode launch, which may still be running)
+    p.ws = region.ws + region.ws_bytes / 2;
+    p.arrive = region.arrive + kArrivePerRegion / 2;
+    p.ws_slots = int(std::min<int64_t>(int64_t(region.ws_bytes / 2) / ki.piece_bytes, kArrivePerRegion / 16));
+    if (num_decodes == 0) {
+      p.ws = region.ws;
+      p.ws_slots = int(std::min<int64_t>(int64_t(region.ws_bytes) / ki.piece_bytes, kArrivePerRegion / 16));
+    }
   }
   p.status = device_status_ptr();
   for (int r = num_decodes; r < a->num_seqs; r += kPrefillMaxReqs) {
     p.num_reqs = std::min(kPrefillMaxReqs, a->num_seqs - r);
+    // nothing here depends on the decode launch: start where its CTAs have left, wait for it at the end
+    p.late_wait = r == num_decodes && num_decodes > 0 ? 1 : 0;
     p.block_tables = a->block_tables + int64_t(r) * a->max_num_blocks_per_seq;
     p.seq_lens = a->seq_lens + r;
     p.q_start = query_start_loc + r;
