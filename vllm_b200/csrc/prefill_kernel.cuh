@@ -175,8 +175,8 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
   auto tiles_of = [&](int len) { return (max(len, 0) + KT - 1) / KT; };
   {
     // groups and key tiles of all requests: with fewer than four groups per SM the groups are cut
-    // into pieces of about half an SM's share of the key tiles (at least four tiles: a piece costs
-    // a Q load, a pipeline fill and a partial)
+    // into pieces of an SM's share of the key tiles, but of no less than 768 keys: a piece costs a Q
+    // load, a pipeline fill, a partial and its merge, about as much as 350 keys
     int groups = 0, work = 0, most = 0;
     for (int r = tid; r < S; r += kPrefillThreads) {
       const int ql = q_len_of(r);
@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
     const int64_t all_work = int64_t(work) * HK, all_groups = int64_t(groups) * HK;
     split_tiles = INT32_MAX;
     if (all_groups < 4 * int64_t(gridDim.x)) {
-      int64_t c = max(int64_t(4), (all_work + 2 * int64_t(gridDim.x) - 1) / (2 * int64_t(gridDim.x)));
+      const int64_t c = max(int64_t(768 / KT), (all_work + gridDim.x - 1) / int64_t(gridDim.x));
       // every piece needs a slot of the workspace: a group of n tiles has at most n / c + 1 pieces
       const int64_t room = p.ws_slots - all_groups;
       if (room > 0) split_tiles = int(min(max(c, int64_t(most) * HK / room + 1), int64_t(INT32_MAX)));
