@@ -68,7 +68,7 @@ __global__ void pa_reduce_kernel(QT* __restrict__ out, const QT* __restrict__ tm
 
 // ------------------------------------------------------------------ generic decode
 // Fallback for every combination the tensor-core kernel is not built for
-// (fp32 tensors, head size 120, block size 8, unaligned strides, G > 32).
+// (fp32 tensors, block size 8, unaligned strides, block-sparse patterns).
 // One warp per (head, sequence, partition); fp32 math throughout.
 template <typename CT, int KV>
 __device__ __forceinline__ float cache_to_f32(CT v) {

@@ -316,8 +316,8 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
     uint32_t n_s = 0, n_pv = 0;  // S tiles received, PV products issued for this row tile
 
     // Each warp brings its own 32 rows: eight rows and four 16-byte granules at a time, 64-byte pieces
-    // of global memory into 128-byte runs of the operand layout.  (One row per thread: 8000 cycles
-    // an item instead of ~2000.)
+    // of global memory into 128-byte runs of the operand layout.  (One row per thread took 8000 cycles
+    // an item at head size 128.)
     // Only for a row tile that has key tiles in this item: a warpgroup without work may be items ahead
     // of the MMAs, and must not complete a phase of q_full that they have not waited for.
     auto load_q = [&](const PrefillItem& it) {
