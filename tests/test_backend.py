@@ -173,3 +173,14 @@ def test_prefill_chunk_and_decode_session(kv_cache_dtype):
             tol = dict(atol=2e-2, rtol=2e-2) if kv_cache_dtype == "fp8" else dict(atol=1e-2, rtol=1e-2)
             torch.testing.assert_close(got, want, **tol)
             off += ln
+
+
+def test_steps_for_capture_are_not_divided_by_a_host_number():
+    b = B200PagedAttentionMetadataBuilder(16, [], None, "cpu")
+    qsl = torch.arange(9, dtype=torch.int32)  # a dummy run: eight requests of one token, chunks allowed
+    common = types.SimpleNamespace(
+        query_start_loc=qsl, query_start_loc_cpu=qsl, seq_lens=torch.full((8,), 9, dtype=torch.int32),
+        num_reqs=8, num_actual_tokens=8, max_query_len=8, max_seq_len=64,
+        block_table_tensor=torch.zeros(8, 4, dtype=torch.int32), slot_mapping=torch.zeros(8, dtype=torch.int64))
+    assert b.build(0, common).num_decodes == 8
+    assert b.build_for_cudagraph_capture(common).num_decodes == 0

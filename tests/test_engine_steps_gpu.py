@@ -1,0 +1,138 @@
+"""Whole engine steps through the backend (KV write and attention in one call) at the places where a
+step is divided between kernels: captured steps replayed with other batches, decodes beside chunks on
+either stream, the native step against the operators one by one."""
+import types
+
+import numpy as np
+import pytest
+import torch
+
+from test_prefill_gpu import _gather
+from vllm_b200.backend import (B200PagedAttentionBackend, B200PagedAttentionImpl,
+                               B200PagedAttentionMetadataBuilder)
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+class Engine:
+    """Static buffers for up to `reqs` requests and `tokens` tokens, and a cache full of old tokens."""
+
+    def __init__(self, reqs, tokens, H=8, HK=2, D=128, B=16, max_blocks=40, kv="auto", alibi=False, seed=0):
+        self.H, self.HK, self.D, self.B, self.kv = H, HK, D, B, kv
+        self.rng = np.random.default_rng(seed)
+        self.gen = torch.Generator(device=DEV).manual_seed(seed)
+        self.dtype = torch.bfloat16
+        self.scale = 0.02 if kv != "auto" else 1.0
+        self.nb = reqs * max_blocks + 1
+        shape = B200PagedAttentionBackend.get_kv_cache_shape(self.nb, B, HK, D, kv)
+        old = torch.randn(shape, generator=self.gen, device=DEV)
+        if kv == "auto":
+            self.cache = old.to(self.dtype)
+        else:
+            t = torch.float8_e5m2 if kv == "fp8_e5m2" else torch.float8_e4m3fn
+            self.cache = (old / self.scale).clamp(-448, 448).to(t).view(torch.uint8)
+        del old
+        self.q, self.k, self.v = (self._randn(tokens, h, D) for h in (H, HK, HK))
+        self.out = torch.zeros(tokens, H * D, dtype=self.dtype, device=DEV)
+        self.qsl = torch.zeros(reqs + 1, dtype=torch.int32, device=DEV)
+        self.lens = torch.zeros(reqs, dtype=torch.int32, device=DEV)
+        self.table = torch.zeros(reqs, max_blocks, dtype=torch.int32, device=DEV)
+        self.slots = torch.full((tokens,), -1, dtype=torch.int64, device=DEV)
+        slopes = [2.0 ** (-(i + 1) / 2) for i in range(H)] if alibi else None
+        self.impl = B200PagedAttentionImpl(H, D, D ** -0.5, HK, alibi_slopes=slopes, kv_cache_dtype=kv)
+        self.builder = B200PagedAttentionMetadataBuilder(types.SimpleNamespace(block_size=B), ["l"], None, DEV)
+        scale = torch.tensor(self.scale, dtype=torch.float32, device=DEV)
+        self.layer = types.SimpleNamespace(_k_scale=scale, _v_scale=scale)
+
+    def _randn(self, *shape):
+        return torch.randn(*shape, generator=self.gen, device=DEV).to(self.dtype)
+
+    def load(self, new, ctx):
+        """Fills the buffers with a batch; the requests behind it bring no token."""
+        self.new, self.ctx = np.array(new), np.array(ctx)
+        n, r = int(self.new.sum()), len(new)
+        for t in (self.q, self.k, self.v):
+            t.copy_(self._randn(*t.shape))
+        table = self.rng.permutation(self.nb - 1)[: self.table.numel()].reshape(self.table.shape) + 1
+        self.table.copy_(torch.from_numpy(table.astype(np.int32)))
+        offsets = np.full(self.qsl.numel(), n, np.int32)
+        offsets[: r + 1] = np.concatenate([[0], np.cumsum(self.new)])
+        lens = np.zeros(self.lens.numel(), np.int32)
+        lens[:r] = self.new + self.ctx
+        slots = np.full(self.slots.numel(), -1, np.int64)
+        seq = np.repeat(np.arange(r), self.new)
+        pos = np.concatenate([np.arange(c, c + t) for t, c in zip(new, ctx)])
+        slots[:n] = table[seq, pos // self.B] * self.B + pos % self.B
+        self.qsl.copy_(torch.from_numpy(offsets))
+        self.lens.copy_(torch.from_numpy(lens))
+        self.slots.copy_(torch.from_numpy(slots))
+        self.out.fill_(float("nan"))
+
+    def common(self, max_query_len=None, max_seq_len=None, tokens=None):
+        qsl = self.qsl.cpu()
+        return types.SimpleNamespace(
+            query_start_loc=self.qsl, query_start_loc_cpu=qsl, seq_lens=self.lens, seq_lens_cpu=self.lens.cpu(),
+            num_reqs=self.lens.numel(), num_actual_tokens=tokens or int(qsl[-1]),
+            max_query_len=max_query_len or int(qsl.diff().max()),
+            max_seq_len=max_seq_len or int(self.lens.max()), block_table_tensor=self.table,
+            slot_mapping=self.slots, causal=True)
+
+    def forward(self, metadata):
+        self.impl.forward(self.layer, self.q, self.k, self.v, self.cache, metadata, output=self.out)
+
+    def check(self):
+        """The rows of the loaded batch against dense attention in fp32 over what the cache holds."""
+        torch.cuda.synchronize()
+        H, HK, D, g = self.H, self.HK, self.D, self.H // self.HK
+        x = 16 // self.cache.element_size()
+        kc = self.cache[0].view(self.nb, HK, D // x, self.B, x)
+        vc = self.cache[1].view(self.nb, HK, D, self.B)
+        slopes = self.impl.alibi_slopes
+        off = 0
+        for r, (t, c) in enumerate(zip(self.new, self.ctx)):
+            if t == 0:
+                continue
+            k, v = _gather(kc, vc, self.table[r], int(t + c), self.kv, self.scale)
+            if self.kv == "auto":
+                assert torch.equal(k[c:], self.k[off:off + t].float())
+            qq = self.q[off:off + t].float().view(t, HK, g, D)
+            s = torch.einsum("tkgd,lkd->kgtl", qq, k) * D ** -0.5
+            pos, key = torch.arange(c, c + t, device=DEV).view(-1, 1), torch.arange(c + t, device=DEV).view(1, -1)
+            if slopes is not None:
+                s = s + slopes.to(DEV).view(HK, g, 1, 1) * (key - pos).float()
+            s = s.masked_fill(key > pos, float("-inf"))
+            want = torch.einsum("kgtl,lkd->tkgd", torch.softmax(s, -1), v).reshape(t, H * D)
+            got = self.out[off:off + t].float()
+            # (P and the result are rounded to 16 bits: 2^-9 each, and 2^-9 of partials that were cut)
+            assert (got - want).norm() < 6e-3 * want.norm(), (r, t, c)
+            torch.testing.assert_close(got, want, atol=2e-2, rtol=2e-2)
+            off += t
+        from vllm_b200 import capi
+        assert capi.device_status() == 0
+
+
+def _capture(e, metadata):
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        e.forward(metadata)
+    torch.cuda.current_stream().wait_stream(s)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        e.forward(metadata)
+    return g
+
+
+@pytest.mark.parametrize("kv", ["auto", "fp8"])
+@pytest.mark.parametrize("for_capture", [True, False], ids=["build_for_cudagraph_capture", "build"])
+def test_a_captured_step_is_replayed_with_other_divisions_of_its_tokens(kv, for_capture):
+    e = Engine(8, 8, kv=kv)
+    e.load([1] * 8, [20 * i for i in range(8)])
+    common = e.common(max_query_len=8, max_seq_len=640)  # as an engine's dummy run has it
+    g = _capture(e, e.builder.build_for_cudagraph_capture(common) if for_capture else e.builder.build(0, common))
+    for new, ctx in (([1, 1, 4, 1, 1], [300, 5, 77, 0, 500]), ([8], [600]), ([1] * 8, [40 * i for i in range(8)]),
+                     ([3, 1, 1, 1, 2], [0, 17, 128, 255, 31]), ([1, 0, 7], [9, 0, 3])):
+        e.load(new, ctx)
+        g.replay()
+        e.check()

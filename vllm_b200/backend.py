@@ -121,6 +121,8 @@ class B200PagedAttentionMetadataBuilder:
         captured launch is cheap (rocm_attn.py:84-99 does the same)."""
         md = self.build(0, common_attn_metadata)
         md.seq_lens.fill_(1)
+        if md.max_query_len > 1:
+            md.num_decodes = 0  # (a host number: the replayed batches are divided otherwise)
         return md
 
 
@@ -167,9 +169,15 @@ class B200PagedAttentionImpl:
         alibi = self.alibi_slopes
         if alibi is not None and alibi.device != query.device:
             alibi = self.alibi_slopes = alibi.to(query.device)
+        # A captured step is replayed with other batches of its token count: what is cut off by a host
+        # number at capture must hold for all of them.  The prefill kernel divides the step by the
+        # offsets and lengths on the device, single tokens among them.
+        num_decodes = md.num_decodes
+        if md.max_query_len > 1 and torch.cuda.is_current_stream_capturing():
+            num_decodes = 0
         if ops.attention_step(
                 output, query, key, value, kv_cache, md.block_table, md.seq_lens, md.slot_mapping,
-                md.query_start_loc, layer._k_scale, layer._v_scale, alibi, n, md.num_decodes,
+                md.query_start_loc, layer._k_scale, layer._v_scale, alibi, n, num_decodes,
                 md.max_query_len, md.max_seq_len, self.num_heads, self.num_kv_heads, self.head_size,
                 self.scale, self.kv_cache_dtype, self.kv_sharing_target_layer_name is None):
             return output
@@ -186,7 +194,7 @@ class B200PagedAttentionImpl:
         elif ops.paged_attention_varlen(
                 output[:n].view(n, self.num_heads, self.head_size), q, key_cache, value_cache,
                 self.num_kv_heads, self.scale, attn_metadata.block_table, attn_metadata.seq_lens,
-                attn_metadata.query_start_loc, attn_metadata.num_decodes, value_cache.shape[3],
+                attn_metadata.query_start_loc, num_decodes, value_cache.shape[3],
                 attn_metadata.max_seq_len, alibi, self.kv_cache_dtype, layer._k_scale, layer._v_scale):
             return output
         else:
