@@ -184,3 +184,17 @@ def test_steps_for_capture_are_not_divided_by_a_host_number():
         block_table_tensor=torch.zeros(8, 4, dtype=torch.int32), slot_mapping=torch.zeros(8, dtype=torch.int64))
     assert b.build(0, common).num_decodes == 8
     assert b.build_for_cudagraph_capture(common).num_decodes == 0
+
+
+def test_the_engine_is_asked_to_put_decodes_in_front():
+    """The split of a step counts the leading single-token requests: without the order that the
+    threshold asks for, a chunk in front leaves the decode kernels none."""
+    from vllm_b200.backend import leading_decodes
+    threshold = B200PagedAttentionMetadataBuilder.reorder_batch_threshold
+    assert threshold == 1
+    new = [5, 1, 1, 40, 1]
+    in_order = sorted(new, key=lambda t: t > threshold)  # (stable: decodes, then the others)
+
+    def count(q):
+        return leading_decodes(torch.tensor([0] + list(np.cumsum(q)), dtype=torch.int32))
+    assert count(new) == 0 and count(in_order) == 3
