@@ -191,6 +191,13 @@ int b200pa_paged_attention_v2(const b200pa_attn_args* args, void* stream);
 int b200pa_paged_attention_v2_noalloc(const b200pa_attn_args* args, void* stream);
 
 /*
+ * Which kernel a call of paged_attention_v1 / v2 with these sizes, types, strides and alignments runs
+ * on; launches nothing and reads no tensor.  *cluster: 1 to 16, the direct kernel with that many CTAs
+ * per (sequence, kv head, head group); 0, the persistent kernel; -1, the generic kernel.
+ */
+int b200pa_decode_route(const b200pa_attn_args* args, int32_t* cluster);
+
+/*
  * Attention of an engine step: request r brings the query rows
  * [query_start_loc[r], query_start_loc[r+1]) of `query` and `out`, the last positions of its
  * sequence, and each of them attends to the cached positions up to its own (causal).  The step's

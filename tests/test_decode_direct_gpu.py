@@ -50,6 +50,12 @@ def test_head_size_120_large_batch():
           "v1", seqs=range(0, 200, 17))
 
 
+@pytest.mark.parametrize("lens", [[32000], [20000, 31999, 7, 513]])
+def test_head_size_120_long_sequences(lens):
+    for heads in ((8, 2), (24, 2)):
+        check(_workload(lens, *heads, 120, 16, torch.bfloat16, "auto"), "v2")
+
+
 def test_lse_and_stale_nans():
     w = _workload([129, 40], 8, 2, 128, 16, torch.bfloat16, "auto")
     for s, n in enumerate((129, 40)):

@@ -1,0 +1,30 @@
+"""The rules that pick a kernel for a call, asked on the host (no GPU: a chip of 148 SMs is assumed)."""
+import pytest
+
+from vllm_b200 import capi
+
+
+def _route(seqs, heads, kv_heads, head_size, max_len, kv=0, dtype=capi.BF16, block=16):
+    a = capi.AttnArgs()
+    a.num_seqs, a.num_heads, a.num_kv_heads, a.head_size = seqs, heads, kv_heads, head_size
+    a.block_size, a.max_seq_len, a.kv_dtype, a.q_dtype = block, max_len, kv, dtype
+    a.q_stride = heads * head_size
+    a.kv_head_stride, a.kv_block_stride = head_size * block, kv_heads * head_size * block
+    return capi.decode_route(a)
+
+
+@pytest.mark.parametrize("seqs,max_len", [(1, 32000), (4, 32000), (1, 131072)])
+def test_head_size_120_keeps_its_cluster_however_long_the_sequences_are(seqs, max_len):
+    # only the direct kernel is built for it: as many CTAs as for sequences where it is the better one
+    assert _route(seqs, 32, 8, 120, max_len) == _route(seqs, 32, 8, 120, 2048) > 1
+
+
+def test_head_size_120_long_sequences_fill_one_wave():
+    # 256 items: a cluster of 2 each would be 512 CTAs for 444 places
+    assert _route(64, 4, 4, 120, 8000) == 1 and _route(32, 4, 4, 120, 8000) == 2
+
+
+def test_head_sizes_with_both_kernels_leave_long_sequences_to_the_persistent_one():
+    assert _route(1, 32, 8, 128, 32000) == 0
+    assert _route(1, 32, 8, 128, 1500) > 1
+    assert _route(1, 32, 8, 128, 1500, dtype=capi.F32) == -1

@@ -88,6 +88,7 @@ def lib() -> C.CDLL:
             getattr(l, name).argtypes = [C.POINTER(CacheArgs), C.c_void_p]
         l.b200pa_convert_fp8.argtypes = [C.c_void_p, C.c_void_p, C.c_int64, C.c_float, C.c_int32,
                                          C.c_int32, C.c_int32, C.c_void_p]
+        l.b200pa_decode_route.argtypes = [C.POINTER(AttnArgs), C.POINTER(C.c_int32)]
         l.b200pa_device_status.argtypes = [C.POINTER(C.c_int32)]
         _lib = l
     return _lib
@@ -118,6 +119,14 @@ def paged_attention_v2_noalloc(args: AttnArgs, stream: int = 0) -> None:
     """v2 with the split-KV scratch taken from a 32 MiB array built into the library (allocates
     nothing; limits and sharing rules in b200pa.h)."""
     check(lib().b200pa_paged_attention_v2_noalloc(C.byref(args), C.c_void_p(stream)))
+
+
+def decode_route(args: AttnArgs) -> int:
+    """The kernel that a decode call runs on: CTAs per cluster of the direct kernel, 0 for the
+    persistent one, -1 for the generic one (see b200pa.h)."""
+    v = C.c_int32(0)
+    check(lib().b200pa_decode_route(C.byref(args), C.byref(v)))
+    return v.value
 
 
 def reshape_and_cache(args: CacheArgs, stream: int = 0) -> None:

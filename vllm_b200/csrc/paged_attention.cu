@@ -382,12 +382,19 @@ static DirectKernelInfo find_direct(int d, int qdt, int kv, int gp) {
                  : d <= 128 ? find_direct_mid(d, qdt, kv, gp) : find_direct_large(d, qdt, kv, gp);
 }
 
-// CTAs per cluster for the direct kernel, or 0 when the persistent kernel is the better one.  Only
-// the bound on the lengths is known here.  Measured on B200, persistent / direct, us: 1 sequence of
-// 1500 (32 / 8 heads of 128, bf16) 21.2 / 7.4, of 8000 23.8 / 15.4, of 32000 37.8 / 44.8; 8 sequences
-// up to 1024 (32 heads) 22.7 / 20.5; 16 up to 4096 37.2 / 34.0; 16 up to 2000 with 16 heads on one kv
-// head 41.7 / 9.8; 256 up to 800 76.9 / 73.3; 600 up to 80 (40 heads) 117.7 / 206.
-static int direct_plan(const DirectKernelInfo& ki, int64_t items, int max_seq_len, const Tuning& tune) {
+// CTAs per cluster for the direct kernel, and whether it is the better one where the persistent kernel
+// is built too.  Only the bound on the lengths is known here.  Measured on B200, persistent / direct,
+// us: 1 sequence of 1500 (32 / 8 heads of 128, bf16) 21.2 / 7.4, of 8000 23.8 / 15.4, of 32000
+// 37.8 / 44.8; 8 sequences up to 1024 (32 heads) 22.7 / 20.5; 16 up to 4096 37.2 / 34.0; 16 up to 2000
+// with 16 heads on one kv head 41.7 / 9.8; 256 up to 800 76.9 / 73.3; 600 up to 80 (40 heads) 117.7 / 206.
+// Head size 120, which has no persistent kernel, us in a CTA each / in clusters (32 / 8 heads): 1
+// sequence of 32000 528 / 49, 4 533 / 94, 16 of 8000 147 / 94.
+struct DirectPlan {
+  int cluster;
+  bool preferred;
+};
+
+static DirectPlan direct_plan(const DirectKernelInfo& ki, int64_t items, int max_seq_len, const Tuning& tune) {
   const int64_t slots = int64_t(sm_count()) * ki.ctas_per_sm;
   const int64_t tiles = (int64_t(std::max(max_seq_len, 1)) + 15) / 16;
   // as many CTAs as the GPU takes at once (a fifth more: short sequences make room early), but no
@@ -397,13 +404,17 @@ static int direct_plan(const DirectKernelInfo& ki, int64_t items, int max_seq_le
   while (cluster < 8 && items * cluster * 10 <= slots * 6 && cluster * kDirectWarps < tiles) cluster *= 2;
   if (cluster == 8 && items <= 8 && tiles >= 128) cluster = 16;
   if (tune.cluster) cluster = tune.cluster;
-  if (tune.direct == 1) return cluster;
+  if (tune.direct == 1) return {cluster, true};
   // A tile costs a warp about 1 us whatever else runs, a CTA 4 us besides; the persistent kernel
   // pays about 15 us once.
   const int64_t per_warp = (tiles + cluster * kDirectWarps - 1) / (cluster * kDirectWarps);
   const int64_t ctas = items * cluster;
-  if (ctas * 10 <= slots * 12) return per_warp <= 20 ? cluster : 0;
-  return ctas <= 5 * slots && per_warp >= 3 && per_warp <= 16 ? cluster : 0;
+  if (ctas * 10 <= slots * 12 ? per_warp <= 20 : ctas <= 5 * slots && per_warp >= 3 && per_warp <= 16)
+    return {cluster, true};
+  // Head size 120 stays here all the same.  With many tiles to a warp a second wave of a few CTAs costs
+  // as much as the first: 64 sequences of 8000 (4 heads) take 207 us in clusters of 2, 176 us one by one.
+  while (cluster > 1 && items * cluster > slots) cluster /= 2;
+  return {cluster, false};
 }
 
 template <typename QT>
@@ -455,6 +466,46 @@ static bool force_generic() {
     v = (e && e[0] == '1') ? 1 : 0;
   }
   return v == 1;
+}
+
+// Which kernel a decode call runs on.
+struct Route {
+  DecodeKernelInfo persistent{nullptr, 0, 1};  // fn: built for this call
+  DirectLaunchFn direct = nullptr;
+  int cluster = 0;      // > 0: the direct kernel, in clusters of this many CTAs
+  int head_tiles = 1;   // of 8 query heads per work item
+  int head_groups = 1;  // work items per (sequence, kv head)
+};
+
+static Route decode_route(const b200pa_attn_args& a, bool split, const Tuning& tune) {
+  Route r;
+  const int group = a.num_heads / a.num_kv_heads;
+  const int gp = group <= 8 ? 1 : 2;
+  r.head_tiles = gp;
+  r.head_groups = (group + 8 * gp - 1) / (8 * gp);
+  const int es = a.kv_dtype == B200PA_KV_AUTO ? 2 : 1;
+  auto aligned = [](const void* ptr, uintptr_t n) { return reinterpret_cast<uintptr_t>(ptr) % n == 0; };
+  // block-sparse attention (unused by any in-tree caller of the reference) runs on the
+  // generic kernel only
+  const bool fast = !force_generic() && a.blocksparse_vert_stride <= 1 && a.q_dtype != B200PA_F32 &&
+                    (a.block_size == 16 || a.block_size == 32) &&
+                    aligned(a.key_cache, 16) && aligned(a.value_cache, 16) && aligned(a.query, 16) &&
+                    aligned(a.out, 16) && (!split || aligned(a.tmp_out, 16)) &&
+                    (a.kv_block_stride * es) % 16 == 0 && (a.kv_head_stride * es) % 16 == 0 &&
+                    a.q_stride % 8 == 0;
+  if (!fast) return r;
+  r.persistent = find_decode(a.head_size, a.q_dtype, a.kv_dtype, gp, a.block_size / 16);
+  if (tune.direct == 2) return r;
+  const DirectKernelInfo di = find_direct(a.head_size, a.q_dtype, a.kv_dtype, gp);
+  if (di.fn == nullptr) return r;
+  const int64_t items = int64_t(a.num_seqs) * a.num_kv_heads * r.head_groups;
+  const DirectPlan plan = direct_plan(di, items, a.max_seq_len, tune);
+  // small batches, and every batch of a head size that only the direct kernel is built for (120)
+  if ((plan.preferred || r.persistent.fn == nullptr) && items * plan.cluster < INT32_MAX) {
+    r.direct = di.fn;
+    r.cluster = plan.cluster;
+  }
+  return r;
 }
 
 // How an attention call may use scratch memory.
@@ -569,46 +620,29 @@ static int attention_entry(const b200pa_attn_args* a, void* stream, Scratch mode
   p.bs_block_size = a->blocksparse_block_size;
   p.bs_head_sliding_step = a->blocksparse_head_sliding_step;
 
-  // ---- can the tensor-core kernel take it?
+  const Route route = decode_route(*a, split, tune);
+  const DecodeKernelInfo ki = route.persistent;
+  const DecodeLaunchFn fn = ki.fn;
   const int es = a->kv_dtype == B200PA_KV_AUTO ? 2 : 1;
-  auto aligned = [](const void* ptr, uintptr_t n) { return reinterpret_cast<uintptr_t>(ptr) % n == 0; };
-  const int gp = p.group <= 8 ? 1 : 2;
-  DecodeKernelInfo ki{nullptr, 0, 1};
-  // block-sparse attention (unused by any in-tree caller of the reference) runs on the
-  // generic kernel only
-  bool fast = !force_generic() && !sparse && a->q_dtype != B200PA_F32 &&
-              (a->block_size == 16 || a->block_size == 32) &&
-              aligned(a->key_cache, 16) && aligned(a->value_cache, 16) && aligned(a->query, 16) &&
-              aligned(a->out, 16) && (!split || aligned(a->tmp_out, 16)) &&
-              (a->kv_block_stride * es) % 16 == 0 && (a->kv_head_stride * es) % 16 == 0 &&
-              a->q_stride % 8 == 0;
-  if (fast) ki = find_decode(a->head_size, a->q_dtype, a->kv_dtype, gp, a->block_size / 16);
-  DecodeLaunchFn fn = ki.fn;
+  const int gp = route.head_tiles;
   int rc;
   bool fused = false;
-  if (fast && tune.direct != 2) {
-    // small batches: the latency-bound form (and head size 120, which only it is built for)
-    const DirectKernelInfo di = find_direct(a->head_size, a->q_dtype, a->kv_dtype, gp);
-    const int head_groups = (p.group + 8 * gp - 1) / (8 * gp);
-    const int64_t items = int64_t(p.num_seqs) * p.num_kv_heads * head_groups;
-    int cluster = di.fn == nullptr ? 0 : direct_plan(di, items, a->max_seq_len, tune);
-    if (di.fn != nullptr && fn == nullptr) cluster = std::max(cluster, 1);
-    if (cluster > 0 && items * cluster < INT32_MAX) {
-      p.head_groups = head_groups;
-      // (lengths beyond what the caller's scratch was sized for are ignored, see below)
-      if (split && mode == Scratch::kCaller)
-        p.len_cap = int(std::min<int64_t>(int64_t(a->max_num_partitions) * kPartitionTokens, INT32_MAX));
-      const cudaError_t e = di.fn(p, int(items), cluster, s);
-      count_launch();
-      if (e != cudaSuccess) {
-        set_error("direct decode kernel launch failed: %s", cudaGetErrorString(e));
-        return B200PA_ECUDA;
-      }
-      return B200PA_OK;
+  if (route.cluster > 0) {
+    p.head_groups = route.head_groups;
+    // (lengths beyond what the caller's scratch was sized for are ignored, see below)
+    if (split && mode == Scratch::kCaller)
+      p.len_cap = int(std::min<int64_t>(int64_t(a->max_num_partitions) * kPartitionTokens, INT32_MAX));
+    const int64_t items = int64_t(p.num_seqs) * p.num_kv_heads * p.head_groups;
+    const cudaError_t e = route.direct(p, int(items), route.cluster, s);
+    count_launch();
+    if (e != cudaSuccess) {
+      set_error("direct decode kernel launch failed: %s", cudaGetErrorString(e));
+      return B200PA_ECUDA;
     }
+    return B200PA_OK;
   }
   if (fn != nullptr) {
-    p.head_groups = (p.group + 8 * gp - 1) / (8 * gp);
+    p.head_groups = route.head_groups;
     const size_t page_bytes = size_t(a->head_size) * a->block_size * es;
     // Ring geometry.  Warps hide the latency of the per-page instruction chain, ring slots
     // the latency of HBM; measured on B200 the first matters more and a shallow ring (about
@@ -778,6 +812,16 @@ extern "C" int b200pa_paged_attention_v1(const b200pa_attn_args* args, void* str
 
 extern "C" int b200pa_paged_attention_v2(const b200pa_attn_args* args, void* stream) {
   return b200pa::attention_entry(args, stream, b200pa::Scratch::kCaller);
+}
+
+extern "C" int b200pa_decode_route(const b200pa_attn_args* args, int32_t* cluster) {
+  using namespace b200pa;
+  B200PA_CHECK_ARG(args != nullptr && cluster != nullptr, "args or cluster is NULL");
+  B200PA_CHECK_ARG(args->num_heads > 0 && args->num_kv_heads > 0 && args->num_heads % args->num_kv_heads == 0,
+                   "bad sizes: num_heads=%d num_kv_heads=%d", args->num_heads, args->num_kv_heads);
+  const Route r = decode_route(*args, args->max_num_partitions > 1, tuning());
+  *cluster = r.cluster > 0 ? r.cluster : r.persistent.fn != nullptr ? 0 : -1;
+  return B200PA_OK;
 }
 
 // ------------------------------------------------------------------ v2 without caller scratch
