@@ -28,3 +28,19 @@ def test_head_sizes_with_both_kernels_leave_long_sequences_to_the_persistent_one
     assert _route(1, 32, 8, 128, 32000) == 0
     assert _route(1, 32, 8, 128, 1500) > 1
     assert _route(1, 32, 8, 128, 1500, dtype=capi.F32) == -1
+
+
+# (sequences, heads, kv heads, head size, longest, fp8 cache), where one of the two kernels took at least a
+# sixth longer on a B200 with all sequences equally long
+@pytest.mark.parametrize("call", [(32, 8, 8, 128, 2500, 1), (256, 8, 8, 128, 200, 1), (32, 8, 8, 80, 2500, 1),
+                                  (256, 32, 8, 80, 200, 1), (64, 32, 32, 96, 1000, 1), (32, 8, 8, 64, 2500, 0),
+                                  (32, 32, 8, 128, 2500, 0)])
+def test_batches_that_the_persistent_kernel_serves_faster(call):
+    assert _route(*call[:5], kv=call[5]) == 0
+
+
+@pytest.mark.parametrize("call", [(1, 32, 8, 128, 1500, 0), (8, 32, 32, 128, 1024, 0), (8, 32, 8, 64, 300, 1),
+                                  (16, 16, 1, 128, 2000, 0), (1, 8, 8, 32, 8000, 0), (64, 64, 4, 128, 300, 1),
+                                  (4, 32, 8, 256, 1000, 1), (32, 64, 4, 112, 2500, 0), (12, 32, 8, 128, 3000, 0)])
+def test_batches_that_the_direct_kernel_serves_faster(call):
+    assert _route(*call[:5], kv=call[5]) > 0

@@ -85,6 +85,8 @@ struct DirectShape {
   // tiles in flight per warp, and resident CTAs per SM that the register budget is set for
   static constexpr int kBufs = 2 * kTileRegs + kOtherRegs <= 120 ? 2 : 1;
   static constexpr int kMinCtas = kBufs * kTileRegs + kOtherRegs <= 128 ? 3 : 2;
+  // CTAs that fit (head size 32 and one head tile needs 117 registers, everything else more than 128)
+  static constexpr int kResident = D == 32 && GP == 1 ? 4 : kMinCtas;
 };
 
 // grid.x = (sequence, kv head, head group) items x cluster size.

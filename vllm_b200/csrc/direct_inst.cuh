@@ -9,7 +9,8 @@ using DirectLaunchFn = cudaError_t (*)(const DecodeParams&, int items, int clust
 
 struct DirectKernelInfo {
   DirectLaunchFn fn;
-  int ctas_per_sm;
+  int ctas_per_sm;  // that the register budget is set for
+  int resident;     // that fit in fact
 };
 
 template <typename QT, int KV, int D, int GP>
@@ -48,9 +49,13 @@ cudaError_t direct_launch(const DecodeParams& p, int items, int cluster, cudaStr
 
 template <typename QT, int KV, int D>
 DirectKernelInfo direct_gp(int gp) {
-  if (gp == 1) return {direct_launch<QT, KV, D, 1>, DirectShape<KV, D, 1>::kMinCtas};
-  if constexpr (D <= 128) return {direct_launch<QT, KV, D, 2>, DirectShape<KV, D, 2>::kMinCtas};
-  return {nullptr, 0};  // (two head tiles of a wide head do not fit the registers)
+  using S1 = DirectShape<KV, D, 1>;
+  if (gp == 1) return {direct_launch<QT, KV, D, 1>, S1::kMinCtas, S1::kResident};
+  if constexpr (D <= 128) {
+    using S2 = DirectShape<KV, D, 2>;
+    return {direct_launch<QT, KV, D, 2>, S2::kMinCtas, S2::kResident};
+  }
+  return {nullptr, 0, 0};  // (two head tiles of a wide head do not fit the registers)
 }
 
 template <typename QT, int D>
@@ -60,7 +65,7 @@ DirectKernelInfo direct_kv(int kv_dtype, int gp) {
     if (kv_dtype == B200PA_KV_FP8_E4M3) return direct_gp<QT, kCacheE4M3, D>(gp);
     if (kv_dtype == B200PA_KV_FP8_E5M2) return direct_gp<QT, kCacheE5M2, D>(gp);
   }
-  return {nullptr, 0};
+  return {nullptr, 0, 0};
 }
 
 // gp: 8-head tiles per work item (1 or 2)
@@ -68,7 +73,7 @@ template <int D>
 DirectKernelInfo find_direct_for(int q_dtype, int kv_dtype, int gp) {
   if (q_dtype == B200PA_BF16) return direct_kv<__nv_bfloat16, D>(kv_dtype, gp);
   if (q_dtype == B200PA_F16) return direct_kv<__half, D>(kv_dtype, gp);
-  return {nullptr, 0};
+  return {nullptr, 0, 0};
 }
 
 // Defined in direct_small.cu (32 .. 96), direct_mid.cu (112 .. 128), direct_large.cu (192, 256).

@@ -385,8 +385,8 @@ static DirectKernelInfo find_direct(int d, int qdt, int kv, int gp) {
 // CTAs per cluster for the direct kernel, and whether it is the better one where the persistent kernel
 // is built too.  Only the bound on the lengths is known here.  Measured on B200, persistent / direct,
 // us: 1 sequence of 1500 (32 / 8 heads of 128, bf16) 21.2 / 7.4, of 8000 23.8 / 15.4, of 32000
-// 37.8 / 44.8; 8 sequences up to 1024 (32 heads) 22.7 / 20.5; 16 up to 4096 37.2 / 34.0; 16 up to 2000
-// with 16 heads on one kv head 41.7 / 9.8; 256 up to 800 76.9 / 73.3; 600 up to 80 (40 heads) 117.7 / 206.
+// 37.8 / 44.8; 8 sequences up to 1024 (32 heads) 22.7 / 20.5; 16 up to 2000 with 16 heads on one kv head
+// 41.7 / 9.8; 256 up to 800 76.9 / 73.3; 600 up to 80 (40 heads) 117.7 / 206.
 // Head size 120, which has no persistent kernel, us in a CTA each / in clusters (32 / 8 heads): 1
 // sequence of 32000 528 / 49, 4 533 / 94, 16 of 8000 147 / 94.
 struct DirectPlan {
@@ -394,9 +394,10 @@ struct DirectPlan {
   bool preferred;
 };
 
-static DirectPlan direct_plan(const DirectKernelInfo& ki, int64_t items, int max_seq_len, const Tuning& tune) {
+static DirectPlan direct_plan(const DirectKernelInfo& ki, const b200pa_attn_args& a, int head_tiles, int64_t items,
+                              const Tuning& tune) {
   const int64_t slots = int64_t(sm_count()) * ki.ctas_per_sm;
-  const int64_t tiles = (int64_t(std::max(max_seq_len, 1)) + 15) / 16;
+  const int64_t tiles = (int64_t(std::max(a.max_seq_len, 1)) + 15) / 16;
   // as many CTAs as the GPU takes at once (a fifth more: short sequences make room early), but no
   // more warps than the longest sequence can have tiles.  Clusters of 16 are placed one to a GPC:
   // worth it for eight items at most, when it takes tiles off the warps.
@@ -405,16 +406,34 @@ static DirectPlan direct_plan(const DirectKernelInfo& ki, int64_t items, int max
   if (cluster == 8 && items <= 8 && tiles >= 128) cluster = 16;
   if (tune.cluster) cluster = tune.cluster;
   if (tune.direct == 1) return {cluster, true};
-  // A tile costs a warp about 1 us whatever else runs, a CTA 4 us besides; the persistent kernel
-  // pays about 15 us once.
   const int64_t per_warp = (tiles + cluster * kDirectWarps - 1) / (cluster * kDirectWarps);
   const int64_t ctas = items * cluster;
-  if (ctas * 10 <= slots * 12 ? per_warp <= 20 : ctas <= 5 * slots && per_warp >= 3 && per_warp <= 16)
-    return {cluster, true};
-  // Head size 120 stays here all the same.  With many tiles to a warp a second wave of a few CTAs costs
-  // as much as the first: 64 sequences of 8000 (4 heads) take 207 us in clusters of 2, 176 us one by one.
-  while (cluster > 1 && items * cluster > slots) cluster /= 2;
-  return {cluster, false};
+  if (ctas * 10 <= slots * 12 ? per_warp > 20 : ctas > 5 * slots || per_warp < 3 || per_warp > 16) {
+    // Head size 120 stays here all the same.  With many tiles to a warp a second wave of a few CTAs costs
+    // as much as the first: 64 sequences of 8000 (4 heads) take 207 us in clusters of 2, 176 us one by one.
+    while (cluster > 1 && items * cluster > slots) cluster /= 2;
+    return {cluster, false};
+  }
+  // What either kernel takes, us, if all sequences are as long as the bound.  Fitted to 4 000 launches
+  // (head sizes 32 to 256, both cache widths, six head counts, 1 to 400 sequences of 100 to 32000 tokens,
+  // all equal or uniform below the bound; 9 and 15 % rms):
+  //   direct       10, and for every wave of CTAs the tiles of a warp, one after the other: their
+  //                latency, or HBM where many warps load; 3 for each wave after the first
+  //   persistent   20, merges that grow with the heads of a kv head, the bytes at HBM's rate
+  // Shorter sequences than the bound favour the direct kernel when it has several waves (their CTAs make
+  // room) and the persistent one when it has one (the longest sequence decides).  Of 2115 equal batches that
+  // the size limits above let through, 144 were slower than on the persistent kernel by more than 10 %
+  // (worst: 32 sequences of 2500, 8 heads of 128, fp8, 45 against 55 us); with the estimate 25 are.
+  const double D = a.head_size, es = a.kv_dtype == B200PA_KV_AUTO ? 2 : 1, us = 1 / 6.5e6;  // (bytes to us)
+  const int64_t resident = int64_t(sm_count()) * ki.resident;
+  const double waves = double((ctas + resident - 1) / resident);
+  const double latency = (es == 1 ? 0.63 + 0.0037 * D : 0.43 + 0.0061 * D) * (head_tiles == 2 ? 1.4 : 1);
+  const double hbm = 0.85 * 32 * D * es * kDirectWarps * double(std::min(ctas, resident)) * us;
+  const double direct = 10 + waves * double(per_warp) * std::max(latency, hbm) + 3 * (waves - 1);
+  const double bytes = double(a.num_seqs) * a.num_kv_heads * a.max_seq_len * 2 * D * es;
+  const double persistent = 20 + 1.25 * (a.num_heads / a.num_kv_heads) + 0.89 * bytes * us * (waves > 1 ? 1 : 0.75);
+  const double margin = waves == 1 ? 1.1 : ctas * 10 <= resident * 12 ? 1.15 : 1.05;
+  return {cluster, direct <= margin * persistent};
 }
 
 template <typename QT>
@@ -499,7 +518,7 @@ static Route decode_route(const b200pa_attn_args& a, bool split, const Tuning& t
   const DirectKernelInfo di = find_direct(a.head_size, a.q_dtype, a.kv_dtype, gp);
   if (di.fn == nullptr) return r;
   const int64_t items = int64_t(a.num_seqs) * a.num_kv_heads * r.head_groups;
-  const DirectPlan plan = direct_plan(di, items, a.max_seq_len, tune);
+  const DirectPlan plan = direct_plan(di, a, gp, items, tune);
   // small batches, and every batch of a head size that only the direct kernel is built for (120)
   if ((plan.preferred || r.persistent.fn == nullptr) && items * plan.cluster < INT32_MAX) {
     r.direct = di.fn;
