@@ -138,3 +138,49 @@ def test_items_whose_second_row_tile_is_empty(kv, alibi):
 @pytest.mark.parametrize("kv", ["auto", "fp8"])
 def test_a_long_prompt(kv):
     _case([1500, 900], [700, 0], 8, 2, 128, 16, torch.bfloat16, kv)
+
+
+# The workspace has 496 slots for pieces on the first stream of a process, 62 on any other, half of them
+# beside a decode launch: what is cut has to fit, and what is not cut must not count.
+@pytest.mark.parametrize("decodes", [0, 5])
+@pytest.mark.parametrize("stream", ["first", "second"])
+@pytest.mark.parametrize("kv", ["auto", "fp8"])
+def test_long_contexts_are_cut_beside_many_whole_groups(kv, stream, decodes):
+    rng = np.random.default_rng(decodes)
+    q = np.concatenate([[1] * decodes, [16], rng.integers(2, 65, size=40), [9, 70], rng.integers(2, 65, size=20)])
+    ctx = rng.integers(0, 700, size=len(q))
+    ctx[decodes], ctx[decodes + 41], ctx[decodes + 42] = 20000, 5000, 900
+    with torch.cuda.stream(torch.cuda.current_stream() if stream == "first" else torch.cuda.Stream()):
+        _case(q.astype(int), ctx, 32, 8, 128, 16, torch.bfloat16, kv, seed=decodes)
+
+
+def test_a_long_context_does_not_run_on_one_sm_beside_many_groups():
+    """Cut into pieces it takes about as long beside 480 other groups as they and it take apart; as one
+    item per kv head it took three times as long."""
+    from vllm_b200 import _custom_ops as ops
+    H, HK, D, B, pool = 32, 8, 128, 16, 2048
+    kc = torch.randn(pool, HK, D // 8, B, 8, device=DEV).bfloat16()
+    vc = torch.randn(pool, HK, D, B, device=DEV).bfloat16()
+    one = torch.tensor(1.0, device=DEV)
+
+    def time(q, lens):
+        n = sum(q)
+        query = torch.randn(n, H, D, device=DEV).bfloat16()
+        out = torch.empty_like(query)
+        table = torch.randint(0, pool, (len(q), -(-max(lens) // B)), dtype=torch.int32, device=DEV)
+        qsl = torch.tensor(np.concatenate([[0], np.cumsum(q)]), dtype=torch.int32, device=DEV)
+        seq_lens = torch.tensor(lens, dtype=torch.int32, device=DEV)
+        best = float("inf")
+        for _ in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(4):
+                assert ops.paged_attention_varlen(out, query, kc, vc, HK, D ** -0.5, table, seq_lens, qsl, 0, B,
+                                                  max(lens), None, "auto", one, one)
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+    long, others = ([16], [32016]), ([32] * 60, [1000] * 60)
+    both = time(long[0] + others[0], long[1] + others[1])
+    assert both < 1.5 * (time(*long) + time(*others))

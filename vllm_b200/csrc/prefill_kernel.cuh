@@ -70,10 +70,11 @@ struct PrefillParams {
 
 constexpr int kPrefillThreads = 16 * 32;  // (three warps beside the MMA warp only complete its warpgroup)
 // Registers per thread: 512 threads start with 128 each; the softmax warpgroups take over what the
-// others give back.  (The producers of an fp8 cache hold a K and a V tile in registers.)
+// others give back.  (The producers of an fp8 cache hold a K and a V tile in registers.  An 8192-token
+// fp8 step of 64 / 8 heads takes 1032 us with 176 / 112 / 48 and 997 with 184 / 104 / 40.)
 template <bool kFp8>
 struct PrefillRegs {
-  static constexpr int kSoftmax = kFp8 ? 176 : 184, kProducer = kFp8 ? 104 : 88, kMma = 56;
+  static constexpr int kSoftmax = 184, kProducer = kFp8 ? 104 : 88, kMma = kFp8 ? 40 : 56;
   static_assert(2 * kSoftmax + kProducer + kMma == 4 * 128, "register split");
 };
 constexpr int kPrefillMaxReqs = 512;    // requests per launch: prefix table in shared memory
@@ -112,7 +113,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
   constexpr int DP = SH::DP, NQ = SH::NQ, KT = SH::KT, NS = SH::kSlots;
   constexpr int kWs = 128 * (D * 2 + 8);  // workspace of one row tile's partial: O, then (m, l)
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  __shared__ int cum[kPrefillMaxReqs + 1];  // items before request r
+  __shared__ int cum[kPrefillMaxReqs + 1];  // 2 x (items before request r), + 1 if it is cut into pieces
   __shared__ uint64_t s_bar[2 * NS + 12];
   __shared__ int s_item[2];
   __shared__ uint32_t s_tmem;
@@ -162,6 +163,8 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
           make_uint4(0, 0, 0, 0);
     fence_proxy_async();
   }
+  if (tid < 16) s_red[2][tid] = 0;  // (see the plan)
+  __syncthreads();
   if (p.late_wait) grid_launch_dependents(); else grid_dependency();
 
   // ---- plan.  T tokens fill a row tile; a request has ceil(q_len / (NQ T)) row-tile groups per kv
@@ -169,51 +172,60 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
   const int G = p.group, HK = p.num_kv_heads, S = p.num_reqs, B = p.block_size;
   const int b_shift = 31 - __clz(B);  // 16 or 32 tokens per block
   const int T = 128 / G, TT = NQ * T;
-  int split_tiles;  // key tiles per piece (INT_MAX: one piece per group)
+  int split_tiles;  // key tiles per piece (1 << 30: one piece per group)
   auto q_len_of = [&](int r) { return p.q_start[r + 1] - p.q_start[r]; };
   auto tiles_of = [&](int len) { return (max(len, 0) + KT - 1) / KT; };
   {
     // groups and key tiles of all requests: with fewer than four groups per SM the groups are cut
     // into pieces of an SM's share of the key tiles, but of no less than 768 keys: a piece costs a Q
-    // load, a pipeline fill, a partial and its merge, about as much as 350 keys
-    int groups = 0, work = 0, most = 0;
+    // load, a pipeline fill, a partial and its merge, about as much as 350 keys.
+    // Every piece of a group that is cut needs a slot of the workspace: s_red[2][k] counts the slots of
+    // cuts of 768 keys x 1, 1.5, 2, 3, 4, 6 ..., and the finest from the share up that fits is taken.
+    // (With a slot for every group, cut or not, nothing was cut beside 496 groups, or 31 on a small
+    // region beside decodes: a 16-token chunk behind 32000 and 60 chunks of 32, 546 -> 169 us.)
+    constexpr int kCut = 768 / KT;
+    int groups = 0, work = 0;
     for (int r = tid; r < S; r += kPrefillThreads) {
       const int ql = q_len_of(r);
       const int n = (ql + TT - 1) / TT;
       const int len = p.seq_lens[r];
+      const int t = tiles_of(len);
       groups += n;
-      work += n * ((tiles_of(len) + tiles_of(len - ql + min(ql, TT)) + 1) / 2);
-      most += n * tiles_of(len);
+      work += n * ((t + tiles_of(len - ql + min(ql, TT)) + 1) / 2);
+      const int q0 = (t + kCut - 1) / kCut, q1 = (t + kCut * 3 / 2 - 1) / (kCut * 3 / 2);
+#pragma unroll 1
+      for (int k = 0; k < 8 && t > kCut << k; ++k) {
+        atomicAdd(&s_red[2][2 * k], n * HK * ((q0 + (1 << k) - 1) >> k));
+        if (t > kCut * 3 / 2 << k) atomicAdd(&s_red[2][2 * k + 1], n * HK * ((q1 + (1 << k) - 1) >> k));
+      }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       groups += __shfl_xor_sync(0xffffffffu, groups, o);
       work += __shfl_xor_sync(0xffffffffu, work, o);
-      most += __shfl_xor_sync(0xffffffffu, most, o);
     }
     if (lane == 0) {
       s_red[0][warp] = groups;
       s_red[1][warp] = work;
-      s_red[2][warp] = most;
     }
     __syncthreads();
-    groups = work = most = 0;
+    groups = work = 0;
     for (int w = 0; w < 16; ++w) {
       groups += s_red[0][w];
       work += s_red[1][w];
-      most += s_red[2][w];
+    }
+    const int64_t all_work = int64_t(work) * HK, all_groups = int64_t(groups) * HK;
+    split_tiles = 1 << 30;
+    if (all_groups < 4 * int64_t(gridDim.x)) {
+      const int want = int((all_work + gridDim.x - 1) / int64_t(gridDim.x));
+      auto cut_of = [&](int k) { return ((k & 1) ? kCut * 3 / 2 : kCut) << (k >> 1); };
+      const unsigned fit = __ballot_sync(
+          0xffffffffu, lane < 16 && s_red[2][lane & 15] <= p.ws_slots && cut_of(lane + 1) > want);
+      if (fit != 0) split_tiles = max(cut_of(__ffs(fit) - 1), want);
     }
     __syncthreads();  // (s_red is written again below)
-    const int64_t all_work = int64_t(work) * HK, all_groups = int64_t(groups) * HK;
-    split_tiles = INT32_MAX;
-    if (all_groups < 4 * int64_t(gridDim.x)) {
-      const int64_t c = max(int64_t(768 / KT), (all_work + gridDim.x - 1) / int64_t(gridDim.x));
-      // every piece needs a slot of the workspace: a group of n tiles has at most n / c + 1 pieces
-      const int64_t room = p.ws_slots - all_groups;
-      if (room > 0) split_tiles = int(min(max(c, int64_t(most) * HK / room + 1), int64_t(INT32_MAX)));
-    }
   }
-  auto pieces_of = [&](int len) { return split_tiles == INT32_MAX ? 1 : max(1, (tiles_of(len) + split_tiles - 1) / split_tiles); };
+  auto pieces_of = [&](int len) { return max(1u, (unsigned(tiles_of(len)) + split_tiles - 1u) / unsigned(split_tiles)); };
   {
     const int per = (S + kPrefillThreads - 1) / kPrefillThreads;
     const int r0 = min(S, tid * per), r1 = min(S, r0 + per);
@@ -231,16 +243,16 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
     int run = incl - mine;
     for (int w = 0; w < warp; ++w) run += s_red[2][w];
     for (int r = r0; r < r1; ++r) {
-      cum[r] = run;
+      cum[r] = 2 * run + (pieces_of(p.seq_lens[r]) > 1 ? 1 : 0);
       run += items_of(r);
     }
-    if (tid == kPrefillThreads - 1) cum[S] = run;
+    if (tid == kPrefillThreads - 1) cum[S] = 2 * run;
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = s_tmem;
-  const int total = cum[S];
+  const int total = cum[S] >> 1;
 
   // item number -> what it covers.  Inside a request the row tiles run from the last to the first
   // (longest first), then the pieces, then the kv heads.
@@ -249,14 +261,14 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
     int lo = 0, hi = S;
     while (hi - lo > 1) {
       const int mid = (lo + hi) >> 1;
-      if (cum[mid] <= item) lo = mid; else hi = mid;
+      if (cum[mid] >> 1 <= item) lo = mid; else hi = mid;
     }
     it.req = lo;
     it.q0 = p.q_start[lo];
     it.q_len = p.q_start[lo + 1] - it.q0;
     it.seq_len = p.seq_lens[lo];
     it.ctx = it.seq_len - it.q_len;
-    const int rel = item - cum[lo];
+    const int rel = item - (cum[lo] >> 1);
     it.kvh = rel % HK;
     const int gp = rel / HK;
     it.npieces = pieces_of(it.seq_len);
@@ -548,7 +560,17 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
       const bool whole = cur.npieces == 1;
       const float inv = v_scale * __fdividef(1.f, l + 1e-6f);
       const int64_t out_row = (int64_t(cur.q0 + tok) * p.num_heads + head) * D;
-      unsigned char* part = p.ws + (size_t(cur.first + cur.piece * HK) * NQ + wg) * kWs;
+      // workspace slot of piece 0: the items of cut requests are counted only.  (A table of the slots takes
+      // the static shared memory past what a carve-out of 196 KiB holds at head size 128, and L1 shrinks to
+      // 28 KiB: 2 chunks of 64 behind 8192 take 98 us instead of 76.)
+      int slot = cur.first;
+      if (!whole) {
+        int others = 0;
+        for (int r = lane; r < cur.req; r += 32)
+          if ((cum[r] & 1) == 0) others += (cum[r + 1] >> 1) - (cum[r] >> 1);
+        slot -= __reduce_add_sync(0xffffffffu, others);
+      }
+      unsigned char* part = p.ws + (size_t(slot + cur.piece * HK) * NQ + wg) * kWs;
       QT* dst = whole ? static_cast<QT*>(p.out) + out_row
                       : reinterpret_cast<QT*>(part) + row * D;
       if (any || whole) {
@@ -579,7 +601,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
         __threadfence();
         __syncwarp();
         unsigned old = 0;
-        unsigned* cnt = p.arrive + (size_t(cur.first) * NQ + wg) * 4 + (warp & 3);
+        unsigned* cnt = p.arrive + (size_t(slot) * NQ + wg) * 4 + (warp & 3);
         if (lane == 0) {
           old = atomicAdd(cnt, 1u);
           if (old == unsigned(cur.npieces - 1)) *cnt = 0;  // re-arm for the next launch
@@ -587,7 +609,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
         old = __shfl_sync(0xffffffffu, old, 0);
         if (old == unsigned(cur.npieces - 1) && valid) {
           __threadfence();
-          const unsigned char* base = p.ws + (size_t(cur.first) * NQ + wg) * kWs;
+          const unsigned char* base = p.ws + (size_t(slot) * NQ + wg) * kWs;
           const size_t step = size_t(HK) * NQ * kWs;
           // statistics of eight pieces at a time (independent loads), online
           float mx = -INFINITY, total_l = 0.f;
