@@ -214,6 +214,10 @@ int b200pa_decode_route(const b200pa_attn_args* args, int32_t* cluster);
 int b200pa_paged_attention_varlen(const b200pa_attn_args* args, const int32_t* query_start_loc,
                                   int32_t num_tokens, int32_t num_decodes, void* stream);
 
+/* 1 if b200pa_paged_attention_varlen has a kernel for requests with several rows of this shape (sizes,
+ * types, strides, alignments), else 0: to be asked before the step's KV is written, for instance. */
+int b200pa_paged_attention_varlen_supported(const b200pa_attn_args* args);
+
 /*
  * Arguments of reshape_and_cache / reshape_and_cache_flash.
  * Replaces: csrc/cache.h:21-32, launchers csrc/cache_kernels.cu:656-683 and :700-738.

@@ -136,3 +136,23 @@ def test_a_captured_step_is_replayed_with_other_divisions_of_its_tokens(kv, for_
         e.load(new, ctx)
         g.replay()
         e.check()
+
+
+def test_a_step_without_a_prefill_kernel_writes_its_kv_once():
+    from vllm_b200 import _custom_ops as ops
+    from vllm_b200 import capi
+    e = Engine(4, 32, B=8)  # (block size 8: decode kernels only)
+    e.load([1, 1, 20, 7], [30, 100, 50, 0])
+    md = e.builder.build(0, e.common())
+
+    def launches(f):
+        capi.launch_count(reset=True)
+        f()
+        return capi.launch_count()
+    step = launches(lambda: e.forward(md))
+    e.check()
+    kc, vc = e.cache[0].view(e.nb, e.HK, e.D // 8, 8, 8), e.cache[1].view(e.nb, e.HK, e.D, 8)
+    write = launches(lambda: ops.reshape_and_cache(e.k, e.v, kc, vc, e.slots, "auto", e.layer._k_scale,
+                                                   e.layer._v_scale))
+    e.impl.kv_sharing_target_layer_name = "another layer writes"
+    assert step == launches(lambda: e.forward(md)) + write

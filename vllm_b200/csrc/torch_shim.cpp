@@ -756,27 +756,6 @@ PyObject* py_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int kv_type = kv_code(kv);
     const at::cuda::OptionalCUDAGuard device_guard(dev);
     void* stream = at::cuda::getCurrentCUDAStream().stream();
-    if (write) {
-      b200pa_cache_args c;
-      std::memset(&c, 0, sizeof(c));
-      c.in_dtype = in_type;
-      c.kv_dtype = kv_type;
-      c.key = k.data_ptr();
-      c.value = v.data_ptr();
-      c.key_cache = base;
-      c.value_cache = vbase;
-      c.slot_mapping = slots.data_ptr<int64_t>();
-      c.k_scale = ks.data_ptr<float>();
-      c.v_scale = vs.data_ptr<float>();
-      c.key_stride = k.stride(0);
-      c.value_stride = v.stride(0);
-      c.num_tokens = static_cast<int32_t>(tokens);
-      c.num_heads = static_cast<int32_t>(HK);
-      c.head_size = static_cast<int32_t>(D);
-      c.block_size = static_cast<int32_t>(B);
-      c.x = static_cast<int32_t>(x);
-      check_rc(b200pa_reshape_and_cache(&c, stream));
-    }
     b200pa_attn_args p;
     std::memset(&p, 0, sizeof(p));
     p.q_dtype = in_type;
@@ -802,6 +781,29 @@ PyObject* py_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p.max_num_blocks_per_seq = static_cast<int32_t>(bt.size(1));
     p.scale = static_cast<float>(scale);
     p.blocksparse_block_size = 64;
+    // (nothing may be done before it is clear that everything can be: the caller would do it again)
+    if (max_q > 1 && decodes < reqs && !b200pa_paged_attention_varlen_supported(&p)) return false;
+    if (write) {
+      b200pa_cache_args c;
+      std::memset(&c, 0, sizeof(c));
+      c.in_dtype = in_type;
+      c.kv_dtype = kv_type;
+      c.key = k.data_ptr();
+      c.value = v.data_ptr();
+      c.key_cache = base;
+      c.value_cache = vbase;
+      c.slot_mapping = slots.data_ptr<int64_t>();
+      c.k_scale = ks.data_ptr<float>();
+      c.v_scale = vs.data_ptr<float>();
+      c.key_stride = k.stride(0);
+      c.value_stride = v.stride(0);
+      c.num_tokens = static_cast<int32_t>(tokens);
+      c.num_heads = static_cast<int32_t>(HK);
+      c.head_size = static_cast<int32_t>(D);
+      c.block_size = static_cast<int32_t>(B);
+      c.x = static_cast<int32_t>(x);
+      check_rc(b200pa_reshape_and_cache(&c, stream));
+    }
     if (max_q > 1) {
       const int rc = b200pa_paged_attention_varlen(&p, qsl.data_ptr<int>(), static_cast<int32_t>(tokens),
                                                    static_cast<int32_t>(decodes), stream);

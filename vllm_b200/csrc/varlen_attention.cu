@@ -6,6 +6,30 @@
 #include "launch_state.cuh"
 #include "prefill_inst.cuh"
 
+namespace b200pa {
+
+// The prefill kernel for a call's shape and alignments, or none.  16-byte accesses: pages, rows of Q and
+// of the output; cache offsets inside a block are shifts.
+static PrefillKernelInfo find_prefill(const b200pa_attn_args& a) {
+  const int es = a.kv_dtype == B200PA_KV_AUTO ? 2 : 1;
+  auto al = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr) % 16 == 0; };
+  const bool fits = (a.block_size == 16 || a.block_size == 32) && a.num_heads / a.num_kv_heads <= 128 &&
+                    al(a.key_cache) && al(a.value_cache) && al(a.query) && al(a.out) &&
+                    (a.kv_block_stride * es) % 16 == 0 && (a.kv_head_stride * es) % 16 == 0 &&
+                    a.q_stride % 8 == 0 && a.blocksparse_vert_stride <= 1 && a.out_lse == nullptr;
+  if (!fits) return {nullptr, 0};
+  return a.head_size <= 96 ? find_prefill_small(a.head_size, a.q_dtype, a.kv_dtype)
+         : a.head_size <= 128 ? find_prefill_mid(a.head_size, a.q_dtype, a.kv_dtype)
+                              : find_prefill_large(a.head_size, a.q_dtype, a.kv_dtype);
+}
+
+}  // namespace b200pa
+
+extern "C" int b200pa_paged_attention_varlen_supported(const b200pa_attn_args* a) {
+  return a != nullptr && a->num_heads > 0 && a->num_kv_heads > 0 && a->num_heads % a->num_kv_heads == 0 &&
+         b200pa::find_prefill(*a).fn != nullptr;
+}
+
 extern "C" int b200pa_paged_attention_varlen(const b200pa_attn_args* a, const int32_t* query_start_loc,
                                              int32_t num_tokens, int32_t num_decodes, void* stream) {
   using namespace b200pa;
@@ -25,18 +49,7 @@ extern "C" int b200pa_paged_attention_varlen(const b200pa_attn_args* a, const in
     B200PA_CHECK_ARG(a->kv_dtype == B200PA_KV_AUTO || (a->k_scale && a->v_scale),
                      "fp8 kv cache needs k_scale and v_scale");
     B200PA_CHECK_ARG(a->max_num_blocks_per_seq > 0, "max_num_blocks_per_seq must be positive");
-    // 16-byte accesses: pages, rows of Q and of the output; cache offsets inside a block are shifts
-    const int es = a->kv_dtype == B200PA_KV_AUTO ? 2 : 1;
-    auto al = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr) % 16 == 0; };
-    const bool fits = (a->block_size == 16 || a->block_size == 32) && a->num_heads / a->num_kv_heads <= 128 &&
-                      al(a->key_cache) && al(a->value_cache) && al(a->query) &&
-                      al(a->out) && (a->kv_block_stride * es) % 16 == 0 && (a->kv_head_stride * es) % 16 == 0 &&
-                      a->q_stride % 8 == 0 && a->blocksparse_vert_stride <= 1 && a->out_lse == nullptr;
-    if (fits) {
-      ki = a->head_size <= 96 ? find_prefill_small(a->head_size, a->q_dtype, a->kv_dtype)
-           : a->head_size <= 128 ? find_prefill_mid(a->head_size, a->q_dtype, a->kv_dtype)
-                                 : find_prefill_large(a->head_size, a->q_dtype, a->kv_dtype);
-    }
+    ki = find_prefill(*a);
     if (ki.fn == nullptr) {
       set_error("paged_attention_varlen: no kernel for head_size=%d block_size=%d q_dtype=%d kv_dtype=%d, "
                 "or unaligned tensors",
