@@ -193,7 +193,8 @@ int b200pa_paged_attention_v2_noalloc(const b200pa_attn_args* args, void* stream
 /*
  * Which kernel a call of paged_attention_v1 / v2 with these sizes, types, strides and alignments runs
  * on; launches nothing and reads no tensor.  *cluster: 1 to 16, the direct kernel with that many CTAs
- * per (sequence, kv head, head group); 0, the persistent kernel; -1, the generic kernel.
+ * per (sequence, kv head, head group), or as many as the GPU can place in one cluster; 0, the
+ * persistent kernel; -1, the generic kernel.
  */
 int b200pa_decode_route(const b200pa_attn_args* args, int32_t* cluster);
 

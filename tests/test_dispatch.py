@@ -1,4 +1,7 @@
 """The rules that pick a kernel for a call, asked on the host (no GPU: a chip of 148 SMs is assumed)."""
+import subprocess
+from pathlib import Path
+
 import pytest
 
 from vllm_b200 import capi
@@ -44,3 +47,20 @@ def test_batches_that_the_persistent_kernel_serves_faster(call):
                                   (4, 32, 8, 256, 1000, 1), (32, 64, 4, 112, 2500, 0), (12, 32, 8, 128, 3000, 0)])
 def test_batches_that_the_direct_kernel_serves_faster(call):
     assert _route(*call[:5], kv=call[5]) > 0
+
+
+def test_a_gpu_without_room_for_clusters_of_16_gets_smaller_ones(tmp_path):
+    """The size is asked from the GPU; here from a stand-in that has room up to some size."""
+    (tmp_path / "t.cpp").write_text("""
+#include <cstdio>
+#include "cluster_fit.h"
+int main() {
+  const int most[] = {16, 15, 8, 7, 4, 1, 0};
+  for (int m : most) std::printf("%d ", b200pa::largest_cluster([&](int n) { return n <= m ? 132 / n : 0; }));
+  std::printf("%d\\n", b200pa::largest_cluster([](int) { return -1; }));
+}
+""")
+    csrc = Path(__file__).resolve().parents[1] / "vllm_b200" / "csrc"
+    subprocess.run(["g++", "-std=c++17", f"-I{csrc}", "t.cpp", "-o", "t"], cwd=tmp_path, check=True, timeout=120)
+    out = subprocess.run(["./t"], cwd=tmp_path, check=True, capture_output=True, text=True, timeout=60).stdout
+    assert out.split() == ["16", "8", "8", "4", "4", "1", "1", "1"]

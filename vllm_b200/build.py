@@ -50,7 +50,7 @@ def _run(cmd: list[str], verbose: bool) -> None:
 
 def build_lib(force: bool = False, verbose: bool = False) -> Path:
     OBJ.mkdir(exist_ok=True)
-    headers = sorted(CSRC.glob("*.cuh")) + [PKG.parent / "include" / "b200pa.h"]
+    headers = sorted([*CSRC.glob("*.cuh"), *CSRC.glob("*.h")]) + [PKG.parent / "include" / "b200pa.h"]
     sources = sorted(CSRC.glob("*.cu"))
     jobs = []
     objs = []

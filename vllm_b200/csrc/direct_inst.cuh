@@ -1,6 +1,7 @@
 // Explicit-instantiation helper of the direct decode kernel (direct_*.cu).
 #pragma once
 
+#include "cluster_fit.h"
 #include "decode_direct.cuh"
 
 namespace b200pa {
@@ -17,33 +18,45 @@ template <typename QT, int KV, int D, int GP>
 cudaError_t direct_launch(const DecodeParams& p, int items, int cluster, cudaStream_t stream) {
   auto kern = pa_decode_direct_kernel<QT, KV, D, GP>;
   constexpr int smem = DirectShape<KV, D, GP>::kSmem;
-  // opt in to clusters of 16 and (for wide heads) more than 48 KiB of shared memory once per device
-  static bool done[64] = {};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= 64 || !done[dev]) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) {
-      (void)cudaGetLastError();
-      return e;
-    }
-    if (dev >= 0 && dev < 64) done[dev] = true;
-  }
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = cluster;
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(unsigned(items) * unsigned(cluster));
   cfg.blockDim = dim3(kDirectWarps * 32);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cfg.attrs = attr;
-  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  auto set_clusters = [&](int n, int size) {
+    attr[1].val.clusterDim.x = size;
+    cfg.gridDim = dim3(unsigned(n) * unsigned(size));
+    cfg.numAttrs = size > 1 ? 2 : 1;
+  };
+  // once per device: opt in to clusters of 16 and (for wide heads) more than 48 KiB of shared memory, and
+  // see what the device has room for
+  static int largest[64] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  int limit = dev >= 0 && dev < 64 ? largest[dev] : 0;
+  if (limit == 0) {
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) {
+      (void)cudaGetLastError();
+      return e;
+    }
+    (void)cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    limit = largest_cluster([&](int size) {
+      set_clusters(1, size);
+      int places = 0;
+      return cudaOccupancyMaxActiveClusters(&places, kern, &cfg) == cudaSuccess ? places : 0;
+    });
+    (void)cudaGetLastError();  // (of sizes that the device refused)
+    if (dev >= 0 && dev < 64) largest[dev] = limit;
+  }
+  if (cluster > limit) cluster = limit;
+  set_clusters(items, cluster);
   return cudaLaunchKernelEx(&cfg, kern, p, cluster);
 }
 
