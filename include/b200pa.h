@@ -161,6 +161,11 @@ int b200pa_paged_attention_v1(const b200pa_attn_args* args, void* stream);
  * instead and leave the caller's scratch untouched. */
 int b200pa_paged_attention_v2(const b200pa_attn_args* args, void* stream);
 
+/* Bytes of the workspace above that every stream can count on (the small parts; the first stream's is
+ * larger): partials of num_seqs * num_heads * P slots of 8 + head_size * sizeof(query element) bytes
+ * that fit need no scratch of the caller. */
+int64_t b200pa_stream_workspace_bytes(void);
+
 /*
  * paged_attention_v2 for callers that cannot hand over scratch memory.  It has no
  * counterpart in the reference, whose caller always allocates exp_sums,

@@ -64,3 +64,13 @@ int main() {
     subprocess.run(["g++", "-std=c++17", f"-I{csrc}", "t.cpp", "-o", "t"], cwd=tmp_path, check=True, timeout=120)
     out = subprocess.run(["./t"], cwd=tmp_path, check=True, capture_output=True, text=True, timeout=60).stdout
     assert out.split() == ["16", "8", "8", "4", "4", "1", "1", "1"]
+
+
+def test_the_choice_of_v1_and_v2_is_the_reference_s():
+    from vllm_b200.paged_attn import PagedAttention
+    for max_len in (0, 1, 511, 512, 513, 8191, 8192, 8193, 100000):
+        for seqs, heads in ((1, 1), (1, 512), (1, 513), (16, 32), (17, 32), (256, 64)):
+            partitions = (max_len + 511) // 512
+            assert PagedAttention.use_v1(max_len, seqs, heads) == (
+                max_len <= 8192 and (partitions == 1 or seqs * heads > 512))
+    assert capi.lib().b200pa_stream_workspace_bytes() == 4 << 20

@@ -183,7 +183,8 @@ class B200PagedAttentionImpl:
                 output, query, key, value, kv_cache, md.block_table, md.seq_lens, md.slot_mapping,
                 md.query_start_loc, layer._k_scale, layer._v_scale, alibi, n, num_decodes,
                 md.max_query_len, md.max_seq_len, self.num_heads, self.num_kv_heads, self.head_size,
-                self.scale, self.kv_cache_dtype, self.kv_sharing_target_layer_name is None):
+                self.scale, self.kv_cache_dtype, self.kv_sharing_target_layer_name is None,
+                PagedAttention.use_v1(md.max_seq_len, n, self.num_heads)):
             return output
         # not a plain call (fp32, odd strides, tracing, ...): operator by operator
         key_cache, value_cache = PagedAttention.split_kv_cache(kv_cache, self.num_kv_heads,

@@ -80,6 +80,7 @@ def lib() -> C.CDLL:
         l.b200pa_last_error.restype = C.c_char_p
         l.b200pa_kv_dtype_from_string.argtypes = [C.c_char_p]
         l.b200pa_launch_count.restype = C.c_int64
+        l.b200pa_stream_workspace_bytes.restype = C.c_int64
         l.b200pa_launch_count.argtypes = [C.c_int]
         for name in ("b200pa_paged_attention_v1", "b200pa_paged_attention_v2",
                      "b200pa_paged_attention_v2_noalloc"):

@@ -833,6 +833,8 @@ extern "C" int b200pa_paged_attention_v2(const b200pa_attn_args* args, void* str
   return b200pa::attention_entry(args, stream, b200pa::Scratch::kCaller);
 }
 
+extern "C" int64_t b200pa_stream_workspace_bytes(void) { return int64_t(b200pa::kSmallRegionBytes); }
+
 extern "C" int b200pa_decode_route(const b200pa_attn_args* args, int32_t* cluster) {
   using namespace b200pa;
   B200PA_CHECK_ARG(args != nullptr && cluster != nullptr, "args or cluster is NULL");

@@ -714,7 +714,7 @@ PyObject* py_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int64_t H = in.integer(), HK = in.integer(), D = in.integer();
   const double scale = in.real();
   const std::string kv = in.text();
-  const int64_t write = in.integer();
+  const int64_t write = in.integer(), prefer_v1 = in.integer();
   return direct(in, [&]() -> bool {
     using at::ScalarType;
     const auto type = q.scalar_type();
@@ -811,11 +811,10 @@ PyObject* py_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
       check_rc(rc);
       return true;
     }
-    // PagedAttention.forward_decode's rule for v1 / v2; and v1 whenever the partials of v2 fit the
-    // library's own workspace (4 MiB for any stream), which saves the scratch allocations
+    // v1 also when the partials of v2 fit the library's own workspace, which saves the scratch allocation
     const int64_t parts = (max_len + 511) / 512, rows_n = tokens * H;
-    const bool use_v1 = (max_len <= 8192 && (parts == 1 || rows_n > 512)) ||
-                        rows_n * parts * (8 + 2 * D) <= (int64_t(4) << 20) - 1024;
+    const bool use_v1 =
+        prefer_v1 != 0 || rows_n * parts * (8 + 2 * D) <= b200pa_stream_workspace_bytes() - 1024;
     if (use_v1) {
       check_rc(b200pa_paged_attention_v1(&p, stream));
       return true;

@@ -42,6 +42,12 @@ class PagedAttention:
                               kv_cache_dtype, k_scale, v_scale)
 
     @staticmethod
+    def use_v1(max_seq_len: int, num_seqs: int, num_heads: int) -> bool:
+        """The reference's choice between v1 and v2 (paged_attn.py:134-136)."""
+        partitions = (max_seq_len + _PARTITION_SIZE - 1) // _PARTITION_SIZE
+        return max_seq_len <= 8192 and (partitions == 1 or num_seqs * num_heads > 512)
+
+    @staticmethod
     def forward_decode(
         query: torch.Tensor,
         key_cache: torch.Tensor,
@@ -71,11 +77,9 @@ class PagedAttention:
         block_size = value_cache.shape[3]
         num_seqs, num_heads, head_size = query.shape
         max_num_partitions = (max_seq_len + _PARTITION_SIZE - 1) // _PARTITION_SIZE
-        # Same rule as the reference (paged_attn.py:134-136).
-        use_v1 = max_seq_len <= 8192 and (max_num_partitions == 1 or num_seqs * num_heads > 512)
         tail = (tp_rank, blocksparse_local_blocks, blocksparse_vert_stride, blocksparse_block_size,
                 blocksparse_head_sliding_step)
-        if use_v1:
+        if PagedAttention.use_v1(max_seq_len, num_seqs, num_heads):
             ops.paged_attention_v1(output, query, key_cache, value_cache, num_kv_heads, scale,
                                    block_tables, seq_lens, block_size, max_seq_len, alibi_slopes,
                                    kv_cache_dtype, k_scale, v_scale, *tail)
