@@ -585,10 +585,12 @@ extern "C" int b200_claim_reference_names(char* err, int err_len) {
 // raises.
 namespace {
 
-// The calling thread's state allows a call that the dispatcher does not see.
+// The calling thread's state allows a call that the dispatcher does not see: no modes, no profiler, and no
+// dispatch keys beyond the usual ones (tracing, functionalization and the function transforms add theirs).
 bool plain_state() {
-  return !c10::impl::TorchDispatchModeTLS::any_modes_set() && !at::impl::torch_function_mode_enabled() &&
-         !at::hasCallbacks();
+  const c10::DispatchKeySet more = c10::impl::tls_local_dispatch_key_set().included_ - c10::default_included_set;
+  return more.empty() && !c10::impl::TorchDispatchModeTLS::any_modes_set() &&
+         !at::impl::torch_function_mode_enabled() && !at::hasCallbacks();
 }
 
 bool plain_tensor(PyObject* o) {
