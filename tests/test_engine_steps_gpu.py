@@ -156,3 +156,52 @@ def test_a_step_without_a_prefill_kernel_writes_its_kv_once():
                                                    e.layer._v_scale))
     e.impl.kv_sharing_target_layer_name = "another layer writes"
     assert step == launches(lambda: e.forward(md)) + write
+
+
+@pytest.mark.parametrize("kv", ["auto", "fp8"])
+@pytest.mark.parametrize("stream", ["first", "second"])
+def test_split_decodes_and_cut_chunks_share_the_workspace(stream, kv):
+    """Long decodes go to the persistent kernel, split across warps through one half of the stream's
+    workspace, while the prefill kernel runs beside it on the other half."""
+    from vllm_b200 import capi
+    e = Engine(6, 400, max_blocks=2000, kv=kv)
+    a = capi.AttnArgs()
+    a.num_seqs, a.num_heads, a.num_kv_heads, a.head_size, a.block_size = 3, e.H, e.HK, e.D, e.B
+    a.max_seq_len, a.q_dtype, a.kv_dtype = 31000, capi.BF16, 0 if kv == "auto" else 1
+    assert capi.decode_route(a) == 0
+    with torch.cuda.stream(torch.cuda.current_stream() if stream == "first" else torch.cuda.Stream()):
+        for _ in range(3):
+            e.load([1, 1, 1, 20, 300, 9], [30999, 20000, 7, 25000, 2000, 9000])
+            e.forward(e.builder.build(0, e.common()))
+            e.check()
+
+
+@pytest.mark.parametrize("new,ctx", [([1, 1, 1], [0, 700, 33]), ([1, 1, 9, 40], [300, 5, 0, 77]),
+                                     ([5, 64], [0, 129]), ([1], [1500])])
+@pytest.mark.parametrize("D,kv,alibi", [(128, "auto", False), (128, "fp8", True), (64, "fp8_e5m2", False),
+                                        (120, "auto", True), (256, "auto", False)])
+def test_the_native_step_does_what_the_operators_do(new, ctx, D, kv, alibi, monkeypatch):
+    from vllm_b200 import _custom_ops as ops
+    e = Engine(4, 80, D=D, kv=kv, alibi=alibi, max_blocks=100)
+    # rows of a fused projection: strided by token
+    fused = torch.empty(80, (e.H + 2 * e.HK) * D, dtype=e.dtype, device=DEV)
+    e.q, e.k, e.v = (t.view(80, -1, D) for t in fused.split([e.H * D, e.HK * D, e.HK * D], dim=1))
+    e.load(new, ctx)
+    before = e.cache.clone()
+    md = e.builder.build(0, e.common())
+    step, taken = ops.attention_step, []
+    monkeypatch.setattr(ops, "attention_step", lambda *args: taken.append(step(*args)) or taken[-1])
+    e.forward(md)
+    assert taken == [True]
+    e.check()
+    native, written = e.out.clone(), e.cache.clone()
+    e.cache.copy_(before)
+    e.out.fill_(float("nan"))
+    monkeypatch.setattr(ops, "attention_step", lambda *args: False)
+    e.forward(md)
+    e.check()
+    assert torch.equal(e.cache, written)
+    n = sum(new)
+    # (the same roundings in another order: two results of 16 bits, and partials of 16 bits in one of them)
+    assert (e.out[:n].float() - native[:n].float()).norm() < 6e-3 * native[:n].float().norm()
+    assert e.out[n:].isnan().all() and native[n:].isnan().all()
