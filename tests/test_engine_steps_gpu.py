@@ -205,3 +205,25 @@ def test_the_native_step_does_what_the_operators_do(new, ctx, D, kv, alibi, monk
     # (the same roundings in another order: two results of 16 bits, and partials of 16 bits in one of them)
     assert (e.out[:n].float() - native[:n].float()).norm() < 6e-3 * native[:n].float().norm()
     assert e.out[n:].isnan().all() and native[n:].isnan().all()
+
+
+def test_a_replay_beside_launches_on_another_stream():
+    """A captured launch does not share its work-distribution words with ordinary ones: more of them
+    than there are rotating slots run beside the replays."""
+    graphed, eager = Engine(4, 512, max_blocks=60, seed=1), Engine(4, 512, max_blocks=60, seed=2)
+    graphed.load([200, 100, 150, 62], [300, 7, 0, 500])
+    eager.load([90, 128, 200, 30], [600, 70, 1, 250])
+    g = _capture(graphed, graphed.builder.build(0, graphed.common()))
+    md = eager.builder.build(0, eager.common())
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    for _ in range(10):
+        graphed.out.fill_(float("nan"))
+        for _ in range(30):
+            g.replay()
+            with torch.cuda.stream(side):
+                eager.forward(md)
+        torch.cuda.current_stream().wait_stream(side)
+        side.wait_stream(torch.cuda.current_stream())
+    graphed.check()
+    eager.check()

@@ -21,7 +21,7 @@ struct StreamRegion {
 };
 
 bool stream_region(cudaStream_t stream, StreamRegion* out);
-unsigned* sched_words();
+unsigned* sched_words(cudaStream_t stream);
 int sm_count();
 
 // paged_attention_v1 on the first half of the stream's workspace and arrival counters.

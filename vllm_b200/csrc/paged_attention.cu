@@ -210,7 +210,8 @@ pa_generic_kernel(const DecodeParams p, int head_size, int x) {
 }
 
 // ------------------------------------------------------------------ host side
-__device__ unsigned g_sched_words[256][2];  // zero-initialised; self-resetting per launch
+constexpr unsigned kSchedOnce = 256, kSchedCaptured = 65536;  // (see sched_words)
+__device__ unsigned g_sched_words[kSchedOnce + kSchedCaptured][2];  // zero-initialised; self-resetting per launch
 // Arrival counters of the fused split-KV merge: one per (sequence, kv head, head
 // group); zero-initialised and re-armed by the warp that performs the merge.
 constexpr int kStreamSlots = 8;
@@ -331,12 +332,14 @@ bool stream_region(cudaStream_t stream, StreamRegion* out) {
   return true;
 }
 
-// Scheduler words of one launch (256 rotating slots; only unsplit launches with more than
-// three items per warp use them).
-unsigned* sched_words() {
+// Scheduler words of one launch.  256 rotating slots serve launches that run once (of those only as many as
+// there are streams are in flight).  A captured launch keeps its slot for as long as its graph lives, and
+// replays run beside anything: it gets one of its own, else a launch on another stream that came round to the
+// same slot would draw from the same counter, and both would leave work out.
+unsigned* sched_words(cudaStream_t stream) {
   constexpr int kMaxDev = 64;
   static unsigned* sbase[kMaxDev] = {};
-  static std::atomic<unsigned> rr{0};
+  static std::atomic<unsigned> rr{0}, captured{0};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) return nullptr;
   unsigned* sb = __atomic_load_n(&sbase[dev], __ATOMIC_ACQUIRE);
@@ -347,7 +350,12 @@ unsigned* sched_words() {
     }
     __atomic_store_n(&sbase[dev], sb, __ATOMIC_RELEASE);
   }
-  return sb + 2 * (rr.fetch_add(1, std::memory_order_relaxed) & 255u);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) (void)cudaGetLastError();
+  const unsigned slot = capture == cudaStreamCaptureStatusActive
+                            ? kSchedOnce + captured.fetch_add(1, std::memory_order_relaxed) % kSchedCaptured
+                            : rr.fetch_add(1, std::memory_order_relaxed) % kSchedOnce;
+  return sb + 2 * size_t(slot);
 }
 
 int sm_count() {
@@ -774,7 +782,7 @@ static int attention_entry(const b200pa_attn_args* a, void* stream, Scratch mode
     }
     p.nstages = ns;
     p.status = device_status_ptr();
-    p.sched = sched_words();
+    p.sched = sched_words(s);
     if (p.sched == nullptr || p.status == nullptr) {
       set_error("could not resolve device-side scheduler/status words");
       return B200PA_ECUDA;

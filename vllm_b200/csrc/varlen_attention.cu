@@ -103,7 +103,7 @@ extern "C" int b200pa_paged_attention_varlen(const b200pa_attn_args* a, const in
     p.block_tables = a->block_tables + int64_t(r) * a->max_num_blocks_per_seq;
     p.seq_lens = a->seq_lens + r;
     p.q_start = query_start_loc + r;
-    p.sched = sched_words();
+    p.sched = sched_words(s);
     if (p.sched == nullptr || p.status == nullptr) {
       set_error("could not resolve device-side scheduler/status words");
       return B200PA_ECUDA;
