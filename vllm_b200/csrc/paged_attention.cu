@@ -422,25 +422,31 @@ static DirectPlan direct_plan(const DirectKernelInfo& ki, const b200pa_attn_args
     while (cluster > 1 && items * cluster > slots) cluster /= 2;
     return {cluster, false};
   }
-  // What either kernel takes, us, if all sequences are as long as the bound.  Fitted to 4 000 launches
-  // (head sizes 32 to 256, both cache widths, six head counts, 1 to 400 sequences of 100 to 32000 tokens,
-  // all equal or uniform below the bound; 9 and 15 % rms):
+  // What either kernel takes, us, if all sequences are as long as the bound.  Fitted to 9 204 batches (head
+  // sizes 32 to 256, both cache widths and block sizes, seven head counts, 1 to 400 sequences of 100 to 8000
+  // tokens, all equal or uniform below the bound):
   //   direct       10, and for every wave of CTAs the tiles of a warp, one after the other: their
-  //                latency, or HBM where many warps load; 3 for each wave after the first
-  //   persistent   20, merges that grow with the heads of a kv head, the bytes at HBM's rate
+  //                latency, or HBM where many warps load (a wide tile comes in smaller runs of a page);
+  //                3 for each wave after the first
+  //   persistent   20, merges that grow with the heads of a kv head while there are fewer work items than
+  //                warps, the bytes at HBM's rate
   // Shorter sequences than the bound favour the direct kernel when it has several waves (their CTAs make
-  // room) and the persistent one when it has one (the longest sequence decides).  Of 2115 equal batches that
-  // the size limits above let through, 144 were slower than on the persistent kernel by more than 10 %
-  // (worst: 32 sequences of 2500, 8 heads of 128, fp8, 45 against 55 us); with the estimate 25 are.
+  // room) and the persistent one when it has one (the longest sequence decides).  Of 4914 equal batches that
+  // the size limits above let through, 450 were slower than on the persistent kernel by more than 10 %
+  // (worst: 256 sequences of 200, 64 / 8 heads of 96, fp8, 28 against 41 us); with the estimate 235 are.
+  // The margins are where the excess over the better kernel, summed over equal and spread batches, is least
+  // (2.7 % a batch without the estimate, 1.6 % with it): 0.1 less loses more on spread batches.
   const double D = a.head_size, es = a.kv_dtype == B200PA_KV_AUTO ? 2 : 1, us = 1 / 6.5e6;  // (bytes to us)
   const int64_t resident = int64_t(sm_count()) * ki.resident;
   const double waves = double((ctas + resident - 1) / resident);
   const double latency = (es == 1 ? 0.63 + 0.0037 * D : 0.43 + 0.0061 * D) * (head_tiles == 2 ? 1.4 : 1);
-  const double hbm = 0.85 * 32 * D * es * kDirectWarps * double(std::min(ctas, resident)) * us;
+  const double wide = 32 * D * es < 16384 ? 1 : a.block_size == 16 ? 1.15 : 1.3;
+  const double hbm = 0.85 * wide * 32 * D * es * kDirectWarps * double(std::min(ctas, resident)) * us;
   const double direct = 10 + waves * double(per_warp) * std::max(latency, hbm) + 3 * (waves - 1);
   const double bytes = double(a.num_seqs) * a.num_kv_heads * a.max_seq_len * 2 * D * es;
-  const double persistent = 20 + 1.25 * (a.num_heads / a.num_kv_heads) + 0.89 * bytes * us * (waves > 1 ? 1 : 0.75);
-  const double margin = waves == 1 ? 1.1 : ctas * 10 <= resident * 12 ? 1.15 : 1.05;
+  const double merge = (items < 12 * int64_t(sm_count()) ? 1.25 : 0.6) * (a.num_heads / a.num_kv_heads);
+  const double persistent = 20 + merge + 0.89 * bytes * us * (waves > 1 ? 1 : 0.75);
+  const double margin = waves == 1 ? 1.1 : ctas * 10 <= resident * 12 ? 1.25 : 1.15;
   return {cluster, direct <= margin * persistent};
 }
 
