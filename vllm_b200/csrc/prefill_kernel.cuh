@@ -19,6 +19,11 @@
 //     transposition.  P goes back to TMEM as the A operand of the second product, over S.
 //   * The two row tiles take turns: while the softmax of one runs, the tensor cores work for the
 //     other.
+//   * A thread takes its whole row of S into registers (one TMEM read, paired fp32 arithmetic,
+//     three-way maxima), so the maximum is known before the first exponential, and P is handed over
+//     in two halves: the product of the first runs under the exponentials of the second.  (Two reads of
+//     S, or exponentials ahead of the maximum: step below 475 us, 443 so; fp8 caches and ALiBi, which
+//     read S twice, 5 to 20 % more than this one on steps of short chunks.)
 //   * The running maximum is only raised (and O rescaled in TMEM) when a row's maximum grew by more
 //     than 2^8: until then P is merely larger than 1, which fp32 sums and 16-bit P hold as exactly.
 //   * fp8 caches are widened to f16 (exact) by the producers on their way to shared memory.
@@ -114,7 +119,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
   constexpr int kWs = 128 * (D * 2 + 8);  // workspace of one row tile's partial: O, then (m, l)
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ int cum[kPrefillMaxReqs + 1];  // 2 x (items before request r), + 1 if it is cut into pieces
-  __shared__ uint64_t s_bar[2 * NS + 12];
+  __shared__ uint64_t s_bar[2 * NS + 14];
   __shared__ int s_item[2];
   __shared__ uint32_t s_tmem;
   __shared__ int s_red[3][16];
@@ -131,6 +136,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
   auto q_full = [&](int i) { return bar0 + 8u * (2 * NS + 6 + i); };
   auto item_full = [&](int i) { return bar0 + 8u * (2 * NS + 8 + i); };
   auto item_empty = [&](int i) { return bar0 + 8u * (2 * NS + 10 + i); };
+  auto p_half = [&](int i) { return bar0 + 8u * (2 * NS + 12 + i); };
 
   const uint32_t sq = smem_u32(smem_raw);
   const uint32_t skv = sq + NQ * SH::kQBytes;
@@ -144,6 +150,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
       }
       for (int i = 0; i < 2; ++i) {
         mbar_init(s_full(i), 1);
+        mbar_init(p_half(i), 4);
         mbar_init(p_full(i), 4);
         mbar_init(pv_done(i), 1);
         mbar_init(q_full(i), 4);
@@ -322,6 +329,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
     const uint32_t t_s = tmem + lane_off + uint32_t(wg * KT);
     const uint32_t t_o = tmem + lane_off + uint32_t(NQ * KT + wg * DP);
     const float c = p.scale * kLog2e * (kFp8 ? *p.k_scale : 1.f);
+    const bool biased = p.alibi != nullptr || !(c > 0.f);  // the maximum is taken of the scaled values then
     const float v_scale = kFp8 ? *p.v_scale : 1.f;
     const bool row_used = wg < NQ && row < T * G;
     const int row_tok = row / G, row_head = row % G;
@@ -395,86 +403,37 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
         if (!wait(s_full(wg), n_s & 1)) break;
         ++n_s;
         tc_fence_after();
+        // The whole row of S goes to registers at once: its maximum is known before the first
+        // exponential, S is read once, and P can be handed over in parts.
+        constexpr int NC = KT / 32;
+        float x[NC][32];
+#pragma unroll
+        for (int ch = 0; ch < NC; ++ch) tmem_ld32(t_s + ch * 32, x[ch]);
         const int key0 = j * KT;
-        // No bias: only the tiles at the causal edge of a row tile need a mask.
-        const bool plain = p.alibi == nullptr && c > 0.f;
-        const bool edge = key0 + KT - 1 > pos_first;
         int last = pos - key0;  // last column of this row that counts
-        float cc = c;           // (goes through the waits for TMEM loads, see tmem_landed)
-        auto mask = [&](float (&x)[32], int ch) {
-          if (edge) {
-#pragma unroll
-            for (int k = 0; k < 32; ++k) x[k] = k <= last - ch * 32 ? x[k] : -INFINITY;
-          }
-        };
-        // with a bias: t = x c + slope (key - pos), and the mask
-        auto biased = [&](float x, int ch, int k) {
-          const int first = ch * 32 - last;  // (of this row: key - pos of column 0)
-          return first + k <= 0 ? fmaf(slope, float(k), fmaf(x, cc, slope * float(first))) : -INFINITY;
-        };
-        float mx = -INFINITY;
-        constexpr int NC = KT / 32;  // 32-column chunks: one is on its way while another is worked on
+        float cc = c;           // (goes through the wait for the TMEM loads, see tmem_landed)
         float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-        float s4[4] = {0.f, 0.f, 0.f, 0.f};
-        float v[2][32];
-        if (!kFp8 && plain && j > b) {
-          // After the first tile the running maximum mostly stands: take it as it is, and look at this
-          // tile's maximum while the exponentials run.  P waits in registers, S stays intact; a
-          // maximum that grew sends the tile through the two passes below.  (3 % at head size 128; not
-          // for fp8 caches, whose producers need the registers.)
-          const float mm = m == -INFINITY ? 0.f : m;
-          uint32_t w[NC][16];
-          tmem_ld32(t_s, v[0]);
+        tmem_landed(m4, cc, last);
+        if (biased) {  // t = x c + slope (key - pos)
+          const float base = slope * -float(last);
 #pragma unroll
-          for (int ch = 0; ch < NC; ++ch) {
-            float (&x)[32] = v[ch & 1];
-            tmem_landed(m4, cc, last);
-            if (ch + 1 < NC) tmem_ld32(t_s + (ch + 1) * 32, v[(ch + 1) & 1]);
-            mask(x, ch);
+          for (int ch = 0; ch < NC; ++ch)
 #pragma unroll
-            for (int k = 0; k < 32; k += 2) {
-              m4[k & 2] = fmaxf(m4[k & 2], x[k]);
-              m4[(k & 2) + 1] = fmaxf(m4[(k & 2) + 1], x[k + 1]);
-              const float p0 = fast_exp2(fmaf(x[k], cc, -mm)), p1 = fast_exp2(fmaf(x[k + 1], cc, -mm));
-              s4[k & 2] += p0;
-              s4[(k & 2) + 1] += p1;
-              w[ch][k / 2] = pack2<kBf>(p0, p1);
-            }
-          }
-          mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * c;
-          if (!__any_sync(0xffffffffu, mx > m + 8.f || (m == -INFINITY && mx > m))) {
-#pragma unroll
-            for (int ch = 0; ch < NC; ++ch) tmem_st16(t_s + ch * 16, w[ch]);
-            l += (s4[0] + s4[1]) + (s4[2] + s4[3]);
-            tmem_wait_st();
-            tc_fence_before();
-            arrive(p_full(wg));
-            ++n_pv;
-            continue;
-          }
-          s4[0] = s4[1] = s4[2] = s4[3] = 0.f;
-        } else if (plain) {
-          tmem_ld32(t_s, v[0]);
-#pragma unroll
-          for (int ch = 0; ch < NC; ++ch) {
-            float (&x)[32] = v[ch & 1];
-            tmem_landed(m4, cc, last);
-            if (ch + 1 < NC) tmem_ld32(t_s + (ch + 1) * 32, v[(ch + 1) & 1]);
-            mask(x, ch);
-#pragma unroll
-            for (int k = 0; k < 32; ++k) m4[k & 3] = fmaxf(m4[k & 3], x[k]);
-          }
-          mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * c;
-        } else {
-#pragma unroll 1
-          for (int ch = 0; ch < NC; ++ch) {
-            tmem_ld32(t_s + ch * 32, v[0]);
-            tmem_landed(m4, cc, last);
-#pragma unroll
-            for (int k = 0; k < 32; ++k) m4[k & 3] = fmaxf(m4[k & 3], biased(v[0][k], ch, k));
-          }
-          mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+            for (int k = 0; k < 32; ++k) x[ch][k] = fmaf(slope, float(ch * 32 + k), fmaf(x[ch][k], cc, base));
+          cc = 1.f;
         }
+        if (key0 + KT - 1 > pos_first) {  // only the tiles at the causal edge of a row tile need a mask
+          asm volatile("");               // (a branch in fact, not 128 selects for every tile)
+#pragma unroll
+          for (int ch = 0; ch < NC; ++ch)
+#pragma unroll
+            for (int k = 0; k < 32; ++k) x[ch][k] = ch * 32 + k <= last ? x[ch][k] : -INFINITY;
+        }
+#pragma unroll
+        for (int ch = 0; ch < NC; ++ch)
+#pragma unroll
+          for (int k = 0; k < 32; k += 2) m4[k / 2 & 3] = fmax3(m4[k / 2 & 3], x[ch][k], x[ch][k + 1]);
+        const float mx = fmax3(fmaxf(m4[0], m4[1]), m4[2], m4[3]) * cc;
         // raise the maximum (and rescale what has been summed) only when it grew by more than 8
         const bool grow = mx > m + 8.f || (m == -INFINITY && mx > m);
         if (__any_sync(0xffffffffu, grow)) {
@@ -496,48 +455,27 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
             tmem_wait_st();
           }
         }
-        const float mm = m == -INFINITY ? 0.f : m;
-        // (P's columns lie over S columns that have been read: 16 a chunk over 32)
-        if (plain) {
-          tmem_ld32(t_s, v[0]);
+        const float nm = m == -INFINITY ? 0.f : -m;
+        float2 sa = make_float2(0.f, 0.f), sb = make_float2(0.f, 0.f);
+        // (P's columns lie over S columns: 16 a chunk of 32)
 #pragma unroll
-          for (int ch = 0; ch < NC; ++ch) {
-            float (&x)[32] = v[ch & 1];
-            tmem_landed(s4, cc, last);
-            if (ch + 1 < NC) tmem_ld32(t_s + (ch + 1) * 32, v[(ch + 1) & 1]);
-            mask(x, ch);
-            uint32_t w[16];
+        for (int ch = 0; ch < NC; ++ch) {
+          uint32_t w[16];
 #pragma unroll
-            for (int k = 0; k < 32; k += 2) {
-              const float p0 = fast_exp2(fmaf(x[k], cc, -mm)), p1 = fast_exp2(fmaf(x[k + 1], cc, -mm));
-              s4[k & 2] += p0;
-              s4[(k & 2) + 1] += p1;
-              w[k / 2] = pack2<kBf>(p0, p1);
-            }
-            tmem_st16(t_s + ch * 16, w);
+          for (int k = 0; k < 32; k += 2) {
+            const float2 t = ffma2(make_float2(x[ch][k], x[ch][k + 1]), make_float2(cc, cc), make_float2(nm, nm));
+            const float2 e2 = make_float2(fast_exp2(t.x), fast_exp2(t.y));
+            if (k & 2) sb = fadd2(sb, e2); else sa = fadd2(sa, e2);
+            w[k / 2] = pack2<kBf>(e2.x, e2.y);
           }
-        } else {
-#pragma unroll 1
-          for (int ch = 0; ch < NC; ++ch) {
-            tmem_ld32(t_s + ch * 32, v[0]);
-            tmem_landed(s4, cc, last);
-            uint32_t w[16];
-#pragma unroll
-            for (int k = 0; k < 32; k += 2) {
-              const float p0 = fast_exp2(biased(v[0][k], ch, k) - mm);
-              const float p1 = fast_exp2(biased(v[0][k + 1], ch, k + 1) - mm);
-              s4[k & 2] += p0;
-              s4[(k & 2) + 1] += p1;
-              w[k / 2] = pack2<kBf>(p0, p1);
-            }
-            tmem_st16(t_s + ch * 16, w);
+          tmem_st16(t_s + ch * 16, w);
+          if (ch == NC / 2 - 1 || ch == NC - 1) {
+            tmem_wait_st();
+            tc_fence_before();
+            arrive(ch == NC - 1 ? p_full(wg) : p_half(wg));
           }
         }
-        const float sum = (s4[0] + s4[1]) + (s4[2] + s4[3]);
-        l += sum;
-        tmem_wait_st();
-        tc_fence_before();
-        arrive(p_full(wg));
+        l += (sa.x + sa.y) + (sb.x + sb.y);
         ++n_pv;
       }
       if (!ok) break;
@@ -890,13 +828,17 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
       }
       __syncwarp();
     };
-    auto pv = [&](int i, uint32_t h, bool more) {
+    // half of the keys of a tile: the first while the softmax works on the second
+    auto pv = [&](int i, uint32_t h, int half, bool more) {
       const uint64_t vd = v_desc + uniform((h % NS) * (SH::kTileBytes >> 4));
       if (elect_one()) {
+        constexpr int NK = KT / 32;
 #pragma unroll
-        for (int ks = 0; ks < KT / 16; ++ks)
+        for (int k = 0; k < NK; ++k) {
+          const int ks = half * NK + k;
           mma_ts(tmem + NQ * KT + i * DP, tmem + i * KT + ks * 8, vd + ks * 2 * DP, idesc_o, more || ks > 0);
-        mma_commit(pv_done(i));
+        }
+        if (half == 1) mma_commit(pv_done(i));
       }
       __syncwarp();
     };
@@ -940,10 +882,13 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
           const int ei = i == 0 ? it.e0 : it.e1;
           uint32_t& n_p = i == 0 ? n_p0 : n_p1;
           if (!ok || j >= ei) continue;
+          if (!wait(p_half(i), n_p & 1)) continue;
+          tc_fence_after();
+          pv(i, n_h, 0, j > it.b);
           if (!wait(p_full(i), n_p & 1)) continue;
           ++n_p;
           tc_fence_after();
-          pv(i, n_h, j > it.b);
+          pv(i, n_h, 1, true);
           if (j + 1 < ei) {
             if (!have_k && !wait_half(n_h + 1)) continue;
             have_k = true;
