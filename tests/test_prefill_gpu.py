@@ -106,6 +106,13 @@ def test_tile_edges(H, HK, q, ctx):
     _case([q, 0, q], [ctx, 7, 0], H, HK, 128, 16, torch.bfloat16, "auto", seed=q)
 
 
+# V comes in pages of 16 keys: the last one of a sequence is cut at every length, the pages behind it do not exist
+@pytest.mark.parametrize("D", [64, 120, 192])
+@pytest.mark.parametrize("B", [16, 32])
+def test_sequences_that_end_anywhere_in_a_page(D, B):
+    _case([3 + i % 7 for i in range(40)], [110 + i for i in range(40)], 8, 2, D, B, torch.bfloat16, "auto", seed=B)
+
+
 @pytest.mark.parametrize("kv", ["auto", "fp8"])
 def test_few_rows_behind_long_contexts_are_split(kv):
     _case([5, 2, 40], [9000, 3000, 20000], 8, 2, 128, 16, torch.bfloat16, kv)

@@ -13,6 +13,11 @@ struct PrefillKernelInfo {
   int piece_bytes;  // workspace of one piece of an item
 };
 
+// Tensor map of a 16-bit V cache: [block][kv head][D][block_size], boxes of 16 keys x D.  The number of
+// blocks is not known here: block ids are taken as they come, as everywhere.  Defined in
+// varlen_attention.cu.
+cudaError_t prefill_v_map(const PrefillParams& p, int head_size, CUtensorMap* map);
+
 template <typename QT, int KV, int D>
 cudaError_t prefill_launch(const PrefillParams& p, int grid, cudaStream_t stream) {
   auto kern = pa_prefill_kernel<QT, KV, D>;
@@ -30,7 +35,12 @@ cudaError_t prefill_launch(const PrefillParams& p, int grid, cudaStream_t stream
     }
     if (dev >= 0 && dev < 64) done[dev] = true;
   }
-  return launch_dependent(kern, dim3(grid), dim3(kPrefillThreads), smem, stream, p);
+  CUtensorMap map = {};
+  if constexpr (KV == kCache16) {
+    e = prefill_v_map(p, D, &map);
+    if (e != cudaSuccess) return e;
+  }
+  return launch_dependent(kern, dim3(grid), dim3(kPrefillThreads), smem, stream, p, map);
 }
 
 template <typename QT, int D>

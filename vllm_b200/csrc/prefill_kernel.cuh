@@ -36,6 +36,8 @@
 // KV write included): 8970 us with one decode work item per token, 525 us here (766 TFLOP/s).
 #pragma once
 
+#include <cuda.h>
+
 #include <type_traits>
 
 #include "decode_kernel.cuh"
@@ -79,7 +81,7 @@ constexpr int kPrefillThreads = 16 * 32;  // (three warps beside the MMA warp on
 // fp8 step of 64 / 8 heads takes 1032 us with 176 / 112 / 48 and 997 with 184 / 104 / 40.)
 template <bool kFp8>
 struct PrefillRegs {
-  static constexpr int kSoftmax = 184, kProducer = kFp8 ? 104 : 88, kMma = kFp8 ? 40 : 56;
+  static constexpr int kSoftmax = kFp8 ? 184 : 192, kProducer = kFp8 ? 104 : 80, kMma = kFp8 ? 40 : 48;
   static_assert(2 * kSoftmax + kProducer + kMma == 4 * 128, "register split");
 };
 constexpr int kPrefillMaxReqs = 512;    // requests per launch: prefix table in shared memory
@@ -94,7 +96,7 @@ struct PrefillShape {
   // ring of K and V tiles in turns (K0, V0, K1, V1, ...): what shared memory holds besides Q
   static constexpr int kRoom = 223 * 1024 - NQ * kQBytes;
   static constexpr int kSlots = kRoom / kTileBytes < 8 ? kRoom / kTileBytes : 8;
-  static constexpr int kSmem = NQ * kQBytes + kSlots * kTileBytes;
+  static constexpr int kSmem = 256 + NQ * kQBytes + kSlots * kTileBytes;  // (256: alignment)
   static_assert(kSlots >= 4, "a K and a V tile in use, another of each on its way");
   static_assert(NQ * (KT + DP) <= 512, "TMEM columns");
 };
@@ -109,7 +111,8 @@ struct PrefillItem {
 };
 
 template <typename QT, int KV, int D>
-__global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const PrefillParams p) {
+__global__ void __launch_bounds__(kPrefillThreads, 1)
+pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vmap) {
   using SH = PrefillShape<D>;
   constexpr bool kFp8 = KV != kCache16;
   constexpr bool kE5 = KV == kCacheE5M2;
@@ -119,7 +122,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
   constexpr int kWs = 128 * (D * 2 + 8);  // workspace of one row tile's partial: O, then (m, l)
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ int cum[kPrefillMaxReqs + 1];  // 2 x (items before request r), + 1 if it is cut into pieces
-  __shared__ uint64_t s_bar[2 * NS + 14];
+  __shared__ uint64_t s_bar[2 * NS + 15];
   __shared__ int s_item[2];
   __shared__ uint32_t s_tmem;
   __shared__ int s_red[3][16];
@@ -137,8 +140,10 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
   auto item_full = [&](int i) { return bar0 + 8u * (2 * NS + 8 + i); };
   auto item_empty = [&](int i) { return bar0 + 8u * (2 * NS + 10 + i); };
   auto p_half = [&](int i) { return bar0 + 8u * (2 * NS + 12 + i); };
+  const uint32_t tail_bar = bar0 + 8u * (2 * NS + 14);
 
-  const uint32_t sq = smem_u32(smem_raw);
+  unsigned char* const smem = smem_raw + (-smem_u32(smem_raw) & 255u);  // (V's swizzle goes by address bits 4 .. 7)
+  const uint32_t sq = smem_u32(smem);
   const uint32_t skv = sq + NQ * SH::kQBytes;
 
   if (warp == 12) {
@@ -157,16 +162,21 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
         mbar_init(item_full(i), 1);
         mbar_init(item_empty(i), 12);
       }
+      mbar_init(tail_bar, 1);
       fence_barrier_init();
     }
     __syncwarp();
     tmem_alloc(smem_u32(&s_tmem), 512);
   }
   if constexpr (DP != D) {
-    // Q's padding granules take part in the product: zero, once (nobody writes them; K's are zeroed
-    // with every tile, V's padding only gives columns that are dropped)
+    // The padding granules of Q and K take part in the product: zero, once (nobody writes them: K sits
+    // in the even slots of the ring, and V's padding only gives columns that are dropped).
+    static_assert(DP - D == 8 && NS % 2 == 0, "one padding granule; K and V in slots of their own");
     for (int i = tid; i < NQ * 128; i += kPrefillThreads)
-      *reinterpret_cast<uint4*>(smem_raw + (i / 128) * SH::kQBytes + (D / 8) * 128 * 16 + (i % 128) * 16) =
+      *reinterpret_cast<uint4*>(smem + (i / 128) * SH::kQBytes + (D / 8) * 128 * 16 + (i % 128) * 16) =
+          make_uint4(0, 0, 0, 0);
+    for (int i = tid; i < NS / 2 * KT; i += kPrefillThreads)
+      *reinterpret_cast<uint4*>(smem + NQ * SH::kQBytes + (i / KT) * 2 * SH::kTileBytes + ((D / 8) * KT + i % KT) * 16) =
           make_uint4(0, 0, 0, 0);
     fence_proxy_async();
   }
@@ -614,24 +624,24 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
     reg_dec<PrefillRegs<kFp8>::kProducer>();
     const int pt = tid - 256;  // 0 .. 127
     uint32_t n_half = 0;       // halves (K or V tiles) put on their way
-    uint32_t n_done = 0;       // ... and announced (16-bit caches)
+    uint32_t n_tail = 0;       // last tiles of a sequence that ended inside a page
     const char* kb = static_cast<const char*>(p.kc);
     const char* vb = static_cast<const char*>(p.vc);
     constexpr int ES = kFp8 ? 1 : 2;
-    // 16-bit caches: halves are announced in order, when their copies have landed.  Up to two stay on
-    // their way while there is something else to issue; before the warp waits for anything, all of
-    // them are announced (the MMAs may be waiting for just those).
+    // K tiles of 16-bit caches are announced when their copies have landed, up to two later; before
+    // the warp waits for anything, all of them are (the MMAs may be waiting for just those).
+    uint32_t n_k = 0, n_told = 0;  // K tiles put on their way, announced
     auto announce = [&]() {
       fence_proxy_async();
-      arrive(kv_full(n_done % NS));
-      ++n_done;
+      arrive(kv_full(2 * n_told % NS));
+      ++n_told;
     };
     auto announce_all = [&]() {
-      if (n_half - n_done >= 2) {
+      if (n_k - n_told >= 2) {
         cp_async_wait<1>();
-        while (n_half - n_done > 1) announce();
+        while (n_k - n_told > 1) announce();
       }
-      if (n_half != n_done) {
+      if (n_k != n_told) {
         cp_async_wait<0>();
         announce();
       }
@@ -656,13 +666,15 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
         return base + int64_t(blk) * p.kv_block_stride * ES + head_off;
       };
       if constexpr (!kFp8) {
-        // K: a thread owns one key and walks along its 16-byte granules; V: a thread owns 8 keys
-        // and every 8th head dimension (128 bytes of shared memory per 8 threads in both cases).
+        // K: a thread owns one key and walks along its 16-byte granules (128 bytes of shared memory per
+        // 8 threads).  V: pages of 16 keys, each one copy by tensor map, whose rows of 16 keys are a K
+        // step of the product (32-byte swizzle); issued by the first warp.  (V by 16-byte cp.async came
+        // in half sectors and kept the load/store unit from the softmax: 8192-token step 444 -> 392 us.  K
+        // by bulk copies of 256 bytes, the run of a granule in a page, takes 835: 128 of them a tile.)
+        constexpr int NP = KT / 16;  // pages per tile
         const int kt = pt % KT, kg = pt / KT;
-        constexpr int VJ = KT / 8;              // 8-key groups per tile
-        const int vj = pt / 8 % VJ, vd = pt % 8 + 8 * (pt / 8 / VJ);
-        int k_blk = block_of(it.b * KT + kt), v_blk = block_of(it.b * KT + vj * 8);
-        for (int j = it.b; j < e; ++j) {
+        int k_blk = block_of(it.b * KT + kt), v_blk = block_of(it.b * KT + lane % NP * 16);
+        for (int j = it.b; j < e && ok; ++j) {
           {
             const int key = j * KT + kt;
             const char* src = page(kb, k_blk) + (kg * B + (key & (B - 1))) * 16;
@@ -671,38 +683,60 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
             if (!wait_slot(n_half)) break;
             uint32_t dst = slot_of(n_half) + (kg * KT + kt) * 16;
 #pragma unroll 4
-            for (int g = kg; g < DP / 8; g += 128 / KT) {
-              cp_async16(dst, src, DP == D || g < D / 8 ? bytes : 0);
+            for (int g = kg; g < D / 8; g += 128 / KT) {
+              cp_async16(dst, src, bytes);
               dst += 128 * 16;
               src += (128 / KT) * B * 16;
             }
             cp_async_commit();
             ++n_half;
-            if (n_half - n_done > 2) {
-              cp_async_wait<2>();
+            ++n_k;
+            if (n_k - n_told > 1) {
+              cp_async_wait<1>();
               announce();
             }
           }
+          const int key = j * KT + lane % NP * 16;
+          const int cur = v_blk;
+          if (j + 1 < e) v_blk = block_of(key + KT);
+          if (!wait_slot(n_half)) break;
           {
-            const int key = j * KT + vj * 8;
-            const char* src = page(vb, v_blk) + (vd * B + (key & (B - 1))) * 2;
-            const int bytes = max(0, min(16, (it.seq_len - key) * 2));  // keys past the end: zeros
-            if (j + 1 < e) v_blk = block_of(key + KT);
-            if (!wait_slot(n_half)) break;
-            uint32_t dst = slot_of(n_half) + (vj * DP + vd) * 16;
-            constexpr int VS = 8 * (16 / VJ);
-#pragma unroll 4
-            for (int d = 0; d < D; d += VS) {
-              if (D % VS == 0 || d + vd < D) cp_async16(dst, src, bytes);
-              dst += VS * 16;
-              src += VS * B * 2;
+            // only pages with a key of the sequence are copied
+            const int pages = min(NP, (it.seq_len - j * KT + 15) / 16);
+            const int left = it.seq_len - j * KT - (pages - 1) * 16;  // keys of the last page that exist
+            const bool cut = left < 16;
+            const uint32_t full = kv_full(n_half % NS), bar = cut ? tail_bar : full;
+            if (warp != 8) {
+              arrive(full);
+              ++n_half;
+              continue;
             }
-            cp_async_commit();
+            if (lane == 0) mbar_expect_tx(bar, pages * D * 32);
+            __syncwarp();
+            if (lane < pages) tma_load4(slot_of(n_half) + lane * DP * 32, &vmap, key & (B - 1), 0, it.kvh, cur, bar);
+            __syncwarp();
+            if (cut) {
+              // keys past the end become zeros (stale bytes could be NaN)
+              announce_all();
+              if (!wait(bar, n_tail++ & 1)) break;
+              const uint32_t last = slot_of(n_half) + (pages - 1) * DP * 32;
+              for (int d = lane; d < D; d += 32) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                  const uint32_t at = last + d * 32 + (h ^ (d >> 2 & 1)) * 16;
+                  const int n = left - 8 * h;  // keys of this half row that exist
+                  uint4 x = ld_shared16(at);
+                  x.x = n >= 2 ? x.x : (n == 1 ? x.x & 0xffffu : 0u);
+                  x.y = n >= 4 ? x.y : (n == 3 ? x.y & 0xffffu : 0u);
+                  x.z = n >= 6 ? x.z : (n == 5 ? x.z & 0xffffu : 0u);
+                  x.w = n >= 8 ? x.w : (n == 7 ? x.w & 0xffffu : 0u);
+                  st_shared16(at, x);
+                }
+              }
+              fence_proxy_async();
+              arrive(full);
+            }
             ++n_half;
-            if (n_half - n_done > 2) {
-              cp_async_wait<2>();
-              announce();
-            }
           }
         }
       } else {
@@ -797,7 +831,11 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
       if constexpr (!kFp8) announce_all();  // (the next item may be drawn only when they have arrived)
       item = next_item();
     }
-    if constexpr (!kFp8) cp_async_wait_all();
+    if constexpr (!kFp8) {  // nobody leaves with copies on their way (after a wait that ran out, too)
+      cp_async_wait_all();
+      if (warp == 8)
+        for (uint32_t h = n_half < NS ? 0 : n_half - NS; h < n_half; ++h) mbar_spin(kv_full(h % NS), (h / NS) & 1);
+    }
   } else {
     reg_dec<PrefillRegs<kFp8>::kMma>();
     if (warp == 12) {
@@ -815,7 +853,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
     };
     const uint64_t q_desc = smem_desc(sq, 128 * 16, 128);
     const uint64_t k_desc = smem_desc(skv, KT * 16, 128);
-    const uint64_t v_desc = smem_desc(skv, DP * 16, 128);
+    const uint64_t v_desc = kFp8 ? smem_desc(skv, DP * 16, 128) : smem_desc_sw32(skv, 256);
     auto wait_half = [&](uint32_t h) { return wait(kv_full(h % NS), (h / NS) & 1); };
     auto qk = [&](int i, uint32_t h) {
       const uint64_t kd = k_desc + uniform((h % NS) * (SH::kTileBytes >> 4));
@@ -828,15 +866,17 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
       }
       __syncwarp();
     };
-    // half of the keys of a tile: the first while the softmax works on the second
-    auto pv = [&](int i, uint32_t h, int half, bool more) {
+    // half of the keys of a tile: the first while the softmax works on the second (`steps`: pages of 16
+    // keys that the tile has)
+    auto pv = [&](int i, uint32_t h, int half, int steps, bool more) {
       const uint64_t vd = v_desc + uniform((h % NS) * (SH::kTileBytes >> 4));
       if (elect_one()) {
         constexpr int NK = KT / 32;
 #pragma unroll
         for (int k = 0; k < NK; ++k) {
           const int ks = half * NK + k;
-          mma_ts(tmem + NQ * KT + i * DP, tmem + i * KT + ks * 8, vd + ks * 2 * DP, idesc_o, more || ks > 0);
+          if (kFp8 || ks < steps)
+            mma_ts(tmem + NQ * KT + i * DP, tmem + i * KT + ks * 8, vd + ks * 2 * DP, idesc_o, more || ks > 0);
         }
         if (half == 1) mma_commit(pv_done(i));
       }
@@ -877,6 +917,7 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
         // V tile j is half n_h, K tile j + 1 half n_h + 1
         if (!wait_half(n_h)) break;
         bool have_k = false;
+        const int steps = (it.seq_len - j * KT + 15) / 16;
 #pragma unroll
         for (int i = 0; i < NQ; ++i) {
           const int ei = i == 0 ? it.e0 : it.e1;
@@ -884,11 +925,11 @@ __global__ void __launch_bounds__(kPrefillThreads, 1) pa_prefill_kernel(const Pr
           if (!ok || j >= ei) continue;
           if (!wait(p_half(i), n_p & 1)) continue;
           tc_fence_after();
-          pv(i, n_h, 0, j > it.b);
+          pv(i, n_h, 0, steps, j > it.b);
           if (!wait(p_full(i), n_p & 1)) continue;
           ++n_p;
           tc_fence_after();
-          pv(i, n_h, 1, true);
+          pv(i, n_h, 1, steps, true);
           if (j + 1 < ei) {
             if (!have_k && !wait_half(n_h + 1)) continue;
             have_k = true;

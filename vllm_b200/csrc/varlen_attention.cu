@@ -8,14 +8,39 @@
 
 namespace b200pa {
 
+cudaError_t prefill_v_map(const PrefillParams& p, int head_size, CUtensorMap* map) {
+  using Encode = decltype(&cuTensorMapEncodeTiled);
+  static const Encode encode = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess)
+      f = nullptr;
+    return reinterpret_cast<Encode>(f);
+  }();
+  if (encode == nullptr) return cudaErrorNotSupported;
+  const cuuint64_t dims[4] = {cuuint64_t(p.block_size), cuuint64_t(head_size), cuuint64_t(p.num_kv_heads),
+                              cuuint64_t(INT32_MAX)};
+  const cuuint64_t strides[3] = {cuuint64_t(p.block_size) * 2, cuuint64_t(p.kv_head_stride) * 2,
+                                 cuuint64_t(p.kv_block_stride) * 2};
+  const cuuint32_t box[4] = {16, cuuint32_t(head_size), 1, 1}, step[4] = {1, 1, 1, 1};
+  const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 4, const_cast<void*>(p.vc), dims, strides, box, step,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
 // The prefill kernel for a call's shape and alignments, or none.  16-byte accesses: pages, rows of Q and
-// of the output; cache offsets inside a block are shifts.
+// of the output; cache offsets inside a block are shifts.  The strides of a 16-bit cache have to fit a tensor
+// map (positive, below 2^40 bytes).
 static PrefillKernelInfo find_prefill(const b200pa_attn_args& a) {
   const int es = a.kv_dtype == B200PA_KV_AUTO ? 2 : 1;
   auto al = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr) % 16 == 0; };
+  auto stride_fits = [](int64_t v) { return v > 0 && v < (int64_t(1) << 39); };  // 2-byte elements
   const bool fits = (a.block_size == 16 || a.block_size == 32) && a.num_heads / a.num_kv_heads <= 128 &&
                     al(a.key_cache) && al(a.value_cache) && al(a.query) && al(a.out) &&
                     (a.kv_block_stride * es) % 16 == 0 && (a.kv_head_stride * es) % 16 == 0 &&
+                    (es == 1 || (stride_fits(a.kv_block_stride) && stride_fits(a.kv_head_stride))) &&
                     a.q_stride % 8 == 0 && a.blocksparse_vert_stride <= 1 && a.out_lse == nullptr;
   if (!fits) return {nullptr, 0};
   return a.head_size <= 96 ? find_prefill_small(a.head_size, a.q_dtype, a.kv_dtype)
