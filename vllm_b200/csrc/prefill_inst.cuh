@@ -13,10 +13,12 @@ struct PrefillKernelInfo {
   int piece_bytes;  // workspace of one piece of an item
 };
 
-// Tensor map of a 16-bit V cache: [block][kv head][D][block_size], boxes of 16 keys x D.  The number of
-// blocks is not known here: block ids are taken as they come, as everywhere.  Defined in
+// Tensor maps.  V of a 16-bit cache: [block][kv head][D][block_size], boxes of 16 keys x D.  The number
+// of blocks is not known here: block ids are taken as they come, as everywhere.  Q: [token][head][D],
+// boxes of `box` head dimensions x the heads of a group x the tokens of a row tile.  Defined in
 // varlen_attention.cu.
 cudaError_t prefill_v_map(const PrefillParams& p, int head_size, CUtensorMap* map);
+cudaError_t prefill_q_map(const PrefillParams& p, int head_size, int box, CUtensorMap* map);
 
 template <typename QT, int KV, int D>
 cudaError_t prefill_launch(const PrefillParams& p, int grid, cudaStream_t stream) {
@@ -35,12 +37,11 @@ cudaError_t prefill_launch(const PrefillParams& p, int grid, cudaStream_t stream
     }
     if (dev >= 0 && dev < 64) done[dev] = true;
   }
-  CUtensorMap map = {};
-  if constexpr (KV == kCache16) {
-    e = prefill_v_map(p, D, &map);
-    if (e != cudaSuccess) return e;
-  }
-  return launch_dependent(kern, dim3(grid), dim3(kPrefillThreads), smem, stream, p, map);
+  CUtensorMap qmap, vmap = {};
+  e = prefill_q_map(p, D, PrefillShape<D>::kQBox, &qmap);
+  if (KV == kCache16 && e == cudaSuccess) e = prefill_v_map(p, D, &vmap);
+  if (e != cudaSuccess) return e;
+  return launch_dependent(kern, dim3(grid), dim3(kPrefillThreads), smem, stream, p, qmap, vmap);
 }
 
 template <typename QT, int D>

@@ -9,14 +9,16 @@
 // 256 query rows.
 //
 //   * One persistent CTA per SM: two softmax warpgroups (one thread per query row), one
-//     producer warpgroup, one warp that issues the MMAs.
+//     producer warpgroup for K and V, one warp that issues the MMAs, one that draws work items and
+//     works out what they cover, one (two for fp8) that brings Q.
 //   * A work item is (request, 2 x 128 query rows, kv head).  A row is one (token, query head of the
 //     group): the heads that share a kv head are packed into the rows of a tile, so K/V are fetched
 //     once for all of them, and the causal edge of a tile is only 128 / group tokens wide.
-//   * S = Q.K^T and O += P.V are tcgen05.mma (M = 128, fp32 accumulators in TMEM).  Q, K and V sit in
-//     shared memory as [16-byte granule along K][row][16 bytes]: the no-swizzle K-major operand
-//     layout, which is what the x-layout of the K cache and 8-token pieces of V rows give without any
-//     transposition.  P goes back to TMEM as the A operand of the second product, over S.
+//   * S = Q.K^T and O += P.V are tcgen05.mma (M = 128, fp32 accumulators in TMEM).  K sits in shared
+//     memory as [16-byte granule along D][key][16 bytes], the no-swizzle K-major operand layout, which the
+//     x-layout of the K cache gives without any transposition; V as its pages lie, with 32-byte swizzle
+//     (fp8 caches: widened, [8 keys][D][16 bytes]); Q as tensor-map boxes with swizzle.  P goes back to
+//     TMEM as the A operand of the second product, over S.
 //   * The two row tiles take turns: while the softmax of one runs, the tensor cores work for the
 //     other.
 //   * A thread takes its whole row of S into registers (one TMEM read, paired fp32 arithmetic,
@@ -33,7 +35,10 @@
 //   * Every mbarrier wait is bounded; on expiry a status code is recorded and all roles leave.
 //
 // Measured on B200, a step of 4 chunks (8192 tokens, contexts up to 4096, 32 / 8 heads of 128, bf16;
-// KV write included): 8970 us with one decode work item per token, 525 us here (766 TFLOP/s).
+// KV write included): 8970 us with one decode work item per token, 361 us here (1110 TFLOP/s).  Start to first
+// product: 15000 cycles when every role worked an item out for itself and Q came with 16-byte copies, 9300
+// now (3400 plan, 2200 item, 500 Q, K beside it), which is what steps of short chunks consist of: 20 to
+// 35 us, 10 to 25 % less.
 #pragma once
 
 #include <cuda.h>
@@ -64,6 +69,7 @@ struct PrefillParams {
   int64_t kv_block_stride;    // elements
   int64_t kv_head_stride;
   int num_reqs;
+  int num_tokens;
   int num_heads;
   int num_kv_heads;
   int group;
@@ -75,7 +81,7 @@ struct PrefillParams {
   float scale;
 };
 
-constexpr int kPrefillThreads = 16 * 32;  // (three warps beside the MMA warp only complete its warpgroup)
+constexpr int kPrefillThreads = 16 * 32;
 // Registers per thread: 512 threads start with 128 each; the softmax warpgroups take over what the
 // others give back.  (The producers of an fp8 cache hold a K and a V tile in registers.  An 8192-token
 // fp8 step of 64 / 8 heads takes 1032 us with 176 / 112 / 48 and 997 with 184 / 104 / 40.)
@@ -96,23 +102,26 @@ struct PrefillShape {
   // ring of K and V tiles in turns (K0, V0, K1, V1, ...): what shared memory holds besides Q
   static constexpr int kRoom = 223 * 1024 - NQ * kQBytes;
   static constexpr int kSlots = kRoom / kTileBytes < 8 ? kRoom / kTileBytes : 8;
-  static constexpr int kSmem = 256 + NQ * kQBytes + kSlots * kTileBytes;  // (256: alignment)
+  static constexpr int kSmem = NQ * kQBytes + kSlots * kTileBytes;
+  // Q comes in boxes of 64 head dimensions (128-byte swizzle) where the head size allows, else of 16
+  static constexpr int kQBox = D % 64 == 0 ? 64 : 16;
   static_assert(kSlots >= 4, "a K and a V tile in use, another of each on its way");
   static_assert(NQ * (KT + DP) <= 512, "TMEM columns");
 };
 
 struct PrefillItem {
-  int req, kvh, piece, npieces;
+  int req;         // < 0: no more items
+  int kvh, piece, npieces;
   int tok0;        // first query token of the item inside its request
   int q_len, ctx;  // ctx: cached positions in front of the chunk (seq_len - q_len)
   int seq_len, q0; // q0: row of the request's first token
-  int first;       // number of the item's piece 0
+  int slot;        // workspace slot of the item's piece 0 (where there are several)
   int b, e0, e1;   // key tiles [b, e0) of row tile 0, [b, e1) of row tile 1
 };
 
 template <typename QT, int KV, int D>
 __global__ void __launch_bounds__(kPrefillThreads, 1)
-pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vmap) {
+pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap vmap) {
   using SH = PrefillShape<D>;
   constexpr bool kFp8 = KV != kCache16;
   constexpr bool kE5 = KV == kCacheE5M2;
@@ -120,10 +129,10 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vma
   constexpr bool kOutBf = std::is_same_v<QT, __nv_bfloat16>;
   constexpr int DP = SH::DP, NQ = SH::NQ, KT = SH::KT, NS = SH::kSlots;
   constexpr int kWs = 128 * (D * 2 + 8);  // workspace of one row tile's partial: O, then (m, l)
-  extern __shared__ __align__(128) unsigned char smem_raw[];
+  extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ int cum[kPrefillMaxReqs + 1];  // 2 x (items before request r), + 1 if it is cut into pieces
-  __shared__ uint64_t s_bar[2 * NS + 15];
-  __shared__ int s_item[2];
+  __shared__ uint64_t s_bar[2 * NS + 19];
+  __shared__ PrefillItem s_item[2];
   __shared__ uint32_t s_tmem;
   __shared__ int s_red[3][16];
 
@@ -141,10 +150,16 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vma
   auto item_empty = [&](int i) { return bar0 + 8u * (2 * NS + 10 + i); };
   auto p_half = [&](int i) { return bar0 + 8u * (2 * NS + 12 + i); };
   const uint32_t tail_bar = bar0 + 8u * (2 * NS + 14);
+  auto q_empty = [&](int i) { return bar0 + 8u * (2 * NS + 15 + i); };
+  auto q_land = [&](int i) { return bar0 + 8u * (2 * NS + 17 + i); };
+  constexpr bool kWiden = kFp8 && kOutBf;  // Q becomes f16, the operand type of an fp8 cache
 
-  unsigned char* const smem = smem_raw + (-smem_u32(smem_raw) & 255u);  // (V's swizzle goes by address bits 4 .. 7)
   const uint32_t sq = smem_u32(smem);
   const uint32_t skv = sq + NQ * SH::kQBytes;
+  if ((sq & 1023u) != 0) {  // (swizzles go by address bits)
+    if (tid == 0) atomicExch(p.status, kStatusNoRing);
+    return;
+  }
 
   if (warp == 12) {
     if (lane == 0) {
@@ -158,9 +173,11 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vma
         mbar_init(p_half(i), 4);
         mbar_init(p_full(i), 4);
         mbar_init(pv_done(i), 1);
-        mbar_init(q_full(i), 4);
+        mbar_init(q_full(i), kWiden ? 2 : 1);
+        mbar_init(q_land(i), 1);
+        mbar_init(q_empty(i), 1);
         mbar_init(item_full(i), 1);
-        mbar_init(item_empty(i), 12);
+        mbar_init(item_empty(i), kWiden ? 15 : 14);
       }
       mbar_init(tail_bar, 1);
       fence_barrier_init();
@@ -169,12 +186,9 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vma
     tmem_alloc(smem_u32(&s_tmem), 512);
   }
   if constexpr (DP != D) {
-    // The padding granules of Q and K take part in the product: zero, once (nobody writes them: K sits
-    // in the even slots of the ring, and V's padding only gives columns that are dropped).
+    // K's padding granule takes part in the product: zero, once (nobody writes it: K sits in the even
+    // slots of the ring.  Q's comes as zeros, V's padding only gives columns that are dropped).
     static_assert(DP - D == 8 && NS % 2 == 0, "one padding granule; K and V in slots of their own");
-    for (int i = tid; i < NQ * 128; i += kPrefillThreads)
-      *reinterpret_cast<uint4*>(smem + (i / 128) * SH::kQBytes + (D / 8) * 128 * 16 + (i % 128) * 16) =
-          make_uint4(0, 0, 0, 0);
     for (int i = tid; i < NS / 2 * KT; i += kPrefillThreads)
       *reinterpret_cast<uint4*>(smem + NQ * SH::kQBytes + (i / KT) * 2 * SH::kTileBytes + ((D / 8) * KT + i % KT) * 16) =
           make_uint4(0, 0, 0, 0);
@@ -189,8 +203,14 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vma
   const int G = p.group, HK = p.num_kv_heads, S = p.num_reqs, B = p.block_size;
   const int b_shift = 31 - __clz(B);  // 16 or 32 tokens per block
   const int T = 128 / G, TT = NQ * T;
+  static_assert(kPrefillThreads == kPrefillMaxReqs, "a thread to a request");
+  int ql = 0, len = 0;
+  if (tid < S) {
+    ql = p.q_start[tid + 1] - p.q_start[tid];
+    len = p.seq_lens[tid];
+  }
+  const int n = (ql + TT - 1) / TT;  // groups
   int split_tiles;  // key tiles per piece (1 << 30: one piece per group)
-  auto q_len_of = [&](int r) { return p.q_start[r + 1] - p.q_start[r]; };
   auto tiles_of = [&](int len) { return (max(len, 0) + KT - 1) / KT; };
   {
     // groups and key tiles of all requests: with fewer than four groups per SM the groups are cut
@@ -202,13 +222,10 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vma
     // region beside decodes: a 16-token chunk behind 32000 and 60 chunks of 32, 546 -> 169 us.)
     constexpr int kCut = 768 / KT;
     int groups = 0, work = 0;
-    for (int r = tid; r < S; r += kPrefillThreads) {
-      const int ql = q_len_of(r);
-      const int n = (ql + TT - 1) / TT;
-      const int len = p.seq_lens[r];
+    if (tid < S) {
       const int t = tiles_of(len);
-      groups += n;
-      work += n * ((t + tiles_of(len - ql + min(ql, TT)) + 1) / 2);
+      groups = n;
+      work = n * ((t + tiles_of(len - ql + min(ql, TT)) + 1) / 2);
       const int q0 = (t + kCut - 1) / kCut, q1 = (t + kCut * 3 / 2 - 1) / (kCut * 3 / 2);
 #pragma unroll 1
       for (int k = 0; k < 8 && t > kCut << k; ++k) {
@@ -234,7 +251,8 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vma
     const int64_t all_work = int64_t(work) * HK, all_groups = int64_t(groups) * HK;
     split_tiles = 1 << 30;
     if (all_groups < 4 * int64_t(gridDim.x)) {
-      const int want = int((all_work + gridDim.x - 1) / int64_t(gridDim.x));
+      const int64_t up = all_work + gridDim.x - 1;
+      const int want = up >> 32 == 0 ? int(uint32_t(up) / gridDim.x) : int(up / int64_t(gridDim.x));
       auto cut_of = [&](int k) { return ((k & 1) ? kCut * 3 / 2 : kCut) << (k >> 1); };
       const unsigned fit = __ballot_sync(
           0xffffffffu, lane < 16 && s_red[2][lane & 15] <= p.ws_slots && cut_of(lane + 1) > want);
@@ -242,13 +260,12 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vma
     }
     __syncthreads();  // (s_red is written again below)
   }
-  auto pieces_of = [&](int len) { return max(1u, (unsigned(tiles_of(len)) + split_tiles - 1u) / unsigned(split_tiles)); };
+  auto pieces_of = [&](int len) -> unsigned {
+    const unsigned t = tiles_of(len);
+    return t <= unsigned(split_tiles) ? 1u : (t + split_tiles - 1u) / unsigned(split_tiles);
+  };
   {
-    const int per = (S + kPrefillThreads - 1) / kPrefillThreads;
-    const int r0 = min(S, tid * per), r1 = min(S, r0 + per);
-    auto items_of = [&](int r) { return ((q_len_of(r) + TT - 1) / TT) * pieces_of(p.seq_lens[r]) * HK; };
-    int mine = 0;
-    for (int r = r0; r < r1; ++r) mine += items_of(r);
+    const int pieces = pieces_of(len), mine = n * pieces * HK;
     int incl = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -259,11 +276,8 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vma
     __syncthreads();
     int run = incl - mine;
     for (int w = 0; w < warp; ++w) run += s_red[2][w];
-    for (int r = r0; r < r1; ++r) {
-      cum[r] = 2 * run + (pieces_of(p.seq_lens[r]) > 1 ? 1 : 0);
-      run += items_of(r);
-    }
-    if (tid == kPrefillThreads - 1) cum[S] = 2 * run;
+    if (tid < S) cum[tid] = 2 * run + (pieces > 1 ? 1 : 0);
+    if (tid == kPrefillThreads - 1) cum[S] = 2 * (run + mine);
   }
   tc_fence_before();
   __syncthreads();
@@ -275,28 +289,45 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vma
   // (longest first), then the pieces, then the kv heads.
   auto decode = [&](int item) {
     PrefillItem it;
-    int lo = 0, hi = S;
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (cum[mid] >> 1 <= item) lo = mid; else hi = mid;
-    }
+    auto starts = [&](int r) { return r < S && cum[r] >> 1 <= item; };  // (true up to the request of the item)
+    int lo = 16 * (31 - __clz(__ballot_sync(0xffffffffu, starts(16 * lane))));
+    lo += 31 - __clz(__ballot_sync(0xffffffffu, lane < 16 && starts(lo + lane)));
     it.req = lo;
     it.q0 = p.q_start[lo];
     it.q_len = p.q_start[lo + 1] - it.q0;
     it.seq_len = p.seq_lens[lo];
     it.ctx = it.seq_len - it.q_len;
-    const int rel = item - (cum[lo] >> 1);
-    it.kvh = rel % HK;
-    const int gp = rel / HK;
+    const unsigned rel = item - (cum[lo] >> 1);
+    unsigned gp = rel / unsigned(HK);
+    it.kvh = rel - gp * HK;
     it.npieces = pieces_of(it.seq_len);
-    it.piece = gp % it.npieces;
+    it.piece = 0;
+    if (it.npieces > 1) {
+      const unsigned q = gp / unsigned(it.npieces);
+      it.piece = gp - q * it.npieces;
+      gp = q;
+    }
     const int ngroups = (it.q_len + TT - 1) / TT;
-    const int grp = ngroups - 1 - gp / it.npieces;
-    it.first = item - it.piece * HK;
+    const int grp = ngroups - 1 - int(gp);
+    // (the items of cut requests are counted only.  A table of the slots takes the static shared memory
+    // past what a carve-out of 196 KiB holds at head size 128, and L1 shrinks to 28 KiB: 2 chunks of 64
+    // behind 8192 take 98 us instead of 76.)
+    it.slot = item - it.piece * HK;
+    if (it.npieces > 1) {
+      int others = 0;
+      for (int r = lane; r < lo; r += 32)
+        if ((cum[r] & 1) == 0) others += (cum[r + 1] >> 1) - (cum[r] >> 1);
+      it.slot -= __reduce_add_sync(0xffffffffu, others);
+    }
     it.tok0 = grp * TT;
     const int n = tiles_of(it.ctx + min(it.q_len, it.tok0 + TT));
-    it.b = int(int64_t(n) * it.piece / it.npieces);
-    const int e = int(int64_t(n) * (it.piece + 1) / it.npieces);
+    int e = n;
+    it.b = 0;
+    if (it.npieces > 1) {  // pieces of n / npieces tiles, the first ones of one more
+      const int per = unsigned(n) / unsigned(it.npieces), more = n - per * it.npieces;
+      it.b = it.piece * per + min(it.piece, more);
+      e = it.b + per + (it.piece < more ? 1 : 0);
+    }
     auto end_of = [&](int i) {
       const int t0 = it.tok0 + i * T;
       return i < NQ && t0 < it.q_len ? max(it.b, min(e, tiles_of(it.ctx + min(it.q_len, t0 + T)))) : it.b;
@@ -319,15 +350,15 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vma
     __syncwarp();
     if (lane == 0) mbar_arrive(bar);
   };
-  // next item of this CTA, for the roles that do not draw it themselves
+  // Items of this CTA: warp 13 draws them, works out what they cover and puts that into a ring of two;
+  // the other roles look there and give the place back when they are through with an item.
   int n_item = 0;  // items received so far
-  auto next_item = [&]() -> int {
-    const int slot = n_item & 1;
-    if (!wait(item_full(slot), (n_item >> 1) & 1)) return INT32_MAX;
-    const int v = *reinterpret_cast<volatile int*>(&s_item[slot]);
-    arrive(item_empty(slot));
+  auto have_item = [&]() -> bool {
+    return wait(item_full(n_item & 1), (n_item >> 1) & 1) && s_item[n_item & 1].req >= 0;
+  };
+  auto item_done = [&]() {
+    arrive(item_empty(n_item & 1));
     ++n_item;
-    return v;
   };
 
   if (warp < 8) {
@@ -345,62 +376,8 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vma
     const int row_tok = row / G, row_head = row % G;
     uint32_t n_s = 0, n_pv = 0;  // S tiles received, PV products issued for this row tile
 
-    // Each warp brings its own 32 rows: eight rows and four 16-byte granules at a time, 64-byte pieces
-    // of global memory into 128-byte runs of the operand layout.  (One row per thread took 8000 cycles
-    // an item at head size 128.)
-    // Only for a row tile that has key tiles in this item: a warpgroup without work may be items ahead
-    // of the MMAs, and must not complete a phase of q_full that they have not waited for.
-    auto load_q = [&](const PrefillItem& it) {
-      if ((wg == 0 ? it.e0 : it.e1) > it.b) {
-#pragma unroll
-        for (int rb = 0; rb < 4; ++rb) {
-          const int from = rb * 8 + (lane & 7);  // the row: this lane's copy of its token and head
-          const int tok = it.tok0 + wg * T + __shfl_sync(0xffffffffu, row_tok, from);
-          const int head = it.kvh * G + __shfl_sync(0xffffffffu, row_head, from);
-          const bool used = __shfl_sync(0xffffffffu, int(row_used), from) != 0 && tok < it.q_len;
-          const QT* src = static_cast<const QT*>(p.q) + int64_t(it.q0 + tok) * p.q_stride + int64_t(head) * D;
-          const uint32_t dst = sq + wg * SH::kQBytes + ((row & ~31) + from) * 16;
-          constexpr int NG = (D / 8 + 3) / 4;
-          if constexpr (kFp8 && kOutBf) {  // the operands of an fp8 cache are f16
-            uint4 v[NG];
-#pragma unroll
-            for (int i = 0; i < NG; ++i) {
-              const int g = 4 * i + (lane >> 3);
-              v[i] = used && (D / 8 % 4 == 0 || g < D / 8) ? __ldg(reinterpret_cast<const uint4*>(src) + g)
-                                                            : make_uint4(0, 0, 0, 0);
-            }
-#pragma unroll
-            for (int i = 0; i < NG; ++i) {
-              const int g = 4 * i + (lane >> 3);
-              const uint32_t w[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
-              uint32_t o[4];
-#pragma unroll
-              for (int k = 0; k < 4; ++k)
-                o[k] = pack2<false>(__uint_as_float(w[k] << 16), __uint_as_float(w[k] & 0xffff0000u));
-              if (D / 8 % 4 == 0 || g < D / 8) st_shared16(dst + g * 128 * 16, make_uint4(o[0], o[1], o[2], o[3]));
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < NG; ++i) {
-              const int g = 4 * i + (lane >> 3);
-              if (used && (D / 8 % 4 == 0 || g < D / 8))
-                cp_async16(dst + g * 128 * 16, reinterpret_cast<const uint4*>(src) + g, 16);
-            }
-          }
-        }
-        if constexpr (!(kFp8 && kOutBf)) cp_async_wait_all();
-        fence_proxy_async();
-        arrive(q_full(wg));
-      }
-    };
-
-    int item = blockIdx.x < unsigned(total) ? int(blockIdx.x) : INT32_MAX;
-    PrefillItem it{};
-    if (item < total) {
-      it = decode(item);
-      load_q(it);
-    }
-    while (item < total && ok) {
+    while (ok && have_item()) {
+      const PrefillItem& it = s_item[n_item & 1];
       const int b = it.b, e = wg == 0 ? it.e0 : it.e1;
       const int tok = it.tok0 + wg * T + row_tok;
       const bool valid = row_used && tok < it.q_len;
@@ -489,58 +466,61 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vma
         ++n_pv;
       }
       if (!ok) break;
-      // ---- the next item's Q goes in while this one's last product runs (S of the last tile has
-      // been received, so nothing reads this tile's Q any more)
-      const PrefillItem cur = it;
-      item = next_item();
-      if (item < total) {
-        it = decode(item);
-        load_q(it);
+      if (wg >= NQ) {
+        item_done();
+        continue;
       }
-      if (!ok) break;
-      if (wg >= NQ) continue;
       // ---- results
       const bool any = e > b;
       if (any) {
         if (!wait(pv_done(wg), (n_pv - 1) & 1)) break;
         tc_fence_after();
       }
-      const bool whole = cur.npieces == 1;
+      const bool whole = it.npieces == 1;
       const float inv = v_scale * __fdividef(1.f, l + 1e-6f);
-      const int64_t out_row = (int64_t(cur.q0 + tok) * p.num_heads + head) * D;
-      // workspace slot of piece 0: the items of cut requests are counted only.  (A table of the slots takes
-      // the static shared memory past what a carve-out of 196 KiB holds at head size 128, and L1 shrinks to
-      // 28 KiB: 2 chunks of 64 behind 8192 take 98 us instead of 76.)
-      int slot = cur.first;
-      if (!whole) {
-        int others = 0;
-        for (int r = lane; r < cur.req; r += 32)
-          if ((cum[r] & 1) == 0) others += (cum[r + 1] >> 1) - (cum[r] >> 1);
-        slot -= __reduce_add_sync(0xffffffffu, others);
-      }
-      unsigned char* part = p.ws + (size_t(slot + cur.piece * HK) * NQ + wg) * kWs;
+      const int64_t out_row = (int64_t(it.q0 + tok) * p.num_heads + head) * D;
+      const int slot = it.slot;
+      unsigned char* part = p.ws + (size_t(slot + it.piece * HK) * NQ + wg) * kWs;
       QT* dst = whole ? static_cast<QT*>(p.out) + out_row
                       : reinterpret_cast<QT*>(part) + row * D;
+      // 32 bytes a store where rows allow it: a row is another 128-byte line for each lane, whatever it
+      // stores there
+      const bool wide = D % 16 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
       if (any || whole) {
+        constexpr int NCO = DP / 16, CH = NCO % 4 == 0 ? 4 : (NCO % 3 == 0 ? 3 : NCO);  // chunks read at a time
+        static_assert(CH <= 7, "registers");
 #pragma unroll 1
-        for (int ch = 0; ch < DP / 16; ++ch) {
-          float o[16];
+        for (int c0 = 0; c0 < NCO; c0 += CH) {
+          float o[CH][16], keep[4] = {inv, 0.f, 0.f, 0.f};
+          float inv2 = inv;
+          int dummy = 0;
           if (any) {
-            tmem_ld16(t_o + ch * 16, o);
+#pragma unroll
+            for (int k = 0; k < CH; ++k) tmem_ld16_start(t_o + (c0 + k) * 16, o[k]);
+            tmem_landed(keep, inv2, dummy);
           } else {
 #pragma unroll
-            for (int k = 0; k < 16; ++k) o[k] = 0.f;
+            for (int k = 0; k < CH; ++k)
+#pragma unroll
+              for (int i = 0; i < 16; ++i) o[k][i] = 0.f;
           }
           if (valid) {
-            uint32_t w[8];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) w[k] = pack2<kOutBf>(o[2 * k] * inv, o[2 * k + 1] * inv);
-            uint4* d4 = reinterpret_cast<uint4*>(dst + ch * 16);
-            d4[0] = make_uint4(w[0], w[1], w[2], w[3]);
-            if (ch * 16 + 8 < D) d4[1] = make_uint4(w[4], w[5], w[6], w[7]);
+            for (int k = 0; k < CH; ++k) {
+              uint32_t w[8];
+#pragma unroll
+              for (int i = 0; i < 8; ++i) w[i] = pack2<kOutBf>(o[k][2 * i] * inv2, o[k][2 * i + 1] * inv2);
+              QT* d = dst + (c0 + k) * 16;
+              if (wide) {
+                st_global32(d, w);
+              } else {
+                reinterpret_cast<uint4*>(d)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+                if (D % 16 == 0 || (c0 + k) * 16 + 8 < D) reinterpret_cast<uint4*>(d)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+              }
+            }
           }
         }
-        tc_fence_before();  // (ordered before the next item's p_full, which frees O)
+        tc_fence_before();  // (ordered before the next item's p_half, which frees O)
       }
       if (!whole) {
         float* stats = reinterpret_cast<float*>(part + 128 * D * 2);
@@ -552,31 +532,31 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vma
         unsigned* cnt = p.arrive + (size_t(slot) * NQ + wg) * 4 + (warp & 3);
         if (lane == 0) {
           old = atomicAdd(cnt, 1u);
-          if (old == unsigned(cur.npieces - 1)) *cnt = 0;  // re-arm for the next launch
+          if (old == unsigned(it.npieces - 1)) *cnt = 0;  // re-arm for the next launch
         }
         old = __shfl_sync(0xffffffffu, old, 0);
-        if (old == unsigned(cur.npieces - 1) && valid) {
+        if (old == unsigned(it.npieces - 1) && valid) {
           __threadfence();
           const unsigned char* base = p.ws + (size_t(slot) * NQ + wg) * kWs;
           const size_t step = size_t(HK) * NQ * kWs;
           // statistics of eight pieces at a time (independent loads), online
           float mx = -INFINITY, total_l = 0.f;
 #pragma unroll 1
-          for (int k0 = 0; k0 < cur.npieces; k0 += 8) {
+          for (int k0 = 0; k0 < it.npieces; k0 += 8) {
             float2 ml[8];
 #pragma unroll
             for (int k = 0; k < 8; ++k)
-              ml[k] = __ldcg(reinterpret_cast<const float2*>(base + min(k0 + k, cur.npieces - 1) * step + 128 * D * 2) + row);
+              ml[k] = __ldcg(reinterpret_cast<const float2*>(base + min(k0 + k, it.npieces - 1) * step + 128 * D * 2) + row);
             float m_new = mx;
 #pragma unroll
             for (int k = 0; k < 8; ++k)
-              if (k0 + k < cur.npieces && ml[k].y > 0.f) m_new = fmaxf(m_new, ml[k].x);
+              if (k0 + k < it.npieces && ml[k].y > 0.f) m_new = fmaxf(m_new, ml[k].x);
             if (m_new == -INFINITY) continue;
             total_l *= fast_exp2(mx - m_new);
             mx = m_new;
 #pragma unroll
             for (int k = 0; k < 8; ++k)
-              if (k0 + k < cur.npieces && ml[k].y > 0.f) total_l += ml[k].y * fast_exp2(ml[k].x - mx);
+              if (k0 + k < it.npieces && ml[k].y > 0.f) total_l += ml[k].y * fast_exp2(ml[k].x - mx);
           }
           const float winv = __fdividef(1.f, total_l + 1e-6f);
           QT* od = static_cast<QT*>(p.out) + out_row;
@@ -587,18 +567,18 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vma
             for (int z = 0; z < 16; ++z) acc[z] = 0.f;
             // four pieces at a time: eight independent loads on their way
 #pragma unroll 1
-            for (int k0 = 0; k0 < cur.npieces; k0 += 4) {
+            for (int k0 = 0; k0 < it.npieces; k0 += 4) {
               uint4 x[4][2];
               float w[4];
 #pragma unroll
               for (int k = 0; k < 4; ++k) {
-                const unsigned char* pk = base + min(k0 + k, cur.npieces - 1) * step;
+                const unsigned char* pk = base + min(k0 + k, it.npieces - 1) * step;
                 const float2 ml = __ldcg(reinterpret_cast<const float2*>(pk + 128 * D * 2) + row);
                 const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const QT*>(pk) + row * D + d0);
                 x[k][0] = __ldcg(src);
                 x[k][1] = D % 16 == 0 || d0 + 8 < D ? __ldcg(src + 1) : make_uint4(0, 0, 0, 0);
                 // (a piece in which this row has no key has written no output)
-                w[k] = k0 + k < cur.npieces && ml.y > 0.f ? ml.y * fast_exp2(ml.x - mx) * winv : 0.f;
+                w[k] = k0 + k < it.npieces && ml.y > 0.f ? ml.y * fast_exp2(ml.x - mx) * winv : 0.f;
               }
 #pragma unroll
               for (int k = 0; k < 4; ++k) {
@@ -618,6 +598,7 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vma
         }
         __syncwarp();
       }
+      item_done();
     }
   } else if (warp < 12) {
     // ================================================= producers: K and V tiles into shared memory
@@ -655,9 +636,8 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vma
       return wait(kv_empty(h % NS), (use - 1) & 1);
     };
     auto slot_of = [&](uint32_t h) { return skv + (h % NS) * SH::kTileBytes; };
-    int item = blockIdx.x < unsigned(total) ? int(blockIdx.x) : INT32_MAX;
-    while (item < total && ok) {
-      const PrefillItem it = decode(item);
+    while (ok && have_item()) {
+      const PrefillItem it = s_item[n_item & 1];
       const int* bt = p.block_tables + int64_t(it.req) * p.max_blocks_per_seq;
       const int64_t head_off = int64_t(it.kvh) * p.kv_head_stride * ES;
       const int e = max(it.e0, it.e1);
@@ -829,7 +809,7 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vma
       }
       if (!ok) break;
       if constexpr (!kFp8) announce_all();  // (the next item may be drawn only when they have arrived)
-      item = next_item();
+      item_done();
     }
     if constexpr (!kFp8) {  // nobody leaves with copies on their way (after a wait that ran out, too)
       cp_async_wait_all();
@@ -845,13 +825,16 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vma
     // warp: after every block of the elected lane the warp converges before anything else runs.
     const uint32_t idesc_s = mma_idesc(kBf, 128, KT);
     const uint32_t idesc_o = mma_idesc(kBf, 128, DP);
-    uint32_t n_h = 0, n_it = 0, n_q0 = 0, n_q1 = 0, n_p0 = 0, n_p1 = 0;  // halves, items, Q tiles, P tiles
+    uint32_t n_h = 0, n_q0 = 0, n_q1 = 0, n_p0 = 0, n_p1 = 0;  // halves, Q tiles, P tiles
     auto uniform = [](uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); };
     auto commit = [&](uint32_t bar) {
       if (elect_one()) mma_commit(bar);
       __syncwarp();
     };
-    const uint64_t q_desc = smem_desc(sq, 128 * 16, 128);
+    const uint64_t q_desc = SH::kQBox == 64 ? smem_desc_sw128(sq) : smem_desc_sw32(sq, 256);
+    auto q_step = [](int ks) {  // where K step ks lies, in 16-byte units
+      return SH::kQBox == 64 ? ks / 4 * (128 * 128 / 16) + ks % 4 * 2 : ks * (128 * 32 / 16);
+    };
     const uint64_t k_desc = smem_desc(skv, KT * 16, 128);
     const uint64_t v_desc = kFp8 ? smem_desc(skv, DP * 16, 128) : smem_desc_sw32(skv, 256);
     auto wait_half = [&](uint32_t h) { return wait(kv_full(h % NS), (h / NS) & 1); };
@@ -861,7 +844,7 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vma
       if (elect_one()) {
 #pragma unroll
         for (int ks = 0; ks < DP / 16; ++ks)
-          mma_ss(tmem + i * KT, qd + ks * 2 * 128, kd + ks * 2 * KT, idesc_s, ks > 0);
+          mma_ss(tmem + i * KT, qd + q_step(ks), kd + ks * 2 * KT, idesc_s, ks > 0);
         mma_commit(s_full(i));
       }
       __syncwarp();
@@ -882,34 +865,28 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vma
       }
       __syncwarp();
     };
-    int item = blockIdx.x < unsigned(total) ? int(blockIdx.x) : INT32_MAX;
-    while (item < total && ok) {
-      // draw the next item now; the other roles pick it up when they are through with this one
-      unsigned ticket = 0;
-      if (lane == 0) ticket = atomicAdd(p.sched, 1u);
-      const PrefillItem it = decode(item);
-      ticket = __shfl_sync(0xffffffffu, ticket, 0);
-      const int nxt = int(min(ticket + gridDim.x, unsigned(INT32_MAX)));
+    while (ok && have_item()) {
+      struct { int b, e0, e1, seq_len; } it;
       {
-        const int slot = n_it & 1;
-        if (n_it >= 2 && !wait(item_empty(slot), ((n_it >> 1) - 1) & 1)) break;
-        if (lane == 0) {
-          *reinterpret_cast<volatile int*>(&s_item[slot]) = nxt;
-          mbar_arrive(item_full(slot));
-        }
-        __syncwarp();
+        const PrefillItem& from = s_item[n_item & 1];
+        it.b = uniform(from.b);
+        it.e0 = uniform(from.e0);
+        it.e1 = uniform(from.e1);
+        it.seq_len = uniform(from.seq_len);
       }
       const int e = max(it.e0, it.e1);
-      if (it.b < it.e0 && !wait(q_full(0), n_q0++ & 1)) break;
-      if (it.b < it.e1 && !wait(q_full(1), n_q1++ & 1)) break;
-      ++n_it;
-      tc_fence_after();
       if (it.b < e) {
         if (!wait_half(n_h)) break;
-        tc_fence_after();
 #pragma unroll
-        for (int i = 0; i < NQ; ++i)
-          if (it.b < (i == 0 ? it.e0 : it.e1)) qk(i, n_h);
+        for (int i = 0; i < NQ; ++i) {
+          const int ei = i == 0 ? it.e0 : it.e1;
+          if (it.b >= ei) continue;
+          if (!wait(q_full(i), (i == 0 ? n_q0++ : n_q1++) & 1)) break;
+          tc_fence_after();
+          qk(i, n_h);
+          if (it.b + 1 == ei) commit(q_empty(i));
+        }
+        if (!ok) break;
         commit(kv_empty(n_h % NS));
         ++n_h;
       }
@@ -934,6 +911,7 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vma
             if (!have_k && !wait_half(n_h + 1)) continue;
             have_k = true;
             qk(i, n_h + 1);
+            if (j + 2 == ei) commit(q_empty(i));
           }
         }
         if (!ok) break;
@@ -944,7 +922,80 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap vma
           ++n_h;
         }
       }
-      item = nxt;
+      if (!ok) break;
+      item_done();
+    }
+    } else if (warp == 13) {
+    // ================================================= draws items and works out what they cover
+    // (when everybody is through with the item before the one in work: any earlier, and the SMs end
+    // less evenly)
+    int item = blockIdx.x < unsigned(total) ? int(blockIdx.x) : INT32_MAX;
+    for (;; ++n_item) {
+      const int slot = n_item & 1;
+      if (n_item >= 2 && !wait(item_empty(slot), ((n_item >> 1) - 1) & 1)) break;
+      if (n_item >= 1) {
+        unsigned ticket = 0;
+        if (lane == 0) ticket = atomicAdd(p.sched, 1u);
+        ticket = __shfl_sync(0xffffffffu, ticket, 0);
+        item = int(min(ticket + gridDim.x, unsigned(INT32_MAX)));
+      }
+      PrefillItem it{};
+      it.req = -1;
+      if (item < total) it = decode(item);
+      if (lane == 0) {
+        s_item[slot] = it;
+        mbar_arrive(item_full(slot));
+      }
+      __syncwarp();
+      if (item >= total) break;
+    }
+    } else {
+    // ================================================= Q into shared memory (warp 14), as soon as the
+    // last product with the Q before it is through: a tile's tokens and heads are a box of a tensor
+    // map.  (16-byte cp.async by two warps: 1600 cycles to issue, 3000 until they landed; by the softmax
+    // warpgroups after their last tile 6500, which nothing hid.)  bf16 becomes f16 in place for an
+    // fp8 cache, half a tile by each of warps 14 and 15.
+    uint32_t n_q[2] = {0, 0};
+    while (ok && (kWiden || warp == 14) && have_item()) {
+      const PrefillItem& it = s_item[n_item & 1];
+      const bool has[2] = {it.e0 > it.b, it.e1 > it.b};
+#pragma unroll
+      for (int i = 0; i < NQ; ++i) {
+        if (!has[i]) continue;
+        const uint32_t land = kWiden ? q_land(i) : q_full(i);
+        if (warp == 14) {
+          if (n_q[i] > 0 && !wait(q_empty(i), (n_q[i] - 1) & 1)) break;
+          constexpr int NB = DP / SH::kQBox;
+          if (lane == 0) {
+            mbar_expect_tx(land, NB * SH::kQBox * 2 * T * G);
+#pragma unroll
+            for (int x = 0; x < NB; ++x)
+              tma_load3(sq + i * SH::kQBytes + x * 128 * SH::kQBox * 2, &qmap, x * SH::kQBox, it.kvh * G,
+                        it.q0 + it.tok0 + i * T, land);
+          }
+          __syncwarp();
+        }
+        if constexpr (kWiden) {
+          if (!wait(land, n_q[i] & 1)) break;
+          const uint32_t at = sq + i * SH::kQBytes + (warp - 14) * (SH::kQBytes / 2) + lane * 16;
+#pragma unroll 4
+          for (int o = 0; o < SH::kQBytes / 2; o += 512) {
+            const uint4 v = ld_shared16(at + o);
+            auto f16 = [](uint32_t w) { return pack2<false>(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); };
+            st_shared16(at + o, make_uint4(f16(v.x), f16(v.y), f16(v.z), f16(v.w)));
+          }
+          fence_proxy_async();
+          arrive(q_full(i));
+        }
+        ++n_q[i];
+      }
+      if (!ok) break;
+      item_done();
+    }
+    if (warp == 14) {  // nobody leaves with copies on their way
+#pragma unroll
+      for (int i = 0; i < NQ; ++i)
+        if (n_q[i] > 0) mbar_spin(kWiden ? q_land(i) : q_full(i), (n_q[i] - 1) & 1);
     }
     }
   }

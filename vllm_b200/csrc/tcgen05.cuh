@@ -125,6 +125,16 @@ __device__ __forceinline__ void tmem_ld16(uint32_t addr, float (&v)[16]) {
       : "r"(addr)
       : "memory");
 }
+// ... without the wait, see tmem_ld32.
+__device__ __forceinline__ void tmem_ld16_start(uint32_t addr, float (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]),
+        "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
+      : "r"(addr)
+      : "memory");
+}
 __device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&v)[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
@@ -160,6 +170,11 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
 // `sbo` bytes apart from the next 8; the 16-byte halves of rows 4 .. 7 of every 8 change places.
 __device__ __forceinline__ uint64_t smem_desc_sw32(uint32_t addr, uint32_t sbo) {
   return smem_desc(addr, 16, sbo) | (uint64_t(6) << 61);
+}
+// ... with the 128-byte swizzle: rows of 64 elements, 8 of them 1024 bytes (which the operand starts at a
+// multiple of); a K step is 32 bytes further.
+__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
+  return smem_desc(addr, 16, 1024) | (uint64_t(2) << 61);
 }
 // D[tmem] (+)= A[shared] . B[shared]^T, one K step of 16 elements.
 __device__ __forceinline__ void mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool accumulate) {
@@ -197,12 +212,25 @@ __device__ __forceinline__ void cp_async_wait() {
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // A box of a tensor map, completion counted in bytes on `bar`.  No cluster multicast: every CTA fetches
 // its own tiles.
+__device__ __forceinline__ void tma_load3(uint32_t dst, const void* map, int x, int y, int z, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+      "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
+      : "memory");
+}
 __device__ __forceinline__ void tma_load4(uint32_t dst, const void* map, int x, int y, int z, int w, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
       "[%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
       "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar)
       : "memory");
+}
+// 32 bytes to an address that is a multiple of 32.
+__device__ __forceinline__ void st_global32(void* dst, const uint32_t (&v)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+               "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
 }
 __device__ __forceinline__ uint4 ld_shared16(uint32_t src) {
   uint4 v;

@@ -8,7 +8,10 @@
 
 namespace b200pa {
 
-cudaError_t prefill_v_map(const PrefillParams& p, int head_size, CUtensorMap* map) {
+// A tensor map of 16-bit elements without interleaving; `strides` in elements.
+template <int N>
+static cudaError_t tensor_map(CUtensorMap* map, const void* base, const int64_t (&dims)[N], const int64_t (&strides)[N - 1],
+                              const int (&box)[N], CUtensorMapSwizzle swizzle) {
   using Encode = decltype(&cuTensorMapEncodeTiled);
   static const Encode encode = [] {
     void* f = nullptr;
@@ -19,20 +22,33 @@ cudaError_t prefill_v_map(const PrefillParams& p, int head_size, CUtensorMap* ma
     return reinterpret_cast<Encode>(f);
   }();
   if (encode == nullptr) return cudaErrorNotSupported;
-  const cuuint64_t dims[4] = {cuuint64_t(p.block_size), cuuint64_t(head_size), cuuint64_t(p.num_kv_heads),
-                              cuuint64_t(INT32_MAX)};
-  const cuuint64_t strides[3] = {cuuint64_t(p.block_size) * 2, cuuint64_t(p.kv_head_stride) * 2,
-                                 cuuint64_t(p.kv_block_stride) * 2};
-  const cuuint32_t box[4] = {16, cuuint32_t(head_size), 1, 1}, step[4] = {1, 1, 1, 1};
-  const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 4, const_cast<void*>(p.vc), dims, strides, box, step,
-                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+  cuuint64_t d[N], st[N - 1];
+  cuuint32_t b[N], step[N];
+  for (int i = 0; i < N; ++i) {
+    d[i] = cuuint64_t(dims[i]);
+    b[i] = cuuint32_t(box[i]);
+    step[i] = 1;
+  }
+  for (int i = 0; i < N - 1; ++i) st[i] = cuuint64_t(strides[i]) * 2;
+  const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, N, const_cast<void*>(base), d, st, b, step,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+cudaError_t prefill_v_map(const PrefillParams& p, int head_size, CUtensorMap* map) {
+  return tensor_map<4>(map, p.vc, {p.block_size, head_size, p.num_kv_heads, INT32_MAX},
+                       {p.block_size, p.kv_head_stride, p.kv_block_stride}, {16, head_size, 1, 1}, CU_TENSOR_MAP_SWIZZLE_32B);
+}
+
+cudaError_t prefill_q_map(const PrefillParams& p, int head_size, int box, CUtensorMap* map) {
+  return tensor_map<3>(map, p.q, {head_size, p.num_heads, p.num_tokens}, {head_size, p.q_stride},
+                       {box, p.group, 128 / p.group}, box == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_32B);
+}
+
 // The prefill kernel for a call's shape and alignments, or none.  16-byte accesses: pages, rows of Q and
-// of the output; cache offsets inside a block are shifts.  The strides of a 16-bit cache have to fit a tensor
-// map (positive, below 2^40 bytes).
+// of the output; cache offsets inside a block are shifts.  The strides of Q and of a 16-bit cache have to
+// fit a tensor map (positive, below 2^40 bytes).
 static PrefillKernelInfo find_prefill(const b200pa_attn_args& a) {
   const int es = a.kv_dtype == B200PA_KV_AUTO ? 2 : 1;
   auto al = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr) % 16 == 0; };
@@ -41,7 +57,7 @@ static PrefillKernelInfo find_prefill(const b200pa_attn_args& a) {
                     al(a.key_cache) && al(a.value_cache) && al(a.query) && al(a.out) &&
                     (a.kv_block_stride * es) % 16 == 0 && (a.kv_head_stride * es) % 16 == 0 &&
                     (es == 1 || (stride_fits(a.kv_block_stride) && stride_fits(a.kv_head_stride))) &&
-                    a.q_stride % 8 == 0 && a.blocksparse_vert_stride <= 1 && a.out_lse == nullptr;
+                    a.q_stride % 8 == 0 && stride_fits(a.q_stride) && a.blocksparse_vert_stride <= 1 && a.out_lse == nullptr;
   if (!fits) return {nullptr, 0};
   return a.head_size <= 96 ? find_prefill_small(a.head_size, a.q_dtype, a.kv_dtype)
          : a.head_size <= 128 ? find_prefill_mid(a.head_size, a.q_dtype, a.kv_dtype)
@@ -104,6 +120,7 @@ extern "C" int b200pa_paged_attention_varlen(const b200pa_attn_args* a, const in
   p.kv_block_stride = a->kv_block_stride;
   p.kv_head_stride = a->kv_head_stride;
   p.num_heads = a->num_heads;
+  p.num_tokens = num_tokens;
   p.num_kv_heads = a->num_kv_heads;
   p.group = a->num_heads / a->num_kv_heads;
   p.block_size = a->block_size;
