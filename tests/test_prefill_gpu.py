@@ -21,7 +21,7 @@ def _gather(key_cache, value_cache, table, n, kv, scale):
     return k, v
 
 
-def _case(q_lens, ctx, H, HK, D, B, dtype, kv, alibi=False, seed=0, poison=True):
+def _case(q_lens, ctx, H, HK, D, B, dtype, kv, alibi=False, seed=0, poison=True, ramp=0.0):
     from vllm_b200 import _custom_ops as ops
     gen = torch.Generator(device=DEV).manual_seed(seed)
     rng = np.random.default_rng(seed)
@@ -41,6 +41,8 @@ def _case(q_lens, ctx, H, HK, D, B, dtype, kv, alibi=False, seed=0, poison=True)
     scale = 0.02 if fp8 else 1.0
     kf = torch.randn((nb, HK, D // x, B, x), generator=gen, device=DEV)
     vf = torch.randn((nb, HK, D, B), generator=gen, device=DEV)
+    for r, k in enumerate(need):  # logits that grow along the sequence
+        kf[table[r, :k].long()] *= 1 + ramp * torch.arange(int(k), device=DEV).view(-1, 1, 1, 1, 1)
     if fp8:
         t = torch.float8_e5m2 if kv == "fp8_e5m2" else torch.float8_e4m3fn
         kc, vc = ((f / scale).clamp(-448, 448).to(t).view(torch.uint8) for f in (kf, vf))
@@ -140,6 +142,15 @@ def test_items_whose_second_row_tile_is_empty(kv, alibi):
     # (the warpgroup of the second row tile runs items ahead of everybody else)
     _case([20 + i % 12 + 64 * (i % 3) for i in range(60)], [i % 19 for i in range(60)], 32, 8, 128, 16,
           torch.bfloat16, kv, alibi=alibi)
+
+
+# A row's running maximum is only raised when a tile shows that it is too low: in its first half (sum of the
+# exponentials) or its second (their maximum)
+@pytest.mark.parametrize("kv,dtype", [("auto", torch.bfloat16), ("auto", torch.float16), ("fp8", torch.bfloat16)])
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("ramp", [0.02, 0.3])
+def test_maxima_that_grow_along_the_sequence(kv, dtype, D, ramp):
+    _case([130, 40, 300], [0, 700, 333], 8, 2, D, 16, dtype, kv, ramp=ramp)
 
 
 @pytest.mark.parametrize("kv", ["auto", "fp8"])

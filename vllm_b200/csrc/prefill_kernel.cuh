@@ -27,7 +27,7 @@
 //     S, or exponentials ahead of the maximum: step below 475 us, 443 so; fp8 caches and ALiBi, which
 //     read S twice, 5 to 20 % more than this one on steps of short chunks.)
 //   * The running maximum is only raised (and O rescaled in TMEM) when a row's maximum grew by more
-//     than 2^8: until then P is merely larger than 1, which fp32 sums and 16-bit P hold as exactly.
+//     than 2^8 to 2^12: until then P is merely larger than 1, which fp32 sums and 16-bit P hold as exactly.
 //   * fp8 caches are widened to f16 (exact) by the producers on their way to shared memory.
 //   * Few items (short chunks behind long contexts): the keys of an item are cut into pieces, every
 //     piece leaves a normalised partial, and the warp that delivers the last piece of its rows merges
@@ -390,72 +390,100 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qma
         if (!wait(s_full(wg), n_s & 1)) break;
         ++n_s;
         tc_fence_after();
-        // The whole row of S goes to registers at once: its maximum is known before the first
-        // exponential, S is read once, and P can be handed over in parts.
+        // The whole row of S goes to registers at once.  After the first tile the running maximum mostly
+        // stands: for 16-bit caches without a bias the exponentials of the first half start with it as it
+        // is; their sum and, beside them, the maximum of the second half tell whether it was too low (by
+        // 2^12: P and its sums hold larger values as exactly).  Then, and for the first tile, the maximum
+        // of the row is taken first.
+        // (8192-token step 363 -> 353 us, with no gain for fp8 caches; with a bias the maximum grows with
+        // every tile, 148 -> 177.  Exponentials by a polynomial on the FMA pipe instead of the special
+        // function unit, a quarter of them: 354 -> 368; the kernel runs into the power limit, and without
+        // any exponentials it would take 336.)
         constexpr int NC = KT / 32;
-        float x[NC][32];
-#pragma unroll
-        for (int ch = 0; ch < NC; ++ch) tmem_ld32(t_s + ch * 32, x[ch]);
         const int key0 = j * KT;
-        int last = pos - key0;  // last column of this row that counts
-        float cc = c;           // (goes through the wait for the TMEM loads, see tmem_landed)
-        float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-        tmem_landed(m4, cc, last);
-        if (biased) {  // t = x c + slope (key - pos)
-          const float base = slope * -float(last);
+        float x[NC][32], cc = c, nm = 0.f;
+        float2 sa, sb;
+        uint32_t w[NC][16];
+        auto exps = [&](int ch, int k) {
+          const float2 t = ffma2(make_float2(x[ch][k], x[ch][k + 1]), make_float2(cc, cc), make_float2(nm, nm));
+          const float2 e2 = make_float2(fast_exp2(t.x), fast_exp2(t.y));
+          if (k & 2) sb = fadd2(sb, e2); else sa = fadd2(sa, e2);
+          w[ch][k / 2] = pack2<kBf>(e2.x, e2.y);
+        };
+        for (bool look = kFp8 || biased || j == b;; look = true) {
 #pragma unroll
-          for (int ch = 0; ch < NC; ++ch)
+          for (int ch = 0; ch < NC; ++ch) tmem_ld32(t_s + ch * 32, x[ch]);
+          int last = pos - key0;  // last column of this row that counts
+          cc = c;                 // (goes through the wait for the TMEM loads, see tmem_landed)
+          float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+          tmem_landed(m4, cc, last);
+          if (biased) {  // t = x c + slope (key - pos)
+            const float base = slope * -float(last);
 #pragma unroll
-            for (int k = 0; k < 32; ++k) x[ch][k] = fmaf(slope, float(ch * 32 + k), fmaf(x[ch][k], cc, base));
-          cc = 1.f;
-        }
-        if (key0 + KT - 1 > pos_first) {  // only the tiles at the causal edge of a row tile need a mask
-          asm volatile("");               // (a branch in fact, not 128 selects for every tile)
+            for (int ch = 0; ch < NC; ++ch)
 #pragma unroll
-          for (int ch = 0; ch < NC; ++ch)
-#pragma unroll
-            for (int k = 0; k < 32; ++k) x[ch][k] = ch * 32 + k <= last ? x[ch][k] : -INFINITY;
-        }
-#pragma unroll
-        for (int ch = 0; ch < NC; ++ch)
-#pragma unroll
-          for (int k = 0; k < 32; k += 2) m4[k / 2 & 3] = fmax3(m4[k / 2 & 3], x[ch][k], x[ch][k + 1]);
-        const float mx = fmax3(fmaxf(m4[0], m4[1]), m4[2], m4[3]) * cc;
-        // raise the maximum (and rescale what has been summed) only when it grew by more than 8
-        const bool grow = mx > m + 8.f || (m == -INFINITY && mx > m);
-        if (__any_sync(0xffffffffu, grow)) {
-          const float m_new = fmaxf(m, mx);
-          const float alpha = m_new == -INFINITY ? 1.f : fast_exp2(m - m_new);
-          m = m_new;
-          l *= alpha;
-          if (j > b) {
-            if (!wait(pv_done(wg), (n_pv - 1) & 1)) break;
-            tc_fence_after();
-#pragma unroll 1
-            for (int ch = 0; ch < DP / 16; ++ch) {
-              float o[16];
-              tmem_ld16(t_o + ch * 16, o);
-#pragma unroll
-              for (int k = 0; k < 16; ++k) o[k] *= alpha;
-              tmem_st16(t_o + ch * 16, o);
-            }
-            tmem_wait_st();
+              for (int k = 0; k < 32; ++k) x[ch][k] = fmaf(slope, float(ch * 32 + k), fmaf(x[ch][k], cc, base));
+            cc = 1.f;
           }
+          if (key0 + KT - 1 > pos_first) {  // only the tiles at the causal edge of a row tile need a mask
+            asm volatile("");               // (a branch in fact, not 128 selects for every tile)
+#pragma unroll
+            for (int ch = 0; ch < NC; ++ch)
+#pragma unroll
+              for (int k = 0; k < 32; ++k) x[ch][k] = ch * 32 + k <= last ? x[ch][k] : -INFINITY;
+          }
+          if (kFp8 || look) {
+            asm volatile("");
+            float h4[4] = {m4[0], m4[1], m4[2], m4[3]};
+#pragma unroll
+            for (int ch = 0; ch < NC; ++ch)
+#pragma unroll
+              for (int k = 0; k < 32; k += 2) h4[k / 2 & 3] = fmax3(h4[k / 2 & 3], x[ch][k], x[ch][k + 1]);
+            const float mx = fmax3(fmaxf(h4[0], h4[1]), h4[2], h4[3]) * cc;
+            // raise the maximum, and rescale what has been summed
+            const bool grow = mx > m + (kFp8 || biased ? 8.f : 0.f) || (m == -INFINITY && mx > m);
+            if (__any_sync(0xffffffffu, grow)) {
+              const float m_new = fmaxf(m, mx);
+              const float alpha = m_new == -INFINITY ? 1.f : fast_exp2(m - m_new);
+              m = m_new;
+              l *= alpha;
+              if (j > b) {
+                if (!wait(pv_done(wg), (n_pv - 1) & 1)) break;
+                tc_fence_after();
+#pragma unroll 1
+                for (int ch = 0; ch < DP / 16; ++ch) {
+                  float o[16];
+                  tmem_ld16(t_o + ch * 16, o);
+#pragma unroll
+                  for (int k = 0; k < 16; ++k) o[k] *= alpha;
+                  tmem_st16(t_o + ch * 16, o);
+                }
+                tmem_wait_st();
+              }
+            }
+          }
+          nm = m == -INFINITY ? 0.f : -m;
+          sa = sb = make_float2(0.f, 0.f);
+#pragma unroll
+          for (int ch = 0; ch < NC / 2; ++ch)
+#pragma unroll
+            for (int k = 0; k < 32; k += 2) {
+              exps(ch, k);
+              if (!kFp8) m4[k / 2 & 3] = fmax3(m4[k / 2 & 3], x[NC / 2 + ch][k], x[NC / 2 + ch][k + 1]);
+            }
+          const float mx = fmax3(fmaxf(m4[0], m4[1]), m4[2], m4[3]) * cc;
+          const bool low = (sa.x + sa.y) + (sb.x + sb.y) > 4096.f || mx > m + 12.f;
+          if (kFp8 || look || !__any_sync(0xffffffffu, low)) break;
         }
-        const float nm = m == -INFINITY ? 0.f : -m;
-        float2 sa = make_float2(0.f, 0.f), sb = make_float2(0.f, 0.f);
+        if (!ok) break;
         // (P's columns lie over S columns: 16 a chunk of 32)
 #pragma unroll
         for (int ch = 0; ch < NC; ++ch) {
-          uint32_t w[16];
+          if (ch >= NC / 2) {
 #pragma unroll
-          for (int k = 0; k < 32; k += 2) {
-            const float2 t = ffma2(make_float2(x[ch][k], x[ch][k + 1]), make_float2(cc, cc), make_float2(nm, nm));
-            const float2 e2 = make_float2(fast_exp2(t.x), fast_exp2(t.y));
-            if (k & 2) sb = fadd2(sb, e2); else sa = fadd2(sa, e2);
-            w[k / 2] = pack2<kBf>(e2.x, e2.y);
+            for (int k = 0; k < 32; k += 2) exps(ch, k);
           }
-          tmem_st16(t_s + ch * 16, w);
+          tmem_st16(t_s + ch * 16, w[ch]);
           if (ch == NC / 2 - 1 || ch == NC - 1) {
             tmem_wait_st();
             tc_fence_before();
