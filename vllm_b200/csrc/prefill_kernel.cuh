@@ -216,13 +216,17 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qma
   const int n = (ql + TT - 1) / TT;  // groups
   int split_tiles;  // key tiles per piece (1 << 30: one piece per group)
   // Longest sequences first, where there are more groups than SMs: the last items of all are short ones
-  // then.  (60 decodes and three chunks of 150 to 700 tokens behind up to 1500, 328 items: 124.5 -> 122 us; 6 fp8 chunks of 200 to 900 with a bias 147 -> 132.)
+  // then.  (60 decodes and three chunks of 150 to 700 tokens behind up to 1500, 328 items: 124.5 -> 122
+  // us; 6 fp8 chunks of 200 to 900 with a bias 147 -> 132.)
   bool sorted = false;
   auto tiles_of = [&](int len) { return (max(len, 0) + KT - 1) / KT; };
   {
     // groups and key tiles of all requests: with fewer than four groups per SM the groups are cut
     // into pieces of an SM's share of the key tiles, but of no less than 768 keys: a piece costs a Q
     // load, a pipeline fill, a partial and its merge, about as much as 350 keys.
+    // (Cuts of 512 keys and less: 128 tokens behind up to 1500 36 -> 33 us, but 550 tokens without context
+    // 26 -> 32 and 1024 tokens behind 2048 at 2 kv heads 35 -> 50, where the pieces no longer run at once.
+    // A search over the sizes with an estimate of the rounds costs every launch 1.4 us.)
     // Every piece of a group that is cut needs a slot of the workspace: s_red[2][k] counts the slots of
     // cuts of 768 keys x 1, 1.5, 2, 3, 4, 6 ..., and the finest from the share up that fits is taken.
     // (With a slot for every group, cut or not, nothing was cut beside 496 groups, or 31 on a small
@@ -531,8 +535,12 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qma
       const int64_t out_row = (int64_t(it.q0 + tok) * p.num_heads + head) * D;
       const int slot = it.slot;
       unsigned char* part = p.ws + (size_t(slot + it.piece * HK) * NQ + wg) * kWs;
-      QT* dst = whole ? static_cast<QT*>(p.out) + out_row
-                      : reinterpret_cast<QT*>(part) + row * D;
+      QT* dst = static_cast<QT*>(p.out) + out_row;
+      // A partial lies as [16 bytes of the head][row] for the 32 rows of a warp, so that a warp's stores,
+      // and its loads when it merges, are whole lines.  (Rows one after the other: 32 lines an
+      // instruction; 64 tokens behind 8192, 9 pieces, 71 us instead of 47.)
+      constexpr int kWarpPart = 32 * D * 2;
+      const int mine = (warp & 3) * kWarpPart + lane * 16;
       // 32 bytes a store where rows allow it: a row is another 128-byte line for each lane, whatever it
       // stores there
       const bool wide = D % 16 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
@@ -561,7 +569,11 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qma
 #pragma unroll
               for (int i = 0; i < 8; ++i) w[i] = pack2<kOutBf>(o[k][2 * i] * inv2, o[k][2 * i + 1] * inv2);
               QT* d = dst + (c0 + k) * 16;
-              if (wide) {
+              if (!whole) {
+                uint4* pd = reinterpret_cast<uint4*>(part + mine + (c0 + k) * 2 * 512);
+                pd[0] = make_uint4(w[0], w[1], w[2], w[3]);
+                if (D % 16 == 0 || (c0 + k) * 16 + 8 < D) pd[32] = make_uint4(w[4], w[5], w[6], w[7]);
+              } else if (wide) {
                 st_global32(d, w);
               } else {
                 reinterpret_cast<uint4*>(d)[0] = make_uint4(w[0], w[1], w[2], w[3]);
@@ -576,17 +588,17 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qma
         float* stats = reinterpret_cast<float*>(part + 128 * D * 2);
         if (valid) reinterpret_cast<float2*>(stats)[row] = make_float2(m, any ? l : 0.f);
         // the rows of a warp are merged by the warp that delivers their last piece
-        __threadfence();
         __syncwarp();
         unsigned old = 0;
         unsigned* cnt = p.arrive + (size_t(slot) * NQ + wg) * 4 + (warp & 3);
         if (lane == 0) {
+          __threadfence();  // (for the whole warp: __syncwarp orders its stores before it)
           old = atomicAdd(cnt, 1u);
           if (old == unsigned(it.npieces - 1)) *cnt = 0;  // re-arm for the next launch
+          __threadfence();
         }
         old = __shfl_sync(0xffffffffu, old, 0);
         if (old == unsigned(it.npieces - 1) && valid) {
-          __threadfence();
           const unsigned char* base = p.ws + (size_t(slot) * NQ + wg) * kWs;
           const size_t step = size_t(HK) * NQ * kWs;
           // statistics of eight pieces at a time (independent loads), online
@@ -609,41 +621,46 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qma
               if (k0 + k < it.npieces && ml[k].y > 0.f) total_l += ml[k].y * fast_exp2(ml[k].x - mx);
           }
           const float winv = __fdividef(1.f, total_l + 1e-6f);
-          QT* od = static_cast<QT*>(p.out) + out_row;
+          // up to 64 bytes of the row and six pieces at a time: 24 independent loads on their way
+          constexpr int NCH = D / 8, MC = NCH % 4 == 0 ? 4 : (NCH % 2 == 0 ? 2 : 3), MP = 6;
+          static_assert(NCH % MC == 0, "no rest");
 #pragma unroll 1
-          for (int d0 = 0; d0 < D; d0 += 16) {
-            float acc[16];
+          for (int c0 = 0; c0 < NCH; c0 += MC) {
+            float acc[MC][8];
 #pragma unroll
-            for (int z = 0; z < 16; ++z) acc[z] = 0.f;
-            // four pieces at a time: eight independent loads on their way
+            for (int c = 0; c < MC; ++c)
+#pragma unroll
+              for (int z = 0; z < 8; ++z) acc[c][z] = 0.f;
 #pragma unroll 1
-            for (int k0 = 0; k0 < it.npieces; k0 += 4) {
-              uint4 x[4][2];
-              float w[4];
+            for (int k0 = 0; k0 < it.npieces; k0 += MP) {
+              uint4 x[MP][MC];
+              float w[MP];
 #pragma unroll
-              for (int k = 0; k < 4; ++k) {
+              for (int k = 0; k < MP; ++k) {
                 const unsigned char* pk = base + min(k0 + k, it.npieces - 1) * step;
                 const float2 ml = __ldcg(reinterpret_cast<const float2*>(pk + 128 * D * 2) + row);
-                const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const QT*>(pk) + row * D + d0);
-                x[k][0] = __ldcg(src);
-                x[k][1] = D % 16 == 0 || d0 + 8 < D ? __ldcg(src + 1) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+                for (int c = 0; c < MC; ++c)
+                  x[k][c] = __ldcg(reinterpret_cast<const uint4*>(pk + mine + (c0 + c) * 512));
                 // (a piece in which this row has no key has written no output)
                 w[k] = k0 + k < it.npieces && ml.y > 0.f ? ml.y * fast_exp2(ml.x - mx) * winv : 0.f;
               }
 #pragma unroll
-              for (int k = 0; k < 4; ++k) {
+              for (int k = 0; k < MP; ++k) {
                 if (w[k] == 0.f) continue;
-                const QT* xe = reinterpret_cast<const QT*>(x[k]);
 #pragma unroll
-                for (int z = 0; z < 16; ++z) acc[z] += w[k] * to_f32(xe[z]);
+                for (int c = 0; c < MC; ++c) {
+                  const QT* xe = reinterpret_cast<const QT*>(&x[k][c]);
+#pragma unroll
+                  for (int z = 0; z < 8; ++z) acc[c][z] += w[k] * to_f32(xe[z]);
+                }
               }
             }
-            uint4* o4 = reinterpret_cast<uint4*>(od + d0);
-            o4[0] = make_uint4(pack2<kOutBf>(acc[0], acc[1]), pack2<kOutBf>(acc[2], acc[3]),
-                               pack2<kOutBf>(acc[4], acc[5]), pack2<kOutBf>(acc[6], acc[7]));
-            if (D % 16 == 0 || d0 + 8 < D)
-              o4[1] = make_uint4(pack2<kOutBf>(acc[8], acc[9]), pack2<kOutBf>(acc[10], acc[11]),
-                                 pack2<kOutBf>(acc[12], acc[13]), pack2<kOutBf>(acc[14], acc[15]));
+#pragma unroll
+            for (int c = 0; c < MC; ++c)
+              *reinterpret_cast<uint4*>(dst + (c0 + c) * 8) =
+                  make_uint4(pack2<kOutBf>(acc[c][0], acc[c][1]), pack2<kOutBf>(acc[c][2], acc[c][3]),
+                             pack2<kOutBf>(acc[c][4], acc[c][5]), pack2<kOutBf>(acc[c][6], acc[c][7]));
           }
         }
         __syncwarp();
