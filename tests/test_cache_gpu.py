@@ -327,6 +327,52 @@ def test_large_mixed_batches_of_chunks_and_single_tokens(seed):
     assert capi.device_status() == 0
 
 
+@pytest.mark.parametrize("kv,dtype", [("auto", torch.bfloat16), ("fp8", torch.bfloat16), ("fp8_e5m2", torch.float16)])
+@pytest.mark.parametrize("H,D", [(4, 64), (8, 128), (12, 128)])
+@pytest.mark.parametrize("block_size", [16, 32])
+def test_tiles_of_large_writes(kv, dtype, H, D, block_size):
+    """Writes of 4096 tokens and more go by tiles of four heads: chunks that start anywhere (windows of a tile,
+    of what it gives up and of what its neighbours give up), single tokens and padding among them, a last tile
+    that is not full, rows of a fused projection, values whose quotient overflows or is NaN, an odd scale."""
+    rng = np.random.default_rng(H * D + block_size)
+    slots, pos = [], 0
+    for n in [700, 16, 16, 16, 17, 31, 1, 1, 2, 300, 128, 128, 128, 5, 600, 129, 64, 33, 15, 250, 1200, 800]:
+        pos = (pos + block_size - 1) // block_size * block_size + int(rng.integers(0, block_size))
+        slots.append(np.arange(pos, pos + n, dtype=np.int64))
+        pos += n + int(rng.integers(0, 3)) * block_size
+        if rng.integers(0, 4) == 0:
+            slots.append(np.full(int(rng.integers(1, 20)), -1, dtype=np.int64))
+    slots = np.concatenate([slots[i] for i in rng.permutation(len(slots))])
+    T, NB, fp8 = len(slots), int(slots.max()) // block_size + 2, kv != "auto"
+    assert T >= 4096 and T % 16
+    g = torch.Generator(device=DEV).manual_seed(5)
+    qkv = torch.randn(T, 3 * H * D, device=DEV, generator=g).mul(2).to(dtype)
+    key, val = (qkv[:, i * H * D:(i + 1) * H * D].unflatten(1, (H, D)) for i in (1, 2))
+    slots_t = torch.from_numpy(slots).to(DEV)
+    same = lambda a, b: torch.equal(a.cpu().contiguous().view(torch.uint8), b.cpu().contiguous().view(torch.uint8))
+    cdt, x = (torch.uint8, 16) if fp8 else (dtype, 8)
+    for odd in (False, True):
+        if odd:
+            key[5, 1, 3], val[77, 0, 1], val[1999, H - 1, D - 1] = float("nan"), float("inf"), float("nan")
+            key[T - 1, 0, 0], val[T - 1, 0, 0] = float("-inf"), 6e4
+        ks, vs = torch.tensor(0.0173, device=DEV), torch.tensor(2.0 ** -70 if odd else 0.0291, device=DEV)
+        kc = torch.zeros(NB, H, D // x, block_size, x, dtype=cdt, device=DEV)
+        vc = torch.zeros(NB, H, D, block_size, dtype=cdt, device=DEV)
+        ops.reshape_and_cache(key, val, kc, vc, slots_t, kv, ks, vs)
+        kco, vco = torch.zeros_like(kc, device="cpu"), torch.zeros_like(vc, device="cpu")
+        O.reshape_and_cache(key.cpu(), val.cpu(), kco, vco, slots_t.cpu(), kv, float(ks), float(vs))
+        assert same(kc, kco) and same(vc, vco), ("x layout", odd)
+        for hnd in (False, True):
+            shape = (NB, H, block_size, D) if hnd else (NB, block_size, H, D)
+            kf, vf = (torch.zeros(shape, dtype=cdt, device=DEV) for _ in range(2))
+            kfo, vfo = (torch.zeros(shape, dtype=cdt) for _ in range(2))
+            view = (lambda c: c.transpose(1, 2)) if hnd else (lambda c: c)
+            ops.reshape_and_cache_flash(key, val, view(kf), view(vf), slots_t, kv, ks, vs)
+            O.reshape_and_cache_flash(key.cpu(), val.cpu(), view(kfo), view(vfo), slots_t.cpu(), kv, float(ks), float(vs))
+            assert same(kf, kfo) and same(vf, vfo), ("flash layout", odd, hnd)
+    assert capi.device_status() == 0
+
+
 @pytest.mark.parametrize("knobs", [
     {"B200PA_TUNE_KVW_STAGED": "0"},
     {"B200PA_TUNE_KVW_STAGED": "1", "B200PA_TUNE_KVW_HSPLIT": "1", "B200PA_TUNE_KVW_SHIFT": "0"},
@@ -336,7 +382,7 @@ def test_large_mixed_batches_of_chunks_and_single_tokens(seed):
 ], ids=["plain", "staged-whole-heads", "staged-half-heads", "staged-whole-heads-moved-tiles",
         "staged-half-heads-moved-tiles"])
 def test_both_kv_write_implementations(knobs):
-    """The library has two implementations of the KV write (plain loads; rows staged through
+    """Beside the tile kernel the library has two implementations of the KV write (plain loads; rows staged through
     shared memory by bulk async copies, with a whole head or half a head of 128 per work item)
     and picks per call by layout, cache type and size; large x-layout writes use a variant that
     moves 16-token tiles onto 16-slot boundaries of the cache.  B200PA_TUNE_KVW_STAGED / _HSPLIT

@@ -164,6 +164,41 @@ def test_reference_names_are_claimed_on_request_and_never_twice():
     assert r.stdout.split() == ["False", "8", "True", "0"]
 
 
+def test_windows_of_the_tile_kv_write_cover_every_token():
+    """The windows of vllm_b200/csrc/kv_write_tiles.cuh: whatever the slots are, every token in one
+    window: its tile's, the tile's before or the one that its tile keeps for itself in front."""
+    rng = np.random.default_rng(11)
+
+    def shift(slots, i):
+        t = slots[16 * i:16 * i + 16] if i >= 0 else []
+        if len(t) < 16 or min(t[0], t[8], t[15]) < 0 or (t[8] - t[0]) % 16 != 8 or (t[15] - t[0]) % 16 != 15:
+            return 0
+        return int(-t[0] % 16)
+
+    for _ in range(300):
+        pieces, pos = [], 0
+        while sum(map(len, pieces)) < 200:
+            pos += int(rng.integers(0, 40))
+            n = int(rng.choice([1, 2, 15, 16, 17, 32, 48, 70]))
+            pieces.append(np.full(n, -1) if rng.random() < 0.15 else np.arange(pos, pos + n))
+            pos += n
+        slots = np.concatenate([pieces[k] for k in rng.permutation(len(pieces))])
+        if rng.random() < 0.2:
+            slots = rng.permutation(slots)
+        n, seen = len(slots), np.zeros(len(slots), int)
+        for i in range((n + 15) // 16):
+            d, before, after = (shift(slots, k) for k in (i, i - 1, i + 1))
+            windows = [(16 * i + d, 0, min(16 if after == d else 16 - d, n - 16 * i - d))]
+            if d > 0 and before != d:
+                windows.append((16 * i + d - 16, 16 - d, 16))
+            for t, lo, hi in windows:
+                assert 0 <= lo < hi <= 16 and 0 <= t + lo and t + hi <= n
+                seen[t + lo:t + hi] += 1
+                if d > 0 and (t, lo) != windows[0][:2]:  # (row r holds the token whose slot is r modulo 16)
+                    assert slots[t + lo] % 16 == lo
+        assert (seen == 1).all()
+
+
 def test_moved_tiles_of_the_kv_write_cover_every_token():
     """The staged KV write may move a 16-token tile onto the next 16-slot boundary of the cache
     (vllm_b200/csrc/kv_write_staged.cuh, `shift_of`): tile i then covers tokens

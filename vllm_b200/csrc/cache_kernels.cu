@@ -230,11 +230,13 @@ __device__ __forceinline__ void convert_words(const uint32_t (&w)[NW], uint32_t 
 
 }  // namespace b200pa
 
-#include "kv_write_staged.cuh"
+#include "kv_write_tiles.cuh"
+#include "tensor_map.cuh"
 
 namespace b200pa {
 
 constexpr int kTokTile = 16;
+constexpr int kTilesFrom = 4096;  // tokens from which the tile kernel takes over
 
 // n / d for small operands (n * d < 2^32) by one multiply-high with a precomputed factor:
 // the index arithmetic below would otherwise spend more instructions on runtime divisions
@@ -767,10 +769,94 @@ static bool launch_staged(const b200pa_cache_args& a, cudaStream_t stream, int* 
   return launch_staged_as<in_t, cache_t, KV, kFlash, false>(a, stream, rc, hsplit);
 }
 
+// The tile kernel for large writes of 4, 8, ... heads.  Returns as launch_staged_as.
+template <typename in_t, typename cache_t, int KV, int D, bool kFlash>
+static bool launch_tiles_as(const b200pa_cache_args& a, cudaStream_t stream, int* rc) {
+  using SH = TileShape<D>;
+  TileWriteParams p{};
+  p.key_cache = a.key_cache;
+  p.value_cache = a.value_cache;
+  p.slot_mapping = a.slot_mapping;
+  p.k_scale = a.k_scale;
+  p.v_scale = a.v_scale;
+  p.status = device_status_ptr();
+  if (p.status == nullptr) return false;
+  p.block_stride = a.block_stride;
+  p.page_stride = a.page_stride;
+  p.head_stride = a.head_stride;
+  p.num_tokens = a.num_tokens;
+  p.num_heads = a.num_heads;
+  p.block_size = a.block_size;
+  p.move = !kFlash;
+  auto kern = kv_write_tiles_kernel<in_t, cache_t, KV, D, kFlash>;
+  static bool done[64] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess && (dev < 0 || dev >= 64 || !done[dev])) {
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SH::kSmem);
+    if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
+  }
+  CUtensorMap kmap, vmap;
+  auto map = [&](CUtensorMap* m, const void* base, int64_t stride) {
+    return tensor_map<3>(m, base, {D, a.num_tokens, a.num_heads}, {stride, D}, {64, 16, kTileHeads}, CU_TENSOR_MAP_SWIZZLE_128B);
+  };
+  if (e == cudaSuccess) e = map(&kmap, a.key, a.key_stride);
+  if (e == cudaSuccess) e = map(&vmap, a.value, a.value_stride);
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  const int64_t items = int64_t((a.num_tokens + 15) / 16) * ((a.num_heads + kTileHeads - 1) / kTileHeads);
+  const int grid = int(std::min<int64_t>(items, int64_t(cache_sm_count()) * SH::kCtas));
+  e = launch_dependent(kern, dim3(grid), dim3(kTileThreads), SH::kSmem, stream, p, kmap, vmap);
+  count_launch();
+  if (e != cudaSuccess) {
+    set_error("KV write kernel launch failed: %s", cudaGetErrorString(e));
+    *rc = B200PA_ECUDA;
+  } else {
+    *rc = B200PA_OK;
+  }
+  return true;
+}
+
+// Which calls it takes: heads of 128, in the x-layout also of 64 (9500 tokens of 8 heads of 64, 16 bit, 13.2 ->
+// 12.1 us; of 4 heads of 256, fp8, 23.3 -> 25.7: one CTA an SM; flash layout, 4 heads of 64, fp8, 5.9 -> 6.1),
+// from 4096 tokens on (32 chunks of 100 to 160 15.1 -> 11.2; 2080 tokens in 16 chunks 6.5 -> 7.4, 2048
+// scattered ones 14.6 -> 16.1, 4608 scattered ones 45.5 -> 46).  Flash with a 16-bit cache is the plain
+// kernel's.
+template <typename in_t, typename cache_t, int KV, bool kFlash>
+static bool launch_tiles(const b200pa_cache_args& a, cudaStream_t stream, int* rc) {
+  if constexpr (sizeof(in_t) != 2 || sizeof(cache_t) > 2 || (kFlash && KV == kKvAuto)) {
+    return false;
+  } else {
+    constexpr int E = sizeof(cache_t);
+    auto al16 = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr) % 16 == 0; };
+    const int B = a.block_size;
+    if (a.num_tokens < kTilesFrom || a.num_heads % kTileHeads != 0 || B <= 0 || (B & (B - 1)) != 0) return false;
+    if (int64_t(a.num_tokens) * a.num_heads > (int64_t(1) << 30)) return false;  // (items are numbered in 32 bits)
+    if (!al16(a.key) || !al16(a.value) || !al16(a.key_cache) || !al16(a.value_cache)) return false;
+    if (a.key_stride % 8 != 0 || a.value_stride % 8 != 0 || !tensor_map_stride(a.key_stride) ||
+        !tensor_map_stride(a.value_stride))
+      return false;
+    if (kFlash) {
+      if ((a.block_stride * E) % 16 != 0 || (a.page_stride * E) % 16 != 0 || (a.head_stride * E) % 16 != 0) return false;
+    } else if (a.x != 16 / E || B % 16 != 0) {
+      return false;
+    }
+    switch (a.head_size) {
+      case 64:
+        if constexpr (!kFlash) return launch_tiles_as<in_t, cache_t, KV, 64, false>(a, stream, rc);
+        return false;
+      case 128: return launch_tiles_as<in_t, cache_t, KV, 128, kFlash>(a, stream, rc);
+    }
+    return false;
+  }
+}
+
 template <typename in_t, typename cache_t, int KV>
 static int launch_reshape(const b200pa_cache_args& a, cudaStream_t stream, bool flash) {
   if (a.num_tokens == 0) return B200PA_OK;
-  // Two implementations; which one is faster was measured per case on B200 (16 384 tokens x 8
+  // Large writes go by tiles (launch_tiles).  Of the two other implementations which one is faster was measured per case on B200 (16 384 tokens x 8
   // heads x 128, us, staged / plain): x-layout fp8 29 / 31, flash fp8 27 / 29, x-layout 16-bit
   // cache 27 / 40, 256 scattered tokens (a decode step) 11 / 17, x-layout fp8 with sequences
   // that start inside a block 38 / 92 - and flash with a 16-bit cache 30 / 25, the
@@ -778,8 +864,11 @@ static int launch_reshape(const b200pa_cache_args& a, cudaStream_t stream, bool 
   // (for the tests that compare the two).
   static const int kn_staged = [] { const char* e = getenv("B200PA_TUNE_KVW_STAGED"); return e ? atoi(e) : -1; }();
   const bool prefer_staged = !(flash && KV == kKvAuto) || a.num_tokens <= 4096;
+  int rc = B200PA_OK;
+  if (kn_staged < 0 && (flash ? launch_tiles<in_t, cache_t, KV, true>(a, stream, &rc)
+                              : launch_tiles<in_t, cache_t, KV, false>(a, stream, &rc)))
+    return rc;
   if (kn_staged == 1 || (kn_staged != 0 && prefer_staged)) {
-    int rc = B200PA_OK;
     const bool took = flash ? launch_staged<in_t, cache_t, KV, true>(a, stream, &rc)
                             : launch_staged<in_t, cache_t, KV, false>(a, stream, &rc);
     if (took) return rc;

@@ -5,36 +5,9 @@
 
 #include "launch_state.cuh"
 #include "prefill_inst.cuh"
+#include "tensor_map.cuh"
 
 namespace b200pa {
-
-// A tensor map of 16-bit elements without interleaving; `strides` in elements.
-template <int N>
-static cudaError_t tensor_map(CUtensorMap* map, const void* base, const int64_t (&dims)[N], const int64_t (&strides)[N - 1],
-                              const int (&box)[N], CUtensorMapSwizzle swizzle) {
-  using Encode = decltype(&cuTensorMapEncodeTiled);
-  static const Encode encode = [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &found) != cudaSuccess ||
-        found != cudaDriverEntryPointSuccess)
-      f = nullptr;
-    return reinterpret_cast<Encode>(f);
-  }();
-  if (encode == nullptr) return cudaErrorNotSupported;
-  cuuint64_t d[N], st[N - 1];
-  cuuint32_t b[N], step[N];
-  for (int i = 0; i < N; ++i) {
-    d[i] = cuuint64_t(dims[i]);
-    b[i] = cuuint32_t(box[i]);
-    step[i] = 1;
-  }
-  for (int i = 0; i < N - 1; ++i) st[i] = cuuint64_t(strides[i]) * 2;
-  const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, N, const_cast<void*>(base), d, st, b, step,
-                            CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
-}
 
 cudaError_t prefill_v_map(const PrefillParams& p, int head_size, CUtensorMap* map) {
   return tensor_map<4>(map, p.vc, {p.block_size, head_size, p.num_kv_heads, INT32_MAX},
@@ -52,12 +25,11 @@ cudaError_t prefill_q_map(const PrefillParams& p, int head_size, int box, CUtens
 static PrefillKernelInfo find_prefill(const b200pa_attn_args& a) {
   const int es = a.kv_dtype == B200PA_KV_AUTO ? 2 : 1;
   auto al = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr) % 16 == 0; };
-  auto stride_fits = [](int64_t v) { return v > 0 && v < (int64_t(1) << 39); };  // 2-byte elements
   const bool fits = (a.block_size == 16 || a.block_size == 32) && a.num_heads / a.num_kv_heads <= 128 &&
                     al(a.key_cache) && al(a.value_cache) && al(a.query) && al(a.out) &&
                     (a.kv_block_stride * es) % 16 == 0 && (a.kv_head_stride * es) % 16 == 0 &&
-                    (es == 1 || (stride_fits(a.kv_block_stride) && stride_fits(a.kv_head_stride))) &&
-                    a.q_stride % 8 == 0 && stride_fits(a.q_stride) && a.blocksparse_vert_stride <= 1 && a.out_lse == nullptr;
+                    (es == 1 || (tensor_map_stride(a.kv_block_stride) && tensor_map_stride(a.kv_head_stride))) &&
+                    a.q_stride % 8 == 0 && tensor_map_stride(a.q_stride) && a.blocksparse_vert_stride <= 1 && a.out_lse == nullptr;
   if (!fits) return {nullptr, 0};
   return a.head_size <= 96 ? find_prefill_small(a.head_size, a.q_dtype, a.kv_dtype)
          : a.head_size <= 128 ? find_prefill_mid(a.head_size, a.q_dtype, a.kv_dtype)
