@@ -268,6 +268,18 @@ int b200pa_reshape_and_cache(const b200pa_cache_args* args, void* stream);
 int b200pa_reshape_and_cache_flash(const b200pa_cache_args* args, void* stream);
 
 /*
+ * One layer of an engine step in one call: the KV write of the step's tokens (b200pa_reshape_and_cache;
+ * `write` NULL: none), then attention on the same stream, which then starts under the write and waits for
+ * it where it first reads the cache.
+ *   query_start_loc, num_tokens, num_decodes: as for b200pa_paged_attention_varlen; query_start_loc NULL:
+ *     a decode batch, one query row per sequence, as for v1, or v2 where `caller_scratch` is not 0
+ * Returns B200PA_EUNSUPPORTED, with nothing launched, where b200pa_paged_attention_varlen has no kernel.
+ */
+int b200pa_attention_step(const b200pa_cache_args* write, const b200pa_attn_args* args,
+                          const int32_t* query_start_loc, int32_t num_tokens, int32_t num_decodes,
+                          int32_t caller_scratch, void* stream);
+
+/*
  * Replaces convert_fp8 (csrc/cache_kernels.cu:826-899): elementwise
  * quantise (src 16/32-bit -> dst fp8) or dequantise (src fp8 -> dst 16/32-bit)
  * of `numel` contiguous elements with a host-side scalar scale.

@@ -227,3 +227,36 @@ def test_a_replay_beside_launches_on_another_stream():
         side.wait_stream(torch.cuda.current_stream())
     graphed.check()
     eager.check()
+
+
+@pytest.mark.parametrize("kv", ["auto", "fp8"])
+@pytest.mark.parametrize("new,ctx", [([1] * 3, [300, 15, 600]), ([1] * 120, list(range(60, 300, 2))),
+                                     ([40, 130, 7], [100, 0, 500]), ([1] * 9 + [70, 33], [200] * 9 + [64, 300])],
+                         ids=["few-decodes", "many-decodes", "chunks", "mixed"])
+def test_attention_starts_under_the_write_of_its_step(new, ctx, kv):
+    """Attention reads lengths, block tables and Q while the KV write in front may still run: what kernels
+    before the write have just stored has to be what it sees, step after step, without a host in between."""
+    eng = Engine(len(new), sum(new), kv=kv)
+    cache, names = eng.cache.clone(), ("q", "k", "v", "table", "lens", "slots", "qsl")
+    steps = []
+    for i in range(4):
+        eng.load(new, [max(0, c - 7 * i) for c in ctx])
+        steps.append({n: getattr(eng, n).clone() for n in names})
+    meta = eng.builder.build(0, eng.common(max_seq_len=max(c + t for t, c in zip(new, ctx))))
+
+    def run(wait):
+        eng.cache.copy_(cache)
+        outs = []
+        for step in steps * 5:
+            for n in names:
+                getattr(eng, n).copy_(step[n])
+            wait()
+            eng.forward(meta)
+            wait()
+            outs.append(eng.out.clone())
+        return torch.stack(outs).float()
+    got, want = run(lambda: None), run(torch.cuda.synchronize)
+    # (the same kernels on the same values: only the order of partial sums may differ)
+    assert ((got - want).norm(dim=-1) < 4e-3 * want.norm(dim=-1)).all()
+    from vllm_b200 import capi
+    assert capi.device_status() == 0

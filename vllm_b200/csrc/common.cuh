@@ -47,6 +47,9 @@ int* device_status_ptr();
 // (programmatic dependent launch).  Such a kernel calls grid_dependency() before its first access to
 // global memory: up to there only its own set-up overlaps.  What it saves is the launch latency
 // between two kernels of a stream, which small launches are mostly made of.
+//   Directly behind the KV write of the same step an attention kernel may do more (its `early`): the
+// write lets it start only when it has itself waited for everything in front, and changes nothing but the
+// cache, so lengths, block tables and Q can be read before grid_dependency() (past L1), K and V after it.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
                                     cudaStream_t stream, Args... args) {

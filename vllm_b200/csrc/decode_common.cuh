@@ -55,6 +55,7 @@ struct DecodeParams {
   int bs_vert_stride;
   int bs_block_size;
   int bs_head_sliding_step;
+  int early;  // 1: the launch in front is the step's KV write, see launch_dependent
 };
 
 // ------------------------------------------------------------------ PTX wrappers

@@ -122,9 +122,9 @@ pa_decode_direct_kernel(const DecodeParams p, const int cluster) {
   const int hq0 = kvh * p.group + hg * HEADS;
   const int nheads = min(HEADS, p.group - hg * HEADS);
   const int B = p.block_size, b_shift = 31 - __clz(B);
-  grid_dependency();
+  if (!p.early) grid_dependency();
 
-  const int len = min(max(p.seq_lens[seq], 0), p.len_cap);
+  const int len = min(max(__ldcg(p.seq_lens + seq), 0), p.len_cap);
   // ---- Q (B operand; n = head g): 16 bytes of K's chunk order per chunk of this lane
   uint32_t qf[GP][NI][SPC][2];
 #pragma unroll
@@ -138,7 +138,7 @@ pa_decode_direct_kernel(const DecodeParams p, const int cluster) {
       const bool ok = hl < nheads && (CHUNKS % 4 == 0 || ch < CHUNKS);
 #pragma unroll
       for (int k = 0; k < X / 8; ++k) {
-        const uint4 v = ok ? __ldg(reinterpret_cast<const uint4*>(q + ch * X) + k) : make_uint4(0, 0, 0, 0);
+        const uint4 v = ok ? __ldcg(reinterpret_cast<const uint4*>(q + ch * X) + k) : make_uint4(0, 0, 0, 0);
         w[4 * k] = v.x;
         w[4 * k + 1] = v.y;
         w[4 * k + 2] = v.z;
@@ -156,14 +156,14 @@ pa_decode_direct_kernel(const DecodeParams p, const int cluster) {
       }
     }
   }
-  const float qk_scale = p.scale * kLog2e * (kFp8 ? *p.k_scale : 1.f);
+  const float qk_scale = p.scale * kLog2e * (kFp8 ? __ldcg(p.k_scale) : 1.f);
   float slope[GP][2];
 #pragma unroll
   for (int nt = 0; nt < GP; ++nt)
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       const int hl = nt * 8 + 2 * c + j;
-      slope[nt][j] = (p.alibi != nullptr && hl < nheads) ? p.alibi[hq0 + hl] * kLog2e : 0.f;
+      slope[nt][j] = (p.alibi != nullptr && hl < nheads) ? __ldcg(p.alibi + hq0 + hl) * kLog2e : 0.f;
     }
 
   // ---- this warp's 16-token tiles [t_begin, t_end)
@@ -176,7 +176,7 @@ pa_decode_direct_kernel(const DecodeParams p, const int cluster) {
   const int64_t bstride = p.kv_block_stride * ES;
   int ids = 0;
   auto load_ids = [&](int t0) {  // block ids of tiles t0 .. t0 + 31
-    ids = t0 + lane < t_end ? __ldg(bt + (((t0 + lane) << 4) >> b_shift)) : 0;
+    ids = t0 + lane < t_end ? __ldcg(bt + (((t0 + lane) << 4) >> b_shift)) : 0;
   };
   // row rho = 8 h + g of the tile's S^T is token 4 (g / 2) + 2 h + g % 2: a lane's V tokens 4c .. 4c+3
   // are then the k indices that its registers of the P.V product stand for
@@ -223,8 +223,9 @@ pa_decode_direct_kernel(const DecodeParams p, const int cluster) {
     m_run[nt][0] = m_run[nt][1] = -INFINITY;
     l_run[nt][0] = l_run[nt][1] = 0.f;
   }
+  if (t_begin < t_end) load_ids(t_begin);
+  if (p.early) grid_dependency();  // (from here on K and V)
   if (t_begin < t_end) {
-    load_ids(t_begin);
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
       if (t_begin + b < t_end) {

@@ -568,7 +568,7 @@ __global__ void __launch_bounds__(MAXW * 32, 1) pa_decode_kernel(const DecodePar
   __shared__ int4 s_iter[MAXW];  // per warp: units left, block offset, sequence, head
   __shared__ int4 s_todo[MAXW][2];  // per warp: merges owed (sequence, head item, pieces, piece | level)
   __shared__ int s_ntodo[MAXW];
-  grid_dependency();
+  if (!p.early) grid_dependency();
   const bool flat = p.use_table != 0;
   const int hsubs = p.num_kv_heads * p.head_groups;
   if (flat) {
@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(MAXW * 32, 1) pa_decode_kernel(const DecodePar
     const int s0 = min(S, int(threadIdx.x) * per);
     const int s1 = min(S, s0 + per);
     auto units_of = [&](int s) {
-      const int len = min(max(p.seq_lens[s], 0), p.len_cap);
+      const int len = min(max(__ldcg(p.seq_lens + s), 0), p.len_cap);
       return max(2, ((len + B - 1) / B + 1) & ~1);
     };
     int mine = 0, mx = 0;
@@ -629,6 +629,7 @@ __global__ void __launch_bounds__(MAXW * 32, 1) pa_decode_kernel(const DecodePar
       s_plan[2] = int((U + C - 1) / C);
     }
   }
+  if (p.early) grid_dependency();
   __syncthreads();
 
   const unsigned grid_warps = gridDim.x * unsigned(nwarps);

@@ -24,7 +24,9 @@ bool stream_region(cudaStream_t stream, StreamRegion* out);
 unsigned* sched_words(cudaStream_t stream);
 int sm_count();
 
-// paged_attention_v1 on the first half of the stream's workspace and arrival counters.
-int attention_half_region(const b200pa_attn_args* a, void* stream);
+// paged_attention_v1 on the first half of the stream's workspace and arrival counters; the attention
+// entries directly behind the KV write of their step (see launch_dependent).
+int attention_half_region(const b200pa_attn_args* a, void* stream, bool behind_write);
+int attention_behind_write(const b200pa_attn_args* a, void* stream, bool caller_scratch);
 
 }  // namespace b200pa

@@ -552,7 +552,7 @@ enum class Scratch {
 
 // `share`: the call may use one `share`-th of the stream's workspace and arrival counters (another
 // launch that may run at the same time has the rest).
-static int attention_entry(const b200pa_attn_args* a, void* stream, Scratch mode, int share = 1) {
+static int attention_entry(const b200pa_attn_args* a, void* stream, Scratch mode, int share = 1, bool behind_write = false) {
   const bool v2 = mode != Scratch::kNone;
   B200PA_CHECK_ARG(a != nullptr, "args is NULL");
   B200PA_CHECK_ARG(a->num_seqs >= 0 && a->num_heads > 0 && a->num_kv_heads > 0 && a->head_size > 0,
@@ -652,6 +652,7 @@ static int attention_entry(const b200pa_attn_args* a, void* stream, Scratch mode
   p.bs_vert_stride = a->blocksparse_vert_stride;
   p.bs_block_size = a->blocksparse_block_size;
   p.bs_head_sliding_step = a->blocksparse_head_sliding_step;
+  p.early = behind_write;
 
   const Route route = decode_route(*a, split, tune);
   const DecodeKernelInfo ki = route.persistent;
@@ -833,8 +834,11 @@ static int attention_entry(const b200pa_attn_args* a, void* stream, Scratch mode
   return B200PA_OK;
 }
 
-int attention_half_region(const b200pa_attn_args* a, void* stream) {
-  return attention_entry(a, stream, Scratch::kNone, 2);
+int attention_half_region(const b200pa_attn_args* a, void* stream, bool behind_write) {
+  return attention_entry(a, stream, Scratch::kNone, 2, behind_write);
+}
+int attention_behind_write(const b200pa_attn_args* a, void* stream, bool caller_scratch) {
+  return attention_entry(a, stream, caller_scratch ? Scratch::kCaller : Scratch::kNone, 1, true);
 }
 
 }  // namespace b200pa

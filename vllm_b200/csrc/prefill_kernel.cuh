@@ -78,6 +78,7 @@ struct PrefillParams {
   int ws_slots;               // pieces that the workspace has room for
   int late_wait;              // 1: independent of the launch in front, waits for it at the end only (the launch in
                               // front has itself waited for all before it)
+  int early;                  // 1: the launch in front is the step's KV write, see launch_dependent
   float scale;
 };
 
@@ -199,7 +200,8 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qma
   }
   if (tid < 16) s_red[2][tid] = 0;  // (see the plan)
   __syncthreads();
-  if (p.late_wait) grid_launch_dependents(); else grid_dependency();
+  if (p.late_wait) grid_launch_dependents();
+  else if (!p.early) grid_dependency();
 
   // ---- plan.  T tokens fill a row tile; a request has ceil(q_len / (NQ T)) row-tile groups per kv
   // head, and each of them npieces pieces.
@@ -209,8 +211,8 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qma
   static_assert(kPrefillThreads == kPrefillMaxReqs, "a thread to a request");
   int ql = 0, len = 0;
   if (tid < S) {
-    ql = p.q_start[tid + 1] - p.q_start[tid];
-    len = p.seq_lens[tid];
+    ql = __ldcg(p.q_start + tid + 1) - __ldcg(p.q_start + tid);
+    len = __ldcg(p.seq_lens + tid);
     if (tid < kPrefillSortReqs) s_sort[tid] = len;
   }
   const int n = (ql + TT - 1) / TT;  // groups
@@ -319,9 +321,9 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qma
     int lo = 16 * (31 - __clz(__ballot_sync(0xffffffffu, starts(16 * lane))));
     lo += 31 - __clz(__ballot_sync(0xffffffffu, lane < 16 && starts(lo + lane)));
     it.req = sorted ? int(s_order[lo]) : lo;
-    it.q0 = p.q_start[it.req];
-    it.q_len = p.q_start[it.req + 1] - it.q0;
-    it.seq_len = p.seq_lens[it.req];
+    it.q0 = __ldcg(p.q_start + it.req);
+    it.q_len = __ldcg(p.q_start + it.req + 1) - it.q0;
+    it.seq_len = __ldcg(p.seq_lens + it.req);
     it.ctx = it.seq_len - it.q_len;
     const unsigned rel = item - (cum[lo] >> 1);
     unsigned gp = rel / unsigned(HK);
@@ -395,9 +397,9 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qma
     const uint32_t lane_off = uint32_t((warp & 3) * 32) << 16;
     const uint32_t t_s = tmem + lane_off + uint32_t(wg * KT);
     const uint32_t t_o = tmem + lane_off + uint32_t(NQ * KT + wg * DP);
-    const float c = p.scale * kLog2e * (kFp8 ? *p.k_scale : 1.f);
+    const float c = p.scale * kLog2e * (kFp8 ? __ldcg(p.k_scale) : 1.f);
     const bool biased = p.alibi != nullptr || !(c > 0.f);  // the maximum is taken of the scaled values then
-    const float v_scale = kFp8 ? *p.v_scale : 1.f;
+    const float v_scale = kFp8 ? __ldcg(p.v_scale) : 1.f;
     const bool row_used = wg < NQ && row < T * G;
     const int row_tok = row / G, row_head = row % G;
     uint32_t n_s = 0, n_pv = 0;  // S tiles received, PV products issued for this row tile
@@ -410,7 +412,7 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qma
       const int pos = valid ? it.ctx + tok : -1;                     // last key of this row
       const int pos_first = it.ctx + it.tok0 + wg * T;               // ... of the tile's first row
       const int head = it.kvh * G + row_head;
-      const float slope = (p.alibi != nullptr && valid) ? p.alibi[head] * kLog2e : 0.f;
+      const float slope = (p.alibi != nullptr && valid) ? __ldcg(p.alibi + head) * kLog2e : 0.f;
       float m = -INFINITY, l = 0.f;
       for (int j = b; j < e; ++j) {
         if (!wait(s_full(wg), n_s & 1)) break;
@@ -708,7 +710,7 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qma
       const int* bt = p.block_tables + int64_t(it.req) * p.max_blocks_per_seq;
       const int64_t head_off = int64_t(it.kvh) * p.kv_head_stride * ES;
       const int e = max(it.e0, it.e1);
-      auto block_of = [&](int key) { return key < it.seq_len ? __ldg(bt + (key >> b_shift)) : 0; };
+      auto block_of = [&](int key) { return key < it.seq_len ? __ldcg(bt + (key >> b_shift)) : 0; };
       auto page = [&](const char* base, int blk) {
         return base + int64_t(blk) * p.kv_block_stride * ES + head_off;
       };
@@ -721,6 +723,7 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qma
         constexpr int NP = KT / 16;  // pages per tile
         const int kt = pt % KT, kg = pt / KT;
         int k_blk = block_of(it.b * KT + kt), v_blk = block_of(it.b * KT + lane % NP * 16);
+        if (p.early) grid_dependency();  // (from here on K and V; returns at once when it has done so before)
         for (int j = it.b; j < e && ok; ++j) {
           {
             const int key = j * KT + kt;
@@ -822,6 +825,7 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qma
           fp8x4_to_f16<kE5>(x.z, hi.x, hi.y);
           fp8x4_to_f16<kE5>(x.w, hi.z, hi.w);
         };
+        if (p.early) grid_dependency();
         if (it.b < e) {
           get_k(it.b);
           get_v(it.b);
@@ -1067,7 +1071,7 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qma
     }
   }
 
-  if (p.late_wait) grid_dependency_wait();
+  if (p.late_wait || p.early) grid_dependency_wait();
   // ---- everything issued has been waited for by the softmax warpgroups (or a wait ran out)
   tc_fence_before();
   __syncthreads();

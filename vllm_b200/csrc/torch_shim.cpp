@@ -785,9 +785,9 @@ PyObject* py_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p.blocksparse_block_size = 64;
     // (nothing may be done before it is clear that everything can be: the caller would do it again)
     if (max_q > 1 && decodes < reqs && !b200pa_paged_attention_varlen_supported(&p)) return false;
+    b200pa_cache_args c;
+    std::memset(&c, 0, sizeof(c));
     if (write) {
-      b200pa_cache_args c;
-      std::memset(&c, 0, sizeof(c));
       c.in_dtype = in_type;
       c.kv_dtype = kv_type;
       c.key = k.data_ptr();
@@ -804,13 +804,13 @@ PyObject* py_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
       c.head_size = static_cast<int32_t>(D);
       c.block_size = static_cast<int32_t>(B);
       c.x = static_cast<int32_t>(x);
-      check_rc(b200pa_reshape_and_cache(&c, stream));
     }
+    auto run = [&](const int* starts, bool caller_scratch) {
+      check_rc(b200pa_attention_step(write ? &c : nullptr, &p, starts, static_cast<int32_t>(tokens),
+                                     static_cast<int32_t>(decodes), caller_scratch, stream));
+    };
     if (max_q > 1) {
-      const int rc = b200pa_paged_attention_varlen(&p, qsl.data_ptr<int>(), static_cast<int32_t>(tokens),
-                                                   static_cast<int32_t>(decodes), stream);
-      if (rc == B200PA_EUNSUPPORTED) return false;
-      check_rc(rc);
+      run(qsl.data_ptr<int>(), false);
       return true;
     }
     // v1 also when the partials of v2 fit the library's own workspace, which saves the scratch allocation
@@ -818,7 +818,7 @@ PyObject* py_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const bool use_v1 =
         prefer_v1 != 0 || rows_n * parts * (8 + 2 * D) <= b200pa_stream_workspace_bytes() - 1024;
     if (use_v1) {
-      check_rc(b200pa_paged_attention_v1(&p, stream));
+      run(nullptr, false);
       return true;
     }
     const int64_t stat = (rows_n * parts * 4 + 255) & ~int64_t(255);
@@ -829,7 +829,7 @@ PyObject* py_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p.max_logits = reinterpret_cast<float*>(sp + stat);
     p.tmp_out = sp + 2 * stat;
     p.max_num_partitions = static_cast<int32_t>(parts);
-    check_rc(b200pa_paged_attention_v2(&p, stream));
+    run(nullptr, true);
     return true;
   });
 }

@@ -43,9 +43,11 @@ extern "C" int b200pa_paged_attention_varlen_supported(const b200pa_attn_args* a
          b200pa::find_prefill(*a).fn != nullptr;
 }
 
-extern "C" int b200pa_paged_attention_varlen(const b200pa_attn_args* a, const int32_t* query_start_loc,
-                                             int32_t num_tokens, int32_t num_decodes, void* stream) {
-  using namespace b200pa;
+namespace b200pa {
+
+// `behind_write`: the launch in front on the stream is the KV write of the same step.
+static int attention_varlen(const b200pa_attn_args* a, const int32_t* query_start_loc, int32_t num_tokens,
+                            int32_t num_decodes, void* stream, bool behind_write) {
   B200PA_CHECK_ARG(a != nullptr, "args is NULL");
   B200PA_CHECK_ARG(a->num_seqs >= 0 && a->num_heads > 0 && a->num_kv_heads > 0 && a->head_size > 0 &&
                        a->num_heads % a->num_kv_heads == 0,
@@ -74,7 +76,8 @@ extern "C" int b200pa_paged_attention_varlen(const b200pa_attn_args* a, const in
     // the decode rows are the first rows of query and out: an ordinary decode batch
     b200pa_attn_args d = *a;
     d.num_seqs = num_decodes;
-    const int rc = reqs > 0 ? attention_half_region(&d, stream) : b200pa_paged_attention_v1(&d, stream);
+    const int rc = reqs > 0 ? attention_half_region(&d, stream, behind_write)
+                   : behind_write ? attention_behind_write(&d, stream, false) : b200pa_paged_attention_v1(&d, stream);
     if (rc != B200PA_OK) return rc;
   }
   if (reqs == 0) return B200PA_OK;
@@ -114,6 +117,7 @@ extern "C" int b200pa_paged_attention_varlen(const b200pa_attn_args* a, const in
     p.num_reqs = std::min(kPrefillMaxReqs, a->num_seqs - r);
     // nothing here depends on the decode launch: start where its CTAs have left, wait for it at the end
     p.late_wait = r == num_decodes && num_decodes > 0 ? 1 : 0;
+    p.early = r == 0 && behind_write ? 1 : 0;
     p.block_tables = a->block_tables + int64_t(r) * a->max_num_blocks_per_seq;
     p.seq_lens = a->seq_lens + r;
     p.q_start = query_start_loc + r;
@@ -130,4 +134,33 @@ extern "C" int b200pa_paged_attention_varlen(const b200pa_attn_args* a, const in
     }
   }
   return B200PA_OK;
+}
+
+}  // namespace b200pa
+
+extern "C" int b200pa_paged_attention_varlen(const b200pa_attn_args* a, const int32_t* query_start_loc,
+                                             int32_t num_tokens, int32_t num_decodes, void* stream) {
+  return b200pa::attention_varlen(a, query_start_loc, num_tokens, num_decodes, stream, false);
+}
+
+extern "C" int b200pa_attention_step(const b200pa_cache_args* write, const b200pa_attn_args* a,
+                                     const int32_t* query_start_loc, int32_t num_tokens, int32_t num_decodes,
+                                     int32_t caller_scratch, void* stream) {
+  using namespace b200pa;
+  B200PA_CHECK_ARG(a != nullptr, "args is NULL");
+  if (query_start_loc != nullptr && num_decodes < a->num_seqs && !b200pa_paged_attention_varlen_supported(a)) {
+    set_error("attention_step: no kernel for head_size=%d block_size=%d q_dtype=%d kv_dtype=%d, or unaligned tensors",
+              a->head_size, a->block_size, a->q_dtype, a->kv_dtype);
+    return B200PA_EUNSUPPORTED;
+  }
+  bool behind_write = false;
+  if (write != nullptr) {
+    const int rc = b200pa_reshape_and_cache(write, stream);
+    if (rc != B200PA_OK) return rc;
+    behind_write = write->num_tokens > 0;
+  }
+  if (query_start_loc != nullptr)
+    return attention_varlen(a, query_start_loc, num_tokens, num_decodes, stream, behind_write);
+  if (behind_write) return attention_behind_write(a, stream, caller_scratch != 0);
+  return caller_scratch != 0 ? b200pa_paged_attention_v2(a, stream) : b200pa_paged_attention_v1(a, stream);
 }
