@@ -328,10 +328,10 @@ def test_large_mixed_batches_of_chunks_and_single_tokens(seed):
 
 
 @pytest.mark.parametrize("kv,dtype", [("auto", torch.bfloat16), ("fp8", torch.bfloat16), ("fp8_e5m2", torch.float16)])
-@pytest.mark.parametrize("H,D", [(4, 64), (8, 128), (12, 128)])
+@pytest.mark.parametrize("H,D", [(4, 64), (8, 128), (2, 128), (4, 256)])
 @pytest.mark.parametrize("block_size", [16, 32])
 def test_tiles_of_large_writes(kv, dtype, H, D, block_size):
-    """Writes of 4096 tokens and more go by tiles of four heads: chunks that start anywhere (windows of a tile,
+    """Writes of 2560 tokens and more go by tiles of two heads: chunks that start anywhere (windows of a tile,
     of what it gives up and of what its neighbours give up), single tokens and padding among them, a last tile
     that is not full, rows of a fused projection, values whose quotient overflows or is NaN, an odd scale."""
     rng = np.random.default_rng(H * D + block_size)

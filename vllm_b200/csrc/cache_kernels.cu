@@ -236,7 +236,7 @@ __device__ __forceinline__ void convert_words(const uint32_t (&w)[NW], uint32_t 
 namespace b200pa {
 
 constexpr int kTokTile = 16;
-constexpr int kTilesFrom = 4096;  // tokens from which the tile kernel takes over
+constexpr int kTilesFrom = 2560;  // tokens from which the tile kernel takes over
 
 // n / d for small operands (n * d < 2^32) by one multiply-high with a precomputed factor:
 // the index arithmetic below would otherwise spend more instructions on runtime divisions
@@ -769,7 +769,7 @@ static bool launch_staged(const b200pa_cache_args& a, cudaStream_t stream, int* 
   return launch_staged_as<in_t, cache_t, KV, kFlash, false>(a, stream, rc, hsplit);
 }
 
-// The tile kernel for large writes of 4, 8, ... heads.  Returns as launch_staged_as.
+// The tile kernel for large writes of an even number of heads.  Returns as launch_staged_as.
 template <typename in_t, typename cache_t, int KV, int D, bool kFlash>
 static bool launch_tiles_as(const b200pa_cache_args& a, cudaStream_t stream, int* rc) {
   using SH = TileShape<D>;
@@ -819,11 +819,11 @@ static bool launch_tiles_as(const b200pa_cache_args& a, cudaStream_t stream, int
   return true;
 }
 
-// Which calls it takes: heads of 128, in the x-layout also of 64 (9500 tokens of 8 heads of 64, 16 bit, 13.2 ->
-// 12.1 us; of 4 heads of 256, fp8, 23.3 -> 25.7: one CTA an SM; flash layout, 4 heads of 64, fp8, 5.9 -> 6.1),
-// from 4096 tokens on (32 chunks of 100 to 160 15.1 -> 11.2; 2080 tokens in 16 chunks 6.5 -> 7.4, 2048
-// scattered ones 14.6 -> 16.1, 4608 scattered ones 45.5 -> 46).  Flash with a 16-bit cache is the plain
-// kernel's.
+// Which calls it takes: heads of whole boxes (64, 128, 256), from 2560 tokens on.  Staged -> tiles, us, 8 heads of
+// 128 to fp8 unless stated: 3000 tokens in 3 chunks 9.2 -> 8.0, the same in the flash layout 7.0 -> 6.2; 2080 in 16
+// chunks 6.5 -> 6.9, 2048 scattered ones 14.7 -> 15.9, 1100 in 2 chunks 5.0 -> 5.4; 8000 tokens of 2 heads 10.7 ->
+// 6.2, 9500 of 4 heads of 256 23.4 -> 21.5, of 4 heads of 64 in the flash layout 5.9 -> 5.5; 4608 scattered
+// ones 45.5 -> 46.5.  Flash with a 16-bit cache is the plain kernel's.
 template <typename in_t, typename cache_t, int KV, bool kFlash>
 static bool launch_tiles(const b200pa_cache_args& a, cudaStream_t stream, int* rc) {
   if constexpr (sizeof(in_t) != 2 || sizeof(cache_t) > 2 || (kFlash && KV == kKvAuto)) {
@@ -845,8 +845,8 @@ static bool launch_tiles(const b200pa_cache_args& a, cudaStream_t stream, int* r
     }
     switch (a.head_size) {
       case 64:
-        if constexpr (!kFlash) return launch_tiles_as<in_t, cache_t, KV, 64, false>(a, stream, rc);
-        return false;
+        return launch_tiles_as<in_t, cache_t, KV, 64, kFlash>(a, stream, rc);
+      case 256: return launch_tiles_as<in_t, cache_t, KV, 256, kFlash>(a, stream, rc);
       case 128: return launch_tiles_as<in_t, cache_t, KV, 128, kFlash>(a, stream, rc);
     }
     return false;

@@ -4,9 +4,10 @@
 // What bounds it: HBM, once the instructions per element are few.  The staged kernel (kv_write_staged.cuh)
 // spends 16 a bf16 element on a quantising write, 9 of them on its work items (16 tokens of one head of K or
 // V, each with its own slot look-up, window search and 16 row copies); here
-//   * a work item is 16 tokens x 4 heads of K and V, fetched with one tensor-map box per 64 head dimensions
-//     (128-byte swizzle) into a ring of three stages;
-//   * one warp walks over the tiles: slots, window (see below), copies; eight warps convert, half a head of
+//   * a work item is 16 tokens x 2 heads of K and V, fetched with one tensor-map box per 64 head dimensions
+//     (128-byte swizzle) into a ring of three stages, four CTAs to an SM (4 heads and two CTAs: 1 to 12 % more
+//     below 10000 tokens; 1 head and eight: up to 13 % less below, 3 % more on the largest);
+//   * one warp walks over the tiles: slots, window (see below), copies; four warps convert, half a head of
 //     K and of V each (V takes longer, so not K in four of them and V in the others), with all loops
 //     unrolled and the head size a constant;
 //   * K (and V of the flash layout): a lane converts 16 bytes of output of one token; V of the x-layout: the
@@ -18,8 +19,8 @@
 // that boundary, unless the tile before is moved as far.  Three slots of a tile decide, the same for it and
 // for its neighbours; whatever the slots are, every token is written, with its own slot.
 // Measured on B200, staged kernel -> this one, us: 128 chunks of 128 tokens that start anywhere, 8 heads of
-// 128, to fp8 36.4 -> 23.6 (4.3 TB/s), 16 bit 43 -> 29.6; 32 chunks of 100 to 160, fp8, 15.1 -> 11.2; flash
-// layout 16384 tokens, fp8, 21.9 -> 20.0.  What is left over 15.6 of traffic: start and end, about 6, and 10
+// 128, to fp8 36.4 -> 23.5 (4.3 TB/s), 16 bit 43 -> 29.8; 32 chunks of 100 to 160, fp8, 15.1 -> 10.0; flash
+// layout 16384 tokens, fp8, 21.9 -> 20.1.  What is left over 15.6 of traffic: start and end, about 6, and 10
 // instructions an element.
 #pragma once
 
@@ -46,7 +47,7 @@ struct TileWriteParams {
   int move;              // 1: tiles may be moved onto 16-slot boundaries
 };
 
-constexpr int kTileHeads = 4;                     // heads per item
+constexpr int kTileHeads = 2;                     // heads per item
 constexpr int kTileStages = 3;
 constexpr int kTileThreads = (2 * kTileHeads + 1) * 32;
 
@@ -56,7 +57,7 @@ struct TileShape {
   static constexpr int kBoxBytes = kTileHeads * 16 * 128;       // [head][token][64 elements]
   static constexpr int kStage = 2 * kBoxes * kBoxBytes;         // K's boxes, then V's
   static constexpr int kSmem = 1024 + kTileStages * kStage;     // (1024: alignment)
-  static constexpr int kCtas = 2;                               // per SM
+  static constexpr int kCtas = D <= 128 ? 4 : 2;                // per SM
   static_assert(D % 64 == 0 && kCtas * (kSmem + 1536) <= 227 * 1024, "shared memory");
 };
 
