@@ -50,6 +50,7 @@ int* device_status_ptr();
 //   Directly behind the KV write of the same step an attention kernel may do more (its `early`): the
 // write lets it start only when it has itself waited for everything in front, and changes nothing but the
 // cache, so lengths, block tables and Q can be read before grid_dependency() (past L1), K and V after it.
+// (One decode of 1500 tokens 9.8 -> 9.1 us, seven chunks of 78 tokens 18 -> 12.8, 512 tokens 21.3 -> 18.2.)
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
                                     cudaStream_t stream, Args... args) {
