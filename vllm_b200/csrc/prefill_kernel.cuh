@@ -35,9 +35,8 @@
 //   * Every mbarrier wait is bounded; on expiry a status code is recorded and all roles leave.
 //
 // Measured on B200, a step of 4 chunks (8192 tokens, contexts up to 4096, 32 / 8 heads of 128, bf16;
-// KV write included): 8970 us with one decode work item per token, 346 us here (1160 TFLOP/s; 400 when it runs for long and the
-// power limit holds the clock down).  Start to first
-// product: 15000 cycles when every role worked an item out for itself and Q came with 16-byte copies, 9300
+// KV write included): 8970 us with one decode work item per token, 346 us here (1160 TFLOP/s; 400 when it
+// runs for long and the power limit holds the clock down).  Start to first product: 15000 cycles when every role worked an item out for itself and Q came with 16-byte copies, 9300
 // now (3400 plan, 2200 item, 500 Q, K beside it), which is what steps of short chunks consist of: 20 to
 // 35 us, 10 to 25 % less.
 #pragma once

@@ -80,7 +80,7 @@ static int attention_varlen(const b200pa_attn_args* a, const int32_t* query_star
                    : behind_write ? attention_behind_write(&d, stream, false) : b200pa_paged_attention_v1(&d, stream);
     if (rc != B200PA_OK) return rc;
   }
-  if (reqs == 0) return B200PA_OK;
+  if (reqs == 0 || num_tokens == num_decodes) return B200PA_OK;  // (a tensor map has no empty dimension)
 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   PrefillParams p{};
