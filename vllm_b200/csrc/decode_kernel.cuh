@@ -605,7 +605,7 @@ __global__ void __launch_bounds__(MAXW * 32, 1) pa_decode_kernel(const DecodePar
     int run = base + incl - mine;
     for (int s = s0; s < s1; ++s) {
       cum[s] = run;
-      run += units_of(s);
+      run += s1 - s0 == 1 ? mine : units_of(s);  // (lengths come from L2)
     }
     if (threadIdx.x == blockDim.x - 1) cum[S] = run;
     if (threadIdx.x == 0) {
