@@ -9,7 +9,8 @@
 
 namespace b200pa {
 
-// A tensor map of 16-bit elements without interleaving; `strides` in elements.
+// A tensor map of 16-bit elements without interleaving; `strides` in elements.  (L2 fetches 256 bytes at a time:
+// large KV writes 1 to 2 % less than with 128, attention the same.)
 template <int N>
 inline cudaError_t tensor_map(CUtensorMap* map, const void* base, const int64_t (&dims)[N], const int64_t (&strides)[N - 1],
                               const int (&box)[N], CUtensorMapSwizzle swizzle) {
@@ -32,7 +33,7 @@ inline cudaError_t tensor_map(CUtensorMap* map, const void* base, const int64_t 
   }
   for (int i = 0; i < N - 1; ++i) st[i] = cuuint64_t(strides[i]) * 2;
   const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, N, const_cast<void*>(base), d, st, b, step,
-                            CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
