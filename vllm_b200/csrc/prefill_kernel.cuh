@@ -220,7 +220,8 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qma
   // Longest sequences first, where there are more groups than SMs: the last items of all are short ones
   // then, whatever the engine's order.  (60 decodes and three chunks of 150 to 700 tokens behind up to
   // 1500, 328 items: 124.5 -> 122 us; 6 fp8 chunks of 200 to 900 with a bias 147 -> 132; 12 bf16 chunks
-  // 112 -> 108.5.  Above 64 requests the count of longer ones would take longer than it gains.)
+  // 112 -> 108.5.  More than 64 requests keep their order: not measured; they make many items, and each
+  // thread would count over all of them.)
   bool sorted = false;
   auto tiles_of = [&](int len) { return (max(len, 0) + KT - 1) / KT; };
   {
