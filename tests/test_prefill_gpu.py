@@ -21,7 +21,7 @@ def _gather(key_cache, value_cache, table, n, kv, scale):
     return k, v
 
 
-def _case(q_lens, ctx, H, HK, D, B, dtype, kv, alibi=False, seed=0, poison=True, ramp=0.0):
+def _case(q_lens, ctx, H, HK, D, B, dtype, kv, alibi=False, seed=0, poison=True, ramp=0.0, dark=None):
     from vllm_b200 import _custom_ops as ops
     gen = torch.Generator(device=DEV).manual_seed(seed)
     rng = np.random.default_rng(seed)
@@ -52,6 +52,19 @@ def _case(q_lens, ctx, H, HK, D, B, dtype, kv, alibi=False, seed=0, poison=True,
     q = (2 * torch.randn((n, H, D), generator=gen, device=DEV)).to(dtype)
     out = torch.full((n, H, D), float("nan"), dtype=dtype, device=DEV)
     slopes = torch.tensor([2.0 ** (-(i + 1) / 2) for i in range(H)], device=DEV) if alibi else None
+    if dark is not None:  # keys whose logits are -inf; those of the others lie around `low`
+        first, low = dark
+        q[..., 0] = q[..., 0].abs() + 0.5
+        q[..., 1] = 4.0
+        for r, n_keys in enumerate(lens):
+            key = torch.arange(int(need[r]) * B, device=DEV)
+            hidden = ((key < first) | (key % 128 >= 20)) & (key < int(ctx[r]))
+            blocks = kc[table[r, :need[r]].long()].view(dtype if kv == "auto" else torch.float8_e5m2)
+            k0 = blocks[:, :, 0, :, 0].float()
+            k0.masked_fill_(hidden.view(-1, 1, B), float("-inf"))
+            blocks[:, :, 0, :, 0] = k0.to(blocks.dtype)
+            blocks[:, :, 0, :, 1] = torch.tensor(low / (4.0 * D ** -0.5 * scale)).to(blocks.dtype)
+            kc[table[r, :need[r]].long()] = blocks.view(kc.dtype)
     if poison:  # stale bytes behind the end of a sequence must not reach the result
         bad = 0x7F if fp8 else float("nan")
         for r, k in enumerate(lens):
@@ -151,6 +164,18 @@ def test_items_whose_second_row_tile_is_empty(kv, alibi):
 @pytest.mark.parametrize("ramp", [0.02, 0.3])
 def test_maxima_that_grow_along_the_sequence(kv, dtype, D, ramp):
     _case([130, 40, 300], [0, 700, 333], 8, 2, D, 16, dtype, kv, ramp=ramp)
+
+
+# Keys with a logit of -inf leave a row without a maximum; whole key tiles of them, and 1 to 20 finite low logits
+# in the first half of the tiles behind
+@pytest.mark.parametrize("kv,dtype", [("auto", torch.bfloat16), ("auto", torch.float16), ("fp8_e5m2", torch.bfloat16)])
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("alibi", [False, True])
+@pytest.mark.parametrize("q,ctx", [([1, 20], [128, 148]), ([40, 2, 3], [300, 257, 128]), ([5, 30], [9000, 3100])],
+                         ids=["few-finite", "whole", "cut"])
+@pytest.mark.parametrize("first,low", [(128, -60.0), (256, -8.0)])
+def test_keys_of_minus_infinity(kv, dtype, D, alibi, q, ctx, first, low):
+    _case(q, ctx, 8, 2, D, 16, dtype, kv, alibi=alibi, dark=(first, low))
 
 
 @pytest.mark.parametrize("kv", ["auto", "fp8"])

@@ -416,6 +416,7 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qma
       const int head = it.kvh * G + row_head;
       const float slope = (p.alibi != nullptr && valid) ? __ldcg(p.alibi + head) * kLog2e : 0.f;
       float m = -INFINITY, l = 0.f;
+      bool unset = true;  // a row of this warp has no maximum yet: every logit so far was masked or -inf
       for (int j = b; j < e; ++j) {
         if (!wait(s_full(wg), n_s & 1)) break;
         ++n_s;
@@ -423,8 +424,9 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qma
         // The whole row of S goes to registers at once.  After the first tile the running maximum mostly
         // stands: for 16-bit caches without a bias the exponentials of the first half start with it as it
         // is; their sum and, beside them, the maximum of the second half tell whether it was too low (by
-        // 2^12: P and its sums hold larger values as exactly).  Then, and for the first tile, the maximum
-        // of the row is taken first.
+        // 2^12: P and its sums hold larger values as exactly).  Then, and as long as a row has no maximum at
+        // all (the first tile, and those behind it while logits are -inf), the maximum of the row is taken
+        // first.
         // (8192-token step 363 -> 353 us, with no gain for fp8 caches; with a bias the maximum grows with
         // every tile, 148 -> 177.  Exponentials by a polynomial on the FMA pipe instead of the special
         // function unit, a quarter of them: 354 -> 368; the kernel runs into the power limit, and without
@@ -440,7 +442,7 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qma
           if (k & 2) sb = fadd2(sb, e2); else sa = fadd2(sa, e2);
           w[ch][k / 2] = pack2<kBf>(e2.x, e2.y);
         };
-        for (bool look = kFp8 || biased || j == b;; look = true) {
+        for (bool look = kFp8 || biased || unset;; look = true) {
 #pragma unroll
           for (int ch = 0; ch < NC; ++ch) tmem_ld32(t_s + ch * 32, x[ch]);
           int last = pos - key0;  // last column of this row that counts
@@ -491,6 +493,7 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qma
                 tmem_wait_st();
               }
             }
+            if (!kFp8) unset = __any_sync(0xffffffffu, valid && m == -INFINITY);
           }
           nm = m == -INFINITY ? 0.f : -m;
           sa = sb = make_float2(0.f, 0.f);
