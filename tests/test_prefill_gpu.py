@@ -133,6 +133,31 @@ def test_few_rows_behind_long_contexts_are_split(kv):
     _case([5, 2, 40], [9000, 3000, 20000], 8, 2, 128, 16, torch.bfloat16, kv)
 
 
+def test_merges_of_cut_rows_launch_after_launch():
+    """The pieces of a row meet in the same workspace in every launch: with other queries each time, and no
+    host in between, a merge that read a piece of the launch before it would give that launch's values."""
+    from vllm_b200 import _custom_ops as ops
+    H, HK, D, B, T, n, runs = 8, 2, 128, 16, 64, 8256, 24
+    gen = torch.Generator(device=DEV).manual_seed(1)
+    kc = torch.randn(n // B, HK, D // 8, B, 8, generator=gen, device=DEV).bfloat16()
+    vc = torch.randn(n // B, HK, D, B, generator=gen, device=DEV).bfloat16()
+    q = (4 * torch.randn(runs, T, H, D, generator=gen, device=DEV)).bfloat16()
+    out = torch.full_like(q, float("nan"))
+    table = torch.randperm(n // B, generator=gen, device=DEV).int().view(1, -1)
+    lens, qsl = (torch.tensor(x, dtype=torch.int32, device=DEV) for x in ([n], [0, T]))
+    one = torch.tensor(1.0, device=DEV)
+    for i in range(runs):
+        assert ops.paged_attention_varlen(out[i], q[i], kc, vc, HK, D ** -0.5, table, lens, qsl, 0, B, n, None,
+                                          "auto", one, one)
+    k, v = _gather(kc, vc, table[0], n, "auto", 1.0)
+    hidden = torch.arange(n, device=DEV).view(1, -1) > torch.arange(n - T, n, device=DEV).view(-1, 1)
+    for i in range(runs):
+        s = torch.einsum("tkgd,lkd->kgtl", q[i].float().view(T, HK, H // HK, D), k) * D ** -0.5
+        want = torch.einsum("kgtl,lkd->tkgd", torch.softmax(s.masked_fill(hidden, float("-inf")), -1), v)
+        # (P, the partials and the result are rounded to 16 bits: 2^-9 each)
+        assert (out[i].float() - want.reshape(T, H, D)).norm() < 6e-3 * want.norm(), i
+
+
 def test_many_requests_and_single_rows_among_them():
     rng = np.random.default_rng(3)
     q = rng.integers(1, 40, size=600)  # (512 requests to a launch)

@@ -604,6 +604,7 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qma
           if (old == unsigned(it.npieces - 1)) *cnt = 0;  // re-arm for the next launch
           __threadfence();
         }
+        __syncwarp();  // the other lanes' loads of partials come after lane 0's fence (a shuffle orders no memory)
         old = __shfl_sync(0xffffffffu, old, 0);
         if (old == unsigned(it.npieces - 1) && valid) {
           const unsigned char* base = p.ws + (size_t(slot) * NQ + wg) * kWs;
