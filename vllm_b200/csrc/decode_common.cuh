@@ -84,6 +84,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
+__device__ __forceinline__ void prefetch_l1(const void* p) {
+  asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+}
+
 // Bounded wait: false if the phase did not complete within ~2^32 SM cycles (about two
 // seconds).  The clock is read only every 64 polls to keep waiting warps cheap.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {

@@ -630,6 +630,11 @@ __global__ void __launch_bounds__(MAXW * 32, 1) pa_decode_kernel(const DecodePar
     }
   }
   if (p.early) grid_dependency();
+  // The plan reads the lengths past L1 (see launch_dependent); from here on every item of a warp looks its
+  // length up again, on the way to its first page.  Without them in L1: 128 sequences of 8192 tokens, 64 / 8
+  // heads, fp8, 334 -> 341 us, as a step with its KV write 340 -> 346.
+  if (flat)
+    for (int s = threadIdx.x; s < p.num_seqs; s += blockDim.x) prefetch_l1(p.seq_lens + s);
   __syncthreads();
 
   const unsigned grid_warps = gridDim.x * unsigned(nwarps);
