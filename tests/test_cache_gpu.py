@@ -328,10 +328,12 @@ def test_large_mixed_batches_of_chunks_and_single_tokens(seed):
 
 
 @pytest.mark.parametrize("kv,dtype", [("auto", torch.bfloat16), ("fp8", torch.bfloat16), ("fp8_e5m2", torch.float16)])
-@pytest.mark.parametrize("H,D", [(4, 64), (8, 128), (2, 128), (4, 256)])
+@pytest.mark.parametrize("H,D,most", [(4, 64, None), (8, 128, None), (2, 128, None), (4, 256, None), (16, 64, None),
+                                      (14, 128, None), (14, 256, None), (20, 128, 2575), (8, 128, 2561), (4, 128, 3205)])
 @pytest.mark.parametrize("block_size", [16, 32])
-def test_tiles_of_large_writes(kv, dtype, H, D, block_size):
-    """Writes of 2560 tokens and more go by tiles of two heads: chunks that start anywhere (windows of a tile,
+def test_tiles_of_large_writes(kv, dtype, H, D, most, block_size):
+    """Large writes go by tiles of two heads (x-layout from 4096 tokens on, and from 2560 tokens and 400 items of 16
+    tokens on, 1600 where it quantises; flash layout from 1600 items on): chunks that start anywhere (windows of a tile,
     of what it gives up and of what its neighbours give up), single tokens and padding among them, a last tile
     that is not full, rows of a fused projection, values whose quotient overflows or is NaN, an odd scale."""
     rng = np.random.default_rng(H * D + block_size)
@@ -343,8 +345,9 @@ def test_tiles_of_large_writes(kv, dtype, H, D, block_size):
         if rng.integers(0, 4) == 0:
             slots.append(np.full(int(rng.integers(1, 20)), -1, dtype=np.int64))
     slots = np.concatenate([slots[i] for i in rng.permutation(len(slots))])
+    slots = slots[:most]
     T, NB, fp8 = len(slots), int(slots.max()) // block_size + 2, kv != "auto"
-    assert T >= 4096 and T % 16
+    assert T >= (most or 4096) and T % 16
     g = torch.Generator(device=DEV).manual_seed(5)
     qkv = torch.randn(T, 3 * H * D, device=DEV, generator=g).mul(2).to(dtype)
     key, val = (qkv[:, i * H * D:(i + 1) * H * D].unflatten(1, (H, D)) for i in (1, 2))

@@ -236,7 +236,8 @@ __device__ __forceinline__ void convert_words(const uint32_t (&w)[NW], uint32_t 
 namespace b200pa {
 
 constexpr int kTokTile = 16;
-constexpr int kTilesFrom = 2560;  // tokens from which the tile kernel takes over
+constexpr int kTilesFrom = 2560;  // tokens from which the tile kernel may take over, see launch_tiles
+constexpr int kMoveFrom = 4096;   // tokens from which the staged kernel moves tiles, see launch_staged
 
 // n / d for small operands (n * d < 2^32) by one multiply-high with a precomputed factor:
 // the index arithmetic below would otherwise spend more instructions on runtime divisions
@@ -761,12 +762,16 @@ static bool launch_staged(const b200pa_cache_args& a, cudaStream_t stream, int* 
   // cache 67 -> 36 us; chunks that start on a boundary are not affected).  Its extra code costs
   // writes of scattered tokens 3-5 us below 4096 tokens (fp8; nothing from 8192 on), and those
   // are decode steps, which have no runs to move.
-  bool shift = !kFlash && a.num_tokens >= 4096 && a.block_size % kStagedTile == 0;
+  bool shift = !kFlash && a.num_tokens >= kMoveFrom && a.block_size % kStagedTile == 0;
   if (kn_shift >= 0) shift = !kFlash && kn_shift != 0 && a.block_size % kStagedTile == 0;
   if constexpr (!kFlash) {
     if (shift) return launch_staged_as<in_t, cache_t, KV, false, true>(a, stream, rc, hsplit);
   }
   return launch_staged_as<in_t, cache_t, KV, kFlash, false>(a, stream, rc, hsplit);
+}
+
+static int64_t tile_items(const b200pa_cache_args& a) {
+  return int64_t((a.num_tokens + 15) / 16) * ((a.num_heads + kTileHeads - 1) / kTileHeads);
 }
 
 // The tile kernel for large writes of an even number of heads.  Returns as launch_staged_as.
@@ -806,8 +811,7 @@ static bool launch_tiles_as(const b200pa_cache_args& a, cudaStream_t stream, int
     (void)cudaGetLastError();
     return false;
   }
-  const int64_t items = int64_t((a.num_tokens + 15) / 16) * ((a.num_heads + kTileHeads - 1) / kTileHeads);
-  const int grid = int(std::min<int64_t>(items, int64_t(cache_sm_count()) * SH::kCtas));
+  const int grid = int(std::min<int64_t>(tile_items(a), int64_t(cache_sm_count()) * SH::kCtas));
   e = launch_dependent(kern, dim3(grid), dim3(kTileThreads), SH::kSmem, stream, p, kmap, vmap);
   count_launch();
   if (e != cudaSuccess) {
@@ -819,11 +823,19 @@ static bool launch_tiles_as(const b200pa_cache_args& a, cudaStream_t stream, int
   return true;
 }
 
-// Which calls it takes: heads of whole boxes (64, 128, 256), from 2560 tokens on.  Staged -> tiles, us, 8 heads of
-// 128 to fp8 unless stated: 3000 tokens in 3 chunks 9.2 -> 8.0, the same in the flash layout 7.0 -> 6.2; 2080 in 16
-// chunks 6.5 -> 6.9, 2048 scattered ones 14.7 -> 15.9, 1100 in 2 chunks 5.0 -> 5.4; 8000 tokens of 2 heads 10.7 ->
-// 6.2, 9500 of 4 heads of 256 23.4 -> 21.5, of 4 heads of 64 in the flash layout 5.9 -> 5.5; 4608 scattered
-// ones 45.5 -> 46.5.  Flash with a 16-bit cache is the plain kernel's.
+// Which calls it takes: heads of whole boxes (64, 128, 256) and, from 2560 tokens on (staged time / its time for
+// runs of 800 tokens, 2 to 40 heads, unless stated),
+//   * x-layout: all from 4096 tokens on, where the staged kernel starts to move tiles, which costs it more than
+//     its items do (1.05 to 1.9, runs of 100 1.3 to 2.3, of 20 1.03 to 1.9).  Below, calls with items enough for a
+//     few rounds of the 592 CTAs: 1600 to fp8 (150 to 1000 items 0.64 to 1.03; 1600 1.04 to 1.16, 3000 and more
+//     1.3 to 1.45), 400 to 16 bits, where the staged kernel moves twice the bytes (160 items 0.98 to 1.08; 400
+//     1.1 to 1.5, 640 and more 1.3 to 1.9);
+//   * flash layout, fp8: 1600 items (600 to 1200 items 0.87 to 1.09, 1600 to 9000 1.04 to 1.27; 15000 of 256-wide
+//     heads 0.94).
+// What it loses, since the slots are not known here and prefill steps matter more than decode batches of so many
+// sequences: scattered tokens and runs of 7 cost 3 to 12 % more to a 16-bit cache of the x-layout (to fp8 the same
+// on average), runs of 20 below 4096 tokens up to 16 % (0.78 for 16 heads of 256 to fp8).  Flash with a 16-bit
+// cache is the plain kernel's.
 template <typename in_t, typename cache_t, int KV, bool kFlash>
 static bool launch_tiles(const b200pa_cache_args& a, cudaStream_t stream, int* rc) {
   if constexpr (sizeof(in_t) != 2 || sizeof(cache_t) > 2 || (kFlash && KV == kKvAuto)) {
@@ -832,7 +844,9 @@ static bool launch_tiles(const b200pa_cache_args& a, cudaStream_t stream, int* r
     constexpr int E = sizeof(cache_t);
     auto al16 = [](const void* ptr) { return reinterpret_cast<uintptr_t>(ptr) % 16 == 0; };
     const int B = a.block_size;
-    if (a.num_tokens < kTilesFrom || a.num_heads % kTileHeads != 0 || B <= 0 || (B & (B - 1)) != 0) return false;
+    if (a.num_heads % kTileHeads != 0 || B <= 0 || (B & (B - 1)) != 0) return false;
+    if (a.num_tokens < kTilesFrom) return false;
+    if ((kFlash || a.num_tokens < kMoveFrom) && tile_items(a) < (KV == kKvAuto ? 400 : 1600)) return false;
     if (int64_t(a.num_tokens) * a.num_heads > (int64_t(1) << 30)) return false;  // (items are numbered in 32 bits)
     if (!al16(a.key) || !al16(a.value) || !al16(a.key_cache) || !al16(a.value_cache)) return false;
     if (a.key_stride % 8 != 0 || a.value_stride % 8 != 0 || !tensor_map_stride(a.key_stride) ||
