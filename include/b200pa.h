@@ -221,7 +221,8 @@ int b200pa_paged_attention_varlen(const b200pa_attn_args* args, const int32_t* q
                                   int32_t num_tokens, int32_t num_decodes, void* stream);
 
 /* 1 if b200pa_paged_attention_varlen has a kernel for requests with several rows of this shape (sizes,
- * types, strides, alignments), else 0: to be asked before the step's KV is written, for instance. */
+ * types, strides, alignments), else 0: to be asked before the step's KV is written, for instance.  Strides
+ * have to be positive, where their dimension is not of size 1. */
 int b200pa_paged_attention_varlen_supported(const b200pa_attn_args* args);
 
 /*

@@ -51,6 +51,17 @@ def _attn(**kw):
     return a
 
 
+@pytest.mark.parametrize("kw,found", [
+    (dict(), 1), (dict(kv_head_stride=0), 0), (dict(kv_block_stride=0), 0), (dict(q_stride=0), 0),
+    (dict(num_kv_heads=1, kv_head_stride=0), 1), (dict(num_kv_heads=1, kv_head_stride=3), 1),
+    (dict(block_size=8), 0), (dict(q_dtype=capi.F32), 0), (dict(q_stride=1025), 0)])
+def test_which_strides_the_prefill_kernel_takes(kw, found):
+    a = _attn(q_stride=1024, kv_block_stride=4096, kv_head_stride=2048)
+    for k, v in kw.items():
+        setattr(a, k, v)
+    assert capi.lib().b200pa_paged_attention_varlen_supported(C.byref(a)) == found
+
+
 @pytest.mark.parametrize("kw,msg", [
     (dict(head_size=48), "Unsupported head size"),
     (dict(block_size=64), "Unsupported block size"),

@@ -121,6 +121,27 @@ def test_tile_edges(H, HK, q, ctx):
     _case([q, 0, q], [ctx, 7, 0], H, HK, 128, 16, torch.bfloat16, "auto", seed=q)
 
 
+@pytest.mark.parametrize("kv", ["auto", "fp8"])
+def test_strides_of_dimensions_of_size_one(kv):
+    """One token, one kv head, one block: whatever strides these come with, the prefill kernel takes the call."""
+    from vllm_b200 import _custom_ops as ops
+    H, D, B, n, x = 4, 128, 16, 11, 8 if kv == "auto" else 16
+    gen = torch.Generator(device=DEV).manual_seed(0)
+    kc, vc = torch.randn(D // x, B, x, generator=gen, device=DEV), torch.randn(D, B, generator=gen, device=DEV)
+    kc, vc = (t.bfloat16() if kv == "auto" else t.to(torch.float8_e4m3fn).view(torch.uint8) for t in (kc, vc))
+    q = torch.randn(H, D, generator=gen, device=DEV).bfloat16()
+    out = torch.full((1, H, D), float("nan"), dtype=q.dtype, device=DEV)
+    table, lens, qsl = (torch.tensor(t, dtype=torch.int32, device=DEV) for t in ([[0]], [n], [0, 1]))
+    one = torch.tensor(1.0, device=DEV)
+    assert ops.paged_attention_varlen(out, q.as_strided((1, H, D), (0, D, 1)),
+                                      kc.as_strided((1, 1, D // x, B, x), (0, 0, B * x, x, 1)),
+                                      vc.as_strided((1, 1, D, B), (0, 0, B, 1)), 1, D ** -0.5, table, lens, qsl, 0, B, n,
+                                      None, kv, one, one)
+    k, v = _gather(kc[None, None], vc[None, None], table[0], n, kv, 1.0)
+    want = torch.softmax(q.float() @ k[:, 0].T * D ** -0.5, -1) @ v[:, 0]
+    assert (out[0].float() - want).norm() < 6e-3 * want.norm()  # (P and the result are rounded to 16 bits)
+
+
 # V comes in pages of 16 keys: the last one of a sequence is cut at every length, the pages behind it do not exist
 @pytest.mark.parametrize("D", [64, 120, 192])
 @pytest.mark.parametrize("B", [16, 32])

@@ -103,8 +103,9 @@ void fill_attn(b200pa_attn_args& a, torch::Tensor& out, torch::Tensor& query,
   }
   a.k_scale = k_scale.defined() && k_scale.is_cuda() ? static_cast<const float*>(k_scale.data_ptr()) : nullptr;
   a.v_scale = v_scale.defined() && v_scale.is_cuda() ? static_cast<const float*>(v_scale.data_ptr()) : nullptr;
-  a.q_stride = query.stride(0);
-  a.kv_block_stride = key_cache.stride(0);
+  // (the stride of a dimension of size 1 means nothing, and may be 0)
+  a.q_stride = query.size(0) == 1 ? query.size(1) * query.size(2) : query.stride(0);
+  a.kv_block_stride = key_cache.size(0) == 1 ? key_cache.numel() : key_cache.stride(0);
   a.kv_head_stride = key_cache.stride(1);
   a.num_seqs = static_cast<int32_t>(query.size(0));
   a.num_heads = static_cast<int32_t>(query.size(1));
@@ -771,7 +772,7 @@ PyObject* py_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p.alibi_slopes = alibi.has_value() ? alibi->data_ptr<float>() : nullptr;
     p.k_scale = ks.data_ptr<float>();
     p.v_scale = vs.data_ptr<float>();
-    p.q_stride = q.stride(0);
+    p.q_stride = tokens == 1 ? H * D : q.stride(0);
     p.kv_block_stride = HK * D * B;
     p.kv_head_stride = D * B;
     p.num_seqs = static_cast<int32_t>(max_q == 1 ? tokens : reqs);

@@ -19,6 +19,14 @@ cudaError_t prefill_q_map(const PrefillParams& p, int head_size, int box, CUtens
                        {box, p.group, 128 / p.group}, box == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_32B);
 }
 
+// A dimension of size 1 may come with any stride, 0 among them; a tensor map wants one that it can hold.
+// (num_tokens 0: not known)
+static b200pa_attn_args with_plain_strides(b200pa_attn_args a, int num_tokens) {
+  if (a.num_kv_heads == 1) a.kv_head_stride = int64_t(a.head_size) * a.block_size;
+  if (num_tokens == 1) a.q_stride = int64_t(a.num_heads) * a.head_size;
+  return a;
+}
+
 // The prefill kernel for a call's shape and alignments, or none.  16-byte accesses: pages, rows of Q and
 // of the output; cache offsets inside a block are shifts.  The strides of Q and of a 16-bit cache have to
 // fit a tensor map (positive, below 2^40 bytes).
@@ -40,15 +48,16 @@ static PrefillKernelInfo find_prefill(const b200pa_attn_args& a) {
 
 extern "C" int b200pa_paged_attention_varlen_supported(const b200pa_attn_args* a) {
   return a != nullptr && a->num_heads > 0 && a->num_kv_heads > 0 && a->num_heads % a->num_kv_heads == 0 &&
-         b200pa::find_prefill(*a).fn != nullptr;
+         b200pa::find_prefill(b200pa::with_plain_strides(*a, 0)).fn != nullptr;
 }
 
 namespace b200pa {
 
 // `behind_write`: the launch in front on the stream is the KV write of the same step.
-static int attention_varlen(const b200pa_attn_args* a, const int32_t* query_start_loc, int32_t num_tokens,
+static int attention_varlen(const b200pa_attn_args* args, const int32_t* query_start_loc, int32_t num_tokens,
                             int32_t num_decodes, void* stream, bool behind_write) {
-  B200PA_CHECK_ARG(a != nullptr, "args is NULL");
+  B200PA_CHECK_ARG(args != nullptr, "args is NULL");
+  const b200pa_attn_args plain = with_plain_strides(*args, num_tokens), *a = &plain;
   B200PA_CHECK_ARG(a->num_seqs >= 0 && a->num_heads > 0 && a->num_kv_heads > 0 && a->head_size > 0 &&
                        a->num_heads % a->num_kv_heads == 0,
                    "bad sizes: num_seqs=%d num_heads=%d num_kv_heads=%d head_size=%d", a->num_seqs,
@@ -148,7 +157,8 @@ extern "C" int b200pa_attention_step(const b200pa_cache_args* write, const b200p
                                      int32_t caller_scratch, void* stream) {
   using namespace b200pa;
   B200PA_CHECK_ARG(a != nullptr, "args is NULL");
-  if (query_start_loc != nullptr && num_decodes < a->num_seqs && !b200pa_paged_attention_varlen_supported(a)) {
+  const b200pa_attn_args plain = with_plain_strides(*a, num_tokens);
+  if (query_start_loc != nullptr && num_decodes < a->num_seqs && !b200pa_paged_attention_varlen_supported(&plain)) {
     set_error("attention_step: no kernel for head_size=%d block_size=%d q_dtype=%d kv_dtype=%d, or unaligned tensors",
               a->head_size, a->block_size, a->q_dtype, a->kv_dtype);
     return B200PA_EUNSUPPORTED;
