@@ -207,6 +207,57 @@ def test_the_native_step_does_what_the_operators_do(new, ctx, D, kv, alibi, monk
     assert e.out[n:].isnan().all() and native[n:].isnan().all()
 
 
+@pytest.mark.parametrize("new,ctx,scratch", [([1, 1, 1], [0, 700, 33], False), ([1] * 3, [9000, 20, 5000], True),
+                                             ([1, 1, 9, 40], [300, 5, 0, 77], False), ([5, 64], [0, 129], False)])
+@pytest.mark.parametrize("kv", ["auto", "fp8"])
+def test_the_step_of_the_c_interface(new, ctx, scratch, kv):
+    """b200pa_attention_step against the write and the attention as two calls, and without a write."""
+    from vllm_b200 import capi
+    e = Engine(len(new), sum(new), kv=kv, max_blocks=600)
+    e.load(new, ctx)
+    n, r = sum(new), len(new)
+    chunks, decodes = max(new) > 1, new.count(1)
+    x = 16 // e.cache.element_size()
+    a = capi.AttnArgs(out=e.out.data_ptr(), query=e.q.data_ptr(), key_cache=e.cache[0].data_ptr(),
+                      value_cache=e.cache[1].data_ptr(), block_tables=e.table.data_ptr(), seq_lens=e.lens.data_ptr(),
+                      k_scale=e.layer._k_scale.data_ptr(), v_scale=e.layer._v_scale.data_ptr(), q_stride=e.H * e.D,
+                      kv_block_stride=e.HK * e.D * e.B, kv_head_stride=e.D * e.B, num_seqs=r, num_heads=e.H,
+                      num_kv_heads=e.HK, head_size=e.D, block_size=e.B, max_seq_len=int(e.lens.max()),
+                      max_num_blocks_per_seq=e.table.shape[1], scale=e.D ** -0.5, q_dtype=capi.BF16,
+                      kv_dtype=capi.kv_dtype_from_string(kv))
+    if scratch:
+        parts = a.max_num_partitions = -(-a.max_seq_len // 512)
+        sums, tops = (torch.empty(r, e.H, parts, device=DEV) for _ in range(2))
+        tmp = torch.empty(r, e.H, parts, e.D, dtype=e.dtype, device=DEV)
+        a.exp_sums, a.max_logits, a.tmp_out = sums.data_ptr(), tops.data_ptr(), tmp.data_ptr()
+    w = capi.CacheArgs(key=e.k.data_ptr(), value=e.v.data_ptr(), key_cache=a.key_cache, value_cache=a.value_cache,
+                       slot_mapping=e.slots.data_ptr(), k_scale=a.k_scale, v_scale=a.v_scale, key_stride=e.HK * e.D,
+                       value_stride=e.HK * e.D, num_tokens=n, num_heads=e.HK, head_size=e.D, block_size=e.B, x=x,
+                       in_dtype=capi.BF16, kv_dtype=a.kv_dtype)
+    before, starts = e.cache.clone(), e.qsl.data_ptr() if chunks else 0
+    st = torch.cuda.current_stream().cuda_stream
+    capi.attention_step(w, a, starts, n, decodes, scratch, st)
+    e.check()
+    got, written = e.out.clone(), e.cache.clone()
+    e.cache.copy_(before)
+    e.out.fill_(float("nan"))
+    capi.reshape_and_cache(w, st)
+    assert torch.equal(e.cache, written)
+    capi.attention_step(None, a, starts, n, decodes, scratch, st)
+    e.check()
+    # (the same kernels on the same values: only the order of partial sums may differ)
+    assert (got.float() - e.out.float()).norm() < 4e-3 * got.float().norm()
+
+    # no kernel for the chunks: nothing is launched, the write neither
+    if chunks:
+        w.block_size = a.block_size = 8
+        e.cache.copy_(before)
+        capi.launch_count(reset=True)
+        with pytest.raises(RuntimeError, match="no kernel"):
+            capi.attention_step(w, a, starts, n, decodes, scratch, st)
+        assert capi.launch_count() == 0 and torch.equal(e.cache, before)
+
+
 def test_a_replay_beside_launches_on_another_stream():
     """A captured launch does not share its work-distribution words with ordinary ones: more of them
     than there are rotating slots run beside the replays."""
@@ -231,12 +282,13 @@ def test_a_replay_beside_launches_on_another_stream():
 
 @pytest.mark.parametrize("kv", ["auto", "fp8"])
 @pytest.mark.parametrize("new,ctx", [([1] * 3, [300, 15, 600]), ([1] * 120, list(range(60, 300, 2))),
-                                     ([40, 130, 7], [100, 0, 500]), ([1] * 9 + [70, 33], [200] * 9 + [64, 300])],
-                         ids=["few-decodes", "many-decodes", "chunks", "mixed"])
+                                     ([40, 130, 7], [100, 0, 500]), ([1] * 9 + [70, 33], [200] * 9 + [64, 300]),
+                                     ([1500, 1400, 1300], [100, 0, 37])],  # (the write goes by tiles)
+                         ids=["few-decodes", "many-decodes", "chunks", "mixed", "large-chunks"])
 def test_attention_starts_under_the_write_of_its_step(new, ctx, kv):
     """Attention reads lengths, block tables and Q while the KV write in front may still run: what kernels
     before the write have just stored has to be what it sees, step after step, without a host in between."""
-    eng = Engine(len(new), sum(new), kv=kv)
+    eng = Engine(len(new), sum(new), kv=kv, max_blocks=max(40, -(-(max(new) + max(ctx)) // 16)))
     cache, names = eng.cache.clone(), ("q", "k", "v", "table", "lens", "slots", "qsl")
     steps = []
     for i in range(4):

@@ -23,6 +23,9 @@ EXPORTS = (
     "b200pa_paged_attention_v2_noalloc",
     "b200pa_reshape_and_cache",
     "b200pa_reshape_and_cache_flash",
+    "b200pa_paged_attention_varlen",
+    "b200pa_paged_attention_varlen_supported",
+    "b200pa_attention_step",
     "b200pa_convert_fp8",
     "b200pa_merge_attn_states",
     "b200pa_copy_blocks",
@@ -90,6 +93,8 @@ def lib() -> C.CDLL:
         l.b200pa_convert_fp8.argtypes = [C.c_void_p, C.c_void_p, C.c_int64, C.c_float, C.c_int32,
                                          C.c_int32, C.c_int32, C.c_void_p]
         l.b200pa_decode_route.argtypes = [C.POINTER(AttnArgs), C.POINTER(C.c_int32)]
+        l.b200pa_attention_step.argtypes = [C.POINTER(CacheArgs), C.POINTER(AttnArgs), C.c_void_p, C.c_int32,
+                                            C.c_int32, C.c_int32, C.c_void_p]
         l.b200pa_device_status.argtypes = [C.POINTER(C.c_int32)]
         _lib = l
     return _lib
@@ -136,6 +141,15 @@ def reshape_and_cache(args: CacheArgs, stream: int = 0) -> None:
 
 def reshape_and_cache_flash(args: CacheArgs, stream: int = 0) -> None:
     check(lib().b200pa_reshape_and_cache_flash(C.byref(args), C.c_void_p(stream)))
+
+
+def attention_step(write: CacheArgs | None, args: AttnArgs, query_start_loc: int, num_tokens: int,
+                   num_decodes: int, caller_scratch: bool = False, stream: int = 0) -> None:
+    """KV write (None: none) and attention of an engine step (see b200pa.h); `query_start_loc` 0: a decode
+    batch."""
+    check(lib().b200pa_attention_step(C.byref(write) if write is not None else None, C.byref(args),
+                                      C.c_void_p(query_start_loc), num_tokens, num_decodes,
+                                      1 if caller_scratch else 0, C.c_void_p(stream)))
 
 
 def device_status() -> int:
