@@ -274,7 +274,9 @@ int b200pa_reshape_and_cache_flash(const b200pa_cache_args* args, void* stream);
  * it where it first reads the cache.
  *   query_start_loc, num_tokens, num_decodes: as for b200pa_paged_attention_varlen; query_start_loc NULL:
  *     a decode batch, one query row per sequence, as for v1, or v2 where `caller_scratch` is not 0
- * Returns B200PA_EUNSUPPORTED, with nothing launched, where b200pa_paged_attention_varlen has no kernel.
+ * What the attention or the write refuses (B200PA_EINVAL; B200PA_EUNSUPPORTED, also where
+ * b200pa_paged_attention_varlen has no kernel) is returned with nothing launched, the write neither.  After
+ * B200PA_ECUDA the write, or the write and the decodes, may be on the stream.
  */
 int b200pa_attention_step(const b200pa_cache_args* write, const b200pa_attn_args* args,
                           const int32_t* query_start_loc, int32_t num_tokens, int32_t num_decodes,

@@ -83,6 +83,37 @@ def test_attention_argument_errors_are_reported_not_thrown(kw, msg):
         capi.paged_attention_v2(_attn(**kw))
 
 
+@pytest.mark.parametrize("kw,chunks,tokens,decodes,scratch,msg", [
+    (dict(head_size=48), False, 3, 3, False, "Unsupported head size"),
+    (dict(block_size=64), False, 3, 3, False, "Unsupported block size"),
+    (dict(seq_lens=0), False, 3, 3, False, "null tensor pointer"),
+    (dict(max_num_blocks_per_seq=0), False, 3, 3, False, "max_num_blocks_per_seq"),
+    (dict(kv_dtype=capi.KV_FP8_E4M3), False, 3, 3, False, "k_scale"),
+    (dict(), False, 3, 3, True, "v2 needs"),
+    (dict(block_size=8), True, 9, 1, False, "no kernel"),
+    (dict(), True, 9, 4, False, "bad counts"),
+    (dict(), True, 1, 2, False, "bad counts"),
+    (dict(out=0), True, 9, 1, False, "null tensor pointer"),
+    (dict(blocksparse_vert_stride=2, blocksparse_block_size=24), True, 3, 3, False, "blocksparse_block_size"),
+])
+def test_a_refused_step_does_not_write(kw, chunks, tokens, decodes, scratch, msg):
+    """What attention refuses is known before the KV write of the step is launched."""
+    buf = C.create_string_buffer(1024)
+    mem = C.addressof(buf) + 255 & ~255  # (any aligned address: nothing is launched)
+    a = _attn(q_stride=1024, kv_block_stride=4096, kv_head_stride=2048, num_seqs=3, max_num_blocks_per_seq=4)
+    for k in ("out", "query", "key_cache", "value_cache", "block_tables", "seq_lens"):
+        setattr(a, k, mem)
+    for k, v in kw.items():
+        setattr(a, k, v)
+    w = capi.CacheArgs(key=mem, value=mem, key_cache=mem, value_cache=mem, slot_mapping=mem, key_stride=256,
+                       value_stride=256, num_tokens=tokens, num_heads=a.num_kv_heads, head_size=128, block_size=16,
+                       x=8, in_dtype=capi.BF16, kv_dtype=0)
+    capi.launch_count(reset=True)
+    with pytest.raises(RuntimeError, match=msg):
+        capi.attention_step(w, a, mem if chunks else 0, tokens, decodes, scratch)
+    assert capi.launch_count() == 0
+
+
 def test_null_args_and_empty_batches():
     lib = capi.lib()
     assert lib.b200pa_paged_attention_v1(None, None) == -1

@@ -28,5 +28,7 @@ int sm_count();
 // entries directly behind the KV write of their step (see launch_dependent).
 int attention_half_region(const b200pa_attn_args* a, void* stream, bool behind_write);
 int attention_behind_write(const b200pa_attn_args* a, void* stream, bool caller_scratch);
+// Whether paged_attention_v1 (v2 with `caller_scratch`) takes the call, without launching anything.
+int attention_check(const b200pa_attn_args* a, bool caller_scratch);
 
 }  // namespace b200pa

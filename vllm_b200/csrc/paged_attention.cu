@@ -550,9 +550,8 @@ enum class Scratch {
               // slots per (sequence, head), not tied to 512 tokens; nothing else is used
 };
 
-// `share`: the call may use one `share`-th of the stream's workspace and arrival counters (another
-// launch that may run at the same time has the rest).
-static int attention_entry(const b200pa_attn_args* a, void* stream, Scratch mode, int share = 1, bool behind_write = false) {
+// What a call is refused for; no more than CUDA errors can come behind it.
+static int check_attention(const b200pa_attn_args* a, Scratch mode) {
   const bool v2 = mode != Scratch::kNone;
   B200PA_CHECK_ARG(a != nullptr, "args is NULL");
   B200PA_CHECK_ARG(a->num_seqs >= 0 && a->num_heads > 0 && a->num_kv_heads > 0 && a->head_size > 0,
@@ -615,6 +614,14 @@ static int attention_entry(const b200pa_attn_args* a, void* stream, Scratch mode
                      "max_num_partitions=%d does not cover max_seq_len=%d", a->max_num_partitions,
                      a->max_seq_len);
   }
+  return B200PA_OK;
+}
+
+// `share`: the call may use one `share`-th of the stream's workspace and arrival counters (another
+// launch that may run at the same time has the rest).
+static int attention_entry(const b200pa_attn_args* a, void* stream, Scratch mode, int share = 1, bool behind_write = false) {
+  if (const int bad = check_attention(a, mode); bad != B200PA_OK || a->num_seqs == 0) return bad;
+  const bool v2 = mode != Scratch::kNone;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const Tuning tune = tuning();
 
@@ -834,6 +841,9 @@ static int attention_entry(const b200pa_attn_args* a, void* stream, Scratch mode
   return B200PA_OK;
 }
 
+int attention_check(const b200pa_attn_args* a, bool caller_scratch) {
+  return check_attention(a, caller_scratch ? Scratch::kCaller : Scratch::kNone);
+}
 int attention_half_region(const b200pa_attn_args* a, void* stream, bool behind_write) {
   return attention_entry(a, stream, Scratch::kNone, 2, behind_write);
 }

@@ -53,34 +53,44 @@ extern "C" int b200pa_paged_attention_varlen_supported(const b200pa_attn_args* a
 
 namespace b200pa {
 
-// `behind_write`: the launch in front on the stream is the KV write of the same step.
-static int attention_varlen(const b200pa_attn_args* args, const int32_t* query_start_loc, int32_t num_tokens,
-                            int32_t num_decodes, void* stream, bool behind_write) {
-  B200PA_CHECK_ARG(args != nullptr, "args is NULL");
-  const b200pa_attn_args plain = with_plain_strides(*args, num_tokens), *a = &plain;
+// What a call is refused for, its decode rows among them; no more than CUDA errors can come behind it.
+static int check_varlen(const b200pa_attn_args* a, const int32_t* query_start_loc, int32_t num_tokens, int32_t num_decodes,
+                        PrefillKernelInfo* ki) {
   B200PA_CHECK_ARG(a->num_seqs >= 0 && a->num_heads > 0 && a->num_kv_heads > 0 && a->head_size > 0 &&
                        a->num_heads % a->num_kv_heads == 0,
                    "bad sizes: num_seqs=%d num_heads=%d num_kv_heads=%d head_size=%d", a->num_seqs,
                    a->num_heads, a->num_kv_heads, a->head_size);
   B200PA_CHECK_ARG(num_decodes >= 0 && num_decodes <= a->num_seqs && num_tokens >= num_decodes,
                    "bad counts: %d requests, %d decodes, %d tokens", a->num_seqs, num_decodes, num_tokens);
-  const int reqs = a->num_seqs - num_decodes;
-  PrefillKernelInfo ki{nullptr, 0};
-  if (reqs > 0) {
+  if (a->num_seqs > num_decodes) {
     B200PA_CHECK_ARG(a->out && a->query && a->key_cache && a->value_cache && a->block_tables &&
                          a->seq_lens && query_start_loc,
                      "null tensor pointer");
     B200PA_CHECK_ARG(a->kv_dtype == B200PA_KV_AUTO || (a->k_scale && a->v_scale),
                      "fp8 kv cache needs k_scale and v_scale");
     B200PA_CHECK_ARG(a->max_num_blocks_per_seq > 0, "max_num_blocks_per_seq must be positive");
-    ki = find_prefill(*a);
-    if (ki.fn == nullptr) {
+    *ki = find_prefill(*a);
+    if (ki->fn == nullptr) {
       set_error("paged_attention_varlen: no kernel for head_size=%d block_size=%d q_dtype=%d kv_dtype=%d, "
                 "or unaligned tensors",
                 a->head_size, a->block_size, a->q_dtype, a->kv_dtype);
       return B200PA_EUNSUPPORTED;
     }
   }
+  if (num_decodes == 0) return B200PA_OK;
+  b200pa_attn_args d = *a;
+  d.num_seqs = num_decodes;
+  return attention_check(&d, false);
+}
+
+// `behind_write`: the launch in front on the stream is the KV write of the same step.
+static int attention_varlen(const b200pa_attn_args* args, const int32_t* query_start_loc, int32_t num_tokens,
+                            int32_t num_decodes, void* stream, bool behind_write) {
+  B200PA_CHECK_ARG(args != nullptr, "args is NULL");
+  const b200pa_attn_args plain = with_plain_strides(*args, num_tokens), *a = &plain;
+  PrefillKernelInfo ki{nullptr, 0};
+  if (const int bad = check_varlen(a, query_start_loc, num_tokens, num_decodes, &ki); bad != B200PA_OK) return bad;
+  const int reqs = a->num_seqs - num_decodes;
   if (num_decodes > 0) {
     // the decode rows are the first rows of query and out: an ordinary decode batch
     b200pa_attn_args d = *a;
@@ -158,11 +168,11 @@ extern "C" int b200pa_attention_step(const b200pa_cache_args* write, const b200p
   using namespace b200pa;
   B200PA_CHECK_ARG(a != nullptr, "args is NULL");
   const b200pa_attn_args plain = with_plain_strides(*a, num_tokens);
-  if (query_start_loc != nullptr && num_decodes < a->num_seqs && !b200pa_paged_attention_varlen_supported(&plain)) {
-    set_error("attention_step: no kernel for head_size=%d block_size=%d q_dtype=%d kv_dtype=%d, or unaligned tensors",
-              a->head_size, a->block_size, a->q_dtype, a->kv_dtype);
-    return B200PA_EUNSUPPORTED;
-  }
+  // (the write is launched only when the attention behind it will be)
+  PrefillKernelInfo ki{nullptr, 0};
+  const int bad = query_start_loc != nullptr ? check_varlen(&plain, query_start_loc, num_tokens, num_decodes, &ki)
+                                             : attention_check(a, caller_scratch != 0);
+  if (bad != B200PA_OK) return bad;
   bool behind_write = false;
   if (write != nullptr) {
     const int rc = b200pa_reshape_and_cache(write, stream);
