@@ -312,3 +312,40 @@ def test_attention_starts_under_the_write_of_its_step(new, ctx, kv):
     assert ((got - want).norm(dim=-1) < 4e-3 * want.norm(dim=-1)).all()
     from vllm_b200 import capi
     assert capi.device_status() == 0
+
+
+@pytest.mark.parametrize("kv", ["auto", "fp8"])
+@pytest.mark.parametrize("new,ctx", [([1] * 3, [300, 15, 600]), ([1] * 3, [9000, 20, 5000]), ([1] * 90, list(range(90, 180))),
+                                     ([40, 130, 7], [100, 0, 500]), ([20, 9], [9000, 4000]),
+                                     ([1, 1, 1, 20, 300], [9000, 700, 7, 8000, 500]), ([1500, 1400, 1300], [100, 0, 37])],
+                         ids=["few-decodes", "split-decodes", "many-decodes", "chunks", "cut-chunks", "mixed", "large-chunks"])
+def test_layers_back_to_back(new, ctx, kv):
+    """Layers with caches of their own on one stream and no other kernel between: the result of a layer is the query
+    of the next, so an attention kernel that read Q before the write in front of it has waited for the layer before,
+    or met scheduler words, counters or partials of that layer's launches, would give other values.  Again with the
+    next step's tokens, lengths and tables."""
+    e = Engine(len(new), sum(new), kv=kv, max_blocks=max(50, -(-(max(new) + max(ctx) + 1) // 16)))
+    n = 5
+    bufs = [{"q": e.q, "k": e.k.clone(), "v": e.v.clone(), "out": e.out.clone(), "cache": e.cache.clone()}
+            for _ in range(n)]
+    for a, b in zip(bufs, bufs[1:]):
+        b["q"] = a["out"].view(e.q.shape)
+
+    def layer(b):
+        for name, t in b.items():
+            setattr(e, name, t)
+    for step in range(3):
+        layer({"q": bufs[0]["q"], "k": bufs[0]["k"], "v": bufs[0]["v"], "out": bufs[0]["out"]})
+        e.load(new, [max(0, c - 7 * step) for c in ctx])
+        for b in bufs:
+            for name in ("k", "v", "out"):
+                b[name].copy_(e._randn(*b[name].shape))
+        meta = e.builder.build(0, e.common())
+        torch.cuda.synchronize()
+        torch.cuda._sleep(20_000_000)  # (all launches are there before the first one runs)
+        for b in bufs:
+            layer(b)
+            e.forward(meta)
+        for b in bufs:
+            layer(b)
+            e.check()

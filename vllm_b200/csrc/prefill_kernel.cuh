@@ -76,8 +76,10 @@ struct PrefillParams {
   int block_size;
   int max_blocks_per_seq;
   int ws_slots;               // pieces that the workspace has room for
-  int late_wait;              // 1: independent of the launch in front, waits for it at the end only (the launch in
-                              // front has itself waited for all before it)
+  // What a kernel reads before its own wait has been written by grids that are complete (the one in front has
+  // waited for them, and lets the next one in only then); copies by tensor map, which are another proxy's
+  // accesses and which no wait of this grid stands in front of, are ordered behind it by a fence.
+  int late_wait;              // 1: independent of the launch in front, waits for it at the end only
   int early;                  // 1: the launch in front is the step's KV write, see launch_dependent
   float scale;
 };
@@ -711,6 +713,7 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qma
       return wait(kv_empty(h % NS), (use - 1) & 1);
     };
     auto slot_of = [&](uint32_t h) { return skv + (h % NS) * SH::kTileBytes; };
+    if (!kFp8 && warp == 8) fence_proxy_async_global();  // (V, under late_wait)
     while (ok && have_item()) {
       const PrefillItem it = s_item[n_item & 1];
       const int* bt = p.block_tables + int64_t(it.req) * p.max_blocks_per_seq;
@@ -1033,6 +1036,7 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qma
     // warpgroups after their last tile 6500, which nothing hid.)  bf16 becomes f16 in place for an
     // fp8 cache, half a tile by each of warps 14 and 15.
     uint32_t n_q[2] = {0, 0};
+    fence_proxy_async_global();  // (Q, under late_wait and early)
     while (ok && (kWiden || warp == 14) && have_item()) {
       const PrefillItem& it = s_item[n_item & 1];
       const bool has[2] = {it.e0 > it.b, it.e1 > it.b};

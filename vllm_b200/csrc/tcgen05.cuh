@@ -210,6 +210,10 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// Orders this thread's tensor-map copies behind what it knows to be written to global memory by ordinary stores.
+__device__ __forceinline__ void fence_proxy_async_global() {
+  asm volatile("fence.proxy.async.global;" ::: "memory");
+}
 // A box of a tensor map, completion counted in bytes on `bar`.  No cluster multicast: every CTA fetches
 // its own tiles.
 __device__ __forceinline__ void tma_load3(uint32_t dst, const void* map, int x, int y, int z, uint32_t bar) {
