@@ -1,6 +1,9 @@
 """Host-side mirror of the reference interface: op schemas, wrappers, helpers,
 workload generators (no GPU needed)."""
+import ctypes as C
 import inspect
+import subprocess
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -164,16 +167,36 @@ def test_reference_names_are_claimed_on_request_and_never_twice():
     assert r.stdout.split() == ["False", "8", "True", "0"]
 
 
-def test_windows_of_the_tile_kv_write_cover_every_token():
+@pytest.fixture(scope="module")
+def windows(tmp_path_factory):
+    """The window arithmetic of the KV write kernels, compiled for the host."""
+    d = tmp_path_factory.mktemp("windows")
+    (d / "w.cpp").write_text("""
+#include "kv_write_windows.h"
+using namespace b200pa;
+extern "C" int shift(int64_t first, int64_t mid, int64_t last) { return tile_shift(first, mid, last); }
+extern "C" TileWindow window(int t0, int n, int d, int after) { return tile_window(t0, n, d, after); }
+extern "C" TileWindow front(int t0, int d, int before) { return tile_front_window(t0, d, before); }
+""")
+    csrc = Path(__file__).resolve().parents[1] / "vllm_b200" / "csrc"
+    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", f"-I{csrc}", "w.cpp", "-o", "w.so"], cwd=d, check=True,
+                   timeout=120)
+    lib = C.CDLL(str(d / "w.so"))
+
+    class Window(C.Structure):
+        _fields_ = [("tok", C.c_int), ("lo", C.c_int), ("hi", C.c_int)]
+    lib.window.restype = lib.front.restype = Window
+    lib.shift.argtypes = [C.c_int64] * 3
+    return lib
+
+
+def test_windows_of_the_tile_kv_write_cover_every_token(windows):
     """The windows of vllm_b200/csrc/kv_write_tiles.cuh: whatever the slots are, every token in one
     window: its tile's, the tile's before or the one that its tile keeps for itself in front."""
     rng = np.random.default_rng(11)
 
-    def shift(slots, i):
-        t = slots[16 * i:16 * i + 16] if i >= 0 else []
-        if len(t) < 16 or min(t[0], t[8], t[15]) < 0 or (t[8] - t[0]) % 16 != 8 or (t[15] - t[0]) % 16 != 15:
-            return 0
-        return int(-t[0] % 16)
+    def shift(slots, i):  # (what the kernel hands over: -1 where there is no token)
+        return windows.shift(*(int(slots[t]) if 0 <= t < len(slots) else -1 for t in (16 * i, 16 * i + 8, 16 * i + 15)))
 
     for _ in range(300):
         pieces, pos = [], 0
@@ -188,20 +211,20 @@ def test_windows_of_the_tile_kv_write_cover_every_token():
         n, seen = len(slots), np.zeros(len(slots), int)
         for i in range((n + 15) // 16):
             d, before, after = (shift(slots, k) for k in (i, i - 1, i + 1))
-            windows = [(16 * i + d, 0, min(16 if after == d else 16 - d, n - 16 * i - d))]
-            if d > 0 and before != d:
-                windows.append((16 * i + d - 16, 16 - d, 16))
-            for t, lo, hi in windows:
+            own, front = windows.window(16 * i, n, d, after), windows.front(16 * i, d, before)
+            assert own.lo < own.hi
+            for w in (own, front) if front.lo < front.hi else (own,):
+                t, lo, hi = w.tok, w.lo, w.hi
                 assert 0 <= lo < hi <= 16 and 0 <= t + lo and t + hi <= n
                 seen[t + lo:t + hi] += 1
-                if d > 0 and (t, lo) != windows[0][:2]:  # (row r holds the token whose slot is r modulo 16)
+                if w is front:  # (row r holds the token whose slot is r modulo 16)
                     assert slots[t + lo] % 16 == lo
         assert (seen == 1).all()
 
 
-def test_moved_tiles_of_the_kv_write_cover_every_token():
+def test_moved_tiles_of_the_kv_write_cover_every_token(windows):
     """The staged KV write may move a 16-token tile onto the next 16-slot boundary of the cache
-    (vllm_b200/csrc/kv_write_staged.cuh, `shift_of`): tile i then covers tokens
+    (vllm_b200/csrc/kv_write_staged.cuh, `tile_shift`): tile i then covers tokens
     [16 i + s_i, 16 i + s_i + 16) and writes the tokens [16 i + s_(i-1), 16 i + s_i) in front of
     its window itself when the tile before it is moved by less.  Whatever the slots are, every
     token must be covered at least once.  This restates the rule on the host and checks the
@@ -209,19 +232,12 @@ def test_moved_tiles_of_the_kv_write_cover_every_token():
     padding)."""
     import numpy as np
 
-    def shift_of(first, mid, last):
-        if first < 0 or mid < 0 or last < 0:
-            return 0
-        if (mid - first) % 16 != 8 or (last - first) % 16 != 15:
-            return 0
-        return (16 - first % 16) % 16
-
     def tile_shift(slots, i):
         T = len(slots)
         tok = [16 * i, 16 * i + 8, 16 * i + 15]
         if i < 0 or tok[2] >= T:
             return 0
-        return shift_of(*(int(slots[t]) for t in tok))
+        return windows.shift(*(int(slots[t]) for t in tok))
 
     rng = np.random.default_rng(5)
     for _ in range(300):

@@ -771,7 +771,7 @@ static bool launch_staged(const b200pa_cache_args& a, cudaStream_t stream, int* 
 }
 
 static int64_t tile_items(const b200pa_cache_args& a) {
-  return int64_t((a.num_tokens + 15) / 16) * ((a.num_heads + kTileHeads - 1) / kTileHeads);
+  return int64_t((a.num_tokens + 15) / 16) * (a.num_heads / kTileHeads);
 }
 
 // The tile kernel for large writes of an even number of heads.  Returns as launch_staged_as.
@@ -792,7 +792,6 @@ static bool launch_tiles_as(const b200pa_cache_args& a, cudaStream_t stream, int
   p.num_tokens = a.num_tokens;
   p.num_heads = a.num_heads;
   p.block_size = a.block_size;
-  p.move = !kFlash;
   auto kern = kv_write_tiles_kernel<in_t, cache_t, KV, D, kFlash>;
   static bool done[64] = {};
   int dev = 0;

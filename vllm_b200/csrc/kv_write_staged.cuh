@@ -24,12 +24,13 @@
 //     the one item a warp then has;
 //   * the kShift instantiation (large x-layout writes) moves a tile whose tokens are consecutive
 //     positions of a sequence onto the next 16-slot boundary of the cache, so that prefill
-//     chunks which start inside a block still write whole rows of V (details at `shift_of`);
+//     chunks which start inside a block still write whole rows of V (details at `tile_shift`);
 //   * every mbarrier wait is bounded; a wait that runs out records a status code and the warp
 //     leaves.
 #pragma once
 
 #include "decode_common.cuh"
+#include "kv_write_windows.h"
 
 namespace b200pa {
 
@@ -161,11 +162,7 @@ __global__ void __launch_bounds__(kStagedMaxWarps * 32, 1) kv_write_staged_kerne
   // otherwise tile i writes them itself from global memory (`head` in the consumer; once per
   // run).  Windows may overlap: a slot is then written twice with the same bytes.  The rule is
   // only a guess about the slots; whatever they are, every token is written, with its own slot.
-  auto shift_of = [&](int64_t first, int64_t mid, int64_t last) -> int {
-    if (first < 0 || mid < 0 || last < 0) return 0;
-    if (((mid - first) & 15) != 8 || ((last - first) & 15) != 15) return 0;
-    return int((kStagedTile - (first & 15)) & 15);
-  };
+
   // Turns the slots of a tile (as load_slot delivers them) into those of its window; `sh` =
   // shift | shift of the tile in front << 8.
   auto to_window = [&](unsigned item, int64_t cand, int& sh) -> int64_t {
@@ -178,10 +175,10 @@ __global__ void __launch_bounds__(kStagedMaxWarps * 32, 1) kv_write_staged_kerne
       const int64_t l = __shfl_sync(0xffffffffu, cand, 15);
       const int64_t pf = __shfl_sync(0xffffffffu, cand, 16), pl = __shfl_sync(0xffffffffu, cand, 17);
       const int64_t pm = __shfl_sync(0xffffffffu, cand, 18);
-      const int d = shift_of(f, m, l);
+      const int d = tile_shift(f, m, l);
       if (d == 0) return cand;  // (the shift of the tile in front does not matter then)
       // the tile in front, by the very rule that its own warp applies
-      const int dp = shift_of(pf, pm, pl);
+      const int dp = tile_shift(pf, pm, pl);
       sh = d | (dp << 8);
       const int tile = int(div_hh(item >= pairs ? item - pairs : item));
       const int tok = tile * kStagedTile + d + (lane & 15);

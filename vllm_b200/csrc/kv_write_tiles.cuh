@@ -27,6 +27,7 @@
 #include <cuda.h>
 
 #include "kv_write_staged.cuh"
+#include "kv_write_windows.h"
 #include "tcgen05.cuh"
 
 namespace b200pa {
@@ -42,9 +43,8 @@ struct TileWriteParams {
   int64_t page_stride;
   int64_t head_stride;
   int num_tokens;
-  int num_heads;
+  int num_heads;         // a multiple of kTileHeads
   int block_size;
-  int move;              // 1: tiles may be moved onto 16-slot boundaries
 };
 
 constexpr int kTileHeads = 2;                     // heads per item
@@ -101,18 +101,13 @@ kv_write_tiles_kernel(const TileWriteParams p, const __grid_constant__ CUtensorM
 
   if (warp == W) {
     // ================================================= slots, windows, copies
-    const int tiles = (N + 15) / 16, groups = (H + kTileHeads - 1) / kTileHeads, items = tiles * groups;
+    const int tiles = (N + 15) / 16, groups = H / kTileHeads, items = tiles * groups;
     auto slot_at = [&](int tok) -> int64_t { return tok >= 0 && tok < N ? __ldg(p.slot_mapping + tok) : int64_t(-1); };
     // Lanes 0 .. 15: the tile's slots, 16 .. 31: those of the next one; and in lanes 0 .. 2 the first, ninth and
     // last of the one before.  Requested an item ahead.
     auto look = [&](int item) -> int64_t { return item < items ? slot_at(item % tiles * 16 + lane) : int64_t(-1); };
     auto look_back = [&](int item) -> int64_t {
       return item < items && lane < 3 ? slot_at(item % tiles * 16 - 16 + (lane == 0 ? 0 : (lane == 1 ? 8 : 15))) : int64_t(-1);
-    };
-    auto shift_of = [&](int64_t first, int64_t mid, int64_t last) -> int {
-      if (first < 0 || mid < 0 || last < 0) return 0;
-      if (((mid - first) & 15) != 8 || ((last - first) & 15) != 15) return 0;
-      return int((16 - (first & 15)) & 15);
     };
     auto from = [&](int64_t v, int l) { return __shfl_sync(0xffffffffu, v, l); };
     bool ok = true;
@@ -148,14 +143,15 @@ kv_write_tiles_kernel(const TileWriteParams p, const __grid_constant__ CUtensorM
       }
       const int t0 = item % tiles * 16, head0 = item / tiles * kTileHeads;
       int d = 0, before = 0, after = 0;
-      if (!kFlash && p.move) {
-        d = shift_of(from(now, 0), from(now, 8), from(now, 15));
-        before = shift_of(from(back, 0), from(back, 1), from(back, 2));
-        after = shift_of(from(now, 16), from(now, 24), from(now, 31));
+      if (!kFlash) {
+        d = tile_shift(from(now, 0), from(now, 8), from(now, 15));
+        before = tile_shift(from(back, 0), from(back, 1), from(back, 2));
+        after = tile_shift(from(now, 16), from(now, 24), from(now, 31));
       }
-      put(t0 + d, 0, min(after == d ? 16 : 16 - d, N - t0 - d), head0, from(now, (lane + d) & 31));
+      const TileWindow own = tile_window(t0, N, d, after), front = tile_front_window(t0, d, before);
+      put(own.tok, own.lo, own.hi, head0, from(now, (lane + d) & 31));
       // (at a negative or a foreign token the box starts with rows that nobody writes)
-      if (ok && d > 0 && before != d) put(t0 + d - 16, 16 - d, 16, head0, from(now, (lane + d) & 15));
+      if (ok && front.lo < front.hi) put(front.tok, front.lo, front.hi, head0, from(now, (lane + d) & 15));
     }
     // the end; then nobody leaves with copies on their way
     if (ok && round > 0) ok = __all_sync(0xffffffffu, mbar_wait(empty(stage), (round - 1) & 1));
@@ -226,83 +222,81 @@ kv_write_tiles_kernel(const TileWriteParams p, const __grid_constant__ CUtensorM
     };
     const uint32_t k_src = smem + stage * SH::kStage + hl * (16 * 128);
     const uint32_t v_src = k_src + SH::kBoxes * SH::kBoxBytes;
-    if (h < H) {
-      rows(k_src, p.key_cache, k_div);
-      if constexpr (kFlash) {
-        rows(v_src, p.value_cache, v_div);
-      } else {
-        // ---- V of the x-layout (kv_write_staged.cuh explains the matrices): lane j = lane % 4 gets tokens
-        // 4 j .. 4 j + 3 of rows d = lane / 4 and 8 more
-        const int j = lane & 3;
-        int64_t sl[4];
+    rows(k_src, p.key_cache, k_div);
+    if constexpr (kFlash) {
+      rows(v_src, p.value_cache, v_div);
+    } else {
+      // ---- V of the x-layout (kv_write_staged.cuh explains the matrices): lane j = lane % 4 gets tokens
+      // 4 j .. 4 j + 3 of rows d = lane / 4 and 8 more
+      const int j = lane & 3;
+      int64_t sl[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) sl[k] = s_slot[stage][4 * j + k];
-        const bool quad = sl[0] >= 0 && (sl[0] & 3) == 0 && sl[1] == sl[0] + 1 && sl[2] == sl[0] + 2 && sl[3] == sl[0] + 3;
-        auto place = [&](int64_t s) {  // of a slot's element of this lane's first row
-          return static_cast<cache_t*>(p.value_cache) + (((s >> b_shift) * H + h) * D + part * (D / 2) + (lane >> 2)) * int64_t(B) +
-                 (s & (B - 1));
-        };
-        const int mr = lane & 7, mi = lane >> 3;
-        const int mtok = (mr >> 1) * 4 + (mr & 1) + (mi & 1) * 2;
-        const uint32_t row = v_src + mtok * 128, chunk = uint32_t((mi >> 1) ^ (mtok & 7)) * 16;
-        auto pass = [&](auto exact_tag) -> uint32_t {
-          constexpr bool kExact = decltype(exact_tag)::value;
-          (void)kExact;
-          uint32_t nan_bits = 0;
-          cache_t* dst = place(sl[0]);
+      for (int k = 0; k < 4; ++k) sl[k] = s_slot[stage][4 * j + k];
+      const bool quad = sl[0] >= 0 && (sl[0] & 3) == 0 && sl[1] == sl[0] + 1 && sl[2] == sl[0] + 2 && sl[3] == sl[0] + 3;
+      auto place = [&](int64_t s) {  // of a slot's element of this lane's first row
+        return static_cast<cache_t*>(p.value_cache) + (((s >> b_shift) * H + h) * D + part * (D / 2) + (lane >> 2)) * int64_t(B) +
+               (s & (B - 1));
+      };
+      const int mr = lane & 7, mi = lane >> 3;
+      const int mtok = (mr >> 1) * 4 + (mr & 1) + (mi & 1) * 2;
+      const uint32_t row = v_src + mtok * 128, chunk = uint32_t((mi >> 1) ^ (mtok & 7)) * 16;
+      auto pass = [&](auto exact_tag) -> uint32_t {
+        constexpr bool kExact = decltype(exact_tag)::value;
+        (void)kExact;
+        uint32_t nan_bits = 0;
+        cache_t* dst = place(sl[0]);
 #pragma unroll
-          for (int i16 = 0; i16 < D / 32; ++i16) {
-            const int d16 = part * (D / 32) + i16;
-            uint32_t r[4];  // (tokens 4j, 4j+1), (4j+2, 4j+3) of row d; the same of row d + 8
-            asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                         : "r"(row + d16 / 4 * SH::kBoxBytes + (chunk ^ (d16 % 4 * 32))));
-            uint32_t w[2][2];  // this lane's piece of row d and of row d + 8 (one word when fp8)
+        for (int i16 = 0; i16 < D / 32; ++i16) {
+          const int d16 = part * (D / 32) + i16;
+          uint32_t r[4];  // (tokens 4j, 4j+1), (4j+2, 4j+3) of row d; the same of row d + 8
+          asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                       : "r"(row + d16 / 4 * SH::kBoxBytes + (chunk ^ (d16 % 4 * 32))));
+          uint32_t w[2][2];  // this lane's piece of row d and of row d + 8 (one word when fp8)
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            if constexpr (KV == kKvAuto) {
+              w[i][0] = r[2 * i];
+              w[i][1] = r[2 * i + 1];
+            } else if constexpr (kExact) {
+              const uint32_t in[2] = {r[2 * i], r[2 * i + 1]};
+              uint32_t o[1];
+              convert_words<in_t, KV, 2>(in, o, v_div);  // (checks its own codes)
+              w[i][0] = o[0];
+            } else {
+              const uint32_t v = neg_quant4<in_t, KV == kKvE5M2>(r[2 * i], r[2 * i + 1], v_div);
+              nan_bits |= (v & 0x7F7F7F7Fu) + 0x01010101u;
+              w[i][0] = v ^ 0x80808080u;
+            }
+          }
+          const int64_t o = int64_t(i16) * 16 * B;
+          if (quad) {
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-              if constexpr (KV == kKvAuto) {
-                w[i][0] = r[2 * i];
-                w[i][1] = r[2 * i + 1];
-              } else if constexpr (kExact) {
-                const uint32_t in[2] = {r[2 * i], r[2 * i + 1]};
-                uint32_t o[1];
-                convert_words<in_t, KV, 2>(in, o, v_div);  // (checks its own codes)
-                w[i][0] = o[0];
-              } else {
-                const uint32_t v = neg_quant4<in_t, KV == kKvE5M2>(r[2 * i], r[2 * i + 1], v_div);
-                nan_bits |= (v & 0x7F7F7F7Fu) + 0x01010101u;
-                w[i][0] = v ^ 0x80808080u;
-              }
+              if constexpr (E == 1) *reinterpret_cast<uint32_t*>(dst + o + 8 * i * B) = w[i][0];
+              else *reinterpret_cast<uint2*>(dst + o + 8 * i * B) = make_uint2(w[i][0], w[i][1]);
             }
-            const int64_t o = int64_t(i16) * 16 * B;
-            if (quad) {
+          } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              if (sl[k] < 0) continue;
+              cache_t* one = place(sl[k]) + o;
 #pragma unroll
               for (int i = 0; i < 2; ++i) {
-                if constexpr (E == 1) *reinterpret_cast<uint32_t*>(dst + o + 8 * i * B) = w[i][0];
-                else *reinterpret_cast<uint2*>(dst + o + 8 * i * B) = make_uint2(w[i][0], w[i][1]);
-              }
-            } else {
-#pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                if (sl[k] < 0) continue;
-                cache_t* one = place(sl[k]) + o;
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                  if constexpr (E == 1) *reinterpret_cast<unsigned char*>(one + 8 * i * B) = static_cast<unsigned char>(w[i][0] >> (8 * k));
-                  else *reinterpret_cast<uint16_t*>(one + 8 * i * B) = static_cast<uint16_t>(w[i][k >> 1] >> (16 * (k & 1)));
-                }
+                if constexpr (E == 1) *reinterpret_cast<unsigned char*>(one + 8 * i * B) = static_cast<unsigned char>(w[i][0] >> (8 * k));
+                else *reinterpret_cast<uint16_t*>(one + 8 * i * B) = static_cast<uint16_t>(w[i][k >> 1] >> (16 * (k & 1)));
               }
             }
           }
-          return nan_bits & 0x80808080u;
-        };
-        if constexpr (KV == kKvAuto) {
-          pass(std::false_type{});
-        } else {
-          // (ldmatrix is warp-collective: the decision to repeat with the division is taken by the warp)
-          const bool again = !v_div.fast || __any_sync(0xffffffffu, pass(std::false_type{}) != 0);
-          if (again) pass(std::true_type{});
         }
+        return nan_bits & 0x80808080u;
+      };
+      if constexpr (KV == kKvAuto) {
+        pass(std::false_type{});
+      } else {
+        // (ldmatrix is warp-collective: the decision to repeat with the division is taken by the warp)
+        const bool again = !v_div.fast || __any_sync(0xffffffffu, pass(std::false_type{}) != 0);
+        if (again) pass(std::true_type{});
       }
     }
     __syncwarp();
