@@ -22,10 +22,10 @@
 //   * The two row tiles take turns: while the softmax of one runs, the tensor cores work for the
 //     other.
 //   * A thread takes its whole row of S into registers (one TMEM read, paired fp32 arithmetic,
-//     three-way maxima), so the maximum is known before the first exponential, and P is handed over
-//     in two halves: the product of the first runs under the exponentials of the second.  (Two reads of
-//     S, or exponentials ahead of the maximum: step below 475 us, 443 so; fp8 caches and ALiBi, which
-//     read S twice, 5 to 20 % more than this one on steps of short chunks.)
+//     three-way maxima; 528 -> 506 us before V and Q came by tensor map) and hands P over in two halves:
+//     the product of the first runs under the exponentials of the second.  With an fp8 cache or a bias the
+//     maximum of the tile comes before its first exponential; otherwise a row that has a maximum starts
+//     with that one, and the tile is done again where it was too low (363 -> 353 us).
 //   * The running maximum is only raised (and O rescaled in TMEM) when a row's maximum grew by more
 //     than 2^8 to 2^12: until then P is merely larger than 1, which fp32 sums and 16-bit P hold as exactly.
 //   * fp8 caches are widened to f16 (exact) by the producers on their way to shared memory.
@@ -94,7 +94,7 @@ struct PrefillRegs {
   static_assert(2 * kSoftmax + kProducer + kMma == 4 * 128, "register split");
 };
 constexpr int kPrefillMaxReqs = 512;    // requests per launch: prefix table in shared memory
-constexpr int kPrefillSortReqs = 64;    // up to so many are taken longest first
+constexpr int kPrefillSortReqs = 64;    // up to so many are taken longest first (the reason is with the plan)
 
 template <int D>
 struct PrefillShape {
@@ -222,8 +222,11 @@ pa_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap qma
   // Longest sequences first, where there are more groups than SMs: the last items of all are short ones
   // then, whatever the engine's order.  (60 decodes and three chunks of 150 to 700 tokens behind up to
   // 1500, 328 items: 124.5 -> 122 us; 6 fp8 chunks of 200 to 900 with a bias 147 -> 132; 12 bf16 chunks
-  // 112 -> 108.5.  More than 64 requests keep their order: not measured; they make many items, and each
-  // thread would count over all of them.)
+  // 112 -> 108.5.  More than 64 requests keep their order, since each
+  // thread would count over all of them.  Measured with a limit of 256: 128 equal prompts of 128 tokens 93.5 -> 95.3,
+  // fp8 96.5 -> 102; requests of various lengths gain, 66 of 50 to 600 tokens behind up to 1500 0 to 4 %, 200 of 20
+  // to 200 behind up to 3000 3 % (fp8 1 % more), 250 of 16 to 64 behind up to 2000 5 %, 100 of 2 to 20 behind up to
+  // 6000 15 to 20 %, 309 -> 262: 64 is too low a line for those.)
   bool sorted = false;
   auto tiles_of = [&](int len) { return (max(len, 0) + KT - 1) / KT; };
   {
